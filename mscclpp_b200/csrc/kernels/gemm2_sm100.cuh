@@ -93,7 +93,7 @@ MSCCLPP_DEVICE_INLINE void gemmCtaPair(const CUtensorMap* tmapA, const CUtensorM
 
   if (warp == 0) {
     // ===================================================== TMA producer (one thread per CTA)
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -132,7 +132,7 @@ MSCCLPP_DEVICE_INLINE void gemmCtaPair(const CUtensorMap* tmapA, const CUtensorM
     }
   } else if (warp == 1) {
     // ===================================================== MMA issuer (one thread of the leader CTA)
-    if (lane == 0 && leader) {
+    if (leader && ptx::elect_one()) {
       constexpr uint32_t idesc = makeInstrDescPair();
       // one thread feeds the tensor cores of both SMs: descriptors are stepped by adds, waits cost one instruction when
       // the data is already there

@@ -269,7 +269,11 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
 
   if (warp == 0) {
     // ===================================================== TMA producer (one thread)
-    if (lane == 0) {
+    // The single threads of this warp and the next are taken with elect.sync, not by lane number: the compiler then knows
+    // that exactly one thread runs the loop and keeps descriptors and barrier addresses uniform. Measured on a B200 (128 x
+    // 128 tiles, K = 4096, operands in L2): 0.41 us per 64-wide k block with `lane == 0`, 0.28 us with elect.sync; 333 x
+    // 6144 x 4096 26.7 -> 18.0 us, 128 x 8192 x 1024 9.5 -> 7.2 us, and with the two-SM core 8192 x 7168 x 8192 779 -> 684 us.
+    if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       uint32_t armed = 0;        // bit s: stage s has a load in flight that nobody has waited for yet
@@ -317,7 +321,7 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
     }
   } else if (warp == 1) {
     // ===================================================== MMA issuer (one thread)
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       constexpr uint32_t idesc = makeInstrDesc<kBlockN>();
       // The issue loop is ONE thread feeding the tensor core: every instruction in it is on the critical path of the
       // whole SM. Descriptors are formed once and stepped by adds; the common case of each wait is one instruction.
