@@ -8,13 +8,16 @@
 //     B. the counts travel to every rank as (value, epoch) pairs - 8-byte stores, no separate flag;
 //     C. every block reads the full [rank][expert] count matrix and derives the first row of each of its groups
 //        at the destination;
-//     D. one warp per token loads the row once and stores it to its top-k destinations (16-byte peer stores);
-//        with fp8 = 1 the row is quantised in registers to e4m3 with one scale per 128 elements, which halves the
-//        bytes on NVLink.
+//     D. a block's tokens are cut into pieces of 128 16-byte words, a warp loads a piece once and stores it to the
+//        token's top-k destinations (16-byte peer stores); with fp8 = 1 the piece is quantised in registers to e4m3
+//        with one scale per 128 elements, which halves the bytes on NVLink.
 // combine: the reverse direction is a PULL - the source rank reads the expert outputs of its tokens out of the
 //   hosting ranks' buffers (16-byte peer loads), applies the routing weights in fp32 and writes the bf16 result.
 //   No staging buffer and no second pass. With fp8 = 1 the expert outputs are e4m3 with 1 x 128 scales (quantised by
 //   the expert GEMM's epilogue or by launchMoeQuantizeRows), half the bytes over NVLink.
+// With one rank both are bound by HBM. Dispatch and combine together on one B200: 4096 tokens x 4096 bf16, top-2 of 64
+// experts 55 us (201 MB, 3.7 TB/s), 777 tokens x 7168 fp8, top-8 of 256 experts 39 us; with 64 blocks, a whole row per
+// warp, one expert's row after the other and system-scope accesses it was 86 and 104 us.
 // Both end with a cross-rank barrier: after dispatch returns every row sent to this rank has landed; after combine
 // returns the peers are done reading this rank's expert outputs.
 //
@@ -32,6 +35,9 @@ namespace {
 using bf16 = __nv_bfloat16;
 constexpr int kThreads = 512;
 constexpr int kMaxWordsPerLane = 32;  // hidden <= 32 lanes * 32 words * 8 elements = 8192
+constexpr int kBatchTokens = 32;      // dispatch: tokens whose destinations are worked out together
+constexpr int kPieceWords = 4;        // dispatch: 16-byte words per lane of the piece of a row that a warp moves at a time
+static_assert(kBatchTokens * kMoeMaxTopk <= kThreads && kMoeMaxExperts < kThreads && kPieceWords % 2 == 0, "one thread per pair and per expert");
 
 struct Workspace {
   uint32_t* cnt;      // [kMoeMaxExperts] pairs of this rank per expert (zero between launches)
@@ -105,7 +111,19 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
 
   __shared__ uint32_t counts[kMaxRanks][kMoeMaxExperts];  // [source rank][expert]
   __shared__ uint32_t firstRow[kMoeMaxExperts];           // first destination row of my group of expert e
+  __shared__ uint32_t prefix[kMoeMaxExperts + 1];         // rows of the experts before e
+  __shared__ uint32_t warpTotal[kThreads / 32];
+  __shared__ uint64_t rowAddr[2][kBatchTokens * kMoeMaxTopk];    // destination row of a pair, 0 = none
+  __shared__ uint64_t scaleAddr[2][kBatchTokens * kMoeMaxTopk];  // its scales
   __shared__ int overflow;
+
+  // this block's tokens; the rows of the first batch start on their way to L2 now, under the exchange of the counts
+  const int words = a.hidden / 8;  // 16-byte words per bf16 row
+  const int chunks = (words + 32 * kPieceWords - 1) / (32 * kPieceWords);
+  const int tokBegin = static_cast<int>(static_cast<int64_t>(a.tokens) * blockIdx.x / gridDim.x);
+  const int tokEnd = static_cast<int>(static_cast<int64_t>(a.tokens) * (blockIdx.x + 1) / gridDim.x);
+  if (threadIdx.x < kBatchTokens && tokBegin + static_cast<int>(threadIdx.x) < tokEnd)
+    ptx::bulk_prefetch_l2(x + static_cast<size_t>(tokBegin + threadIdx.x) * a.hidden, static_cast<uint32_t>(a.hidden) * 2);
 
   // ---- A. position of every pair inside its (me, expert) group
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += gridDim.x * blockDim.x) {
@@ -146,22 +164,40 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
     }
   }
   __syncthreads();
-  if (healthy && overflow == 0) {
-    for (int e = threadIdx.x; e < E; e += blockDim.x) {
-      const int d = e / El;
-      uint32_t row = 0, rankTotal = 0;
-      for (int e2 = d * El; e2 < (d + 1) * El; e2++) {
-        uint32_t tot = 0;
-        for (int s = 0; s < world; s++) tot += counts[s][e2];
-        if (e2 < e) row += tot;
-        rankTotal += tot;
+  {
+    // prefix[e] = rows of all experts before e, over all source ranks (one expert per thread, kMoeMaxExperts <= blockDim.x):
+    // a scan of shuffles, where summing up the experts before each one took 4 us with 256 experts on one rank
+    const bool known = healthy && overflow == 0;
+    const int e = threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t tot = 0, before = 0;
+    if (known && e < E) {
+      for (int s = 0; s < world; s++) {
+        const uint32_t n = counts[s][e];
+        if (s < rank) before += n;
+        tot += n;
       }
-      for (int s = 0; s < rank; s++) row += counts[s][e];
-      firstRow[e] = row;
+    }
+    uint32_t incl = tot;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    if (lane == 31) warpTotal[warp] = incl;
+    __syncthreads();
+    if (e <= E && e <= kMoeMaxExperts) {
+      uint32_t base = 0;
+      for (int q = 0; q < warp; q++) base += warpTotal[q];
+      prefix[e] = base + incl - tot;
+    }
+    __syncthreads();
+    if (known && e < E) {
+      const int d = e / El;
+      const uint32_t first = prefix[d * El];
+      firstRow[e] = prefix[e] - first + before;
+      const uint32_t rankTotal = prefix[(d + 1) * El] - first;
       if (rankTotal > static_cast<uint32_t>(a.capacity)) atomicExch(&overflow, 1);
       if (blockIdx.x == 0 && d == rank) {
-        uint32_t tot = 0;
-        for (int s = 0; s < world; s++) tot += counts[s][e];
         recvCounts[e - d * El] = static_cast<int32_t>(tot);
         if (e == d * El) recvCounts[El] = static_cast<int32_t>(rankTotal);
       }
@@ -175,85 +211,111 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
   }
   const bool send = healthy && overflow == 0;
 
-  // ---- D. one warp per token: load the row once, store it to each destination
+  // ---- D. rows to their destinations. Every block has a contiguous share of the tokens. Destinations of a batch of tokens
+  // are worked out by one thread per pair (the only reader and writer of its slotMap entry), then the warps take the
+  // (token, piece) units of the batch in turn, with the next unit's loads in flight while the current one is stored.
   const int lane = threadIdx.x & 31;
-  const int warpsPerBlock = blockDim.x >> 5;
-  const int warp = blockIdx.x * warpsPerBlock + (threadIdx.x >> 5);
-  const int numWarps = gridDim.x * warpsPerBlock;
-  const int words = a.hidden / 8;  // 16-byte words per bf16 row
+  const int warp = threadIdx.x >> 5;
+  const int warps = blockDim.x >> 5;
   const int scalesPerRow = a.hidden / kMoeScaleGroup;
+  const bool wide = (recvXOff & 15) == 0;  // the quantised rows may be stored in 16-byte words
   if (send) {
-    for (int t = warp; t < a.tokens; t += numWarps) {
-      int dstRank[kMoeMaxTopk], dstRow[kMoeMaxTopk], dstK[kMoeMaxTopk];
-      int nd = 0;
-      for (int k = 0; k < a.topk; k++) {
-        const int e = topkIdx[t * a.topk + k];
-        if (e < 0 || e >= E) continue;
-        dstRank[nd] = e / El;
-        dstRow[nd] = static_cast<int>(firstRow[e]) + slotMap[t * a.topk + k];  // slotMap holds the position in the group
-        dstK[nd] = k;
-        nd++;
+    auto stage = [&](int t0, int n, int buf) {
+      const int i = threadIdx.x;
+      if (i >= n * a.topk) return;
+      const int p = t0 * a.topk + i;
+      const int e = topkIdx[p];
+      uint64_t row = 0, scales = 0;
+      if (e >= 0 && e < E) {
+        const uint64_t peer = c.peerBase[e / El];
+        const uint32_t r = firstRow[e] + static_cast<uint32_t>(slotMap[p]);  // slotMap holds the position in the group
+        slotMap[p] = static_cast<int32_t>(r);
+        row = peer + recvXOff + static_cast<uint64_t>(r) * a.hidden * (a.fp8 ? 1 : 2);
+        scales = peer + recvScalesOff + static_cast<uint64_t>(r) * scalesPerRow * 4;
+        ptx::st_relaxed_sys(reinterpret_cast<uint32_t*>(peer + recvSrcOff) + r,
+                            (static_cast<uint32_t>(rank) << 24) | static_cast<uint32_t>(t0 + i / a.topk));
       }
-      __syncwarp();  // every lane has read the positions before lane 0 replaces them by the final rows
-      if (lane == 0) {
-        for (int q = 0; q < nd; q++) slotMap[t * a.topk + dstK[q]] = dstRow[q];
-      }
-      if (nd == 0) continue;
-      const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(t) * a.hidden);
-      if (!a.fp8) {
-#pragma unroll 1
-        for (int w0 = 0; w0 < words; w0 += 32 * 8) {
-          uint4 v[8];
+      rowAddr[buf][i] = row;
+      scaleAddr[buf][i] = scales;
+    };
+    if (tokBegin < tokEnd) stage(tokBegin, min(kBatchTokens, tokEnd - tokBegin), 0);
+    int buf = 0;
+    for (int t0 = tokBegin; t0 < tokEnd; t0 += kBatchTokens, buf ^= 1) {
+      const int n = min(kBatchTokens, tokEnd - t0);
+      __syncthreads();
+      if (t0 + n < tokEnd) stage(t0 + n, min(kBatchTokens, tokEnd - t0 - n), buf ^ 1);
+      const int units = n * chunks;
+      uint4 cur[kPieceWords];
+      auto load = [&](int u, uint4 (&v)[kPieceWords]) {
+        const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(t0 + u / chunks) * a.hidden);
+        const int w0 = (u % chunks) * (32 * kPieceWords) + lane;
 #pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const int w = w0 + j * 32 + lane;
-            v[j] = w < words ? ptx::ld_nc_na_v4(src + w) : make_uint4(0, 0, 0, 0);
-          }
-          for (int q = 0; q < nd; q++) {
-            const uint64_t rowBase = c.peerBase[dstRank[q]] + recvXOff + static_cast<uint64_t>(dstRow[q]) * a.hidden * 2;
+        for (int j = 0; j < kPieceWords; j++) {
+          v[j] = make_uint4(0, 0, 0, 0);
+          if (w0 + j * 32 < words) v[j] = ptx::ld_input_v4(src + w0 + j * 32);
+        }
+      };
+      if (warp < units) load(warp, cur);
+      for (int u = warp; u < units; u += warps) {
+        uint4 next[kPieceWords];
+        if (u + warps < units) load(u + warps, next);
+        const int w0 = (u % chunks) * (32 * kPieceWords);
+        const uint64_t* rows = &rowAddr[buf][(u / chunks) * a.topk];
+        if (!a.fp8) {
+          for (int k = 0; k < a.topk; k++) {
+            const uint64_t row = rows[k];
+            if (row == 0) continue;
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
+            for (int j = 0; j < kPieceWords; j++) {
               const int w = w0 + j * 32 + lane;
-              if (w < words) ptx::st_na_v4(reinterpret_cast<void*>(rowBase + static_cast<uint64_t>(w) * 16), v[j]);
+              if (w < words) ptx::st_weak_v4(reinterpret_cast<void*>(row + static_cast<uint64_t>(w) * 16), cur[j]);
             }
           }
-        }
-      } else {
-        // 32 lanes x 8 elements = 256 elements per step = two scale groups (lanes 0-15, 16-31). Eight steps are loaded
-        // before the first is quantised, so a lane keeps 128 bytes of the row in flight instead of 16.
-#pragma unroll 1
-        for (int w0 = 0; w0 < words; w0 += 32 * 8) {
-          uint4 v[8];
+        } else {
+          // 32 lanes x 8 elements = 256 elements per step = two scale groups (lanes 0-15, 16-31)
+          uint2 q8[kPieceWords];
+          float scale = 0.f;  // lane 2 j + g: the scale of step j's group g
 #pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const int w = w0 + j * 32 + lane;
-            v[j] = w < words ? ptx::ld_nc_na_v4(src + w) : make_uint4(0, 0, 0, 0);
-          }
-#pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const int w = w0 + j * 32 + lane;
+          for (int j = 0; j < kPieceWords; j++) {
             float f[8];
-            Vec16<bf16>::toFloat(v[j], f);
-            float scale;
-            const uint2 packed = quantizeWordE4m3(f, scale);
-            if (w < words) {
-              for (int q = 0; q < nd; q++) {
-                const uint64_t peer = c.peerBase[dstRank[q]];
-                ptx::st_volatile_v2(reinterpret_cast<void*>(peer + recvXOff + static_cast<uint64_t>(dstRow[q]) * a.hidden + static_cast<uint64_t>(w) * 8), packed);
-                if ((lane & 15) == 0) {
-                  float* sc = reinterpret_cast<float*>(peer + recvScalesOff) + static_cast<uint64_t>(dstRow[q]) * scalesPerRow + w / 16;
-                  ptx::st_relaxed_sys(reinterpret_cast<uint32_t*>(sc), __float_as_uint(scale));
-                }
+            Vec16<bf16>::toFloat(cur[j], f);
+            float sc;
+            q8[j] = quantizeWordE4m3(f, sc);
+            sc = __shfl_sync(0xffffffffu, sc, (lane & 1) * 16);
+            if ((lane >> 1) == j) scale = sc;
+          }
+          // neighbouring lanes swap halves: even lanes end up with 16 bytes of step j, odd lanes with 16 bytes of step j + 1
+          uint4 out16[kPieceWords / 2];
+#pragma unroll
+          for (int j = 0; j < kPieceWords; j += 2) {
+            const uint2 give = (lane & 1) ? q8[j] : q8[j + 1];
+            const uint32_t gx = __shfl_xor_sync(0xffffffffu, give.x, 1), gy = __shfl_xor_sync(0xffffffffu, give.y, 1);
+            out16[j / 2] = (lane & 1) ? make_uint4(gx, gy, q8[j + 1].x, q8[j + 1].y) : make_uint4(q8[j].x, q8[j].y, gx, gy);
+          }
+          const uint64_t* scaleRows = &scaleAddr[buf][(u / chunks) * a.topk];
+          for (int k = 0; k < a.topk; k++) {
+            const uint64_t row = rows[k];
+            if (row == 0) continue;
+            if (wide) {
+#pragma unroll
+              for (int j = 0; j < kPieceWords; j += 2) {
+                const int w = w0 + (j + (lane & 1)) * 32 + (lane & ~1);
+                if (w < words) ptx::st_weak_v4(reinterpret_cast<void*>(row + static_cast<uint64_t>(w) * 8), out16[j / 2]);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < kPieceWords; j++) {
+                const int w = w0 + j * 32 + lane;
+                if (w < words) ptx::st_volatile_v2(reinterpret_cast<void*>(row + static_cast<uint64_t>(w) * 8), q8[j]);
               }
             }
+            const int sw = w0 / 16 + lane;
+            if (lane < 2 * kPieceWords && sw < scalesPerRow)
+              ptx::st_relaxed_sys(reinterpret_cast<uint32_t*>(scaleRows[k]) + sw, __float_as_uint(scale));
           }
         }
-      }
-      if (lane == 0) {
-        for (int q = 0; q < nd; q++) {
-          int32_t* dst = reinterpret_cast<int32_t*>(c.peerBase[dstRank[q]] + recvSrcOff) + dstRow[q];
-          ptx::st_relaxed_sys(reinterpret_cast<uint32_t*>(dst), (static_cast<uint32_t>(rank) << 24) | static_cast<uint32_t>(t));
-        }
+#pragma unroll
+        for (int j = 0; j < kPieceWords; j++) cur[j] = next[j];
       }
     }
   } else {
@@ -264,6 +326,10 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
   finishLaunch(c, rank, epoch);
 }
 
+// A unit of the combine is 32 x kWords 16-byte words of one token's result (kFp8: of its quantised rows). A warp takes the
+// units in turn over the whole grid; the rows of kRows experts are requested together (kWords x kRows = 8 loads per lane
+// in flight), and the expert ids, rows and weights of its next unit while it waits for them (lane k holds the k-th).
+template <int kWords, int kRows, bool kFp8>
 __global__ void __launch_bounds__(kThreads, 1) moeCombineKernel(MoeCombineArgs a) {
   const DeviceComm& c = a.comm;
   const int rank = deviceRank(c);
@@ -276,10 +342,13 @@ __global__ void __launch_bounds__(kThreads, 1) moeCombineKernel(MoeCombineArgs a
   const int32_t* slotMap = reinterpret_cast<const int32_t*>(local + (reinterpret_cast<uint64_t>(a.slotMap) - base));
   bf16* y = reinterpret_cast<bf16*>(local + (reinterpret_cast<uint64_t>(a.y) - base));
   const uint64_t outOff = reinterpret_cast<uint64_t>(a.expertOut) - base;
-  const uint64_t scalesOff = a.fp8 ? reinterpret_cast<uint64_t>(a.outScales) - base : 0;
+  const uint64_t scalesOff = kFp8 ? reinterpret_cast<uint64_t>(a.outScales) - base : 0;
   const int scalesPerRow = a.hidden / kMoeScaleGroup;
   const int El = a.numExperts / world;
-  const int words = a.hidden / 8;
+  constexpr int kElems = kFp8 ? 16 : 8;  // values in a 16-byte word
+  const int words = a.hidden / kElems;
+  const int chunks = (words + 32 * kWords - 1) / (32 * kWords);
+  const int64_t units = static_cast<int64_t>(a.tokens) * chunks;
 
   // the peers' expert outputs are final once their kernels run
   const bool healthy = rankBarrier(c, rank, 0, blockIdx.x, epoch);
@@ -287,98 +356,89 @@ __global__ void __launch_bounds__(kThreads, 1) moeCombineKernel(MoeCombineArgs a
   const int warpsPerBlock = blockDim.x >> 5;
   const int numWarps = gridDim.x * warpsPerBlock;
   if (healthy) {
-    for (int t = blockIdx.x * warpsPerBlock + (threadIdx.x >> 5); t < a.tokens; t += numWarps) {
-      uint64_t rowBase[kMoeMaxTopk];
-      uint64_t scaleBase[kMoeMaxTopk];
-      float wgt[kMoeMaxTopk];
-      int nd = 0;
-      for (int k = 0; k < a.topk; k++) {
-        const int e = topkIdx[t * a.topk + k];
-        const int row = slotMap[t * a.topk + k];
-        if (e < 0 || e >= a.numExperts || row < 0) continue;
-        rowBase[nd] = c.peerBase[e / El] + outOff + static_cast<uint64_t>(row) * a.hidden * (a.fp8 ? 1 : 2);
-        scaleBase[nd] = c.peerBase[e / El] + scalesOff + static_cast<uint64_t>(row) * scalesPerRow * 4;
-        wgt[nd] = weights[t * a.topk + k];
-        nd++;
+    int e = -1, row = -1;
+    float wgt = 0.f;
+    auto fetch = [&](int64_t u) {  // lane k: the k-th expert of unit u's token
+      e = row = -1;
+      if (u < units && lane < a.topk) {
+        const size_t p = static_cast<size_t>(u / chunks) * a.topk + lane;
+        e = topkIdx[p];
+        row = slotMap[p];
+        wgt = weights[p];
+      }
+    };
+    int64_t u = blockIdx.x * warpsPerBlock + (threadIdx.x >> 5);
+    fetch(u);
+    for (; u < units; u += numWarps) {
+      const int t = static_cast<int>(u / chunks);
+      const int w0 = static_cast<int>(u % chunks) * (32 * kWords) + lane;
+      uint64_t rowBase = 0, scaleBase = 0;  // 0 = this lane's slot is not in use
+      const float weight = wgt;
+      if (e >= 0 && e < a.numExperts && row >= 0) {
+        const uint64_t peer = c.peerBase[e / El];
+        rowBase = peer + outOff + static_cast<uint64_t>(row) * a.hidden * (kFp8 ? 1 : 2);
+        scaleBase = peer + scalesOff + static_cast<uint64_t>(row) * scalesPerRow * 4;
+      }
+      fetch(u + numWarps);
+      float acc[kWords][kElems];
+#pragma unroll
+      for (int j = 0; j < kWords; j++) {
+#pragma unroll
+        for (int i = 0; i < kElems; i++) acc[j][i] = 0.f;
+      }
+#pragma unroll 1
+      for (int k0 = 0; k0 < a.topk; k0 += kRows) {
+        uint4 v[kRows][kWords];
+        [[maybe_unused]] float sc[kRows][kWords];
+        bool used[kRows];
+        float wq[kRows];
+#pragma unroll
+        for (int q = 0; q < kRows; q++) {  // (slots at or beyond topk carry rowBase 0)
+          const uint64_t rb = __shfl_sync(0xffffffffu, rowBase, k0 + q);
+          [[maybe_unused]] const uint64_t sb = kFp8 ? __shfl_sync(0xffffffffu, scaleBase, k0 + q) : 0;
+          wq[q] = __shfl_sync(0xffffffffu, weight, k0 + q);
+          used[q] = rb != 0;
+#pragma unroll
+          for (int j = 0; j < kWords; j++) {
+            const int w = w0 + j * 32;
+            v[q][j] = make_uint4(0, 0, 0, 0);
+            sc[q][j] = 0.f;
+            if (used[q] && w < words) {
+              v[q][j] = ptx::ld_weak_v4(reinterpret_cast<const void*>(rb + static_cast<uint64_t>(w) * 16));
+              if constexpr (kFp8) sc[q][j] = __uint_as_float(ptx::ld_weak_u32(reinterpret_cast<const uint32_t*>(sb) + w / 8));
+            }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < kRows; q++) {
+          if (!used[q]) continue;
+#pragma unroll
+          for (int j = 0; j < kWords; j++) {
+            float f[kElems];
+            float m = wq[q];
+            if constexpr (kFp8) {
+              // the 8 lanes of a 128-element group share one scale
+              e4m3x16ToFloat(v[q][j], f);
+              m *= sc[q][j];
+            } else {
+              Vec16<bf16>::toFloat(v[q][j], f);
+            }
+#pragma unroll
+            for (int i = 0; i < kElems; i++) acc[j][i] += m * f[i];
+          }
+        }
       }
       uint4* dst = reinterpret_cast<uint4*>(y + static_cast<size_t>(t) * a.hidden);
-      if (a.fp8) {
-        // a lane's 16-byte word holds 16 values; the 8 lanes of a 128-element group share one scale
-        const int words16 = a.hidden / 16;
-#pragma unroll 1
-        for (int w0 = 0; w0 < words16; w0 += 32 * 4) {
-          float acc[4][16];
 #pragma unroll
-          for (int j = 0; j < 4; j++) {
+      for (int j = 0; j < kWords; j++) {
+        const int w = w0 + j * 32;
+        if (w >= words) continue;
 #pragma unroll
-            for (int i = 0; i < 16; i++) acc[j][i] = 0.f;
-          }
-          for (int q = 0; q < nd; q++) {
-            uint4 v[4];
-            float sc[4];
+        for (int h = 0; h < kElems / 8; h++) {
+          float part[8];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-              const int w = w0 + j * 32 + lane;
-              v[j] = make_uint4(0, 0, 0, 0);
-              sc[j] = 0.f;
-              if (w < words16) {
-                v[j] = ptx::ld_nc_na_v4(reinterpret_cast<const void*>(rowBase[q] + static_cast<uint64_t>(w) * 16));
-                sc[j] = __uint_as_float(ptx::ld_relaxed_sys(reinterpret_cast<const uint32_t*>(scaleBase[q]) + w / 8));
-              }
-            }
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-              float f[16];
-              e4m3x16ToFloat(v[j], f);
-              const float m = wgt[q] * sc[j];
-#pragma unroll
-              for (int i = 0; i < 16; i++) acc[j][i] += m * f[i];
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const int w = w0 + j * 32 + lane;
-            if (w < words16) {
-              float lo[8], hi[8];
-#pragma unroll
-              for (int i = 0; i < 8; i++) {
-                lo[i] = acc[j][i];
-                hi[i] = acc[j][8 + i];
-              }
-              dst[2 * w] = Vec16<bf16>::fromFloat(lo);
-              dst[2 * w + 1] = Vec16<bf16>::fromFloat(hi);
-            }
-          }
-        }
-        continue;
-      }
-#pragma unroll 1
-      for (int w0 = 0; w0 < words; w0 += 32 * 4) {
-        float acc[4][8];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-#pragma unroll
-          for (int i = 0; i < 8; i++) acc[j][i] = 0.f;
-        }
-        for (int q = 0; q < nd; q++) {
-          uint4 v[4];
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const int w = w0 + j * 32 + lane;
-            v[j] = w < words ? ptx::ld_nc_na_v4(reinterpret_cast<const void*>(rowBase[q] + static_cast<uint64_t>(w) * 16)) : make_uint4(0, 0, 0, 0);
-          }
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            float f[8];
-            Vec16<bf16>::toFloat(v[j], f);
-#pragma unroll
-            for (int i = 0; i < 8; i++) acc[j][i] += wgt[q] * f[i];
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const int w = w0 + j * 32 + lane;
-          if (w < words) dst[w] = Vec16<bf16>::fromFloat(acc[j]);
+          for (int i = 0; i < 8; i++) part[i] = acc[j][8 * h + i];
+          dst[w * (kElems / 8) + h] = Vec16<bf16>::fromFloat(part);
         }
       }
     }
@@ -429,11 +489,12 @@ cudaError_t launchCoop(Kernel kernel, const Args& args, int nBlocks, int emu, cu
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), grid, block, params, 0, stream);
 }
 
-int defaultBlocks(int emu) {
+int defaultBlocks(int emu, int world) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int n = sms / (emu > 1 ? emu : 1);
-  if (n > 64) n = 64;  // NVLink-bound: 64 blocks x 16 warps x 8 KB rows keep several MB in flight
+  // several GPUs: bound by NVLink, 64 blocks keep several MB in flight. One rank: bound by HBM, which takes every SM
+  if (world > 1 && n > 64) n = 64;
   return n < 1 ? 1 : n;
 }
 
@@ -450,7 +511,7 @@ cudaError_t launchMoeDispatch(const MoeDispatchArgs& args, int nBlocks, cudaStre
   const int emu = args.emuRanks > 1 ? args.emuRanks : 1;
   if (!validCommon(args.comm, args.tokens, args.hidden, args.topk, args.numExperts, emu)) return cudaErrorInvalidValue;
   if (args.capacity <= 0 || (args.fp8 && args.recvScales == nullptr)) return cudaErrorInvalidValue;
-  if (nBlocks <= 0) nBlocks = defaultBlocks(emu);
+  if (nBlocks <= 0) nBlocks = defaultBlocks(emu, args.comm.world);
   if (nBlocks > kBarrierSlots) return cudaErrorInvalidValue;
   return launchCoop(moeDispatchKernel, args, nBlocks, emu, stream);
 }
@@ -469,9 +530,18 @@ cudaError_t launchMoeCombine(const MoeCombineArgs& args, int nBlocks, cudaStream
   const int emu = args.emuRanks > 1 ? args.emuRanks : 1;
   if (!validCommon(args.comm, args.tokens, args.hidden, args.topk, args.numExperts, emu)) return cudaErrorInvalidValue;
   if (args.fp8 && args.outScales == nullptr) return cudaErrorInvalidValue;
-  if (nBlocks <= 0) nBlocks = defaultBlocks(emu);
+  if (nBlocks <= 0) nBlocks = defaultBlocks(emu, args.comm.world);
   if (nBlocks > kBarrierSlots) return cudaErrorInvalidValue;
-  return launchCoop(moeCombineKernel, args, nBlocks, emu, stream);
+  if (args.topk <= 2) {
+    return args.fp8 ? launchCoop(moeCombineKernel<4, 2, true>, args, nBlocks, emu, stream)
+                    : launchCoop(moeCombineKernel<4, 2, false>, args, nBlocks, emu, stream);
+  }
+  if (args.topk <= 4) {
+    return args.fp8 ? launchCoop(moeCombineKernel<2, 4, true>, args, nBlocks, emu, stream)
+                    : launchCoop(moeCombineKernel<2, 4, false>, args, nBlocks, emu, stream);
+  }
+  return args.fp8 ? launchCoop(moeCombineKernel<1, 8, true>, args, nBlocks, emu, stream)
+                  : launchCoop(moeCombineKernel<1, 8, false>, args, nBlocks, emu, stream);
 }
 
 }  // namespace mscclpp

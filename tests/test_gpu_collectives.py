@@ -507,6 +507,56 @@ def test_moe_dispatch_combine(world, experts, tokens, hidden, topk, fp8):
     symm.destroy()
 
 
+@pytest.mark.parametrize("tokens,hidden,experts,topk,fp8", [
+    (1, 256, 8, 1, False),      # the smallest: one token, less than one piece of a row
+    (33, 768, 16, 3, True),     # an odd number of 256-element steps in a row's last piece
+    (149, 1280, 256, 8, False),  # one token more than thread blocks, all counters
+    (148 * 32 + 5, 512, 64, 2, True),  # more tokens per block than one batch of destinations
+    (700, 8192, 128, 5, False),  # the widest rows
+])
+def test_moe_one_rank(tokens, hidden, experts, topk, fp8):
+    """One rank: rows grouped by expert in expert order, every pair's slot pointing at its row, and the weighted sum back.
+    The result of identity experts is exact up to one bf16 rounding of an fp32 sum of `topk` terms."""
+    from mscclpp_b200 import SymmetricMemory
+    from mscclpp_b200.parallel.moe import ExpertParallelDispatcher, dequantize_rows
+
+    symm = SymmetricMemory.emulated(1, nbytes=tokens * topk * hidden * 5 + tokens * hidden * 4 + (64 << 20), timeout_ms=3000)
+    disp = ExpertParallelDispatcher(symm, num_experts=experts, hidden=hidden, max_tokens=tokens, topk=topk, capacity=tokens * topk, fp8=fp8,
+                                    fp8_combine=fp8)
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    for _ in range(2):
+        x = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+        idx = torch.rand((tokens, experts), generator=g, device="cuda").topk(topk, dim=1).indices.to(torch.int32)
+        idx[0, -1] = -1  # an unused slot
+        weights = torch.rand((tokens, topk), generator=g, device="cuda")
+        recv, counts, slots = disp.dispatch(x, idx)
+        used = idx >= 0
+        expect = torch.bincount(idx[used].long(), minlength=experts)
+        assert torch.equal(counts.long().cpu(), torch.cat([expect, expect.sum(0, keepdim=True)]).cpu())
+        first = torch.cumsum(expect, 0) - expect
+        assert torch.equal(slots[used].sort().values.long(), torch.arange(int(used.sum()), device="cuda"))
+        e = idx[used].long()
+        assert bool(((slots[used] >= first[e]) & (slots[used] < first[e] + expect[e])).all())
+        assert bool((slots[~used] == -1).all())
+        token = torch.arange(tokens, device="cuda")[:, None].expand(-1, topk)[used]
+        assert torch.equal(disp.recv_src[slots[used].long()].long(), token)
+        rows = dequantize_rows(recv, disp.recv_scales) if fp8 else recv.float()
+        got = rows[slots[used].long()]
+        # e4m3 keeps three mantissa bits: half a unit in the last place is 2^-4 of the value, at least 2^-10 of the scaled range
+        slack = x.float()[token].abs() / 16 + x.float()[token].abs().amax(1, keepdim=True) / 448 / 1024 if fp8 else torch.zeros_like(got)
+        assert bool(((got - x.float()[token]).abs() <= slack * 1.001).all())
+        if fp8:
+            disp.expert_out_q, disp.expert_out_scales = disp.recv_x, disp.recv_scales
+        y = disp.combine(idx, weights, slots, expert_out=None if fp8 else recv)
+        ref = torch.zeros((tokens, hidden), dtype=torch.float64, device="cuda")
+        ref.index_add_(0, token, rows[slots[used].long()].double() * weights[used].double()[:, None])
+        bound = ref.abs() * 2.0 ** -8 + torch.zeros_like(ref).index_add_(
+            0, token, rows[slots[used].long()].double().abs() * weights[used].double()[:, None]) * (topk + 1) * 2.0 ** -23
+        assert bool(((y.double() - ref).abs() <= bound).all())
+        symm.check()
+    symm.destroy()
+
+
 @pytest.mark.parametrize("world,experts,tokens,hidden,topk", [(2, 8, 120, 512, 2), (8, 64, 48, 4096, 2), (4, 16, 64, 1024, 4)])
 def test_moe_combine_fp8_payload(world, experts, tokens, hidden, topk):
     """Combine with e4m3 expert outputs (1 x 128 scales): the stand-alone quantiser against a PyTorch model of it, then the
