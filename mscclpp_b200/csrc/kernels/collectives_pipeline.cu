@@ -11,9 +11,13 @@
 //   4. barrier B   (every rank's part of my scratch-out slice has landed)
 //   5. copy-out    scratch-out -> user output                                  (local loads, L1 bypassed)
 //
-// Blocks never wait for other blocks of their own rank, so while one block sits in a barrier the others copy and
-// reduce: with a few blocks per SM the NVLink transfers, the local copies and the barrier latencies overlap. Scratch is
-// double buffered per block (round parity), which is what makes two barriers per round enough.
+// The barriers are split into a signal and a wait, and the copy-in of round r + 1 (with its signal) sits between round r's
+// reduction and its wait for barrier B, so a block copies while its peers reduce. Blocks never wait for other blocks of
+// their own rank, so while one block sits in a barrier the others copy and reduce as well: with a few blocks per SM the
+// NVLink transfers, the local copies and the barrier latencies overlap. Scratch is double buffered per block (round
+// parity), which is what makes two barriers per round enough.
+// Four ranks on one B200 (one HBM; 32 MB bf16 each): 121 us; 629 us with one copy load in flight per thread, system-scope
+// accesses, the barriers unsplit and 16 blocks per rank instead of the 74 that fit.
 // One round that covers the whole message is the un-pipelined "reduce-scatter + all-gather through scratch" form.
 //
 // Role of the reference's allreduce_nvls_block_pipeline.cu:16-147 / allreduce_nvls_warp_pipeline.cu:14-112 (NVLS) and
@@ -21,6 +25,8 @@
 // and chain them with device semaphores; here every block runs all legs on its own slice and the overlap comes from
 // the blocks being out of step with one another.
 #include "collectives.cuh"
+
+#include <type_traits>
 
 namespace mscclpp {
 
@@ -37,38 +43,63 @@ MSCCLPP_DEVICE_INLINE uint64_t* pipeFlag(const DeviceComm& c, int owner, int pha
          ((static_cast<uint64_t>(phase) * kBarrierSlots + slot) * kMaxRanks + src);
 }
 
-// All threads of the block call it. Stores made by the block before the call are visible to the peers' blocks of the same
-// slot after their call returns.
-MSCCLPP_DEVICE_INLINE bool pipeBarrier(const DeviceComm& c, int rank, int phase, int slot, uint64_t token, int* okSmem) {
+// The two halves of a barrier with the blocks of the same slot on every rank; all threads of the block call both. What the
+// block stored before pipeSignal is visible to a peer's block of this slot after its pipeWait for the same token. As in
+// rankBarrier, one fence and a relaxed flag store publish, and one acquire follows relaxed polls.
+MSCCLPP_DEVICE_INLINE void pipeSignal(const DeviceComm& c, int rank, int phase, int slot, uint64_t token) {
   __syncthreads();
   const int t = threadIdx.x;
   if (t < c.world && t != rank) {
     ptx::fence_acq_rel_sys();
-    ptx::st_release_sys(pipeFlag(c, t, phase, slot, rank), token);
-    if (!waitGreaterEqual(pipeFlag(c, rank, phase, slot, t), token, c.status, c.timeoutNs, kDevTimeoutBarrier, rank,
-                          20000 + phase * 1000 + slot, t)) {
-      *okSmem = 0;
+    ptx::st_relaxed_sys(pipeFlag(c, t, phase, slot, rank), token);
+  }
+}
+MSCCLPP_DEVICE_INLINE bool pipeWait(const DeviceComm& c, int rank, int phase, int slot, uint64_t token, int* okSmem) {
+  const int t = threadIdx.x;
+  if (t < c.world && t != rank) {
+    const uint64_t* mine = pipeFlag(c, rank, phase, slot, t);
+    SpinGuard g(c.status, c.timeoutNs);
+    uint64_t v;
+    bool here = true;
+    while ((v = ptx::ld_relaxed_sys(mine)) < token) {
+      if (!g.keepSpinning()) {
+        g.report(kDevTimeoutBarrier, rank, 20000 + phase * 1000 + slot, t, token, v);
+        here = false;
+        break;
+      }
     }
+    if (here) (void)ptx::ld_acquire_sys(mine);
+    else *okSmem = 0;
   }
   __syncthreads();
   return *okSmem != 0;
 }
 
-MSCCLPP_DEVICE_INLINE uint4 loadUnitTail(const char* base, uint64_t u, uint64_t bytes) {
-  const uint64_t off = u * 16;
-  if (off + 16 <= bytes) return *reinterpret_cast<const uint4*>(base + off);
-  uint32_t w[4] = {0, 0, 0, 0};
-  for (uint64_t i = off; i < bytes; i++) w[(i - off) >> 2] |= static_cast<uint32_t>(static_cast<uint8_t>(base[i])) << (8 * ((i - off) & 3));
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
-MSCCLPP_DEVICE_INLINE void storeUnitTail(char* base, uint64_t u, uint64_t bytes, uint4 v) {
-  const uint64_t off = u * 16;
-  if (off + 16 <= bytes) {
-    *reinterpret_cast<uint4*>(base + off) = v;
-    return;
+// `n` 16-byte units from src to dst, kCopyUnroll loads in flight per thread.
+constexpr uint32_t kCopyUnroll = 4;
+MSCCLPP_DEVICE_INLINE void copyUnits(char* dst, const char* src, uint32_t n) {
+  for (uint32_t u0 = threadIdx.x; u0 < n; u0 += blockDim.x * kCopyUnroll) {
+    uint4 v[kCopyUnroll];
+#pragma unroll
+    for (uint32_t k = 0; k < kCopyUnroll; k++) {
+      const uint32_t u = u0 + k * blockDim.x;  // (loads beyond the end repeat the last unit: no branch around them)
+      v[k] = ptx::ld_weak_v4(src + static_cast<uint64_t>(u < n ? u : n - 1) * 16);
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kCopyUnroll; k++) {
+      const uint32_t u = u0 + k * blockDim.x;
+      if (u < n) ptx::st_weak_v4(dst + static_cast<uint64_t>(u) * 16, v[k]);
+    }
   }
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-  for (uint64_t i = off; i < bytes; i++) base[i] = static_cast<char>(w[(i - off) >> 2] >> (8 * ((i - off) & 3)));
+}
+// The last bytes of a message whose size is not a multiple of 16: one thread, byte by byte; the scratch unit is padded
+// with zeros.
+MSCCLPP_DEVICE_INLINE void copyTail(char* dst, const char* src, uint32_t n, uint32_t padTo) {
+  if (threadIdx.x != 0) return;
+#pragma unroll 1
+  for (uint32_t i = 0; i < n; i++) *reinterpret_cast<volatile char*>(dst + i) = *reinterpret_cast<const volatile char*>(src + i);
+#pragma unroll 1
+  for (uint32_t i = n; i < padTo; i++) *reinterpret_cast<volatile char*>(dst + i) = 0;
 }
 
 template <typename T, ReduceOp Op>
@@ -132,73 +163,121 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
   const uint64_t scratchOff = reinterpret_cast<uint64_t>(a.scratch) - c.peerBase[c.rank];
   const uint64_t local = c.peerBase[rank];
   __shared__ int okSmem;
+  __shared__ uint64_t heaps[8];  // (in shared memory: as kernel parameters their sums with the slices live in registers all along)
+  if (threadIdx.x < 8) heaps[threadIdx.x] = c.peerBase[threadIdx.x];
   if (threadIdx.x == 0) okSmem = 1;
   __syncthreads();
 
-  bool healthy = true;
-  for (uint64_t r = 0; r < rounds && healthy; r++) {
-    const uint64_t first = r * roundUnits + static_cast<uint64_t>(slot) * sliceUnits;  // first global unit of my slice
-    const uint64_t parityOff = scratchOff + (r & 1) * (2ull * gridDim.x * a.sliceBytes);
-    const uint64_t inSlice = parityOff + static_cast<uint64_t>(slot) * a.sliceBytes;
-    const uint64_t outSlice = parityOff + (static_cast<uint64_t>(gridDim.x) + slot) * a.sliceBytes;
-    const uint64_t token = (static_cast<uint64_t>(epoch) << 32) | (r + 1);
-    const uint64_t have = first < nunits ? (nunits - first < sliceUnits ? nunits - first : sliceUnits) : 0;  // units of this slice that exist
+  const uint64_t roundBytes = 2ull * gridDim.x * a.sliceBytes;  // scratch of one parity
+  const uint32_t tailBytes = static_cast<uint32_t>(bytes & 15);   // of the message's last unit, 0 = it is whole
+  auto inSliceOf = [&](uint64_t r) { return scratchOff + (r & 1) * roundBytes + static_cast<uint64_t>(slot) * a.sliceBytes; };
+  auto firstOf = [&](uint64_t r) { return r * roundUnits + static_cast<uint64_t>(slot) * sliceUnits; };  // first global unit of my slice
+  auto haveOf = [&](uint64_t r) {  // units of my slice that exist, the last of them possibly not whole
+    const uint64_t first = firstOf(r);
+    return static_cast<uint32_t>(first < nunits ? (nunits - first < sliceUnits ? nunits - first : sliceUnits) : 0);
+  };
+  auto tailOf = [&](uint64_t r, uint32_t have) { return have != 0 && firstOf(r) + have == nunits ? tailBytes : 0u; };
+  // 1. copy-in (nothing to do for a slice beyond the end of the message, but the barriers still run: peers may not know)
+  auto copyIn = [&](uint64_t r) {
+    const uint32_t have = haveOf(r), tail = tailOf(r, have), whole = have - (tail != 0 ? 1 : 0);
+    const char* src = in + firstOf(r) * 16;
+    char* dst = reinterpret_cast<char*>(local + inSliceOf(r));
+    copyUnits(dst, src, whole);
+    if (tail != 0) copyTail(dst + static_cast<uint64_t>(whole) * 16, src + static_cast<uint64_t>(whole) * 16, tail, 16);
+  };
+  auto tokenOf = [&](uint64_t r) { return (static_cast<uint64_t>(epoch) << 32) | (r + 1); };
 
-    // 1. copy-in (nothing to do for a slice beyond the end of the message, but the barriers still run: peers may not know)
-    for (uint64_t u = threadIdx.x; u < have; u += blockDim.x) {
-      *reinterpret_cast<uint4*>(local + inSlice + u * 16) = loadUnitTail(in, first + u, bytes);
-    }
+  bool healthy = true;
+  if (rounds > 0) {
+    copyIn(0);
+    pipeSignal(c, rank, 0, slot, tokenOf(0));
+  }
+#pragma unroll 1
+  for (uint64_t r = 0; r < rounds; r++) {
+    const uint64_t inSlice = inSliceOf(r);
+    const uint64_t outSlice = inSlice + static_cast<uint64_t>(gridDim.x) * a.sliceBytes;
+    const uint32_t have = haveOf(r);
     // 2. every rank has staged its slice of this index
-    healthy = pipeBarrier(c, rank, 0, slot, token, &okSmem);
+    healthy = pipeWait(c, rank, 0, slot, tokenOf(r), &okSmem);
     if (!healthy) break;
     // 3. reduce my part of the slice, result to everybody's scratch-out
     {
-      const uint64_t begin = static_cast<uint64_t>(rank) * subUnits;
-      const uint64_t end = begin + subUnits < have ? begin + subUnits : have;
-      constexpr int kUnroll = kNvls ? 4 : 2;  // peer loads hold `world` words per unit in registers
-      for (uint64_t u0 = begin + threadIdx.x; u0 < end; u0 += static_cast<uint64_t>(blockDim.x) * kUnroll) {
-        uint4 v[kUnroll];
-#pragma unroll
-        for (int k = 0; k < kUnroll; k++) {
-          const uint64_t u = u0 + static_cast<uint64_t>(k) * blockDim.x;
-          if (u >= end) continue;
+      const uint32_t begin = static_cast<uint32_t>(rank) * static_cast<uint32_t>(subUnits);
+      const uint32_t end = begin + static_cast<uint32_t>(subUnits) < have ? begin + static_cast<uint32_t>(subUnits) : have;
+      // eight loads in flight per thread: kUnroll units of up to kSources ranks each (with the switch, four sums)
+      auto sweep = [&](auto unrollTag, auto sourcesTag) {
+        constexpr int kUnroll = decltype(unrollTag)::value, kSources = decltype(sourcesTag)::value;
+#pragma unroll 1
+        for (uint32_t u0 = begin + threadIdx.x; u0 < end; u0 += blockDim.x * kUnroll) {
+          uint4 v[kUnroll];
           if constexpr (kNvls) {
-            v[k] = switchReduce<T, Op>(reinterpret_cast<const void*>(c.mcBase + inSlice + u * 16));
+#pragma unroll
+            for (int k = 0; k < kUnroll; k++) {
+              const uint32_t u = u0 + k * blockDim.x;
+              if (u < end) v[k] = switchReduce<T, Op>(reinterpret_cast<const void*>(c.mcBase + inSlice + static_cast<uint64_t>(u) * 16));
+            }
           } else {
-            PipeAccum<T, Op> acc;
-            uint4 w[8];
+            uint4 w[kUnroll][kSources];
 #pragma unroll
-            for (int p = 0; p < 8; p++)
-              if (p < world) w[p] = ptx::ld_nc_na_v4(reinterpret_cast<const void*>(c.peerBase[p] + inSlice + u * 16));
-            acc.init(w[0]);
+            for (int k = 0; k < kUnroll; k++) {
+              const uint32_t u = u0 + k * blockDim.x;
+              const uint64_t off = inSlice + static_cast<uint64_t>(u < end ? u : end - 1) * 16;
 #pragma unroll
-            for (int p = 1; p < 8; p++)
-              if (p < world) acc.add(w[p]);
-            v[k] = acc.result();
+              for (int p = 0; p < kSources; p++)  // (slots beyond the last rank read local memory and are not added)
+                w[k][p] = ptx::ld_weak_v4(reinterpret_cast<const void*>(heaps[p < world ? p : rank] + off));
+            }
+#pragma unroll
+            for (int k = 0; k < kUnroll; k++) {
+              PipeAccum<T, Op> acc;
+              acc.init(w[k][0]);
+#pragma unroll
+              for (int p = 1; p < kSources; p++)
+                if (p < world) acc.add(w[k][p]);
+              v[k] = acc.result();
+            }
           }
-        }
 #pragma unroll
-        for (int k = 0; k < kUnroll; k++) {
-          const uint64_t u = u0 + static_cast<uint64_t>(k) * blockDim.x;
-          if (u >= end) continue;
-          if constexpr (kNvls) {
-            ptx::multimem_st_v4(reinterpret_cast<void*>(c.mcBase + outSlice + u * 16), v[k]);
-          } else {
-            for (int i = 0; i < world; i++) {
-              const int p = (rank + i) % world;
-              ptx::st_na_v4(reinterpret_cast<void*>(c.peerBase[p] + outSlice + u * 16), v[k]);
+          for (int k = 0; k < kUnroll; k++) {
+            const uint32_t u = u0 + k * blockDim.x;
+            if (u >= end) continue;
+            const uint64_t off = outSlice + static_cast<uint64_t>(u) * 16;
+            if constexpr (kNvls) {
+              ptx::multimem_st_v4(reinterpret_cast<void*>(c.mcBase + off), v[k]);
+            } else {
+#pragma unroll 1
+              for (int i = 0; i < world; i++) {
+                const int p = rank + i < world ? rank + i : rank + i - world;
+                ptx::st_weak_v4(reinterpret_cast<void*>(heaps[p] + off), v[k]);
+              }
             }
           }
         }
+      };
+      using std::integral_constant;
+      if constexpr (kNvls) {
+        sweep(integral_constant<int, 4>{}, integral_constant<int, 1>{});
+      } else {
+        if (world <= 2) sweep(integral_constant<int, 4>{}, integral_constant<int, 2>{});
+        else if (world <= 4) sweep(integral_constant<int, 2>{}, integral_constant<int, 4>{});
+        else sweep(integral_constant<int, 1>{}, integral_constant<int, 8>{});
       }
     }
+    pipeSignal(c, rank, 1, slot, tokenOf(r));
+    // the next round's copy-in, under the peers' reductions. Its scratch was last read in round r - 1, and the end of that
+    // round told this block that every rank had reduced it.
+    if (r + 1 < rounds) {
+      copyIn(r + 1);
+      pipeSignal(c, rank, 0, slot, tokenOf(r + 1));
+    }
     // 4. every rank's part of my scratch-out slice has landed
-    healthy = pipeBarrier(c, rank, 1, slot, token, &okSmem);
+    healthy = pipeWait(c, rank, 1, slot, tokenOf(r), &okSmem);
     if (!healthy) break;
     // 5. copy-out
-    for (uint64_t u = threadIdx.x; u < have; u += blockDim.x) {
-      storeUnitTail(out, first + u, bytes, ptx::ld_nc_na_v4(reinterpret_cast<const void*>(local + outSlice + u * 16)));
-    }
+    const uint32_t tail = tailOf(r, have), whole = have - (tail != 0 ? 1 : 0);
+    const char* src = reinterpret_cast<const char*>(local + outSlice);
+    char* dst = out + firstOf(r) * 16;
+    copyUnits(dst, src, whole);
+    if (tail != 0) copyTail(dst + static_cast<uint64_t>(whole) * 16, src + static_cast<uint64_t>(whole) * 16, tail, 0);
   }
   finishLaunch(c, rank, epoch);
 }

@@ -158,7 +158,9 @@ def all_reduce(symm: SymmetricMemory, inp: torch.Tensor, out: Optional[torch.Ten
             assert inp.shape[0] == symm.world and out.shape[0] == symm.world
             nbytes //= symm.world
             emu_stride = nbytes
-            blocks = min(blocks, 16)
+            # all ranks run at the same time on one GPU; the kernel is built for two resident blocks per SM
+            sms = torch.cuda.get_device_properties(symm.device).multi_processor_count
+            blocks = max(1, min(blocks, 2 * sms // symm.world))
         n.pipeline_allreduce(symm.heap, inp.data_ptr(), out.data_ptr(), nbytes, torch_dtype_to_native(inp.dtype), _op(op), scratch.data_ptr(),
                              slice_bytes, blocks, n_threads or 512, _stream(stream), algo == "nvls_block_pipeline", emu_stride)
         return out

@@ -83,6 +83,31 @@ def test_allreduce_pipeline_buffers_outside_the_heap(world, dtype, numel):
     symm.destroy()
 
 
+@pytest.mark.parametrize("world,numel,n_blocks", [(1, 3, 1), (1, 100003, 2), (3, 1009, 2), (5, 70001, 3), (7, 40000, 0), (2, 5000003, 0), (4, 2100001, 0)])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.float16])
+def test_allreduce_pipeline_ragged(world, numel, n_blocks, dtype):
+    """Messages that end inside a 16-byte unit and inside a slice, ranks that fill no batch of sources, one round and many,
+    in place and not. Integers are exact; fp16 sums in fp32 round once (2^-11 of the value) after `world` fp32 additions."""
+    from mscclpp_b200.ops import all_reduce
+
+    # (the rows of emulated ranks follow one another and start on 16-byte boundaries: only one rank can end inside a unit)
+    stride = numel if world == 1 else (numel * dtype.itemsize + 15) // 16 * 16 // dtype.itemsize
+    symm = _symm(world)
+    g = torch.Generator(device="cuda").manual_seed(numel)
+    x = torch.randn((world, stride), generator=g, device="cuda")
+    x = (x * 1000).to(dtype) if not dtype.is_floating_point else x.to(dtype)
+    expect = x.double().sum(0)
+    bound = 0 if not dtype.is_floating_point else expect.abs() * 2.0 ** -11 + x.double().abs().sum(0) * world * 2.0 ** -23 + 2.0 ** -25
+    for in_place in (False, True):
+        src = x.clone()
+        out = src if in_place else torch.zeros_like(src)
+        all_reduce(symm, src, out, algo="rsag_pipeline", n_blocks=n_blocks)
+        torch.cuda.synchronize()
+        symm.check()
+        assert bool(((out.double() - expect).abs() <= bound).all())
+    symm.destroy()
+
+
 @pytest.mark.parametrize("world", [2, 8])
 def test_allreduce_ll_int_and_min(world):
     from mscclpp_b200.ops import all_reduce
