@@ -14,6 +14,8 @@
 //     reference silently skips them on CUDA).
 #include "execution_kernel.hpp"
 
+#include <type_traits>
+
 #include <mscclpp/copy_device.hpp>
 #include <mscclpp/npkit/npkit.hpp>
 #include <mscclpp/packet_device.hpp>
@@ -187,19 +189,54 @@ MSCCLPP_DEVICE_INLINE void portRequests(Ctx& x, const DevOp& op, uint32_t kind, 
   if (!portOk) x.healthy = false;
 }
 
+// The vector body of a reduction, a function of its own: inlined into the interpreter it has to share 64 registers with
+// every other operation's state, and the loads in flight are what gets spilled.
+template <typename T>
+__noinline__ __device__ void reduceWords(char* const* src, int nSrc, char* const* dst, int nDst, uint64_t nvec) {
+#pragma unroll 1
+  for (uint64_t i = threadIdx.x; i < nvec; i += blockDim.x) {
+    ExecAccum<T> acc;
+    auto batch = [&](int s, auto count) {
+      constexpr int kCount = decltype(count)::value;
+      uint4 v[kCount];
+#pragma unroll
+      for (int k = 0; k < kCount; k++) v[k] = ptx::ld_weak_v4(src[s + k] + i * 16);
+      if (s == 0) acc.init(v[0]);
+      else acc.add(v[0]);
+#pragma unroll
+      for (int k = 1; k < kCount; k++) acc.add(v[k]);
+    };
+    int s = 0;
+#pragma unroll 1
+    for (; s + 4 <= nSrc; s += 4) batch(s, std::integral_constant<int, 4>{});
+    if (s + 2 <= nSrc) {
+      batch(s, std::integral_constant<int, 2>{});
+      s += 2;
+    }
+    if (s < nSrc) batch(s, std::integral_constant<int, 1>{});
+    const uint4 r = acc.result();
+#pragma unroll 1
+    for (int d = 0; d < nDst; d++) ptx::st_weak_v4(dst[d] + i * 16, r);
+  }
+}
+
 // dst[k] (all of them) = sum over src[*]. Sizes are multiples of 16 bytes (plans align chunks to 16).
 template <typename T>
 MSCCLPP_DEVICE_INLINE void reduceOp(const Ctx& x, const DevOp& op) {
   uint64_t skip;
   const uint64_t bytes = sliced(x, op, op.src[0], skip);
   const uint64_t nvec = bytes / 16;
-  for (uint64_t i = threadIdx.x; i < nvec; i += blockDim.x) {
-    ExecAccum<T> acc;
-    acc.init(ptx::ld_nc_na_v4(plainAddr(x, op.src[0], skip) + i * 16));
-    for (int s = 1; s < op.nSrc; s++) acc.add(ptx::ld_nc_na_v4(plainAddr(x, op.src[s], skip) + i * 16));
-    const uint4 r = acc.result();
-    for (int d = 0; d < op.nDst; d++) ptx::st_na_v4(plainAddr(x, op.dst[d], skip) + i * 16, r);
-  }
+  // Operand addresses are worked out once per operation, by one thread each, and the sources of a word are requested
+  // up to four at a time: one after the other they cost a dependent round trip each, with a walk over the operand's fields in
+  // the plan (global memory) in front of it. Reduce-scatter of 16 MB fp16 over eight ranks on one B200, 64 blocks: 89 -> 48 us.
+  __shared__ char* srcAddr[kExecMaxOperands];
+  __shared__ char* dstAddr[kExecMaxOperands];
+  const int nSrc = op.nSrc, nDst = op.nDst;
+  __syncthreads();  // the previous operation's readers are done with the addresses
+  if (threadIdx.x < static_cast<uint32_t>(nSrc)) srcAddr[threadIdx.x] = plainAddr(x, op.src[threadIdx.x], skip);
+  if (threadIdx.x >= 32 - static_cast<uint32_t>(nDst) && threadIdx.x < 32) dstAddr[31 - threadIdx.x] = plainAddr(x, op.dst[31 - threadIdx.x], skip);
+  __syncthreads();
+  reduceWords<T>(srcAddr, nSrc, dstAddr, nDst, nvec);
   // tail shorter than one vector (only with alignment < 16): element-wise through a zero-padded word
   const uint64_t tail = bytes - nvec * 16;
   if (tail != 0 && threadIdx.x == 0) {

@@ -230,3 +230,13 @@ def test_guard_bands_around_executor_buffers(monkeypatch):
         assert symm.heap.bytes_free() > free_before  # the buffers went back to the heap all the same
     assert executor.canary_regions() == []
     symm.destroy()
+
+
+@pytest.mark.parametrize("world", [2, 3, 4, 5, 6, 7, 8])
+def test_reductions_of_every_number_of_sources(world):
+    """The interpreter requests a reduction's sources in groups of four, two and one: every remainder of that split."""
+    from mscclpp_b200.default_algos import single_node
+
+    for per in (8, 1040):
+        _run_both(single_node.build("reducescatter_allpairs", world).to_json(), world, world * per, per, np.float16, inplace=False)
+        _run_both(single_node.build("reducescatter_allpairs", world).to_json(), world, world * per, per, np.int32, inplace=False)
