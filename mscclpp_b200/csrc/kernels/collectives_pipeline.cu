@@ -16,8 +16,9 @@
 // their own rank, so while one block sits in a barrier the others copy and reduce as well: with a few blocks per SM the
 // NVLink transfers, the local copies and the barrier latencies overlap. Scratch is double buffered per block (round
 // parity), which is what makes two barriers per round enough.
-// Four ranks on one B200 (one HBM; 32 MB bf16 each): 121 us; 629 us with one copy load in flight per thread, system-scope
-// accesses, the barriers unsplit and 16 blocks per rank instead of the 74 that fit.
+// Four ranks on one B200 (one HBM; 32 MB bf16 each): 102 us, 121 us when a rank's own part went through the scratch as well;
+// 629 us with one copy load in flight per thread, system-scope accesses, the barriers unsplit and 16 blocks per rank
+// instead of the 74 that fit.
 // One round that covers the whole message is the un-pipelined "reduce-scatter + all-gather through scratch" form.
 //
 // Role of the reference's allreduce_nvls_block_pipeline.cu:16-147 / allreduce_nvls_warp_pipeline.cu:14-112 (NVLS) and
@@ -75,10 +76,10 @@ MSCCLPP_DEVICE_INLINE bool pipeWait(const DeviceComm& c, int rank, int phase, in
   return *okSmem != 0;
 }
 
-// `n` 16-byte units from src to dst, kCopyUnroll loads in flight per thread.
+// 16-byte units [first, n) from src to dst, kCopyUnroll loads in flight per thread.
 constexpr uint32_t kCopyUnroll = 4;
-MSCCLPP_DEVICE_INLINE void copyUnits(char* dst, const char* src, uint32_t n) {
-  for (uint32_t u0 = threadIdx.x; u0 < n; u0 += blockDim.x * kCopyUnroll) {
+MSCCLPP_DEVICE_INLINE void copyUnits(char* dst, const char* src, uint32_t first, uint32_t n) {
+  for (uint32_t u0 = first + threadIdx.x; u0 < n; u0 += blockDim.x * kCopyUnroll) {
     uint4 v[kCopyUnroll];
 #pragma unroll
     for (uint32_t k = 0; k < kCopyUnroll; k++) {
@@ -177,12 +178,23 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
     return static_cast<uint32_t>(first < nunits ? (nunits - first < sliceUnits ? nunits - first : sliceUnits) : 0);
   };
   auto tailOf = [&](uint64_t r, uint32_t have) { return have != 0 && firstOf(r) + have == nunits ? tailBytes : 0u; };
+  // The part of a slice that this rank reduces is read by nobody else, and nobody else writes its result: with peer loads
+  // its whole units skip the scratch both ways (1 / world of the copies).
+  const uint32_t ownBegin = static_cast<uint32_t>(rank) * static_cast<uint32_t>(subUnits), ownEnd = ownBegin + static_cast<uint32_t>(subUnits);
+  auto copyOthers = [&](char* dst, const char* src, uint32_t whole) {
+    if constexpr (kNvls) {
+      copyUnits(dst, src, 0, whole);
+    } else {
+      copyUnits(dst, src, 0, ownBegin < whole ? ownBegin : whole);
+      copyUnits(dst, src, ownEnd, whole);
+    }
+  };
   // 1. copy-in (nothing to do for a slice beyond the end of the message, but the barriers still run: peers may not know)
   auto copyIn = [&](uint64_t r) {
     const uint32_t have = haveOf(r), tail = tailOf(r, have), whole = have - (tail != 0 ? 1 : 0);
     const char* src = in + firstOf(r) * 16;
     char* dst = reinterpret_cast<char*>(local + inSliceOf(r));
-    copyUnits(dst, src, whole);
+    copyOthers(dst, src, whole);
     if (tail != 0) copyTail(dst + static_cast<uint64_t>(whole) * 16, src + static_cast<uint64_t>(whole) * 16, tail, 16);
   };
   auto tokenOf = [&](uint64_t r) { return (static_cast<uint64_t>(epoch) << 32) | (r + 1); };
@@ -202,8 +214,11 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
     if (!healthy) break;
     // 3. reduce my part of the slice, result to everybody's scratch-out
     {
-      const uint32_t begin = static_cast<uint32_t>(rank) * static_cast<uint32_t>(subUnits);
-      const uint32_t end = begin + static_cast<uint32_t>(subUnits) < have ? begin + static_cast<uint32_t>(subUnits) : have;
+      const uint32_t begin = ownBegin;
+      const uint32_t end = ownEnd < have ? ownEnd : have;
+      [[maybe_unused]] const uint32_t direct = have - (tailOf(r, have) != 0 ? 1 : 0);  // units below it are whole
+      [[maybe_unused]] const uint64_t inDirect = reinterpret_cast<uint64_t>(in) + firstOf(r) * 16;
+      [[maybe_unused]] const uint64_t outDirect = reinterpret_cast<uint64_t>(out) + firstOf(r) * 16;
       // eight loads in flight per thread: kUnroll units of up to kSources ranks each (with the switch, four sums)
       auto sweep = [&](auto unrollTag, auto sourcesTag) {
         constexpr int kUnroll = decltype(unrollTag)::value, kSources = decltype(sourcesTag)::value;
@@ -221,10 +236,12 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
 #pragma unroll
             for (int k = 0; k < kUnroll; k++) {
               const uint32_t u = u0 + k * blockDim.x;
-              const uint64_t off = inSlice + static_cast<uint64_t>(u < end ? u : end - 1) * 16;
+              const uint32_t uc = u < end ? u : end - 1;
+              const uint64_t off = static_cast<uint64_t>(uc) * 16;
+              const uint64_t own = (uc < direct ? inDirect : local + inSlice) + off;
 #pragma unroll
               for (int p = 0; p < kSources; p++)  // (slots beyond the last rank read local memory and are not added)
-                w[k][p] = ptx::ld_weak_v4(reinterpret_cast<const void*>(heaps[p < world ? p : rank] + off));
+                w[k][p] = ptx::ld_weak_v4(reinterpret_cast<const void*>(p < world && p != rank ? heaps[p] + inSlice + off : own));
             }
 #pragma unroll
             for (int k = 0; k < kUnroll; k++) {
@@ -245,10 +262,11 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
               ptx::multimem_st_v4(reinterpret_cast<void*>(c.mcBase + off), v[k]);
             } else {
 #pragma unroll 1
-              for (int i = 0; i < world; i++) {
+              for (int i = 1; i < world; i++) {
                 const int p = rank + i < world ? rank + i : rank + i - world;
                 ptx::st_weak_v4(reinterpret_cast<void*>(heaps[p] + off), v[k]);
               }
+              ptx::st_weak_v4(reinterpret_cast<void*>(u < direct ? outDirect + static_cast<uint64_t>(u) * 16 : local + off), v[k]);
             }
           }
         }
@@ -276,7 +294,7 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
     const uint32_t tail = tailOf(r, have), whole = have - (tail != 0 ? 1 : 0);
     const char* src = reinterpret_cast<const char*>(local + outSlice);
     char* dst = out + firstOf(r) * 16;
-    copyUnits(dst, src, whole);
+    copyOthers(dst, src, whole);
     if (tail != 0) copyTail(dst + static_cast<uint64_t>(whole) * 16, src + static_cast<uint64_t>(whole) * 16, tail, 0);
   }
   finishLaunch(c, rank, epoch);
