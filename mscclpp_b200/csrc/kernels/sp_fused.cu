@@ -235,13 +235,14 @@ __global__ void __launch_bounds__(gemm::kNumThreads, 1)
     };
     auto epi = makeEpilogue();
     gemm::Shape shape = a.shape;
-    shape.mOrder = 2;
+    if (c.world > 1) {  // own rows first, then the peers' in the order in which the copiers bring them
+      shape.mOrder = 2;
+      shape.mOrderParam = kBlockN == 0 ? rank * per / 2 : rank * per;  // (the pair core orders 256-row blocks)
+    }
     if constexpr (kBlockN == 0) {
-      shape.mOrderParam = rank * per / 2;  // the pair core orders 256-row blocks
       gemm::gemmCtaPair(&maps.aFull[blockIdx.y], &maps.b[blockIdx.y], shape, blockIdx.x / 2, a.numGemmCtas / 2, gate, epi, c.status,
                         c.timeoutNs, smemRaw);
     } else {
-      shape.mOrderParam = rank * per;
       gemm::gemmCta<kBlockN>(&maps.aFull[blockIdx.y], &maps.b[blockIdx.y], shape, blockIdx.x, a.numGemmCtas, gate, epi, c.status,
                              c.timeoutNs, smemRaw);
     }
@@ -337,7 +338,19 @@ cudaError_t launchAllGatherGemm(const AgGemmArgs& argsIn, const void* const* B, 
   }
   const int tiles = numMBlk * (N / tileN);
   const int sms = gemm::smCount() / emu;
-  if (numCopiers <= 0) numCopiers = world == 1 ? 1 : (sms >= 64 ? 12 : 2);
+  // One rank has nothing to gather: no copier takes an SM from the GEMM, and the tiles are walked in bands of 2048 rows (the
+  // order of a plain GEMM) instead of one row block after the other, which re-reads all of W for every wave.
+  // The gated MLP of 8192 tokens x 8192 x 3584 on one B200, together with the plain product of its second half (see mode 2 in
+  // tp_fused.cu): 1274 -> 1120 us.
+  if (numCopiers <= 0) numCopiers = world == 1 ? 0 : (sms >= 64 ? 12 : 2);
+  if (world == 1) {
+    const int rowBlocks = M / (twoSm ? gemm::Config2::kPairM : gemm::kBlockM), band = 2048 / (twoSm ? gemm::Config2::kPairM : gemm::kBlockM);
+    args.shape.rowMajorTiles = 0;
+    if (rowBlocks > band) {
+      args.shape.mOrder = 3;
+      args.shape.mOrderParam = band;
+    }
+  }
   if (numCopiers > kBarrierSlots) numCopiers = kBarrierSlots;
   int gemmCtas = args.numGemmCtas > 0 ? args.numGemmCtas : sms - numCopiers;
   if (gemmCtas > tiles) gemmCtas = tiles;

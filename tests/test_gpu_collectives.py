@@ -452,6 +452,53 @@ def test_gemm_reduce_scatter_one_kernel(world, rows_per_rank, k, n_cols):
     symm.destroy()
 
 
+@pytest.mark.parametrize("rows,k,n_cols,act", [
+    (128, 128, 128, "none"),      # one tile
+    (256, 256, 512, "gelu"),      # one pair of SMs' tile in each direction
+    (2304, 128, 256, "silu"),     # a band of 2048 rows and a last one of one tile, two-SM core
+    (2176, 128, 384, "none"),     # the same on one-SM tiles
+    (2304, 128, 512, "swiglu"),
+])
+def test_sequence_parallel_halves_on_one_rank(rows, k, n_cols, act):
+    """One rank: no copiers, the band order, and the product stored where the reduce-scatter leaves it. Bounds: fp32
+    accumulation (k * 2^-24 of the products' magnitudes, twice that through an activation of slope below 1.13 and the other
+    factor of a gate), the activation's own error, one bf16 rounding."""
+    from mscclpp_b200 import SymmetricMemory
+    from mscclpp_b200.parallel.sp_layer import all_gather_gemm, gemm_reduce_scatter
+
+    symm = SymmetricMemory.emulated(1, nbytes=64 << 20, timeout_ms=3000)
+    g = torch.Generator(device="cuda").manual_seed(rows + n_cols)
+    x = symm.tensor((rows, k), torch.bfloat16)
+    x.copy_(torch.randn((rows, k), generator=g, device="cuda"))
+    w = (torch.randn((n_cols, k), generator=g, device="cuda") * 0.1).to(torch.bfloat16)
+    full = symm.tensor((rows, k), torch.bfloat16)
+    out = symm.tensor((rows, n_cols // 2 if act == "swiglu" else n_cols), torch.bfloat16)
+    back = symm.tensor((rows, n_cols), torch.bfloat16)
+    partial = symm.tensor((rows, n_cols), torch.bfloat16)
+    p = x.double() @ w.double().t()
+    slack = (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24
+    ref, extra = p, slack
+    if act == "gelu":
+        ref = torch.nn.functional.gelu(p, approximate="tanh")
+    elif act == "silu":
+        ref = torch.nn.functional.silu(p)
+    elif act == "swiglu":
+        gate, up = (t.reshape(rows, -1) for t in p.view(rows, -1, 2, 32).unbind(2))
+        sg, su = (t.reshape(rows, -1) for t in slack.view(rows, -1, 2, 32).unbind(2))
+        ref = torch.nn.functional.silu(gate) * up
+        extra = sg * up.abs() + su * gate.abs()
+    for _ in range(2):
+        out.fill_(float("nan"))
+        back.fill_(float("nan"))
+        all_gather_gemm(symm, x, full, w, out, activation=act)
+        gemm_reduce_scatter(symm, x, w, partial, back)
+        torch.cuda.synchronize()
+        symm.check()
+        assert bool(((out.double() - ref).abs() <= ref.abs() * (2.0 ** -8) + 2 * extra + 1e-6).all())
+        assert bool(((back.double() - p).abs() <= p.abs() * 2.0 ** -8 + slack).all())
+    symm.destroy()
+
+
 def _moe_reference(xs, idxs, wts, world, experts, f):
     """fp32 PyTorch model of dispatch -> expert function f(e, rows) -> combine, for all ranks."""
     ys = []
