@@ -16,19 +16,24 @@
 namespace mscclpp {
 namespace gemm {
 
-struct Config2 {
+template <int kStages_, int kStagingBytes_, int kBarrierBytes_>
+struct Config2Of {
   static constexpr int kBlockN = 256;
   static constexpr int kPairM = 2 * kBlockM;                       // 256 rows per tile
   static constexpr int kStageABytes = kBlockM * kBlockK * 2;       // this CTA's A half: 16 KB
   static constexpr int kStageBBytes = (kBlockN / 2) * kBlockK * 2;  // this CTA's B half: 16 KB
   static constexpr int kStageBytes = kStageABytes + kStageBBytes;
-  static constexpr int kStages = 6;
+  static constexpr int kStages = kStages_;
   static constexpr int kTmemCols = 2 * kBlockN;  // two accumulator buffers of 256 columns
-  static constexpr int kBarrierBytes = 256;
+  static constexpr int kBarrierBytes = kBarrierBytes_;
+  static constexpr int kStagingBytes = kStagingBytes_;  // of the epilogue
   static constexpr int kEpiWarps = kNumEpilogueWarps;
   static constexpr int kColsPerWarp = kBlockN / 2;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kEpilogueStagingBytes + kBarrierBytes + 1024;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + kBarrierBytes + 1024;
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
 };
+using Config2 = Config2Of<6, kEpilogueStagingBytes, 256>;
+using Config2Rows = Config2Of<5, 2 * kEpilogueStagingBytes, 512>;  // row epilogues: every block of a warp's tile is staged
 
 MSCCLPP_HOST_DEVICE_INLINE constexpr uint32_t makeInstrDescPair() {
   return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(Config2::kBlockN >> 3) << 17) |
@@ -37,10 +42,9 @@ MSCCLPP_HOST_DEVICE_INLINE constexpr uint32_t makeInstrDescPair() {
 
 // Body of one CTA of a pair. All threads call it; `pairIdx` / `numPairs` index the persistent tile loop.
 // shape.mOrder / mOrderParam apply to 256-row blocks here.
-template <typename AGate, typename Epilogue>
+template <typename Cfg = Config2, typename AGate, typename Epilogue>
 MSCCLPP_DEVICE_INLINE void gemmCtaPair(const CUtensorMap* tmapA, const CUtensorMap* tmapB, Shape shape, int pairIdx, int numPairs,
                                        AGate& gate, Epilogue& epi, DeviceStatus* status, uint64_t budgetNs, uint8_t* smemRaw) {
-  using Cfg = Config2;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t ctaRank = ptx::cluster_ctarank();
@@ -49,7 +53,7 @@ MSCCLPP_DEVICE_INLINE void gemmCtaPair(const CUtensorMap* tmapA, const CUtensorM
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
   uint8_t* tiles = smem;
   uint8_t* staging = smem + Cfg::kStages * Cfg::kStageBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(staging + kEpilogueStagingBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(staging + Cfg::kStagingBytes);
   SharedState st;
   st.full = bars;
   st.empty = bars + Cfg::kStages;
@@ -78,6 +82,9 @@ MSCCLPP_DEVICE_INLINE void gemmCtaPair(const CUtensorMap* tmapA, const CUtensorM
     ptx::fence_mbar_init();
     ptx::tma_prefetch_desc(tmapA);
     ptx::tma_prefetch_desc(tmapB);
+  }
+  if constexpr (IsRowEpilogue<Epilogue>::value) {
+    if (warp >= 2) epi.setup(staging + (warp - 2) * Epilogue::kBlocks * kStagingBytesPerWarp, bars + 20 + (warp - 2) * Epilogue::kBlocks, lane);
   }
   __syncthreads();
   // the peer's barriers must exist before anything of mine can signal them
@@ -188,14 +195,28 @@ MSCCLPP_DEVICE_INLINE void gemmCtaPair(const CUtensorMap* tmapA, const CUtensorM
       const int row0 = mBlk * kBlockM + quarter * 32;
       const int col0 = nBlk * Cfg::kBlockN + part * Cfg::kColsPerWarp;
       // lets the epilogue put loads it will need (a residual, a bias) in flight while the MMAs of this tile still run
-      epi.tileBegin(row0, col0, lane);
+      if constexpr (IsRowEpilogue<Epilogue>::value) {
+        if (it == 0) epi.request(row0, col0, lane);
+      } else {
+        epi.tileBegin(row0, col0, lane);
+      }
       ok = mbarWait(&st.tmemFull[acc], accPhase, status, budgetNs, 400 + acc);
       ok = __all_sync(0xffffffffu, ok) && (*st.abortFlag == 0);
       if (!ok) break;
       ptx::tcgen05_fence_after_sync();
       const uint32_t taddr = tmemBase + (static_cast<uint32_t>(quarter * 32) << 16) + acc * Cfg::kBlockN + part * Cfg::kColsPerWarp;
       const uint32_t leaderEmpty = ptx::mapa_shared(ptx::smem_u32(&st.tmemEmpty[acc]), 0);
-      stagedEpilogueTile<Cfg::kColsPerWarp>(epi, taddr, stage, row0, col0, lane, [&] { ptx::mbar_arrive_cluster(leaderEmpty); }, shape.probe);
+      if constexpr (IsRowEpilogue<Epilogue>::value) {
+        ok = epi.tile(taddr, row0, col0, it, lane, [&] { ptx::mbar_arrive_cluster(leaderEmpty); });
+        if (!ok) break;
+        if (tile + numPairs < numTiles) {  // the next tile's residual, under its MMAs
+          int m, n;
+          tileCoord(shape, tile + numPairs, numMBlk2, numNBlk, m, n);
+          epi.request((2 * m + static_cast<int>(ctaRank)) * kBlockM + quarter * 32, n * Cfg::kBlockN + part * Cfg::kColsPerWarp, lane);
+        }
+      } else {
+        stagedEpilogueTile<Cfg::kColsPerWarp>(epi, taddr, stage, row0, col0, lane, [&] { ptx::mbar_arrive_cluster(leaderEmpty); }, shape.probe);
+      }
       if constexpr (Epilogue::kNeedsTileBarrier) {
         __syncwarp();
         if (lane == 0) {
@@ -223,6 +244,9 @@ MSCCLPP_DEVICE_INLINE void gemmCtaPair(const CUtensorMap* tmapA, const CUtensorM
     }
     if (ok) epi.warpDrain(lane);  // follow-up work that is left once the warp has no tile of its own any more
     if (!ok && lane == 0) *st.abortFlag = 1;
+    if constexpr (IsRowEpilogue<Epilogue>::value) {
+      if (!ok) epi.drain(it);
+    }
     if constexpr (Epilogue::kBulkStore) {
       if (lane == 0) ptx::bulk_wait<0>();
     }

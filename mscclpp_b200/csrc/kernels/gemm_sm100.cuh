@@ -164,6 +164,13 @@ struct IsGatedEpilogue : std::false_type {};
 template <typename E>
 struct IsGatedEpilogue<E, std::void_t<decltype(E::kGatedPairs)>> : std::bool_constant<E::kGatedPairs> {};
 
+// Epilogues that do a whole tile themselves, with a row of the accumulator per lane and their own staging memory and
+// barriers, say so with `static constexpr bool kRowEpilogue = true` (two-SM core only; see ResidualSumsqRows).
+template <typename E, typename = void>
+struct IsRowEpilogue : std::false_type {};
+template <typename E>
+struct IsRowEpilogue<E, std::void_t<decltype(E::kRowEpilogue)>> : std::bool_constant<E::kRowEpilogue> {};
+
 // One epilogue warp, one tile: `taddr` is the TMEM address of the warp's lane quarter at its first column,
 // (row0, col0) the global coordinates of that corner. Calls arriveEmpty() as soon as the warp's last accumulator
 // read has completed, i.e. before the last block is written out.

@@ -943,11 +943,116 @@ __global__ void __launch_bounds__(gemm::kNumThreads, 1)
                             ResidualSumsqStore epi, DeviceStatus* status, uint64_t budgetNs) {
   extern __shared__ uint8_t smemRaw[];
   gemm::NoGate gate;
-  if constexpr (kBlockN == 0) {
-    gemm::gemmCtaPair(&tmapA, &tmapB, shape, blockIdx.x / 2, gridDim.x / 2, gate, epi, status, budgetNs, smemRaw);
-  } else {
-    gemm::gemmCta<kBlockN>(&tmapA, &tmapB, shape, blockIdx.x, gridDim.x, gate, epi, status, budgetNs, smemRaw);
+  gemm::gemmCta<kBlockN>(&tmapA, &tmapB, shape, blockIdx.x, gridDim.x, gate, epi, status, budgetNs, smemRaw);
+}
+
+// The same for the two-SM core, where a CTA works through many tiles and the epilogue above took longer than a tile's MMAs
+// (9.8 us of 4.5 at full clock: some 500 instructions per warp and 64 columns, half of them addresses, shuffles and
+// conversions between the accumulator's row-per-lane layout and a row-contiguous one). Here everything stays in the
+// row-per-lane layout: the residual comes in by tiled bulk loads, one 32 x 64 box per block, a tile ahead of its use; a lane
+// adds it to its row of the accumulator, sums up the squares by itself and leaves h in place of the residual, from where a
+// tiled bulk store takes it. The boxes of a tile need twice the staging memory, which takes one of the six operand stages.
+// One B200, 8192 x 8192 x 1024 with residual: 131 -> 111 us (the plain product 97 us); 2048 rows 38 -> 31 us. Requesting the
+// residual further ahead in the epilogue above changed nothing there.
+struct ResidualSumsqRows {
+  static constexpr bool kNeedsTileBarrier = false;
+  static constexpr bool kBulkStore = true;
+  static constexpr bool kRowEpilogue = true;
+  static constexpr int kBlocks = gemm::Config2Rows::kColsPerWarp / 64;
+  const CUtensorMap* tmapResidual;  // boxes of 64 columns x 32 rows; null = no residual
+  const CUtensorMap* tmapH;
+  float* sumsq;  // [N / 128][M]
+  int M;
+  DeviceStatus* status;
+  uint64_t budgetNs;
+  uint8_t* boxes = nullptr;  // this warp's kBlocks boxes
+  uint64_t* here = nullptr;  // ... and the barriers of their loads
+  int nextRow0 = -1, nextCol0 = 0;
+  int loads = 0;  // of tiles requested so far
+  MSCCLPP_DEVICE_INLINE void tileBegin(int, int, int) const {}
+  // Before the block-wide barrier of the set-up: this warp's barriers.
+  MSCCLPP_DEVICE_INLINE void setup(uint8_t* boxes_, uint64_t* here_, int lane) {
+    boxes = boxes_;
+    here = here_;
+    if (lane == 0) {
+      for (int b = 0; b < kBlocks; b++) ptx::mbar_init(&here[b], 1);
+      ptx::fence_mbar_init();
+    }
+    __syncwarp();
   }
+  MSCCLPP_DEVICE_INLINE void request(int row0, int col0, int lane) {
+    loads++;
+    if (tmapResidual == nullptr || lane != 0) return;
+#pragma unroll
+    for (int b = 0; b < kBlocks; b++) {
+      // the box is free once the store that left from it has been read
+      if (b == 0) ptx::bulk_wait_read<kBlocks - 1>();
+      else ptx::bulk_wait_read<0>();
+      ptx::mbar_expect_tx(&here[b], gemm::kStagingBytesPerWarp);
+      ptx::tma_load_2d(boxes + b * gemm::kStagingBytesPerWarp, tmapResidual, col0 + b * 64, row0, &here[b]);
+    }
+  }
+  // One tile. Returns false if the residual did not come.
+  template <typename ArriveEmpty>
+  MSCCLPP_DEVICE_INLINE bool tile(uint32_t taddr, int row0, int col0, int it, int lane, ArriveEmpty&& arriveEmpty) {
+    float ss[2] = {0.f, 0.f};
+    bool ok = true;
+#pragma unroll
+    for (int b = 0; b < kBlocks; b++) {
+      uint32_t v0[32], v1[32];
+      ptx::tmem_ld_32x32b_x32(taddr + b * 64, v0);
+      ptx::tmem_ld_32x32b_x32(taddr + b * 64 + 32, v1);
+      ptx::tmem_ld_wait();
+      if (b == kBlocks - 1) {
+        ptx::tcgen05_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) arriveEmpty();
+      }
+      uint8_t* box = boxes + b * gemm::kStagingBytesPerWarp;
+      if (tmapResidual != nullptr) {
+        ok = ok && mbarWait(&here[b], it & 1, status, budgetNs, 450 + b);
+        ok = __all_sync(0xffffffffu, ok);
+      } else {
+        if (lane == 0) ptx::bulk_wait_read<0>();  // the store of the tile before
+        __syncwarp();
+      }
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        uint4* word = reinterpret_cast<uint4*>(box + gemm::stagedOffset(lane, c));
+        uint4 x = c < 4 ? gemm::packChunk<ResidualSumsqRows>(v0, c & 3) : gemm::packChunk<ResidualSumsqRows>(v1, c & 3);
+        if (tmapResidual != nullptr) x = addBf16x8(x, *word);
+        ss[c & 1] += sumSquaresBf16x8(x);
+        *word = x;
+      }
+      ptx::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0 && row0 < M) ptx::tma_store_2d(tmapH, box, col0 + b * 64, row0);
+      if (lane == 0) ptx::bulk_commit();  // (an empty group keeps the count of groups the same in every tile)
+    }
+    const int row = row0 + lane;
+    if (row < M) sumsq[static_cast<size_t>(col0 / (64 * kBlocks)) * M + row] = ss[0] + ss[1];
+    return ok;
+  }
+  // After an abort: what is still on its way into the boxes must land before the CTA may end.
+  MSCCLPP_DEVICE_INLINE void drain(int done) const {
+    if (tmapResidual == nullptr || loads <= done) return;
+    for (int b = 0; b < kBlocks; b++) (void)mbarWait(&here[b], (loads - 1) & 1, nullptr, 2000000ull, 0);
+  }
+  MSCCLPP_DEVICE_INLINE static float convert(float x) { return x; }
+  MSCCLPP_DEVICE_INLINE void warpTileDone(int, int) const {}
+  MSCCLPP_DEVICE_INLINE void tileDone(int, int, int) const {}
+  MSCCLPP_DEVICE_INLINE void warpDrain(int) const {}
+  MSCCLPP_DEVICE_INLINE void auxWarp(int, int) const {}
+};
+
+__global__ void __launch_bounds__(gemm::kNumThreads, 1)
+    gemmResidualSumsqPairKernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
+                                const __grid_constant__ CUtensorMap tmapResidual, const __grid_constant__ CUtensorMap tmapH, gemm::Shape shape,
+                                int hasResidual, float* sumsq, DeviceStatus* status, uint64_t budgetNs) {
+  extern __shared__ uint8_t smemRaw[];
+  gemm::NoGate gate;
+  ResidualSumsqRows epi{hasResidual ? &tmapResidual : nullptr, &tmapH, sumsq, shape.M, status, budgetNs};
+  gemm::gemmCtaPair<gemm::Config2Rows>(&tmapA, &tmapB, shape, blockIdx.x / 2, gridDim.x / 2, gate, epi, status, budgetNs, smemRaw);
 }
 
 // out[row] = h[row] * rsqrt(sum of the row's parts / N + eps) * gamma. `tpr` threads (a multiple of 32) share a row; every
@@ -1181,20 +1286,28 @@ cudaError_t launchLocalTyped(const CUtensorMap& ta, const CUtensorMap& tb, gemm:
   cudaError_t e = gemm::ensureDynamicSmem(reinterpret_cast<const void*>(kernel), Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
   uint64_t budget = 2000000000ull;
-  if constexpr (kBlockN == 0) {
-    const int tiles = ((shape.M + gemm::Config2::kPairM - 1) / gemm::Config2::kPairM) * (shape.N / gemm::Config2::kBlockN);
-    int grid = gemm::smCount() & ~1;
-    if (grid > 2 * tiles) grid = 2 * tiles;
-    void* params[] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), &shape, &epi, &status, &budget};
-    return gemm::launchClusterPair(reinterpret_cast<const void*>(kernel), dim3(grid), dim3(gemm::kNumThreads), Cfg::kSmemBytes, params, false,
-                                   stream);
-  } else {
-    const int tiles = ((shape.M + gemm::kBlockM - 1) / gemm::kBlockM) * (shape.N / kBlockN);
-    int grid = gemm::smCount();
-    if (grid > tiles) grid = tiles;
-    kernel<<<grid, gemm::kNumThreads, Cfg::kSmemBytes, stream>>>(ta, tb, shape, epi, status, budget);
-    return cudaGetLastError();
-  }
+  const int tiles = ((shape.M + gemm::kBlockM - 1) / gemm::kBlockM) * (shape.N / kBlockN);
+  int grid = gemm::smCount();
+  if (grid > tiles) grid = tiles;
+  kernel<<<grid, gemm::kNumThreads, Cfg::kSmemBytes, stream>>>(ta, tb, shape, epi, status, budget);
+  return cudaGetLastError();
+}
+
+static cudaError_t launchLocalPair(const CUtensorMap& ta, const CUtensorMap& tb, gemm::Shape shape, const void* residual, void* h, float* sumsq,
+                                   DeviceStatus* status, cudaStream_t stream) {
+  CUtensorMap tr, th;
+  cudaError_t e = gemm::makeTensorMapBf16(&th, h, shape.M, shape.N, static_cast<uint64_t>(shape.N) * 2, 32);
+  if (e == cudaSuccess) e = gemm::makeTensorMapBf16(&tr, residual != nullptr ? residual : h, shape.M, shape.N, static_cast<uint64_t>(shape.N) * 2, 32);
+  const void* kernel = reinterpret_cast<const void*>(gemmResidualSumsqPairKernel);
+  if (e == cudaSuccess) e = gemm::ensureDynamicSmem(kernel, gemm::Config2Rows::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  const int tiles = ((shape.M + gemm::Config2::kPairM - 1) / gemm::Config2::kPairM) * (shape.N / gemm::Config2::kBlockN);
+  int grid = gemm::smCount() & ~1;
+  if (grid > 2 * tiles) grid = 2 * tiles;
+  int hasResidual = residual != nullptr;
+  uint64_t budget = 2000000000ull;
+  void* params[] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), &tr, &th, &shape, &hasResidual, &sumsq, &status, &budget};
+  return gemm::launchClusterPair(kernel, dim3(grid), dim3(gemm::kNumThreads), gemm::Config2Rows::kSmemBytes, params, false, stream);
 }
 
 int tpSumsqParts(int N, int blockN, bool twoSm) {
@@ -1211,19 +1324,26 @@ cudaError_t launchGemmResidualSumsq(const void* A, const void* B, const void* re
   cudaError_t e = cudaSuccess;
   gemm::Shape shape{M, N, K, M < gemm::kBlockM ? M : gemm::kBlockM, 0, 0, 0};
   if (twoSm) shape.aBoxRows = gemm::kBlockM;
+  // bands of 2048 rows, the order of a plain GEMM of this size: a wave re-reads its operands from L2, and the rows that are
+  // finished last are complete and still in L2 when the scale pass starts with them
+  const int band = 2048 / (twoSm ? gemm::Config2::kPairM : gemm::kBlockM);
+  if ((M + (twoSm ? gemm::Config2::kPairM : gemm::kBlockM) - 1) / (twoSm ? gemm::Config2::kPairM : gemm::kBlockM) > band) {
+    shape.mOrder = 3;
+    shape.mOrderParam = band;
+  }
   CUtensorMap ta, tb;
   e = gemm::makeTensorMapBf16(&ta, A, M, K, static_cast<uint64_t>(K) * 2, shape.aBoxRows);
   if (e != cudaSuccess) return e;
   e = gemm::makeTensorMapBf16(&tb, B, N, K, static_cast<uint64_t>(K) * 2, twoSm ? gemm::Config2::kBlockN / 2 : blockN);
   if (e != cudaSuccess) return e;
+  if (twoSm) return launchLocalPair(ta, tb, shape, residual, h, sumsq, status, stream);
   ResidualSumsqStore epi{};
   epi.residual = static_cast<const bf16*>(residual);
   epi.h = static_cast<bf16*>(h);
   epi.sumsq = sumsq;
   epi.M = M;
   epi.N = N;
-  epi.blocksPerWarp = twoSm ? gemm::Config2::kColsPerWarp / 64 : (blockN >= 128 ? blockN / 128 : 1);
-  if (twoSm) return launchLocalTyped<0>(ta, tb, shape, epi, status, stream);
+  epi.blocksPerWarp = blockN >= 128 ? blockN / 128 : 1;
   switch (blockN) {
     case 64:
       return launchLocalTyped<64>(ta, tb, shape, epi, status, stream);

@@ -168,7 +168,10 @@ class RowParallelLinearNorm:
         if residual is not None:
             self.residual_in[rows].copy_(residual)
         if two_sm is None:
-            two_sm = t >= 1024 and self.out_features % 256 == 0
+            # from 1024 tokens on, and for shorter prompts that fill at least 64 pairs of SMs (two launches, graph replay: 512
+            # tokens x 8192 17.8 us against 18.7 on one-SM tiles, 1000 x 4096 with K = 2048 23.7 against 24.8)
+            pairs = (t + 255) // 256 * (self.out_features // 256)
+            two_sm = self.out_features % 256 == 0 and (t >= 1024 or (t >= 256 and pairs >= 64 and not one_kernel))
         s = (stream or torch.cuda.current_stream()).cuda_stream
         if one_kernel:
             ws_bytes = (n.tp_local_fused_workspace_bytes(self.max_tokens, self.out_features) + 255) // 256 * 256

@@ -84,3 +84,48 @@ def test_single_gpu_layer_gemm_epilogue_residual_sumsq(tokens, hidden, k, two_sm
     assert (res.float() - h).abs().max().item() <= 0.02 * h.abs().max().item() + 0.05
     assert (out.float() - y).abs().max().item() <= 0.1
     symm.destroy()
+
+
+@pytest.mark.parametrize("tokens,hidden,k", [
+    (256, 256, 64),      # one tile, one block of the reduction
+    (257, 2048, 192),    # a row block with one row, warps without rows
+    (1333, 2048, 256),   # rows beyond M inside a box
+    (2305, 8192, 128),   # several tiles per pair of SMs, a band of 2048 rows and a rest
+    (1000, 4096, 2048),
+])
+@pytest.mark.parametrize("with_residual", [True, False])
+def test_single_gpu_layer_on_pairs_of_sms(tokens, hidden, k, with_residual):
+    """The two-launch layer on two-SM tiles: residual boxes by bulk loads, h by bulk stores, sums of squares per lane, then
+    the scale pass. Bounds: fp32 accumulation (k * 2^-24 of the products' magnitudes), one bf16 rounding before and one
+    after the residual is added, one of the output."""
+    from mscclpp_b200 import SymmetricMemory, native
+    from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
+
+    n = native()
+    symm = SymmetricMemory.emulated(1, nbytes=256 << 20, timeout_ms=3000)
+    layer = RowParallelLinearNorm(symm, out_features=hidden, k_shard=k, max_tokens=tokens)
+    g = torch.Generator(device="cuda").manual_seed(tokens + k)
+    layer.gamma.copy_((1 + 0.1 * torch.randn((hidden,), generator=g, device="cuda")).to(torch.bfloat16))
+    parts = torch.full((tokens * hidden // 128,), float("nan"), device="cuda")
+    for _ in range(2):
+        x = torch.randn((tokens, k), generator=g, device="cuda").to(torch.bfloat16)
+        residual = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+        layer.out.fill_(float("nan"))
+        layer.residual_out.fill_(float("nan"))
+        if with_residual:
+            out, res = layer.forward_local(x, residual, two_sm=True, one_kernel=False)
+        else:
+            out, res = layer.out, layer.residual_out
+            s = torch.cuda.current_stream().cuda_stream
+            num = n.gemm_residual_sumsq(x.data_ptr(), layer.weight.data_ptr(), 0, res.data_ptr(), parts.data_ptr(), tokens, hidden, k, 256, True, s)
+            n.tp_scale_rows_from_sumsq(res.data_ptr(), parts.data_ptr(), num, layer.gamma.data_ptr(), out.data_ptr(), tokens, hidden, layer.eps, s)
+        torch.cuda.synchronize()
+        p = x.double() @ layer.weight.double().t()
+        h = p + residual.double() if with_residual else p
+        slack = (x.double().abs() @ layer.weight.double().abs().t()) * k * 2.0 ** -24 + p.abs() * 2.0 ** -8 + h.abs() * 2.0 ** -8
+        assert bool(((res.double() - h).abs() <= slack).all())
+        y = res.double() * torch.rsqrt(res.double().square().mean(-1, keepdim=True) + layer.eps) * layer.gamma.double()
+        assert bool(((out.double() - y).abs() <= y.abs() * 2.0 ** -8).all())
+    symm.destroy()
+
+
