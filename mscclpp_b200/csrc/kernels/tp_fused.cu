@@ -1055,47 +1055,74 @@ __global__ void __launch_bounds__(gemm::kNumThreads, 1)
   gemm::gemmCtaPair<gemm::Config2Rows>(&tmapA, &tmapB, shape, blockIdx.x / 2, gridDim.x / 2, gate, epi, status, budgetNs, smemRaw);
 }
 
-// out[row] = h[row] * rsqrt(sum of the row's parts / N + eps) * gamma. `tpr` threads (a multiple of 32) share a row; every
-// warp adds up the parts for itself. Eight 16-byte loads are in flight per thread.
-__global__ void __launch_bounds__(512) tpScaleRowsPartsKernel(const bf16* h, const float* parts, int numParts, const bf16* gamma, bf16* out,
-                                                              int M, int N, float eps, int tpr) {
-  const int lane = threadIdx.x & 31;
-  const int groupsPerBlock = blockDim.x / tpr;
-  const int inGroup = threadIdx.x % tpr;
+// out[row] = h[row] * rsqrt(sum of the row's parts / N + eps) * gamma. A block takes kScaleRows (or fewer) consecutive rows:
+// first all their 1/rms, from coalesced pieces of the table of parts, then the rows, `tpr` threads (a power of two from 32
+// on, a quarter of the row's words) to a row and four words in flight per thread. Few registers, so that three blocks fit an SM: with 64
+// registers and eight words in flight in half as many threads, and every warp adding up its row's parts, this pass ran at
+// 4.7-5.0 TB/s. One B200, alone: 2048 x 8192 14.4 -> 11.4 us (5.9 TB/s), 8192 x 4096 26.3 -> 22.4 us, 8192 x 8192 53 -> 50 us.
+// The blocks start with the last rows: the GEMM before this launch finishes them in ascending order, so the last ones are
+// those that L2 still holds.
+constexpr int kScaleThreads = 512;
+constexpr int kScaleRows = 32;
+__global__ void __launch_bounds__(kScaleThreads, 3) tpScaleRowsPartsKernel(const bf16* h, const float* parts, int numParts, const bf16* gamma, bf16* out,
+                                                                           int M, int N, float eps, int tpr, int rowsPerBlock) {
+  __shared__ float partial[kScaleThreads / 32][kScaleRows];
+  __shared__ float rinv[kScaleRows];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int words = N / 8;
   const uint4* g4 = reinterpret_cast<const uint4*>(gamma);
-  for (int row = blockIdx.x * groupsPerBlock + threadIdx.x / tpr; row < M; row += gridDim.x * groupsPerBlock) {
+  const int row0 = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) * rowsPerBlock;
+  const int rows = M - row0 < rowsPerBlock ? M - row0 : rowsPerBlock;
+  {
+    // a lane per row, the parts dealt out to the warps
+    static_assert(kScaleRows == 32, "one lane per row");
+    float sum = 0.f;
+    if (lane < rows) {
+      for (int p = warp; p < numParts; p += kScaleThreads / 32) sum += parts[static_cast<size_t>(p) * M + row0 + lane];
+    }
+    partial[warp][lane] = sum;
+  }
+  __syncthreads();
+  if (threadIdx.x < kScaleRows) {
     float total = 0.f;
-    for (int p = lane; p < numParts; p += 32) total += parts[static_cast<size_t>(p) * M + row];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-    const float sc = rsqrtf(total / static_cast<float>(N) + eps);
-    const uint4* src = reinterpret_cast<const uint4*>(h + static_cast<size_t>(row) * N);
-    uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * N);
-    for (int w0 = inGroup; w0 < words; w0 += tpr * 8) {
-      uint4 v[8];
+    for (int w = 0; w < kScaleThreads / 32; w++) total += partial[w][threadIdx.x];
+    rinv[threadIdx.x] = rsqrtf(total / static_cast<float>(N) + eps);
+  }
+  __syncthreads();
+  const int groups = kScaleThreads / tpr;
+  const int inGroup = threadIdx.x % tpr;
+  const uint4* src = reinterpret_cast<const uint4*>(h) + static_cast<size_t>(row0) * words;
+  uint4* dst = reinterpret_cast<uint4*>(out) + static_cast<size_t>(row0) * words;
+  // (32-bit offsets from the block's first row: kScaleRows rows are far below 2^31 words)
+  auto scale = [&](uint4& v, int w, float sc) {
+    float f[8];
+    Vec16<bf16>::toFloat(v, f);
+    if (gamma != nullptr) {
+      float g[8];
+      Vec16<bf16>::toFloat(__ldg(g4 + w), g);
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const int w = w0 + k * tpr;
-        if (w < words) v[k] = ptx::ld_input_v4(src + w);
-      }
+      for (int i = 0; i < 8; i++) f[i] = f[i] * sc * g[i];
+    } else {
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const int w = w0 + k * tpr;
-        if (w < words) {
-          float f[8];
-          Vec16<bf16>::toFloat(v[k], f);
-          if (gamma != nullptr) {
-            float g[8];
-            Vec16<bf16>::toFloat(__ldg(g4 + w), g);
+      for (int i = 0; i < 8; i++) f[i] = f[i] * sc;
+    }
+    v = Vec16<bf16>::fromFloat(f);
+  };
+#pragma unroll 1
+  for (int r = threadIdx.x / tpr; r < rows; r += groups) {
+    const int base = r * words;
+#pragma unroll 1
+    for (int w = inGroup; w < words; w += 4 * tpr) {
+      // (words beyond the row repeat its last one: no branch around the loads)
+      uint4 v[4];
 #pragma unroll
-            for (int i = 0; i < 8; i++) f[i] = f[i] * sc * g[i];
-          } else {
+      for (int k = 0; k < 4; k++) v[k] = ptx::ld_input_v4(src + base + min(w + k * tpr, words - 1));
 #pragma unroll
-            for (int i = 0; i < 8; i++) f[i] = f[i] * sc;
-          }
-          dst[w] = Vec16<bf16>::fromFloat(f);
-        }
+      for (int k = 0; k < 4; k++) {
+        if (w + k * tpr >= words) break;
+        scale(v[k], w + k * tpr, rinv[r]);
+        dst[base + w + k * tpr] = v[k];
       }
     }
   }
@@ -1447,14 +1474,15 @@ cudaError_t launchTpLocalFused(const void* A, const void* B, const void* residua
 cudaError_t launchTpScaleRowsFromSumsq(const void* h, const float* sumsqParts, int numParts, const void* gamma, void* out, int M, int N,
                                        float eps, cudaStream_t stream) {
   if (N % 8 != 0 || numParts < 1 || M < 1) return cudaErrorInvalidValue;
-  // few rows: a whole thread block per row (one batch of loads); many rows: a warp per row
-  const int sms = gemm::smCount();
-  const int tpr = M <= 2 * sms ? 512 : (M <= 16 * sms ? 128 : 32);
-  const int groupsPerBlock = 512 / tpr;
-  int blocks = (M + groupsPerBlock - 1) / groupsPerBlock;
-  if (blocks > sms * 4) blocks = sms * 4;
-  tpScaleRowsPartsKernel<<<blocks, 512, 0, stream>>>(static_cast<const bf16*>(h), sumsqParts, numParts, static_cast<const bf16*>(gamma),
-                                                      static_cast<bf16*>(out), M, N, eps, tpr);
+  // enough rows per block to pay for its start, few enough that every SM has its three blocks
+  const int resident = 3 * gemm::smCount();
+  int rowsPerBlock = (M + resident - 1) / resident;
+  if (rowsPerBlock > kScaleRows) rowsPerBlock = kScaleRows;
+  int tpr = 32;
+  while (tpr < kScaleThreads && (tpr * 4 < N / 8 || rowsPerBlock * tpr < kScaleThreads)) tpr *= 2;
+  const int blocks = (M + rowsPerBlock - 1) / rowsPerBlock;
+  tpScaleRowsPartsKernel<<<blocks, kScaleThreads, 0, stream>>>(static_cast<const bf16*>(h), sumsqParts, numParts, static_cast<const bf16*>(gamma),
+                                                               static_cast<bf16*>(out), M, N, eps, tpr, rowsPerBlock);
   return cudaGetLastError();
 }
 

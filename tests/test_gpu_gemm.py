@@ -129,3 +129,20 @@ def test_single_gpu_layer_on_pairs_of_sms(tokens, hidden, k, with_residual):
     symm.destroy()
 
 
+@pytest.mark.parametrize("rows,n,parts", [(1, 8, 1), (3, 72, 2), (445, 1000, 5), (444 * 32 + 7, 256, 4), (900, 8192, 64), (37, 16392, 128)])
+def test_scale_pass_sizes(rows, n, parts):
+    """out = h * rsqrt(sum of the row's parts / n + eps) * gamma at the edges of the pass: rows of less than a warp's words,
+    of several batches per thread, more rows than resident blocks take at once. One bf16 rounding of an fp32 product."""
+    from mscclpp_b200 import native
+
+    nat = native()
+    g = torch.Generator(device="cuda").manual_seed(rows + n)
+    h = torch.randn((rows, n), generator=g, device="cuda").to(torch.bfloat16)
+    table = torch.rand((parts, rows), generator=g, device="cuda") * n
+    gamma = (1 + 0.1 * torch.randn((n,), generator=g, device="cuda")).to(torch.bfloat16)
+    out = torch.full((rows, n), float("nan"), device="cuda", dtype=torch.bfloat16)
+    for gam in (gamma, None):
+        nat.tp_scale_rows_from_sumsq(h.data_ptr(), table.data_ptr(), parts, 0 if gam is None else gam.data_ptr(), out.data_ptr(), rows, n, 1e-5,
+                                     torch.cuda.current_stream().cuda_stream)
+        y = h.double() * torch.rsqrt(table.double().sum(0) / n + 1e-5)[:, None] * (1.0 if gam is None else gam.double())
+        assert bool(((out.double() - y).abs() <= y.abs() * (2.0 ** -8)).all())
