@@ -51,8 +51,9 @@ cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   const int tiles = ((shape.M + kBlockM - 1) / kBlockM) * (shape.N / kBlockN);
   int grid = numCtas > 0 ? numCtas : smCount();
   if (grid > tiles) grid = tiles;
-  gemmBf16Kernel<kBlockN><<<grid, kNumThreads, Cfg::kSmemBytes, stream>>>(ta, tb, td, shape, status, 2000000000ull);
-  return cudaGetLastError();
+  uint64_t budget = 2000000000ull;
+  void* params[] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), const_cast<CUtensorMap*>(&td), &shape, &status, &budget};
+  return launchOverlapped(reinterpret_cast<const void*>(gemmBf16Kernel<kBlockN>), dim3(grid), dim3(kNumThreads), Cfg::kSmemBytes, params, stream);
 }
 
 __global__ void __launch_bounds__(kNumThreads, 1)
@@ -91,7 +92,7 @@ cudaError_t ensureDynamicSmem(const void* kernel, int bytes) {
 }
 
 cudaError_t launchClusterPair(const void* kernel, dim3 grid, dim3 block, size_t smemBytes, void** params, bool cooperative,
-                              cudaStream_t stream) {
+                              cudaStream_t stream, bool overlapped) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -102,10 +103,29 @@ cudaError_t launchClusterPair(const void* kernel, dim3 grid, dim3 block, size_t 
   attrs[0].val.clusterDim.x = 2;
   attrs[0].val.clusterDim.y = 1;
   attrs[0].val.clusterDim.z = 1;
-  attrs[1].id = cudaLaunchAttributeCooperative;
-  attrs[1].val.cooperative = 1;
   cfg.attrs = attrs;
-  cfg.numAttrs = cooperative ? 2 : 1;
+  cfg.numAttrs = 1;
+  if (cooperative) {
+    attrs[cfg.numAttrs].id = cudaLaunchAttributeCooperative;
+    attrs[cfg.numAttrs++].val.cooperative = 1;
+  } else if (overlapped) {
+    attrs[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  return cudaLaunchKernelExC(&cfg, kernel, params);
+}
+
+cudaError_t launchOverlapped(const void* kernel, dim3 grid, dim3 block, size_t smemBytes, void** params, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
   return cudaLaunchKernelExC(&cfg, kernel, params);
 }
 
@@ -132,7 +152,7 @@ cudaError_t gemmBf16TwoSm(const void* A, const void* B, void* D, int M, int N, i
   uint64_t budget = 2000000000ull;
   void* params[] = {&ta, &tb, &td, &shape, &status, &budget};
   return launchClusterPair(reinterpret_cast<const void*>(gemmBf16PairKernel), dim3(grid), dim3(kNumThreads), Config2::kSmemBytes, params,
-                           false, stream);
+                           false, stream, true);
 }
 
 int smCount() {

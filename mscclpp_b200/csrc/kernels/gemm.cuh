@@ -51,9 +51,15 @@ cudaError_t gemmBf16TwoSm(const void* A, const void* B, void* D, int M, int N, i
 // Raises the kernel's dynamic shared-memory limit once per (kernel, device); call before every launch that needs > 48 KB.
 cudaError_t ensureDynamicSmem(const void* kernel, int bytes);
 
-// Launch helper for kernels built on the two-SM core: clusters of two CTAs along x, optionally cooperative.
+// Launch helper for kernels built on the two-SM core: clusters of two CTAs along x, optionally cooperative. overlapped: see
+// launchOverlapped (not for cooperative launches).
 cudaError_t launchClusterPair(const void* kernel, dim3 grid, dim3 block, size_t smemBytes, void** params, bool cooperative,
-                              cudaStream_t stream);
+                              cudaStream_t stream, bool overlapped = false);
+
+// Launch with programmatic stream serialisation: the kernel may be set up while the one before it on the stream still runs.
+// Only for kernels that call ptx::grid_dependency_wait() before they touch any memory but their own.
+// One B200, graph replay: 128 x 8192 x 64 4.1 -> 3.3 us, 128 x 8192 x 1024 7.2 -> 6.3 us.
+cudaError_t launchOverlapped(const void* kernel, dim3 grid, dim3 block, size_t smemBytes, void** params, cudaStream_t stream);
 
 int smCount();
 

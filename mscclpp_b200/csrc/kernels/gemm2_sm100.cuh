@@ -97,6 +97,9 @@ MSCCLPP_DEVICE_INLINE void gemmCtaPair(const CUtensorMap* tmapA, const CUtensorM
   __syncthreads();
   ptx::tcgen05_fence_after_sync();
   const uint32_t tmemBase = *st.tmemBase;
+  // everything up to here is this pair's own: with a programmatic dependent launch it ran under the kernel before
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
 
   if (warp == 0) {
     // ===================================================== TMA producer (one thread per CTA)

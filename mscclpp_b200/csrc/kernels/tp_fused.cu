@@ -1073,6 +1073,8 @@ __global__ void __launch_bounds__(kScaleThreads, 3) tpScaleRowsPartsKernel(const
   const uint4* g4 = reinterpret_cast<const uint4*>(gamma);
   const int row0 = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) * rowsPerBlock;
   const int rows = M - row0 < rowsPerBlock ? M - row0 : rowsPerBlock;
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   {
     // a lane per row, the parts dealt out to the warps
     static_assert(kScaleRows == 32, "one lane per row");
@@ -1316,8 +1318,8 @@ cudaError_t launchLocalTyped(const CUtensorMap& ta, const CUtensorMap& tb, gemm:
   const int tiles = ((shape.M + gemm::kBlockM - 1) / gemm::kBlockM) * (shape.N / kBlockN);
   int grid = gemm::smCount();
   if (grid > tiles) grid = tiles;
-  kernel<<<grid, gemm::kNumThreads, Cfg::kSmemBytes, stream>>>(ta, tb, shape, epi, status, budget);
-  return cudaGetLastError();
+  void* params[] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), &shape, &epi, &status, &budget};
+  return gemm::launchOverlapped(reinterpret_cast<const void*>(kernel), dim3(grid), dim3(gemm::kNumThreads), Cfg::kSmemBytes, params, stream);
 }
 
 static cudaError_t launchLocalPair(const CUtensorMap& ta, const CUtensorMap& tb, gemm::Shape shape, const void* residual, void* h, float* sumsq,
@@ -1334,7 +1336,7 @@ static cudaError_t launchLocalPair(const CUtensorMap& ta, const CUtensorMap& tb,
   int hasResidual = residual != nullptr;
   uint64_t budget = 2000000000ull;
   void* params[] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), &tr, &th, &shape, &hasResidual, &sumsq, &status, &budget};
-  return gemm::launchClusterPair(kernel, dim3(grid), dim3(gemm::kNumThreads), gemm::Config2Rows::kSmemBytes, params, false, stream);
+  return gemm::launchClusterPair(kernel, dim3(grid), dim3(gemm::kNumThreads), gemm::Config2Rows::kSmemBytes, params, false, stream, true);
 }
 
 int tpSumsqParts(int N, int blockN, bool twoSm) {
@@ -1481,9 +1483,11 @@ cudaError_t launchTpScaleRowsFromSumsq(const void* h, const float* sumsqParts, i
   int tpr = 32;
   while (tpr < kScaleThreads && (tpr * 4 < N / 8 || rowsPerBlock * tpr < kScaleThreads)) tpr *= 2;
   const int blocks = (M + rowsPerBlock - 1) / rowsPerBlock;
-  tpScaleRowsPartsKernel<<<blocks, kScaleThreads, 0, stream>>>(static_cast<const bf16*>(h), sumsqParts, numParts, static_cast<const bf16*>(gamma),
-                                                               static_cast<bf16*>(out), M, N, eps, tpr, rowsPerBlock);
-  return cudaGetLastError();
+  const bf16* hp = static_cast<const bf16*>(h);
+  const bf16* gp = static_cast<const bf16*>(gamma);
+  bf16* op = static_cast<bf16*>(out);
+  void* params[] = {&hp, &sumsqParts, &numParts, &gp, &op, &M, &N, &eps, &tpr, &rowsPerBlock};
+  return gemm::launchOverlapped(reinterpret_cast<const void*>(tpScaleRowsPartsKernel), dim3(blocks), dim3(kScaleThreads), 0, params, stream);
 }
 
 cudaError_t launchTpScaleRows(const void* h, const float* rinv, const void* gamma, void* out, int M, int N,
