@@ -967,9 +967,7 @@ struct ResidualSumsqRows {
   uint64_t budgetNs;
   uint8_t* boxes = nullptr;  // this warp's kBlocks boxes
   uint64_t* here = nullptr;  // ... and the barriers of their loads
-  int nextRow0 = -1, nextCol0 = 0;
   int loads = 0;  // of tiles requested so far
-  MSCCLPP_DEVICE_INLINE void tileBegin(int, int, int) const {}
   // Before the block-wide barrier of the set-up: this warp's barriers.
   MSCCLPP_DEVICE_INLINE void setup(uint8_t* boxes_, uint64_t* here_, int lane) {
     boxes = boxes_;
@@ -1040,7 +1038,6 @@ struct ResidualSumsqRows {
   }
   MSCCLPP_DEVICE_INLINE static float convert(float x) { return x; }
   MSCCLPP_DEVICE_INLINE void warpTileDone(int, int) const {}
-  MSCCLPP_DEVICE_INLINE void tileDone(int, int, int) const {}
   MSCCLPP_DEVICE_INLINE void warpDrain(int) const {}
   MSCCLPP_DEVICE_INLINE void auxWarp(int, int) const {}
 };
