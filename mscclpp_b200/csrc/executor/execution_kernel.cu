@@ -52,8 +52,16 @@ struct Ctx {
   uint64_t pipeOff;   // byte offset of the current pipeline iteration inside each operand
   uint64_t pipeUnit;  // bytes per pipeline iteration (0 = not in a pipeline)
   uint32_t* barrierPasses;  // shared memory: grid barriers this block has passed in this launch, per barrier id
-  bool healthy;
+  bool healthy;  // the same in every thread of the block: operations run as a whole block or not at all
 };
+
+// End of an operation whose threads wait on their own (packets: a thread without one has nothing to miss): the block agrees on
+// whether all of them got what they waited for. Without the vote the threads that gave up leave the operation loop alone, and
+// the rest run on into block barriers and shared memory (a reduction's operand addresses) that the missing threads should have
+// filled. All threads of the block call it.
+MSCCLPP_DEVICE_INLINE void voteHealthy(Ctx& x, bool ok) {
+  if (!__syncthreads_and(ok ? 1 : 0)) x.healthy = false;
+}
 
 // Byte range of an operand after pipeline slicing: returns size, sets `skip` to the offset inside the operand.
 MSCCLPP_DEVICE_INLINE uint64_t sliced(const Ctx& x, const DevOp& op, const DevOperand& o, uint64_t& skip) {
@@ -232,7 +240,7 @@ MSCCLPP_DEVICE_INLINE void reduceOp(const Ctx& x, const DevOp& op) {
   __shared__ char* srcAddr[kExecMaxOperands];
   __shared__ char* dstAddr[kExecMaxOperands];
   const int nSrc = op.nSrc, nDst = op.nDst;
-  __syncthreads();  // the previous operation's readers are done with the addresses
+  __syncthreads();  // the previous operation's readers are done with the addresses (the whole block is here: see voteHealthy)
   if (threadIdx.x < static_cast<uint32_t>(nSrc)) srcAddr[threadIdx.x] = plainAddr(x, op.src[threadIdx.x], skip);
   if (threadIdx.x >= 32 - static_cast<uint32_t>(nDst) && threadIdx.x < 32) dstAddr[31 - threadIdx.x] = plainAddr(x, op.dst[31 - threadIdx.x], skip);
   __syncthreads();
@@ -305,7 +313,7 @@ MSCCLPP_DEVICE_INLINE void reducePacketsOp(Ctx& x, const DevOp& op, bool copyPac
   };
   for (uint64_t i = threadIdx.x; i < nvec && ok; i += blockDim.x) unit(i, 4);
   if (ok && tailWords != 0 && threadIdx.x == 0) unit(nvec, tailWords);
-  if (!ok) x.healthy = false;
+  voteHealthy(x, ok);
 }
 
 template <typename T>
@@ -441,11 +449,8 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
           Payload v;
           ok = in[i].read(x.epoch, v, x.c->status, x.c->timeoutNs, x.rank, 0);
         }
-        if (!__syncthreads_and(ok ? 1 : 0)) {
-          x.healthy = false;
-          break;
-        }
-        portRequests(x, op, kPortData, true);
+        voteHealthy(x, ok);
+        if (x.healthy) portRequests(x, op, kPortData, true);
         break;
       }
       for (uint64_t i = threadIdx.x; i < n && ok; i += blockDim.x) {
@@ -454,7 +459,7 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
         if (!ok) break;
         for (int d = 0; d < op.nDst; d++) pktAddr<Pkt>(x, op.dst[d], skip, op.dst[d].rank)[i].write(v, x.epoch);
       }
-      if (!ok) x.healthy = false;
+      voteHealthy(x, ok);
       break;
     }
     case OpType::COPY_PACKETS: {
@@ -464,10 +469,8 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
     }
     case OpType::UNPACK_PACKETS: {
       const uint64_t n = sliced(x, op, op.src[0], skip);
-      if (!copyFromPackets<Pkt>(plainAddr(x, op.dst[0], skip), pktAddr<Pkt>(x, op.src[0], skip, x.rank), n, threadIdx.x, blockDim.x,
-                                       x.epoch, x.c->status, x.c->timeoutNs)) {
-        x.healthy = false;
-      }
+      voteHealthy(x, copyFromPackets<Pkt>(plainAddr(x, op.dst[0], skip), pktAddr<Pkt>(x, op.src[0], skip, x.rank), n, threadIdx.x, blockDim.x,
+                                          x.epoch, x.c->status, x.c->timeoutNs));
       break;
     }
     case OpType::REDUCE_PACKETS:
@@ -513,7 +516,7 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
           for (int r = 0; r < g.nRanks; r++) pktAddr<Pkt>(x, op.dst[0], skip, g.ranks[r])[i].write(v, x.epoch);
         }
       }
-      if (!ok) x.healthy = false;
+      voteHealthy(x, ok);
       break;
     }
     case OpType::SEM_ACQUIRE:
@@ -564,9 +567,7 @@ MSCCLPP_DEVICE_INLINE void tracedOp(Ctx& x, const DevOp& op) {
     npkitCollectGpuEvent(trace, NPKIT_EVENT_EXECUTOR_OP_BASE_ENTRY + op.type, static_cast<uint32_t>(op.nSrc ? op.src[0].size : 0), x.rank);
   execOp<T, Pkt>(x, op);
   if (trace != nullptr) {
-    // the exit stamp is taken when the whole block is done with the operation; the vote also keeps the
-    // health flag uniform, so that every thread leaves the operation loop at the same place
-    x.healthy = __syncthreads_and(x.healthy ? 1 : 0) != 0;
+    __syncthreads();  // the exit stamp is taken when the whole block is done with the operation
     if (threadIdx.x == 0)
       npkitCollectGpuEvent(trace, NPKIT_EVENT_EXECUTOR_OP_BASE_EXIT + op.type, static_cast<uint32_t>(op.nSrc ? op.src[0].size : 0), x.rank);
   }

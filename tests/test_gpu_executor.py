@@ -240,3 +240,81 @@ def test_reductions_of_every_number_of_sources(world):
     for per in (8, 1040):
         _run_both(single_node.build("reducescatter_allpairs", world).to_json(), world, world * per, per, np.float16, inplace=False)
         _run_both(single_node.build("reducescatter_allpairs", world).to_json(), world, world * per, per, np.int32, inplace=False)
+
+
+def _packets_then_reduction(kind):
+    """Two ranks, one thread block each: a packet operation of fewer packets than threads, then a reduction of other
+    chunks, which the DSL puts directly behind it (their chunks do not overlap)."""
+    from mscclpp_b200.default_algos.single_node import make_spec
+    from mscclpp_b200.language.channel import MemoryChannel
+    from mscclpp_b200.language.collectives import AllReduce
+    from mscclpp_b200.language.program import CollectiveProgram
+    from mscclpp_b200.language.rank import Buffer, Rank
+
+    prog = CollectiveProgram.from_spec(make_spec(f"packets_then_reduction_{kind}", AllReduce(2, 2, True), 2, protocol="LL"))
+    with prog:
+        scratch = [Buffer(r, 4) for r in range(2)]
+        chan = [MemoryChannel(1 - r, r) for r in range(2)]
+        for r in range(2):
+            chan[r].put_packets(scratch[1 - r][0:1], Rank(r).get_input_buffer()[0:1], tb=0)
+        for r in range(2):
+            inp = Rank(r).get_input_buffer()
+            if kind == "unpack":
+                Rank(r).unpack_packets(inp[1:2], scratch[r][0:1], tb=0)
+            elif kind == "reduce":
+                Rank(r).reduce(inp[1:2], [scratch[r][0:1]], tb=0, packet=True)
+            else:
+                chan[r].read_put_packets(scratch[1 - r][1:2], scratch[r][0:1], tb=0)
+            Rank(r).reduce(inp[2:3], [inp[3:4]], tb=0)
+    return json.loads(prog.to_json())
+
+
+@pytest.mark.parametrize("kind", ["unpack", "reduce", "forward"])
+@pytest.mark.parametrize("packet_type", ["LL8", "LL16"])
+def test_packets_that_never_come_end_the_block_before_a_reduction(monkeypatch, kind, packet_type):
+    """The peers' puts are left out of the plan, so the wait for packets runs out in the threads that have one. The error is
+    reported, the reduction behind it has run in no thread (its destination and everything else are as before, the guard bands
+    intact), and the complete plan works afterwards."""
+    from mscclpp_b200 import SymmetricMemory, native
+
+    monkeypatch.setenv("MSCCLPP_EXECUTOR_CANARY", "1")
+    n = native()
+    plan = _packets_then_reduction(kind)
+    complete = n.ExecutionPlan.from_string(json.dumps(plan), 0)
+    plan["name"] += "_without_puts"  # (an executor knows a plan by its name)
+    for gpu in plan["gpus"]:
+        for tb in gpu["threadblocks"]:
+            names = [op["name"] for op in tb["ops"]]
+            assert names[0] == "ppkt" and names[-1] == "re" and len(names) == 3
+            tb["ops"] = tb["ops"][1:]
+    symm = SymmetricMemory.emulated(2, nbytes=64 << 20, timeout_ms=300)
+    per = 128  # elements of a chunk: at most 128 packets, 1024 threads
+    t = symm.tensor((4 * per,), torch.float32)
+    before = [torch.arange(4 * per, device="cuda", dtype=torch.float32) + 1000 * r for r in range(2)]
+    executor = n.Executor(symm.heap)
+
+    def run(loaded):
+        for r in range(2):
+            symm.rank_view(t, r).copy_(before[r])
+        executor.execute(0, t.data_ptr(), t.data_ptr(), 16 * per, 16 * per, n.DataType.float32, loaded,
+                         torch.cuda.current_stream().cuda_stream, getattr(n.PacketType, packet_type))
+        torch.cuda.synchronize()
+
+    lacking = n.ExecutionPlan.from_string(json.dumps(plan), 0)
+    run(lacking)
+    with pytest.raises(Exception, match="gave up"):
+        symm.check()
+    assert executor.check_canaries() > 0
+    for r in range(2):
+        assert torch.equal(symm.rank_view(t, r), before[r])
+    symm.heap.reset_status()
+    run(complete)
+    symm.check()
+    for r in range(2):
+        expect = before[r].view(4, per).clone()
+        if kind != "forward":
+            expect[1] = before[1 - r][:per] + (expect[1] if kind == "reduce" else 0)
+        expect[2] += expect[3]
+        assert torch.equal(symm.rank_view(t, r).view(4, per), expect)
+    executor.reset()
+    symm.destroy()
