@@ -106,7 +106,6 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
   const uint64_t recvScalesOff = a.recvScales ? reinterpret_cast<uint64_t>(a.recvScales) - base : 0;
   const uint64_t recvSrcOff = reinterpret_cast<uint64_t>(a.recvSrc) - base;
   const int E = a.numExperts, El = E / world;
-  const int pairs = a.tokens * a.topk;
   SymmControl* ctl = control(c, rank);
 
   __shared__ uint32_t counts[kMaxRanks][kMoeMaxExperts];  // [source rank][expert]
@@ -120,13 +119,13 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
   // this block's tokens; the rows of the first batch start on their way to L2 now, under the exchange of the counts
   const int words = a.hidden / 8;  // 16-byte words per bf16 row
   const int chunks = (words + 32 * kPieceWords - 1) / (32 * kPieceWords);
-  const int tokBegin = static_cast<int>(static_cast<int64_t>(a.tokens) * blockIdx.x / gridDim.x);
-  const int tokEnd = static_cast<int>(static_cast<int64_t>(a.tokens) * (blockIdx.x + 1) / gridDim.x);
+  const MoeTokenShare share = moeTokenShare(a.tokens, blockIdx.x, gridDim.x);
+  const int tokBegin = share.begin, tokEnd = share.end;
   if (threadIdx.x < kBatchTokens && tokBegin + static_cast<int>(threadIdx.x) < tokEnd)
     ptx::bulk_prefetch_l2(x + static_cast<size_t>(tokBegin + threadIdx.x) * a.hidden, static_cast<uint32_t>(a.hidden) * 2);
 
   // ---- A. position of every pair inside its (me, expert) group
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += gridDim.x * blockDim.x) {
+  for (int i = tokBegin * a.topk + threadIdx.x; i < tokEnd * a.topk; i += blockDim.x) {
     const int e = topkIdx[i];
     slotMap[i] = (e >= 0 && e < E) ? static_cast<int32_t>(atomicAdd(&ws.cnt[e], 1u)) : -1;
   }
@@ -211,8 +210,9 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
   }
   const bool send = healthy && overflow == 0;
 
-  // ---- D. rows to their destinations. Every block has a contiguous share of the tokens. Destinations of a batch of tokens
-  // are worked out by one thread per pair (the only reader and writer of its slotMap entry), then the warps take the
+  // ---- D. rows to their destinations. Every block has a contiguous share of the tokens, and their slotMap entries to itself:
+  // a block that gave up above may not take back what another one, which got through, is about to read. Destinations of a
+  // batch of tokens are worked out by one thread per pair (one reader and writer per entry), then the warps take the
   // (token, piece) units of the batch in turn, with the next unit's loads in flight while the current one is stored.
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -226,10 +226,10 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
       const int p = t0 * a.topk + i;
       const int e = topkIdx[p];
       uint64_t row = 0, scales = 0;
-      if (e >= 0 && e < E) {
+      const int r = e >= 0 && e < E ? moeDestinationRow(firstRow[e], slotMap[p], a.capacity) : -1;  // slotMap holds the position in the group
+      slotMap[p] = r;
+      if (r >= 0) {
         const uint64_t peer = c.peerBase[e / El];
-        const uint32_t r = firstRow[e] + static_cast<uint32_t>(slotMap[p]);  // slotMap holds the position in the group
-        slotMap[p] = static_cast<int32_t>(r);
         row = peer + recvXOff + static_cast<uint64_t>(r) * a.hidden * (a.fp8 ? 1 : 2);
         scales = peer + recvScalesOff + static_cast<uint64_t>(r) * scalesPerRow * 4;
         ptx::st_relaxed_sys(reinterpret_cast<uint32_t*>(peer + recvSrcOff) + r,
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
       }
     }
   } else {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += gridDim.x * blockDim.x) slotMap[i] = -1;
+    for (int i = tokBegin * a.topk + threadIdx.x; i < tokEnd * a.topk; i += blockDim.x) slotMap[i] = -1;
   }
   // every row of mine is on its way: after this barrier the rows sent TO me have landed
   if (healthy) rankBarrier(c, rank, 0, blockIdx.x, epoch);

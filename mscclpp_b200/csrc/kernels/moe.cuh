@@ -16,6 +16,22 @@ constexpr int kMoeScaleGroup = 128;  // elements per fp8 scale (1 x 128 blocks a
 // Bytes of symmetric workspace the dispatch kernel needs (counters + count matrix).
 constexpr size_t moeWorkspaceBytes() { return (kMoeMaxExperts + 2ull * kMaxRanks * kMoeMaxExperts) * sizeof(uint32_t) + 256; }
 
+// Tokens [begin, end) of one of a rank's thread blocks. A block assigns positions to these tokens' pairs, sends them and,
+// after a wait that ran out, marks them as not sent; it never touches a slotMap entry of another block's tokens, which may
+// have got further than it has.
+struct MoeTokenShare {
+  int begin, end;
+};
+MSCCLPP_HOST_DEVICE_INLINE MoeTokenShare moeTokenShare(int tokens, int block, int blocks) {
+  return {static_cast<int>(static_cast<int64_t>(tokens) * block / blocks), static_cast<int>(static_cast<int64_t>(tokens) * (block + 1) / blocks)};
+}
+// Row of the receive buffer for the pair at `position` of a group whose first row is `first`; -1 = there is none: the pair is
+// not in use, or the row would lie beyond the buffer.
+MSCCLPP_HOST_DEVICE_INLINE int moeDestinationRow(uint32_t first, int32_t position, int capacity) {
+  const uint64_t row = static_cast<uint64_t>(first) + static_cast<uint32_t>(position);
+  return position >= 0 && row < static_cast<uint64_t>(capacity) ? static_cast<int>(row) : -1;
+}
+
 struct MoeDispatchArgs {
   DeviceComm comm;
   int tokens, hidden, topk, numExperts;  // numExperts over all ranks; rank r hosts experts [r * E/world, (r+1) * E/world)

@@ -28,6 +28,7 @@
 #include "core/range_allocator.hpp"
 #include "core/socket.hpp"
 #include "core/unix_socket.hpp"
+#include "kernels/moe.cuh"
 #include <mscclpp/ext/collectives/algorithm_collection_builder.hpp>
 
 #include "framework.hpp"
@@ -407,6 +408,30 @@ TEST(RangeAllocator, FirstFitReleaseAndCoalescing) {
   }
   EXPECT_THROW(r.release(12345), std::invalid_argument);
   EXPECT_EQ(r.allocate(0), RangeAllocator::npos);
+}
+
+// A dispatch block that gives up marks its own tokens as not sent while other blocks, which got through, read the positions of
+// theirs: the blocks' shares of the tokens cover each one once, and a position that marks "not sent" leads to no row.
+TEST(MoeDispatch, BlocksShareNoTokenAndRowsStayInTheBuffer) {
+  for (int tokens : {0, 1, 3, 147, 148, 149, 4096, 4741, (1 << 24) - 1}) {
+    for (int blocks : {1, 2, 64, 148}) {
+      int next = 0;
+      for (int b = 0; b < blocks; b++) {
+        const MoeTokenShare share = moeTokenShare(tokens, b, blocks);
+        EXPECT_EQ(share.begin, next);
+        EXPECT_TRUE(share.end >= share.begin && share.end - share.begin <= tokens / blocks + 1);
+        next = share.end;
+      }
+      EXPECT_EQ(next, tokens);
+    }
+  }
+  EXPECT_EQ(moeDestinationRow(5, 7, 100), 12);
+  EXPECT_EQ(moeDestinationRow(0, 99, 100), 99);
+  EXPECT_EQ(moeDestinationRow(0, 100, 100), -1);
+  EXPECT_EQ(moeDestinationRow(0, -1, 100), -1);  // not sent, first group
+  EXPECT_EQ(moeDestinationRow(5, -1, 100), -1);  // not sent, another group's row
+  EXPECT_EQ(moeDestinationRow(0xffffffffu, 1, 100), -1);
+  EXPECT_EQ(moeDestinationRow(0xffffffffu, 0x7fffffff, 0x7fffffff), -1);
 }
 
 TEST(Numa, CpuListsAndBinding) {
