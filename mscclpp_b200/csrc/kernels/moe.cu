@@ -16,7 +16,7 @@
 //   No staging buffer and no second pass. With fp8 = 1 the expert outputs are e4m3 with 1 x 128 scales (quantised by
 //   the expert GEMM's epilogue or by launchMoeQuantizeRows), half the bytes over NVLink.
 // With one rank both are bound by HBM. Dispatch and combine together on one B200: 4096 tokens x 4096 bf16, top-2 of 64
-// experts 55 us (201 MB, 3.7 TB/s), 777 tokens x 7168 fp8, top-8 of 256 experts 39 us; with 64 blocks, a whole row per
+// experts 51 us (201 MB, 3.9 TB/s), 777 tokens x 7168 fp8, top-8 of 256 experts 39 us; with 64 blocks, a whole row per
 // warp, one expert's row after the other and system-scope accesses it was 86 and 104 us.
 // Both end with a cross-rank barrier: after dispatch returns every row sent to this rank has landed; after combine
 // returns the peers are done reading this rank's expert outputs.
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
 
 // A unit of the combine is 32 x kWords 16-byte words of one token's result (kFp8: of its quantised rows). A warp takes the
 // units in turn over the whole grid; the rows of kRows experts are requested together (kWords x kRows = 8 loads per lane
-// in flight), and the expert ids, rows and weights of its next unit while it waits for them (lane k holds the k-th).
+// in flight; launchMoeCombine picks the form), and the expert ids, rows and weights of its next unit while it waits for them (lane k holds the k-th).
 template <int kWords, int kRows, bool kFp8>
 __global__ void __launch_bounds__(kThreads, 1) moeCombineKernel(MoeCombineArgs a) {
   const DeviceComm& c = a.comm;
@@ -532,16 +532,39 @@ cudaError_t launchMoeCombine(const MoeCombineArgs& args, int nBlocks, cudaStream
   if (args.fp8 && args.outScales == nullptr) return cudaErrorInvalidValue;
   if (nBlocks <= 0) nBlocks = defaultBlocks(emu, args.comm.world);
   if (nBlocks > kBarrierSlots) return cudaErrorInvalidValue;
-  if (args.topk <= 2) {
-    return args.fp8 ? launchCoop(moeCombineKernel<4, 2, true>, args, nBlocks, emu, stream)
-                    : launchCoop(moeCombineKernel<4, 2, false>, args, nBlocks, emu, stream);
+  // How much of a row a warp takes at a time. Long pieces of one or two rows stream best: a word costs about a fifth more in
+  // the next shorter form. They leave warps idle where there are few of them, or where most warps have no unit in the last
+  // round. The form is the one with the smallest product of that cost and the busiest warp's words (units x words per unit).
+  // One B200, eight ranks, microseconds by form (words x rows):
+  //   256 tokens x 8192 bf16, top-8: 8x1 56, 4x2 63, 2x4 65, 1x8 90;  2048 tokens, top-1: 102, 116, 176, 338
+  //   256 tokens x 7168 fp8, top-8: 8x1 70 (no registers left for loads), 4x2 42, 2x4 44, 1x8 49
+  //   86 tokens x 8192 fp8, top-4 (1.2 units of four words per warp): 4x2 21.8, 2x4 20.9;  115 x 1024, top-8: 18.4, 16.2, 1x8 13.6
+  // Forms of more rows than there are experts per token only keep fewer loads in flight.
+  const int words = args.hidden / (args.fp8 ? 16 : 8);
+  const int64_t warps = static_cast<int64_t>(nBlocks) * (kThreads / 32);
+  auto cost = [&](int wordsPerLane) {
+    const int64_t units = static_cast<int64_t>(args.tokens) * ((words + 32 * wordsPerLane - 1) / (32 * wordsPerLane));
+    const int perWord = wordsPerLane == 8 ? 100 : (wordsPerLane == 4 ? 120 : (wordsPerLane == 2 ? 135 : 165));
+    return (units + warps - 1) / warps * wordsPerLane * perWord;
+  };
+  int form = args.fp8 ? 4 : 8;
+  const int shortest = args.topk <= 2 ? 4 : (args.topk <= 4 ? 2 : 1);
+  for (int w = form / 2; w >= shortest; w /= 2) {
+    if (cost(w) < cost(form)) form = w;
   }
-  if (args.topk <= 4) {
-    return args.fp8 ? launchCoop(moeCombineKernel<2, 4, true>, args, nBlocks, emu, stream)
-                    : launchCoop(moeCombineKernel<2, 4, false>, args, nBlocks, emu, stream);
+  switch (form) {
+    case 8:
+      return launchCoop(moeCombineKernel<8, 1, false>, args, nBlocks, emu, stream);
+    case 4:
+      return args.fp8 ? launchCoop(moeCombineKernel<4, 2, true>, args, nBlocks, emu, stream)
+                      : launchCoop(moeCombineKernel<4, 2, false>, args, nBlocks, emu, stream);
+    case 2:
+      return args.fp8 ? launchCoop(moeCombineKernel<2, 4, true>, args, nBlocks, emu, stream)
+                      : launchCoop(moeCombineKernel<2, 4, false>, args, nBlocks, emu, stream);
+    default:
+      return args.fp8 ? launchCoop(moeCombineKernel<1, 8, true>, args, nBlocks, emu, stream)
+                      : launchCoop(moeCombineKernel<1, 8, false>, args, nBlocks, emu, stream);
   }
-  return args.fp8 ? launchCoop(moeCombineKernel<1, 8, true>, args, nBlocks, emu, stream)
-                  : launchCoop(moeCombineKernel<1, 8, false>, args, nBlocks, emu, stream);
 }
 
 }  // namespace mscclpp

@@ -629,6 +629,44 @@ def test_moe_one_rank(tokens, hidden, experts, topk, fp8):
     symm.destroy()
 
 
+@pytest.mark.parametrize("tokens,hidden,topk", [(5, 256, 1), (19, 768, 2), (21, 2304, 3), (40, 8192, 5), (17, 1280, 8), (300, 2048, 8)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_moe_combine_piece_sizes(tokens, hidden, topk, fp8):
+    """The combine takes longer or shorter pieces of the rows, and of more or fewer rows together, by how many warps the launch
+    has: from one thread block to 148, with ragged last pieces. Each element is the same fp32 sum in the same order in all of
+    them; its distance from the 64-bit sum is bounded by topk + 1 fp32 roundings and one of bf16."""
+    from mscclpp_b200 import SymmetricMemory
+    from mscclpp_b200.parallel.moe import ExpertParallelDispatcher, dequantize_rows
+
+    experts = 16
+    symm = SymmetricMemory.emulated(1, nbytes=tokens * topk * hidden * 8 + tokens * hidden * 4 + (64 << 20), timeout_ms=3000)
+    disp = ExpertParallelDispatcher(symm, num_experts=experts, hidden=hidden, max_tokens=tokens, topk=topk, capacity=tokens * topk,
+                                    fp8_combine=fp8)
+    g = torch.Generator(device="cuda").manual_seed(tokens + hidden)
+    x = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+    idx = torch.rand((tokens, experts), generator=g, device="cuda").topk(topk, dim=1).indices.to(torch.int32)
+    idx[tokens // 2, topk // 2] = -1  # an unused slot
+    weights = torch.rand((tokens, topk), generator=g, device="cuda")
+    _, _, slots = disp.dispatch(x, idx)
+    rows = tokens * topk
+    disp.expert_out.copy_(torch.randn((rows, hidden), generator=g, device="cuda"))
+    if fp8:
+        disp.quantize_expert_out(rows)
+    values = dequantize_rows(disp.expert_out_q, disp.expert_out_scales) if fp8 else disp.expert_out.float()
+    w = torch.where(idx >= 0, weights, torch.zeros_like(weights)).double()
+    terms = values.double()[slots.clamp(min=0).long()] * w[:, :, None]
+    ref, bound = terms.sum(1), terms.sum(1).abs() * 2.0 ** -8 + terms.abs().sum(1) * (topk + 2) * 2.0 ** -23
+    first = None
+    for n_blocks in (1, 2, 6, 30, 148):
+        disp.y.fill_(float("nan"))
+        y = disp.combine(idx, weights, slots, n_blocks=n_blocks)
+        symm.check()
+        assert bool(((y.double() - ref).abs() <= bound).all())
+        first = y.clone() if first is None else first
+        assert torch.equal(y, first)
+    symm.destroy()
+
+
 @pytest.mark.parametrize("world,experts,tokens,hidden,topk", [(2, 8, 120, 512, 2), (8, 64, 48, 4096, 2), (4, 16, 64, 1024, 4)])
 def test_moe_combine_fp8_payload(world, experts, tokens, hidden, topk):
     """Combine with e4m3 expert outputs (1 x 128 scales): the stand-alone quantiser against a PyTorch model of it, then the
