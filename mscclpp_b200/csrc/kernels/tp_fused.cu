@@ -739,7 +739,8 @@ struct ResidualSumsqStore {
     for (int i = 0; i < 8; i++) {
       const int row = row0 + gemm::stagedRow(i, lane);
       pre[i] = make_uint4(0, 0, 0, 0);
-      if (row < M) pre[i] = ptx::ld_input_v4(residual + static_cast<size_t>(row) * N + col0 + gemm::stagedCol(lane));
+      // (not .nc: the launch before may have written the residual while this one was already resident, and it may be h)
+      if (row < M) pre[i] = ptx::ld_weak_v4(residual + static_cast<size_t>(row) * N + col0 + gemm::stagedCol(lane));
     }
   }
   MSCCLPP_DEVICE_INLINE void tileBegin(int row0, int col0, int lane) { prefetch(row0, col0, lane); }
@@ -1099,7 +1100,7 @@ __global__ void __launch_bounds__(kScaleThreads, 3) tpScaleRowsPartsKernel(const
     Vec16<bf16>::toFloat(v, f);
     if (gamma != nullptr) {
       float g[8];
-      Vec16<bf16>::toFloat(__ldg(g4 + w), g);
+      Vec16<bf16>::toFloat(g4[w], g);
 #pragma unroll
       for (int i = 0; i < 8; i++) f[i] = f[i] * sc * g[i];
     } else {
@@ -1113,10 +1114,11 @@ __global__ void __launch_bounds__(kScaleThreads, 3) tpScaleRowsPartsKernel(const
     const int base = r * words;
 #pragma unroll 1
     for (int w = inGroup; w < words; w += 4 * tpr) {
-      // (words beyond the row repeat its last one: no branch around the loads)
+      // (words beyond the row repeat its last one: no branch around the loads; not .nc: the GEMM before wrote h while this
+      // block was already resident)
       uint4 v[4];
 #pragma unroll
-      for (int k = 0; k < 4; k++) v[k] = ptx::ld_input_v4(src + base + min(w + k * tpr, words - 1));
+      for (int k = 0; k < 4; k++) v[k] = ptx::ld_weak_v4(src + base + min(w + k * tpr, words - 1));
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         if (w + k * tpr >= words) break;
