@@ -146,3 +146,95 @@ def test_scale_pass_sizes(rows, n, parts):
                                      torch.cuda.current_stream().cuda_stream)
         y = h.double() * torch.rsqrt(table.double().sum(0) / n + 1e-5)[:, None] * (1.0 if gam is None else gam.double())
         assert bool(((out.double() - y).abs() <= y.abs() * (2.0 ** -8)).all())
+
+
+def _same_without_waiting(launches, outputs):
+    """Runs `launches` with a synchronisation after each, then without one between them, eagerly and replayed from a CUDA
+    graph: the contents of `outputs` have to be the same bits every time."""
+    def run(each=lambda: None):
+        for launch in launches:
+            launch()
+            each()
+
+    def results():
+        torch.cuda.synchronize()
+        got = [o.clone() for o in outputs]
+        for o in outputs:
+            o.fill_(float("nan"))
+        torch.cuda.synchronize()
+        return got
+
+    run(torch.cuda.synchronize)
+    expect = results()
+    assert all(bool(torch.isfinite(e).all()) for e in expect)
+    for _ in range(5):
+        run()
+        assert all(torch.equal(a, b) for a, b in zip(results(), expect))
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        with torch.cuda.graph(graph, stream=side):
+            run()
+    torch.cuda.current_stream().wait_stream(side)
+    for _ in range(5):
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(results(), expect))
+
+
+@pytest.mark.parametrize("tokens,two_sm", [(100, False), (333, False), (1000, False), (333, True), (2305, True)])
+def test_chained_layers_wait_for_one_another(tokens, two_sm):
+    """Launches that overlap the one before them, back to back: a GEMM that reads what the scale pass just before it writes
+    (x) and what the GEMM before that wrote (its residual), and a second pass over the same layer, whose GEMM overwrites the
+    sums and h that the first scale pass reads."""
+    from mscclpp_b200 import SymmetricMemory
+    from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
+
+    hidden = 1024
+    symm = SymmetricMemory.emulated(1, nbytes=256 << 20, timeout_ms=3000)
+    layers = [RowParallelLinearNorm(symm, out_features=hidden, k_shard=hidden, max_tokens=tokens, seed=i) for i in range(4)]
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+    other = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+    first = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+    for i, layer in enumerate(layers):
+        layer.residual_in = first if i == 0 else layers[i - 1].residual_out
+
+    def step(i, a):
+        return lambda: layers[i].forward_local(a, two_sm=two_sm, one_kernel=False)
+
+    chain = [step(i, x if i == 0 else layers[i - 1].out[:tokens]) for i in range(4)]
+    _same_without_waiting(chain, [t for layer in layers for t in (layer.out, layer.residual_out)])
+    _same_without_waiting([step(0, other), step(0, x), step(1, layers[0].out[:tokens]), step(0, other), step(2, layers[0].out[:tokens])],
+                          [t for layer in layers[:3] for t in (layer.out, layer.residual_out)])
+    symm.destroy()
+
+
+@pytest.mark.parametrize("m,two_sm", [(100, False), (777, False), (777, True), (2304, True)])
+def test_chained_gemms_wait_for_one_another(m, two_sm):
+    """Each product is the A operand of the next one, or its residual; every second buffer is written again while the launch
+    before may still read it. A copy (a node that is no kernel) stands in the middle."""
+    from mscclpp_b200 import native
+    from mscclpp_b200.ops import gemm_bf16
+
+    n, size = native(), 512
+    g = torch.Generator(device="cuda").manual_seed(m)
+    w = (torch.randn((size, size), generator=g, device="cuda") * size ** -0.5).to(torch.bfloat16)
+    x = torch.randn((m, size), generator=g, device="cuda").to(torch.bfloat16)
+    bufs = [torch.full((m, size), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(4)]
+    parts = [torch.full((size // (128 if two_sm else 64), m), float("nan"), device="cuda") for _ in range(2)]
+
+    def product(a, d):
+        return lambda: gemm_bf16(a, w, d, two_sm=two_sm)
+
+    def added(a, residual, h, sums):
+        def launch():
+            num = n.gemm_residual_sumsq(a.data_ptr(), w.data_ptr(), residual.data_ptr(), h.data_ptr(), sums.data_ptr(), m, size, size, 128,
+                                        two_sm, torch.cuda.current_stream().cuda_stream)
+            assert num == sums.shape[0]
+        return launch
+
+    _same_without_waiting([product(x, bufs[0]), product(bufs[0], bufs[1]), product(bufs[1], bufs[0]), lambda: bufs[2].copy_(bufs[0]),
+                           product(bufs[2], bufs[1]), product(bufs[1], bufs[3])], bufs)
+    _same_without_waiting([added(x, x, bufs[0], parts[0]), added(x, bufs[0], bufs[1], parts[1]), added(bufs[1], bufs[1], bufs[2], parts[0]),
+                           added(x, bufs[2], bufs[0], parts[1]), added(bufs[0], bufs[0], bufs[3], parts[0])], bufs + parts)
