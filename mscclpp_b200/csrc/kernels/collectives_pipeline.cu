@@ -55,6 +55,8 @@ MSCCLPP_DEVICE_INLINE void pipeSignal(const DeviceComm& c, int rank, int phase, 
     ptx::st_relaxed_sys(pipeFlag(c, t, phase, slot, rank), token);
   }
 }
+// (A flag per phase: no barrier stands between a round's last wait and the next round's first one, which could otherwise clear
+// the flag before a slow warp has read it for the wait before.)
 MSCCLPP_DEVICE_INLINE bool pipeWait(const DeviceComm& c, int rank, int phase, int slot, uint64_t token, int* okSmem) {
   const int t = threadIdx.x;
   if (t < c.world && t != rank) {
@@ -70,10 +72,10 @@ MSCCLPP_DEVICE_INLINE bool pipeWait(const DeviceComm& c, int rank, int phase, in
       }
     }
     if (here) (void)ptx::ld_acquire_sys(mine);
-    else *okSmem = 0;
+    else okSmem[phase] = 0;
   }
   __syncthreads();
-  return *okSmem != 0;
+  return okSmem[phase] != 0;
 }
 
 // 16-byte units [first, n) from src to dst, kCopyUnroll loads in flight per thread.
@@ -163,10 +165,10 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
   // scratch (heap offset, equal on every rank): [parity][in | out][slot][sliceBytes]
   const uint64_t scratchOff = reinterpret_cast<uint64_t>(a.scratch) - c.peerBase[c.rank];
   const uint64_t local = c.peerBase[rank];
-  __shared__ int okSmem;
+  __shared__ int okSmem[2];
   __shared__ uint64_t heaps[8];  // (in shared memory: as kernel parameters their sums with the slices live in registers all along)
   if (threadIdx.x < 8) heaps[threadIdx.x] = c.peerBase[threadIdx.x];
-  if (threadIdx.x == 0) okSmem = 1;
+  if (threadIdx.x < 2) okSmem[threadIdx.x] = 1;
   __syncthreads();
 
   const uint64_t roundBytes = 2ull * gridDim.x * a.sliceBytes;  // scratch of one parity
@@ -210,7 +212,7 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
     const uint64_t outSlice = inSlice + static_cast<uint64_t>(gridDim.x) * a.sliceBytes;
     const uint32_t have = haveOf(r);
     // 2. every rank has staged its slice of this index
-    healthy = pipeWait(c, rank, 0, slot, tokenOf(r), &okSmem);
+    healthy = pipeWait(c, rank, 0, slot, tokenOf(r), okSmem);
     if (!healthy) break;
     // 3. reduce my part of the slice, result to everybody's scratch-out
     {
@@ -288,7 +290,7 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
       pipeSignal(c, rank, 0, slot, tokenOf(r + 1));
     }
     // 4. every rank's part of my scratch-out slice has landed
-    healthy = pipeWait(c, rank, 1, slot, tokenOf(r), &okSmem);
+    healthy = pipeWait(c, rank, 1, slot, tokenOf(r), okSmem);
     if (!healthy) break;
     // 5. copy-out
     const uint32_t tail = tailOf(r, have), whole = have - (tail != 0 ? 1 : 0);
