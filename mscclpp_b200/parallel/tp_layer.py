@@ -157,7 +157,8 @@ class RowParallelLinearNorm:
         counters first, and its few extra warps wait out a loaded L2 for every row (B200, graph replay, hidden 8192, K
         1024: 128 tokens 13.0 us against 35, 2048 tokens 52 against 74, 8192 tokens 169 against 190).
         timeline (one-kernel path, one-SM tiles): zeroed int64 CUDA tensor [148, 16] that receives per-CTA time stamps in ns
-        (start, last MMA issued, MMA waits, epilogue waits and work, drain, first extra warp's rows / waits / work)."""
+        (start, last MMA issued, MMA waits, epilogue waits and work, drain, first extra warp's rows / waits / work). Only the
+        one-kernel form has it and `probe`; given either of them, one_kernel=None is that form up to 512 tokens."""
         from .._core import native
 
         assert self.symm.world == 1, "forward_local is the single-GPU path"
@@ -167,6 +168,8 @@ class RowParallelLinearNorm:
         rows = slice(row_offset, row_offset + t)
         if residual is not None:
             self.residual_in[rows].copy_(residual)
+        if one_kernel is None:
+            one_kernel = t <= 512 and (timeline is not None or probe != 0)
         if two_sm is None:
             # from 1024 tokens on, and for shorter prompts that fill at least 64 pairs of SMs (two launches, graph replay: 512
             # tokens x 8192 17.8 us against 18.7 on one-SM tiles, 1000 x 4096 with K = 2048 23.7 against 24.8)

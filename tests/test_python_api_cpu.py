@@ -422,3 +422,50 @@ def test_raw_buffer_dlpack_helper_parses_types(native):
     with pytest.raises(ValueError):
         parse_torch_dtype("torch.nope")
     assert callable(native.RawGpuBuffer.to_dlpack)
+
+
+def test_forward_local_forms_by_arguments(monkeypatch):
+    """Which kernels a call of the single-GPU layer launches, told by a stand-in for the native module: two launches by default;
+    one up to 512 tokens when the caller wants its time line or probe, which only that form has."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from mscclpp_b200._core import native as native_module
+    from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
+
+    calls = []
+
+    class FakeNative:
+        def __getattr__(self, name):
+            def call(*args):
+                calls.append((name, args))
+                return 1
+            return call
+
+    monkeypatch.setattr(native_module, "load", lambda: FakeNative())
+    layer = object.__new__(RowParallelLinearNorm)
+    layer.symm = SimpleNamespace(world=1, device="cpu")
+    layer.out_features, layer.k_shard, layer.max_tokens, layer.eps = 256, 64, 1024, 1e-5
+    for name in ("residual_in", "residual_out", "out"):
+        setattr(layer, name, torch.zeros((1024, 256), dtype=torch.bfloat16))
+    layer.weight, layer.gamma = torch.zeros((256, 64), dtype=torch.bfloat16), torch.ones((256,), dtype=torch.bfloat16)
+    layer._local_ws = layer._sumsq_parts = None
+    stamps = torch.zeros((148, 16), dtype=torch.int64)
+
+    def launched(tokens, **kwargs):
+        calls.clear()
+        layer.forward_local(torch.zeros((tokens, 64), dtype=torch.bfloat16), stream=SimpleNamespace(cuda_stream=0), **kwargs)
+        return [name for name, _ in calls if not name.endswith("workspace_bytes")]
+
+    one, two = ["tp_local_fused"], ["gemm_residual_sumsq", "tp_scale_rows_from_sumsq"]
+    for tokens in (1, 512, 513, 1024):
+        assert launched(tokens) == two
+        assert launched(tokens, one_kernel=True) == one
+        assert launched(tokens, one_kernel=False, timeline=stamps) == two
+    for tokens in (1, 512):
+        assert launched(tokens, timeline=stamps) == one
+        assert calls[-1][1][-1] == stamps.data_ptr()
+        assert launched(tokens, probe=4) == one
+        assert calls[-1][1][-2] == 4
+    assert launched(513, timeline=stamps) == two
