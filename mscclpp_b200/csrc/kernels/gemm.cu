@@ -44,15 +44,14 @@ __global__ void __launch_bounds__(kNumThreads, 1)
 
 template <int kBlockN>
 cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, Shape shape, int numCtas,
-                   DeviceStatus* status, cudaStream_t stream) {
+                   DeviceStatus* status, cudaStream_t stream, uint64_t budgetNs) {
   using Cfg = Config<kBlockN>;
   cudaError_t e = ensureDynamicSmem(reinterpret_cast<const void*>(gemmBf16Kernel<kBlockN>), Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
   const int tiles = ((shape.M + kBlockM - 1) / kBlockM) * (shape.N / kBlockN);
   int grid = numCtas > 0 ? numCtas : smCount();
   if (grid > tiles) grid = tiles;
-  uint64_t budget = 2000000000ull;
-  void* params[] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), const_cast<CUtensorMap*>(&td), &shape, &status, &budget};
+  void* params[] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), const_cast<CUtensorMap*>(&td), &shape, &status, &budgetNs};
   return launchOverlapped(reinterpret_cast<const void*>(gemmBf16Kernel<kBlockN>), dim3(grid), dim3(kNumThreads), Cfg::kSmemBytes, params, stream);
 }
 
@@ -130,7 +129,7 @@ cudaError_t launchOverlapped(const void* kernel, dim3 grid, dim3 block, size_t s
 }
 
 cudaError_t gemmBf16TwoSm(const void* A, const void* B, void* D, int M, int N, int K, int ldd, int numCtas, DeviceStatus* status,
-                          cudaStream_t stream, int probe, int band) {
+                          cudaStream_t stream, int probe, int band, uint64_t budgetNs) {
   if (M <= 0 || N <= 0 || K <= 0 || K % kBlockK != 0 || N % Config2::kBlockN != 0 || ldd % 8 != 0) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(D) & 15) != 0) return cudaErrorInvalidValue;
   Shape shape{M, N, K, kBlockM, 0, 0, 0, probe};
@@ -149,8 +148,7 @@ cudaError_t gemmBf16TwoSm(const void* A, const void* B, void* D, int M, int N, i
   grid &= ~1;
   if (grid > 2 * tiles) grid = 2 * tiles;
   if (grid < 2) grid = 2;
-  uint64_t budget = 2000000000ull;
-  void* params[] = {&ta, &tb, &td, &shape, &status, &budget};
+  void* params[] = {&ta, &tb, &td, &shape, &status, &budgetNs};
   return launchClusterPair(reinterpret_cast<const void*>(gemmBf16PairKernel), dim3(grid), dim3(kNumThreads), Config2::kSmemBytes, params,
                            false, stream, true);
 }
@@ -183,7 +181,7 @@ cudaError_t makeTensorMapBf16(CUtensorMap* map, const void* ptr, uint64_t rows, 
 }
 
 cudaError_t gemmBf16(const void* A, const void* B, void* D, int M, int N, int K, int ldd, int blockN, int numCtas,
-                     DeviceStatus* status, cudaStream_t stream, int probe, int band) {
+                     DeviceStatus* status, cudaStream_t stream, int probe, int band, uint64_t budgetNs) {
   if (M <= 0 || N <= 0 || K <= 0 || K % kBlockK != 0 || N % blockN != 0 || ldd % 8 != 0) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(D) & 15) != 0) return cudaErrorInvalidValue;
   Shape shape{M, N, K, M < kBlockM ? M : kBlockM, 0, 0, 0, probe};
@@ -197,11 +195,11 @@ cudaError_t gemmBf16(const void* A, const void* B, void* D, int M, int N, int K,
   if (e != cudaSuccess) return e;
   switch (blockN) {
     case 64:
-      return launch<64>(ta, tb, td, shape, numCtas, status, stream);
+      return launch<64>(ta, tb, td, shape, numCtas, status, stream, budgetNs);
     case 128:
-      return launch<128>(ta, tb, td, shape, numCtas, status, stream);
+      return launch<128>(ta, tb, td, shape, numCtas, status, stream, budgetNs);
     case 256:
-      return launch<256>(ta, tb, td, shape, numCtas, status, stream);
+      return launch<256>(ta, tb, td, shape, numCtas, status, stream, budgetNs);
     default:
       return cudaErrorInvalidValue;
   }

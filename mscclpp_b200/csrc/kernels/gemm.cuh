@@ -32,6 +32,8 @@ struct Shape {
 constexpr int kStampWords = 16;
 
 
+constexpr uint64_t kDefaultBudgetNs = 2000000000ull;  // how long a wait inside a GEMM may take
+
 // Encodes a 2-D bf16 tensor map (row-major [rows, cols], 128-byte swizzle, box = [boxRows, 64]).
 // Returns cudaErrorNotSupported when the driver entry point is unavailable.
 cudaError_t makeTensorMapBf16(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t cols, uint64_t rowStrideBytes,
@@ -41,12 +43,12 @@ cudaError_t makeTensorMapBf16(CUtensorMap* map, const void* ptr, uint64_t rows, 
 // blockN in {64, 128, 256}; N % blockN == 0; K % 64 == 0; numCtas <= 0 picks one CTA per SM.
 // band: row blocks per band of the tile order (0 = default, < 0 = none); probe: see Shape::probe.
 cudaError_t gemmBf16(const void* A, const void* B, void* D, int M, int N, int K, int ldd, int blockN, int numCtas,
-                     DeviceStatus* status, cudaStream_t stream, int probe = 0, int band = 0);
+                     DeviceStatus* status, cudaStream_t stream, int probe = 0, int band = 0, uint64_t budgetNs = kDefaultBudgetNs);
 
 // Same product on 256 x 256 tiles shared by pairs of SMs (tcgen05 cta_group::2, clusters of two CTAs).
 // N % 256 == 0; K % 64 == 0; numCtas <= 0 picks one CTA per SM (rounded down to an even number).
 cudaError_t gemmBf16TwoSm(const void* A, const void* B, void* D, int M, int N, int K, int ldd, int numCtas, DeviceStatus* status,
-                          cudaStream_t stream, int probe = 0, int band = 0);
+                          cudaStream_t stream, int probe = 0, int band = 0, uint64_t budgetNs = kDefaultBudgetNs);
 
 // Raises the kernel's dynamic shared-memory limit once per (kernel, device); call before every launch that needs > 48 KB.
 cudaError_t ensureDynamicSmem(const void* kernel, int bytes);

@@ -1221,11 +1221,12 @@ cudaError_t launchTpFused(const TpFusedArgs& argsIn, const void* const* A, const
     // reduce-scatter: rank r owns rows [r * M / world, (r + 1) * M / world); the GEMM visits the row blocks
     // interleaved over the owners so that every owner's reducers have a finished block per round
     if (M % (world * (twoSm ? gemm::Config2::kPairM : gemm::kBlockM)) != 0) return cudaErrorInvalidValue;
-    if (world == 1 && emu == 1 && args.timeline == nullptr && (reinterpret_cast<uintptr_t>(args.out) & 15) == 0) {
+    if (world == 1 && emu == 1 && args.timeline == nullptr && numReducers <= 0 && (reinterpret_cast<uintptr_t>(args.out) & 15) == 0) {
       // one rank: the product is the result, and the plain GEMM writes it where it belongs. Through `partial` and the
-      // reducers the same bits cost a second pass over it.
-      return twoSm ? gemm::gemmBf16TwoSm(A[0], B[0], args.out, M, N, K, N, args.numGemmCtas, args.comm.status, stream)
-                   : gemm::gemmBf16(A[0], B[0], args.out, M, N, K, N, args.blockN, args.numGemmCtas, args.comm.status, stream);
+      // reducers the same bits cost a second pass over it; a caller that asks for reducers gets them.
+      const uint64_t budget = args.comm.timeoutNs;
+      return twoSm ? gemm::gemmBf16TwoSm(A[0], B[0], args.out, M, N, K, N, args.numGemmCtas, args.comm.status, stream, 0, 0, budget)
+                   : gemm::gemmBf16(A[0], B[0], args.out, M, N, K, N, args.blockN, args.numGemmCtas, args.comm.status, stream, 0, 0, budget);
     }
     args.rowsPerUnit = M / world;
     args.shape.mOrder = 1;

@@ -53,7 +53,9 @@ def gemm_reduce_scatter(symm: SymmetricMemory, a, weight, partial: torch.Tensor,
                         block_n: int = -1, num_reducers: int = 0, num_gemm_ctas: int = 0,
                         stream: Optional[torch.cuda.Stream] = None) -> torch.Tensor:
     """out_r[S/tp, N] = rows of sum_r(a_r @ weight_r^T) that rank r owns. `partial` [S, N] and `out` [S/tp, N] are
-    symmetric-heap tensors; `a` [S, K] and `weight` [N, K] are local (lists with one entry per rank for emulated heaps)."""
+    symmetric-heap tensors; `a` [S, K] and `weight` [N, K] are local (lists with one entry per rank for emulated heaps).
+    `partial` is workspace. One rank writes the product straight into `out` and leaves it alone, unless num_reducers (> 0)
+    asks for the form with reducers."""
     n = native.load()
     a_list = a if isinstance(a, (list, tuple)) else [a]
     w_list = weight if isinstance(weight, (list, tuple)) else [weight]

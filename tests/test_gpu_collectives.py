@@ -499,6 +499,27 @@ def test_sequence_parallel_halves_on_one_rank(rows, k, n_cols, act):
     symm.destroy()
 
 
+@pytest.mark.parametrize("rows,k,n_cols", [(256, 128, 256), (384, 192, 128)])
+def test_gemm_reduce_scatter_on_one_rank_with_reducers(rows, k, n_cols):
+    """num_reducers on one rank: the product goes through `partial` and the reducers, to the same bits as without."""
+    from mscclpp_b200 import SymmetricMemory
+    from mscclpp_b200.parallel.sp_layer import gemm_reduce_scatter
+
+    symm = SymmetricMemory.emulated(1, nbytes=64 << 20, timeout_ms=3000)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn((rows, k), generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn((n_cols, k), generator=g, device="cuda") * 0.1).to(torch.bfloat16)
+    outs = [symm.tensor((rows, n_cols), torch.bfloat16) for _ in range(2)]
+    partial = symm.tensor((rows, n_cols), torch.bfloat16)
+    partial.fill_(float("nan"))
+    gemm_reduce_scatter(symm, x, w, partial, outs[0])
+    gemm_reduce_scatter(symm, x, w, partial, outs[1], num_reducers=2)
+    torch.cuda.synchronize()
+    symm.check()
+    assert torch.equal(outs[0], outs[1]) and torch.equal(partial, outs[1])
+    symm.destroy()
+
+
 def _moe_reference(xs, idxs, wts, world, experts, f):
     """fp32 PyTorch model of dispatch -> expert function f(e, rows) -> combine, for all ranks."""
     ys = []
