@@ -650,6 +650,37 @@ def test_moe_one_rank(tokens, hidden, experts, topk, fp8):
     symm.destroy()
 
 
+@pytest.mark.parametrize("offset", [0, 8])
+@pytest.mark.parametrize("tokens,hidden,topk", [(3, 256, 1), (70, 768, 3), (160, 2304, 8)])
+def test_moe_dispatch_fp8_rows_at_eight_byte_offsets(tokens, hidden, topk, offset):
+    """Quantised rows are stored in 16-byte words where the receive buffer allows it and in 8-byte words where it does not. Either
+    way they are the bytes and scales of the stand-alone quantiser, and the bytes around the buffer stay as they are."""
+    from mscclpp_b200 import SymmetricMemory, native
+    from mscclpp_b200.parallel.moe import ExpertParallelDispatcher
+
+    n, experts, rows = native(), 16, tokens * topk
+    symm = SymmetricMemory.emulated(1, nbytes=rows * hidden * 8 + tokens * hidden * 4 + (64 << 20), timeout_ms=3000)
+    disp = ExpertParallelDispatcher(symm, num_experts=experts, hidden=hidden, max_tokens=tokens, topk=topk, capacity=rows + 1, fp8=True)
+    whole = disp.recv_x.view(-1)
+    whole.fill_(0xA5)
+    disp.recv_x, disp.capacity = whole[offset:offset + rows * hidden].view(rows, hidden), rows
+    assert disp.recv_x.data_ptr() % 16 == offset
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+    idx = torch.rand((tokens, experts), generator=g, device="cuda").topk(topk, dim=1).indices.to(torch.int32)
+    recv, _, slots = disp.dispatch(x, idx)
+    q = torch.empty((tokens, hidden), dtype=torch.uint8, device="cuda")
+    scales = torch.empty((tokens, hidden // 128), dtype=torch.float32, device="cuda")
+    n.moe_quantize_rows(x.data_ptr(), q.data_ptr(), scales.data_ptr(), tokens, hidden, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    symm.check()
+    for k in range(topk):
+        assert torch.equal(recv[slots[:, k].long()], q)
+        assert torch.equal(disp.recv_scales[slots[:, k].long()], scales)
+    assert bool((whole[:offset] == 0xA5).all()) and bool((whole[offset + rows * hidden:] == 0xA5).all())
+    symm.destroy()
+
+
 @pytest.mark.parametrize("tokens,hidden,topk", [(5, 256, 1), (19, 768, 2), (21, 2304, 3), (40, 8192, 5), (17, 1280, 8), (300, 2048, 8)])
 @pytest.mark.parametrize("fp8", [False, True])
 def test_moe_combine_piece_sizes(tokens, hidden, topk, fp8):
