@@ -59,7 +59,8 @@ cudaError_t launchClusterPair(const void* kernel, dim3 grid, dim3 block, size_t 
                               cudaStream_t stream, bool overlapped = false);
 
 // Launch with programmatic stream serialisation: the kernel may be set up while the one before it on the stream still runs.
-// Only for kernels that call ptx::grid_dependency_wait() before they touch any memory but their own.
+// Only for kernels that call ptx::grid_dependency_wait() before they touch any memory but their own: every kernel built on the
+// two GEMM cores lets the next launch start as soon as its own CTAs are set up, the cooperative and fused ones included.
 // One B200, graph replay: 128 x 8192 x 64 4.1 -> 3.3 us, 128 x 8192 x 1024 7.2 -> 6.3 us.
 cudaError_t launchOverlapped(const void* kernel, dim3 grid, dim3 block, size_t smemBytes, void** params, cudaStream_t stream);
 

@@ -171,8 +171,11 @@ class RowParallelLinearNorm:
         if one_kernel is None:
             one_kernel = t <= 512 and (timeline is not None or probe != 0)
         if two_sm is None:
-            # from 1024 tokens on, and for shorter prompts that fill at least 64 pairs of SMs (two launches, graph replay: 512
-            # tokens x 8192 17.8 us against 18.7 on one-SM tiles, 1000 x 4096 with K = 2048 23.7 against 24.8)
+            # From 1024 tokens on, and for shorter prompts that fill at least 64 pairs of SMs. Two launches, graph replay, weights
+            # from HBM, K = 1024, us on one-SM / two-SM tiles by pairs: 16 (512 x 2048) 11.5 / 14.4, 32 (512 x 4096) 13.1 / 15.8,
+            # 48 (512 x 6144) 18.7 / 17.5, 63 (768 x 5376) 20.5 / 17.5, 64 (512 x 8192) 21.2 / 18.1, 96 (700 x 8192) 28.3 / 22.8,
+            # 128 (1023 x 8192) 30.5 / 25.2; K = 256 and 2048 alike. The forms cross where the one-SM tiles no longer fit one
+            # wave, between 32 and 48 pairs; up to 63 the one-SM form is kept.
             pairs = (t + 255) // 256 * (self.out_features // 256)
             two_sm = self.out_features % 256 == 0 and (t >= 1024 or (t >= 256 and pairs >= 64 and not one_kernel))
         s = (stream or torch.cuda.current_stream()).cuda_stream
