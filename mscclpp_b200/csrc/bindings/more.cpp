@@ -205,6 +205,20 @@ void registerMoreBindings(py::module_& m) {
       py::arg("n"), py::arg("k"), py::arg("eps") = 1e-5f, py::arg("block_n") = 256, py::arg("two_sm") = false, py::arg("status") = 0,
       py::arg("stream") = 0, py::arg("probe") = 0, py::arg("stamps") = 0);
   m.def(
+      "tp_layer_wave",
+      [](SymmetricHeap& heap, uintptr_t a, uintptr_t b, uintptr_t residual, uintptr_t h, uintptr_t out, uintptr_t gamma, uintptr_t parts,
+         uintptr_t counters, int M, int N, int K, float eps, uintptr_t stream) {
+        const DeviceComm comm = heap.deviceComm();  // for the status word and the time limit of the waits
+        checkCudaMore(launchTpLayerWave(reinterpret_cast<const void*>(a), reinterpret_cast<const void*>(b), reinterpret_cast<const void*>(residual),
+                                        reinterpret_cast<void*>(h), reinterpret_cast<void*>(out), reinterpret_cast<const void*>(gamma),
+                                        reinterpret_cast<float*>(parts), reinterpret_cast<uint32_t*>(counters), M, N, K, eps, comm.status,
+                                        comm.timeoutNs, reinterpret_cast<cudaStream_t>(stream)),
+                      "tp_layer_wave");
+      },
+      py::arg("heap"), py::arg("a"), py::arg("b"), py::arg("residual"), py::arg("h"), py::arg("out"), py::arg("gamma"), py::arg("parts"),
+      py::arg("counters"), py::arg("m"), py::arg("n"), py::arg("k"), py::arg("eps") = 1e-5f, py::arg("stream") = 0);
+  m.def("tp_layer_wave_counter_words", [](int M) { return tpLayerWaveCounterWords(M); }, py::arg("m"));
+  m.def(
       "tp_scale_rows_from_sumsq",
       [](uintptr_t h, uintptr_t sumsq, int numParts, uintptr_t gamma, uintptr_t out, int M, int N, float eps, uintptr_t stream) {
         checkCudaMore(launchTpScaleRowsFromSumsq(reinterpret_cast<const void*>(h), reinterpret_cast<const float*>(sumsq), numParts,

@@ -28,6 +28,7 @@
 
 #include <mscclpp/gpu_data_types.hpp>
 
+#include "bf16x8.cuh"
 #include "gemm2_sm100.cuh"
 #include "gemm_sm100.cuh"
 
@@ -37,35 +38,6 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 constexpr int kMaxNBlk = 128;
-
-// Packed bf16 arithmetic for the element-wise parts of the single-GPU layer. With a dozen warps per SM these loops are
-// bound by instruction latency, not by memory: one HADD2 / HMUL2 / HFMA2 per two elements instead of a convert - operate -
-// convert chain per element is what makes them fit in the shadow of the MMAs.
-MSCCLPP_DEVICE_INLINE __nv_bfloat162 asBf162(uint32_t w) { return *reinterpret_cast<__nv_bfloat162*>(&w); }
-MSCCLPP_DEVICE_INLINE uint32_t asWord(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
-// a + b per element, each sum rounded once to bf16 (the adder works in fp32 internally: same result as an fp32 add + round)
-MSCCLPP_DEVICE_INLINE uint4 addBf16x8(uint4 a, uint4 b) {
-  return make_uint4(asWord(__hadd2(asBf162(a.x), asBf162(b.x))), asWord(__hadd2(asBf162(a.y), asBf162(b.y))),
-                    asWord(__hadd2(asBf162(a.z), asBf162(b.z))), asWord(__hadd2(asBf162(a.w), asBf162(b.w))));
-}
-MSCCLPP_DEVICE_INLINE float sumSquaresBf16x8(uint4 v) {
-  const float2 a = __bfloat1622float2(asBf162(v.x)), b = __bfloat1622float2(asBf162(v.y));
-  const float2 c = __bfloat1622float2(asBf162(v.z)), d = __bfloat1622float2(asBf162(v.w));
-  float s0 = a.x * a.x, s1 = b.x * b.x;
-  s0 = fmaf(a.y, a.y, s0);
-  s1 = fmaf(b.y, b.y, s1);
-  s0 = fmaf(c.x, c.x, s0);
-  s1 = fmaf(d.x, d.x, s1);
-  s0 = fmaf(c.y, c.y, s0);
-  s1 = fmaf(d.y, d.y, s1);
-  return s0 + s1;
-}
-// v * g * s with the fp32 scale s split into a bf16 head and a bf16 tail (s = hi + lo up to 2^-17 relative), so that the
-// result carries the two product roundings of bf16 arithmetic but not a third from rounding s itself.
-MSCCLPP_DEVICE_INLINE uint32_t scaleBf16x2(uint32_t v, uint32_t g, __nv_bfloat162 hi, __nv_bfloat162 lo, bool hasGamma) {
-  const __nv_bfloat162 p = hasGamma ? __hmul2(asBf162(v), asBf162(g)) : asBf162(v);
-  return asWord(__hfma2(p, lo, __hmul2(p, hi)));
-}
 
 struct TmapSet {
   CUtensorMap a[8];

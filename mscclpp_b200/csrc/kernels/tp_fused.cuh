@@ -93,6 +93,14 @@ cudaError_t launchTpLocalFused(const void* A, const void* B, const void* residua
                                int M, int N, int K, float eps, int blockN, bool twoSm, DeviceStatus* status, cudaStream_t stream,
                                int probe = 0, unsigned long long* stamps = nullptr);
 
+// The same layer in ONE launch that keeps each 256 x 256 tile of h on chip until its rows' sums of squares are complete (see
+// tp_wave.cu): M >= 256, N % 256 == 0, at most as many 256-column tiles per row as pairs of SMs that run at the same time.
+// parts: M rounded up to 256 rows x N / 128 floats, never cleared; counters: tpLayerWaveCounterWords(M) words, zero before the
+// first launch and left zero by every launch. Launches that may run at the same time want their own of both.
+size_t tpLayerWaveCounterWords(int M);
+cudaError_t launchTpLayerWave(const void* A, const void* B, const void* residual, void* h, void* out, const void* gamma, float* parts,
+                              uint32_t* counters, int M, int N, int K, float eps, DeviceStatus* status, uint64_t budgetNs, cudaStream_t stream);
+
 // The layer for a handful of tokens (decode): one launch, no tensor-core tiles - every SM streams the weight rows of its
 // slab of output columns, the slabs meet the other ranks in a one-shot LL packet allreduce done by the same thread
 // blocks, residual add and RMSNorm follow in registers (see tp_decode.cu). Every rank ends up with the whole result.

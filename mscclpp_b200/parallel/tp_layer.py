@@ -42,7 +42,10 @@ class RowParallelLinearNorm:
         self.gamma.fill_(1.0)
         self.rinv = symm.tensor((max_tokens,), torch.float32)
         self._local_ws = None  # workspace of the one-kernel single-GPU path, made on first use
-        self._sumsq_parts = None  # parts of the rows' sums of squares between the two launches of the two-kernel path
+        self._sumsq_parts = None  # parts of the rows' sums of squares on their way from the GEMM's epilogue to the norm
+        # counters of the long-prompt form of forward_local: zero before and after every launch (so made here, where no graph is being
+        # captured); a launch on rows [r, r + t) uses words from r on
+        self._wave_counters = torch.zeros((max_tokens,), dtype=torch.int32, device=dev)
         self.launches_per_forward = 1  # forward_fused, mode 0
 
     def forward(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None, algo: Optional[str] = None,
@@ -147,15 +150,27 @@ class RowParallelLinearNorm:
                     0 if timeline is None else timeline.data_ptr())
         return self.out[:t], self.residual_out[:t]
 
+    @staticmethod
+    def _wave_form(t: int, n: int, k: int) -> bool:
+        """Whether forward_local takes the one-launch form that keeps h on chip until its rows are complete (tp_wave.cu). It saves
+        reading h back, but its launch is cooperative (about 3 us that the two overlapped launches do not have) and every wave
+        of its 256 x 256 tiles ends in an exchange, which only the matrix products of the next wave hide. B200, graph replay, time
+        of two launches / of this form by waves of 74 tiles, widths 1024 to 8192: K = 2048 up to 1.5 waves 0.69-1.11, 2-2.7
+        0.95-1.08, 3.2-5.4 1.02-1.14, 6.9 and more 1.06-1.19; K = 1024 likewise 0.72-1.12, 0.94-1.08, 1.08-1.20, 1.13-1.25; K = 512
+        0.69-1.08, 0.82-1.00, 0.91-1.10, 0.97-1.05; K = 256 0.71-1.07, 0.79-1.01, 0.89-1.09, 1.01-1.14."""
+        return t >= 256 and n % 256 == 0 and n <= 8192 and k >= 1024 and (t + 255) // 256 * (n // 256) >= 222
+
     def forward_local(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None, two_sm: Optional[bool] = None,
                       stream: Optional[torch.cuda.Stream] = None, one_kernel: Optional[bool] = None, row_offset: int = 0,
                       probe: int = 0, timeline: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
         """World size 1 (no collective). one_kernel: ONE launch - the GEMM's epilogue adds the residual, stores h and
         accumulates every row's sum of squares, and extra warps normalise each 128-row block as soon as it is complete,
         while the MMAs of the later blocks run. one_kernel=False: the same epilogue, then a second, memory-bound launch
-        that applies 1/rms and gamma, the faster form at every size and the default: one launch saves a launch but clears
+        that applies 1/rms and gamma. It is the faster of these two at every size: one launch saves a launch but clears
         counters first, and its few extra warps wait out a loaded L2 for every row (B200, graph replay, hidden 8192, K
-        1024: 128 tokens 13.0 us against 35, 2048 tokens 52 against 74, 8192 tokens 169 against 190).
+        1024: 128 tokens 13.0 us against 35, 2048 tokens 46 against 74, 8192 tokens 160 against 190). By default (both None) it
+        is taken up to a few thousand tokens; longer prompts take a third form, one launch whose extra warps hold h on chip
+        until its rows are complete (2048 tokens 43 us, 8192 139; see _wave_form).
         timeline (one-kernel path, one-SM tiles): zeroed int64 CUDA tensor [148, 16] that receives per-CTA time stamps in ns
         (start, last MMA issued, MMA waits, epilogue waits and work, drain, first extra warp's rows / waits / work). Only the
         one-kernel form has it and `probe`; given either of them, one_kernel=None is that form up to 512 tokens."""
@@ -168,6 +183,16 @@ class RowParallelLinearNorm:
         rows = slice(row_offset, row_offset + t)
         if residual is not None:
             self.residual_in[rows].copy_(residual)
+        s = (stream or torch.cuda.current_stream()).cuda_stream
+        # the rows' sums of squares travel in parts ([parts][t] floats, nothing to clear); launches on disjoint row ranges
+        # use disjoint pieces of the buffer
+        per_row = self.out_features // 64
+        if one_kernel is None and two_sm is None and timeline is None and probe == 0 and self._wave_form(t, self.out_features, self.k_shard):
+            n.tp_layer_wave(self.symm.heap, x.data_ptr(), self.weight.data_ptr(), self.residual_in[rows].data_ptr(),
+                            self.residual_out[rows].data_ptr(), self.out[rows].data_ptr(), self.gamma.data_ptr(),
+                            self._parts()[row_offset * per_row:].data_ptr(), self._wave_counters[row_offset:].data_ptr(), t,
+                            self.out_features, self.k_shard, self.eps, s)
+            return self.out[rows], self.residual_out[rows]
         if one_kernel is None:
             one_kernel = t <= 512 and (timeline is not None or probe != 0)
         if two_sm is None:
@@ -178,7 +203,6 @@ class RowParallelLinearNorm:
             # wave, between 32 and 48 pairs; up to 63 the one-SM form is kept.
             pairs = (t + 255) // 256 * (self.out_features // 256)
             two_sm = self.out_features % 256 == 0 and (t >= 1024 or (t >= 256 and pairs >= 64 and not one_kernel))
-        s = (stream or torch.cuda.current_stream()).cuda_stream
         if one_kernel:
             ws_bytes = (n.tp_local_fused_workspace_bytes(self.max_tokens, self.out_features) + 255) // 256 * 256
             if self._local_ws is None:  # one workspace per 256-row-aligned launch that may be in flight: indexed by row offset
@@ -188,17 +212,17 @@ class RowParallelLinearNorm:
                              self.out[rows].data_ptr(), self.gamma.data_ptr(), ws.data_ptr(), t, self.out_features, self.k_shard,
                              self.eps, pick_block_n(t, self.out_features), two_sm, 0, s, probe, 0 if timeline is None else timeline.data_ptr())
             return self.out[rows], self.residual_out[rows]
-        # the rows' sums of squares travel between the two launches in parts ([parts][t] floats, nothing to clear); launches
-        # on disjoint row ranges use disjoint pieces of the buffer
-        per_row = self.out_features // 64
-        if self._sumsq_parts is None:
-            self._sumsq_parts = torch.empty((self.max_tokens * per_row,), dtype=torch.float32, device=self.symm.device)
-        parts_buf = self._sumsq_parts[row_offset * per_row:]
+        parts_buf = self._parts()[row_offset * per_row:]
         parts = n.gemm_residual_sumsq(x.data_ptr(), self.weight.data_ptr(), self.residual_in[rows].data_ptr(), self.residual_out[rows].data_ptr(),
                                       parts_buf.data_ptr(), t, self.out_features, self.k_shard, pick_block_n(t, self.out_features), two_sm, s)
         n.tp_scale_rows_from_sumsq(self.residual_out[rows].data_ptr(), parts_buf.data_ptr(), parts, self.gamma.data_ptr(),
                                    self.out[rows].data_ptr(), t, self.out_features, self.eps, s)
         return self.out[rows], self.residual_out[rows]
+
+    def _parts(self) -> torch.Tensor:
+        if self._sumsq_parts is None:
+            self._sumsq_parts = torch.empty((self.max_tokens * (self.out_features // 64),), dtype=torch.float32, device=self.symm.device)
+        return self._sumsq_parts
 
     def forward_from_host(self, x_host: torch.Tensor, chunks: int = 4, **fused_kwargs) -> Tuple[torch.Tensor, torch.Tensor]:
         """The layer on activations that are still in (pinned) host memory. The rows are cut into `chunks` pieces of whole

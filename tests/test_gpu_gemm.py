@@ -129,6 +129,47 @@ def test_single_gpu_layer_on_pairs_of_sms(tokens, hidden, k, with_residual):
     symm.destroy()
 
 
+@pytest.mark.parametrize("tokens,hidden,k", [
+    (256, 256, 64),      # one tile
+    (257, 2048, 192),    # a row block with one row
+    (2305, 8192, 128),   # several waves, and row blocks that straddle two of them
+    (1999, 6400, 1024),  # 25 tiles per row block; rows beyond M inside a scale warp's sixteen
+    (8192, 2048, 1088),
+])
+def test_single_gpu_layer_in_waves(tokens, hidden, k):
+    """The one-launch layer that keeps h on chip: with and without residual and gamma, twice in a row (the counters it leaves are
+    those it needs). Bounds as for the two-launch form above."""
+    from mscclpp_b200 import SymmetricMemory, native
+
+    n = native()
+    symm = SymmetricMemory.emulated(1, nbytes=64 << 20, timeout_ms=3000)
+    g = torch.Generator(device="cuda").manual_seed(tokens + k)
+    w = (0.05 * torch.randn((hidden, k), generator=g, device="cuda")).to(torch.bfloat16)
+    gamma = (1 + 0.1 * torch.randn((hidden,), generator=g, device="cuda")).to(torch.bfloat16)
+    parts = torch.full(((tokens + 255) // 256 * 256 * hidden // 128,), float("nan"), device="cuda")
+    counters = torch.zeros((n.tp_layer_wave_counter_words(tokens),), dtype=torch.int32, device="cuda")
+    for residual, gam in ((True, gamma), (True, None), (False, gamma), (True, gamma)):
+        x = torch.randn((tokens, k), generator=g, device="cuda").to(torch.bfloat16)
+        r = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+        out, res = (torch.full((tokens, hidden), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        n.tp_layer_wave(symm.heap, x.data_ptr(), w.data_ptr(), r.data_ptr() if residual else 0, res.data_ptr(), out.data_ptr(),
+                        0 if gam is None else gam.data_ptr(), parts.data_ptr(), counters.data_ptr(), tokens, hidden, k, 1e-5,
+                        torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        symm.check()
+        assert not bool(counters.any())
+        p = x.double() @ w.double().t()
+        h = p + r.double() if residual else p
+        slack = (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24 + p.abs() * 2.0 ** -8 + h.abs() * 2.0 ** -8
+        assert bool(((res.double() - h).abs() <= slack).all())
+        y = res.double() * torch.rsqrt(res.double().square().mean(-1, keepdim=True) + 1e-5) * (1.0 if gam is None else gam.double())
+        assert bool(((out.double() - y).abs() <= y.abs() * 2.0 ** -8).all())
+    with pytest.raises(Exception):  # a row block has to fit two waves
+        n.tp_layer_wave(symm.heap, x.data_ptr(), w.data_ptr(), 0, res.data_ptr(), out.data_ptr(), 0, parts.data_ptr(), counters.data_ptr(), 256,
+                        256 * 149, 64, 1e-5, torch.cuda.current_stream().cuda_stream)
+    symm.destroy()
+
+
 @pytest.mark.parametrize("rows,n,parts", [(1, 8, 1), (3, 72, 2), (445, 1000, 5), (444 * 32 + 7, 256, 4), (900, 8192, 64), (37, 16392, 128)])
 def test_scale_pass_sizes(rows, n, parts):
     """out = h * rsqrt(sum of the row's parts / n + eps) * gamma at the edges of the pass: rows of less than a warp's words,

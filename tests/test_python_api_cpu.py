@@ -469,3 +469,13 @@ def test_forward_local_forms_by_arguments(monkeypatch):
         assert launched(tokens, probe=4) == one
         assert calls[-1][1][-2] == 4
     assert launched(513, timeline=stamps) == two
+
+
+def test_forward_local_long_prompts_by_size():
+    """The line between two launches and the one-launch form for long prompts: 222 tiles of 256 x 256 and 1024 reduction elements."""
+    from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
+
+    wave = RowParallelLinearNorm._wave_form
+    assert wave(1537, 8192, 1024) and wave(8192, 8192, 1024) and wave(14337, 1024, 2048)
+    assert not wave(1536, 8192, 1024)  # 192 tiles
+    assert not wave(8192, 8192, 960) and not wave(8192, 8200, 1024) and not wave(8192, 8448, 1024) and not wave(255, 8192, 1024)
