@@ -37,4 +37,36 @@ MSCCLPP_DEVICE_INLINE uint32_t scaleBf16x2(uint32_t v, uint32_t g, __nv_bfloat16
   return asWord(__hfma2(p, lo, __hmul2(p, hi)));
 }
 
+// Two fp32 values per instruction.
+MSCCLPP_DEVICE_INLINE uint64_t pairOf(uint32_t bf16x2) {
+  uint64_t p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "r"(bf16x2 << 16), "r"(bf16x2 & 0xffff0000u));
+  return p;
+}
+MSCCLPP_DEVICE_INLINE uint64_t pairOf(float a, float b) {
+  uint64_t p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a), "f"(b));
+  return p;
+}
+MSCCLPP_DEVICE_INLINE float2 valuesOf(uint64_t p) {
+  float2 v;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+MSCCLPP_DEVICE_INLINE uint64_t mulPair(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+MSCCLPP_DEVICE_INLINE uint64_t fmaPair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// ... rounded to bf16
+MSCCLPP_DEVICE_INLINE uint32_t packPair(uint64_t p) {
+  const float2 f = valuesOf(p);
+  return asWord(__floats2bfloat162_rn(f.x, f.y));
+}
+
 }  // namespace mscclpp

@@ -129,6 +129,13 @@ struct TpDecodeArgs {
 };
 cudaError_t launchTpDecode(const TpDecodeArgs& args, cudaStream_t stream);
 
+// The same for one rank, with launches that overlap (see tp_decode_local.cu): of `args` it takes the operands, the status and
+// the time limit. workspace: tpDecodeLocalWorkspaceWords() 32-bit words, zero before the first launch; launches that
+// may run at the same time want their own. cudaErrorInvalidValue or cudaErrorInvalidConfiguration, with nothing launched, for what it does
+// not cover: no residualOut, an operand that is not 16-byte aligned, pieces of the weights that do not fit shared memory.
+size_t tpDecodeLocalWorkspaceWords();
+cudaError_t launchTpDecodeLocal(const TpDecodeArgs& args, void* workspace, cudaStream_t stream);
+
 // Local pass of mode 1: out = h * rinv[row] * gamma.
 cudaError_t launchTpScaleRows(const void* h, const float* rinv, const void* gamma, void* out, int M, int N,
                               cudaStream_t stream);

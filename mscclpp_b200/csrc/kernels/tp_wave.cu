@@ -47,32 +47,6 @@ constexpr int kBarWords = 20 + gemm::kNumEpilogueWarps * kBoxesOfWarp + 6;
 using ConfigWave = gemm::Config2Of<5, kBoxesOfWarp * gemm::kEpilogueStagingBytes, kBarWords * 8>;
 static_assert(kBoxesOfWarp * 64 == ConfigWave::kColsPerWarp && kScaleWarps * 16 == gemm::kBlockM, "");
 
-// Two fp32 values per instruction.
-MSCCLPP_DEVICE_INLINE uint64_t pairOf(uint32_t bf16x2) {
-  uint64_t p;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "r"(bf16x2 << 16), "r"(bf16x2 & 0xffff0000u));
-  return p;
-}
-MSCCLPP_DEVICE_INLINE uint64_t pairOf(float a, float b) {
-  uint64_t p;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a), "f"(b));
-  return p;
-}
-MSCCLPP_DEVICE_INLINE float2 valuesOf(uint64_t p) {
-  float2 v;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
-  return v;
-}
-MSCCLPP_DEVICE_INLINE uint64_t mulPair(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-MSCCLPP_DEVICE_INLINE uint64_t fmaPair(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 MSCCLPP_DEVICE_INLINE uint4 lds128(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
@@ -302,8 +276,7 @@ struct LayerRows {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
           if (gamma != nullptr) p[i] = mulPair(p[i], g[i]);
-          const float2 f = valuesOf(p[i]);
-          o[i] = asWord(__floats2bfloat162_rn(f.x, f.y));
+          o[i] = packPair(p[i]);
         }
         if (row0 + j < M) ptx::st_weak_v4_hint(to, make_uint4(o[0], o[1], o[2], o[3]), once);
         to += words;

@@ -25,6 +25,8 @@ class RowParallelLinearNorm:
 
     def __init__(self, symm: SymmetricMemory, out_features: int = 8192, k_shard: int = 1024, max_tokens: int = 8192,
                  eps: float = 1e-5, seed: int = 0, init_std: float = 0.02):
+        from .._core import native
+
         self.symm = symm
         self.out_features = out_features
         self.k_shard = k_shard
@@ -45,6 +47,7 @@ class RowParallelLinearNorm:
         self._sumsq_parts = None  # parts of the rows' sums of squares on their way from the GEMM's epilogue to the norm
         # counters of the long-prompt form of forward_local: zero before and after every launch (so made here, where no graph is being
         # captured); a launch on rows [r, r + t) uses words from r on
+        self._decode_ws = torch.zeros((native.load().tp_decode_workspace_words(),), dtype=torch.int32, device=dev) if symm.world == 1 else None
         self._wave_counters = torch.zeros((max_tokens,), dtype=torch.int32, device=dev)
         self.launches_per_forward = 1  # forward_fused, mode 0
 
@@ -127,7 +130,7 @@ class RowParallelLinearNorm:
         of output columns, the slabs are all-reduced with LL packets by the same thread blocks (no barrier between the
         ranks), residual add and RMSNorm follow in registers. Any world size, 1 included. k_shard must be a multiple of 256.
         nvls: packets leave through one multimem.st instead of one store per peer (default: where the heap has it and
-        there are more than two ranks). timeline: optional zeroed int64 CUDA tensor [thread blocks, 8] that receives each
+        there are more than two ranks). On one rank the launches of a chain of layers overlap (tp_decode_local.cu). timeline: optional zeroed int64 CUDA tensor [thread blocks, 8] that receives each
         block's time stamps in ns (entry, activations staged, weight pieces consumed, all warps done, allreduce + residual
         done, row-sum shares read, last store)."""
         from .._core import native
@@ -147,7 +150,7 @@ class RowParallelLinearNorm:
             xp, wp = [x.data_ptr()], [self.weight.data_ptr()]
         n.tp_decode(self.symm.heap, xp, wp, self.residual_in.data_ptr(), self.residual_out.data_ptr(), self.out.data_ptr(),
                     self.gamma.data_ptr(), t, self.out_features, self.k_shard, self.eps, nvls, num_ctas, s,
-                    0 if timeline is None else timeline.data_ptr())
+                    0 if timeline is None else timeline.data_ptr(), 0 if self._decode_ws is None else self._decode_ws.data_ptr())
         return self.out[:t], self.residual_out[:t]
 
     @staticmethod

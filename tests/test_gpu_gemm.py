@@ -279,3 +279,67 @@ def test_chained_gemms_wait_for_one_another(m, two_sm):
                            product(bufs[2], bufs[1]), product(bufs[1], bufs[3])], bufs)
     _same_without_waiting([added(x, x, bufs[0], parts[0]), added(x, bufs[0], bufs[1], parts[1]), added(bufs[1], bufs[1], bufs[2], parts[0]),
                            added(x, bufs[2], bufs[0], parts[1]), added(bufs[0], bufs[0], bufs[3], parts[0])], bufs + parts)
+
+
+@pytest.mark.parametrize("tokens,hidden,k", [
+    (1, 8, 256),        # one block, eight columns
+    (2, 1032, 256),     # the last block has eight columns of what others have
+    (3, 1032, 512),     # pairs of blocks, the odd one out without columns
+    (8, 5120, 2560),
+    (5, 18944, 3072),   # the widest slab, whose tiles go six times around the ring
+    (4, 18952, 256),    # wider: the cooperative form
+])
+def test_decode_layer_one_gpu(tokens, hidden, k):
+    """The layer for a few tokens on one rank: with and without residual and gamma, launches back to back (the count they leave is
+    the one they need). Bounds: fp32 accumulation, one bf16 rounding before and one after the residual, one of the output."""
+    from mscclpp_b200 import SymmetricMemory, native
+    from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
+
+    n = native()
+    symm = SymmetricMemory.emulated(1, nbytes=64 << 20, timeout_ms=3000)
+    layer = RowParallelLinearNorm(symm, out_features=hidden, k_shard=k, max_tokens=tokens, init_std=0.05)
+    g = torch.Generator(device="cuda").manual_seed(tokens + hidden)
+    layer.gamma.copy_((1 + 0.1 * torch.randn((hidden,), generator=g, device="cuda")).to(torch.bfloat16))
+    for plain in (False, True, False):
+        x = torch.randn((tokens, k), generator=g, device="cuda").to(torch.bfloat16)
+        residual = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+        layer.out.fill_(float("nan"))
+        layer.residual_out.fill_(float("nan"))
+        if plain:
+            n.tp_decode(symm.heap, [x.data_ptr()], [layer.weight.data_ptr()], 0, layer.residual_out.data_ptr(), layer.out.data_ptr(), 0, tokens, hidden,
+                        k, layer.eps, False, 0, torch.cuda.current_stream().cuda_stream, 0, layer._decode_ws.data_ptr())
+        else:
+            for _ in range(3):
+                layer.forward_decode(x, residual)
+        torch.cuda.synchronize()
+        symm.check()
+        p = x.double() @ layer.weight.double().t()
+        h = p if plain else p + residual.double()
+        res, out = layer.residual_out[:tokens].double(), layer.out[:tokens].double()
+        slack = (x.double().abs() @ layer.weight.double().abs().t()) * k * 2.0 ** -24 + p.abs() * 2.0 ** -8 + h.abs() * 2.0 ** -8
+        assert bool(((res - h).abs() <= slack).all())
+        y = res * torch.rsqrt(res.square().mean(-1, keepdim=True) + layer.eps) * (1.0 if plain else layer.gamma.double())
+        assert bool(((out - y).abs() <= y.abs() * 2.0 ** -8).all())
+    symm.destroy()
+
+
+@pytest.mark.parametrize("tokens", [1, 8])
+def test_chained_decode_layers_wait_for_one_another(tokens):
+    """Decode launches overlap the one before them and prefetch their operands under it: activations that the layer before
+    writes, a residual that it writes, and weights that a copy right before writes."""
+    from mscclpp_b200 import SymmetricMemory
+    from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
+
+    hidden = 2048
+    symm = SymmetricMemory.emulated(1, nbytes=64 << 20, timeout_ms=3000)
+    layers = [RowParallelLinearNorm(symm, out_features=hidden, k_shard=hidden, max_tokens=tokens, seed=i) for i in range(3)]
+    weights = [layer.weight.clone() for layer in layers]
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x, first = (torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    layers[0].residual_in.copy_(first)
+    layers[1].residual_in, layers[2].residual_in = layers[0].residual_out, layers[1].residual_out
+    chain = [lambda: layers[0].weight.copy_(weights[1]), lambda: layers[0].forward_decode(x), lambda: layers[0].weight.copy_(weights[0]),
+             lambda: layers[0].forward_decode(x), lambda: layers[1].forward_decode(layers[0].out), lambda: layers[2].forward_decode(layers[1].out)]
+    _same_without_waiting(chain, [t for layer in layers for t in (layer.out, layer.residual_out)])
+    symm.check()
+    symm.destroy()
