@@ -1032,10 +1032,16 @@ __global__ void __launch_bounds__(gemm::kNumThreads, 1)
 // 4.7-5.0 TB/s. One B200, alone: 2048 x 8192 14.4 -> 11.4 us (5.9 TB/s), 8192 x 4096 26.3 -> 22.4 us, 8192 x 8192 53 -> 50 us.
 // The blocks start with the last rows: the GEMM before this launch finishes them in ascending order, so the last ones are
 // those that L2 still holds.
+// What a block needs first, the parts of its rows and their first words, is requested together. kShort: gamma's words too, for
+// which there are registers with fewer blocks per SM: passes of at most one, which are all latency. Layers of both launches
+// in a CUDA graph, weights from memory, us a layer: 16 x 8192 x 1024 12.0 -> 11.3, 128 x 8192 x 1024 14.4 -> 14.1, 300 x 5120 x 1024 14.9 ->
+// 14.3, 450 x 8192 x 512 17.9 -> 16.7.
 constexpr int kScaleThreads = 512;
 constexpr int kScaleRows = 32;
-__global__ void __launch_bounds__(kScaleThreads, 3) tpScaleRowsPartsKernel(const bf16* h, const float* parts, int numParts, const bf16* gamma, bf16* out,
-                                                                           int M, int N, float eps, int tpr, int rowsPerBlock) {
+template <bool kShort>
+__global__ void __launch_bounds__(kScaleThreads, kShort ? 2 : 3)
+    tpScaleRowsPartsKernel(const bf16* h, const float* parts, int numParts, const bf16* gamma, bf16* out, int M, int N, float eps, int tpr,
+                           int rowsPerBlock, int rowSlots) {
   __shared__ float partial[kScaleThreads / 32][kScaleRows];
   __shared__ float rinv[kScaleRows];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1043,61 +1049,71 @@ __global__ void __launch_bounds__(kScaleThreads, 3) tpScaleRowsPartsKernel(const
   const uint4* g4 = reinterpret_cast<const uint4*>(gamma);
   const int row0 = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) * rowsPerBlock;
   const int rows = M - row0 < rowsPerBlock ? M - row0 : rowsPerBlock;
-  ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();
-  {
-    // a lane per row, the parts dealt out to the warps
-    static_assert(kScaleRows == 32, "one lane per row");
-    float sum = 0.f;
-    if (lane < rows) {
-      for (int p = warp; p < numParts; p += kScaleThreads / 32) sum += parts[static_cast<size_t>(p) * M + row0 + lane];
-    }
-    partial[warp][lane] = sum;
-  }
-  __syncthreads();
-  if (threadIdx.x < kScaleRows) {
-    float total = 0.f;
-#pragma unroll
-    for (int w = 0; w < kScaleThreads / 32; w++) total += partial[w][threadIdx.x];
-    rinv[threadIdx.x] = rsqrtf(total / static_cast<float>(N) + eps);
-  }
-  __syncthreads();
   const int groups = kScaleThreads / tpr;
   const int inGroup = threadIdx.x % tpr;
   const uint4* src = reinterpret_cast<const uint4*>(h) + static_cast<size_t>(row0) * words;
   uint4* dst = reinterpret_cast<uint4*>(out) + static_cast<size_t>(row0) * words;
-  // (32-bit offsets from the block's first row: kScaleRows rows are far below 2^31 words)
-  auto scale = [&](uint4& v, int w, float sc) {
-    float f[8];
-    Vec16<bf16>::toFloat(v, f);
-    if (gamma != nullptr) {
-      float g[8];
-      Vec16<bf16>::toFloat(g4[w], g);
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+  // (32-bit offsets from the block's first row: kScaleRows rows are far below 2^31 words. Words beyond the row repeat its last one: no
+  // branch around the loads. Not .nc: the GEMM before wrote h while this block was already resident.)
+  uint4 v[4], g[4];
+  int r = threadIdx.x / tpr, w = inGroup;
+  bool more = r < rows && w < words;
+  auto load = [&] {
 #pragma unroll
-      for (int i = 0; i < 8; i++) f[i] = f[i] * sc * g[i];
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; i++) f[i] = f[i] * sc;
+    for (int k = 0; k < 4; k++) {
+      const int at = min(w + k * tpr, words - 1);
+      v[k] = ptx::ld_weak_v4(src + r * words + at);
+      if (kShort && gamma != nullptr) g[k] = ptx::ld_weak_v4(g4 + at);
     }
-    v = Vec16<bf16>::fromFloat(f);
   };
-#pragma unroll 1
-  for (int r = threadIdx.x / tpr; r < rows; r += groups) {
-    const int base = r * words;
-#pragma unroll 1
-    for (int w = inGroup; w < words; w += 4 * tpr) {
-      // (words beyond the row repeat its last one: no branch around the loads; not .nc: the GEMM before wrote h while this
-      // block was already resident)
-      uint4 v[4];
-#pragma unroll
-      for (int k = 0; k < 4; k++) v[k] = ptx::ld_weak_v4(src + base + min(w + k * tpr, words - 1));
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        if (w + k * tpr >= words) break;
-        scale(v[k], w + k * tpr, rinv[r]);
-        dst[base + w + k * tpr] = v[k];
-      }
+  if (more) load();
+  {
+    // the parts of a row are dealt out to the threads of the same number modulo rowSlots, a power of two
+    float sum = 0.f;
+    const int row = threadIdx.x & (rowSlots - 1);
+    if (row < rows) {
+      for (int p = threadIdx.x / rowSlots; p < numParts; p += kScaleThreads / rowSlots) sum += parts[static_cast<size_t>(p) * M + row0 + row];
     }
+    for (int o = 16; o >= rowSlots; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane < rowSlots) partial[warp][lane] = sum;
+  }
+  __syncthreads();
+  if (threadIdx.x < rowSlots) {
+    float total = 0.f;
+#pragma unroll
+    for (int i = 0; i < kScaleThreads / 32; i++) total += partial[i][threadIdx.x];
+    rinv[threadIdx.x] = rsqrtf(total / static_cast<float>(N) + eps);
+  }
+  __syncthreads();
+#pragma unroll 1
+  while (more) {
+    const float sc = rinv[r];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int at = w + k * tpr;
+      if (at >= words) break;
+      float f[8];
+      Vec16<bf16>::toFloat(v[k], f);
+      if (gamma != nullptr) {
+        float gm[8];
+        Vec16<bf16>::toFloat(kShort ? g[k] : g4[at], gm);
+#pragma unroll
+        for (int i = 0; i < 8; i++) f[i] = f[i] * sc * gm[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) f[i] = f[i] * sc;
+      }
+      dst[r * words + at] = Vec16<bf16>::fromFloat(f);
+    }
+    w += 4 * tpr;
+    if (w >= words) {
+      w = inGroup;
+      r += groups;
+      more = r < rows;
+    }
+    if (more) load();
   }
 }
 
@@ -1458,8 +1474,13 @@ cudaError_t launchTpScaleRowsFromSumsq(const void* h, const float* sumsqParts, i
   const bf16* hp = static_cast<const bf16*>(h);
   const bf16* gp = static_cast<const bf16*>(gamma);
   bf16* op = static_cast<bf16*>(out);
-  void* params[] = {&hp, &sumsqParts, &numParts, &gp, &op, &M, &N, &eps, &tpr, &rowsPerBlock};
-  return gemm::launchOverlapped(reinterpret_cast<const void*>(tpScaleRowsPartsKernel), dim3(blocks), dim3(kScaleThreads), 0, params, stream);
+  int rowSlots = 1;
+  while (rowSlots < rowsPerBlock) rowSlots *= 2;
+  void* params[] = {&hp, &sumsqParts, &numParts, &gp, &op, &M, &N, &eps, &tpr, &rowsPerBlock, &rowSlots};
+  // (one block per SM: at two, the larger blocks are in each other's way, 512 x 4096 15.6 us a layer against 14.8)
+  const void* kernel = blocks <= gemm::smCount() ? reinterpret_cast<const void*>(tpScaleRowsPartsKernel<true>)
+                                                     : reinterpret_cast<const void*>(tpScaleRowsPartsKernel<false>);
+  return gemm::launchOverlapped(kernel, dim3(blocks), dim3(kScaleThreads), 0, params, stream);
 }
 
 cudaError_t launchTpScaleRows(const void* h, const float* rinv, const void* gamma, void* out, int M, int N,
