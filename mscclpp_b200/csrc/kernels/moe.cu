@@ -15,10 +15,11 @@
 //   hosting ranks' buffers (16-byte peer loads), applies the routing weights in fp32 and writes the bf16 result.
 //   No staging buffer and no second pass. With fp8 = 1 the expert outputs are e4m3 with 1 x 128 scales (quantised by
 //   the expert GEMM's epilogue or by launchMoeQuantizeRows), half the bytes over NVLink.
-// With one rank both are bound by HBM. Dispatch and combine together on one B200: 4096 tokens x 4096 bf16, top-2 of 64
-// experts 51 us (201 MB, 3.9 TB/s), 777 tokens x 7168 fp8, top-8 of 256 experts 39 us; with 64 blocks, a whole row per
-// warp, one expert's row after the other and system-scope accesses it was 86 and 104 us.
-// Both end with a cross-rank barrier: after dispatch returns every row sent to this rank has landed; after combine
+// With one rank there is nobody to exchange counts with or to wait for: neither launch is cooperative, both overlap the kernel
+// before them, and every block of the dispatch counts all pairs by itself (up to 16384 of them). Dispatch and combine together
+// on one B200, before / now: 4096 tokens x 4096 bf16, top-2 of 64 experts 51 / 42 us (201 MB, 4.8 TB/s), 777 tokens x 7168
+// fp8, top-8 of 256 experts 39 / 33 us.
+// With several ranks both end with a cross-rank barrier: after dispatch returns every row sent to this rank has landed; after combine
 // returns the peers are done reading this rank's expert outputs.
 //
 // The reference library has no MoE kernels of its own; its bulk-copy device primitives
@@ -27,6 +28,8 @@
 
 #include <mscclpp/gpu_data_types.hpp>
 #include <mscclpp/poll_device.hpp>
+
+#include "gemm.cuh"
 
 namespace mscclpp {
 
@@ -88,11 +91,16 @@ MSCCLPP_DEVICE_INLINE void e4m3x16ToFloat(const uint4& v, float (&f)[16]) {
   }
 }
 
+// kOne: one rank and few enough pairs that every block counts them all by itself (moeCountsAlone). No block waits for another
+// then, so the launch is not cooperative and overlaps the kernel before it, and the heap's epoch plays no part.
+template <bool kOne>
 __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs a) {
   const DeviceComm& c = a.comm;
   const int rank = deviceRank(c);
-  const int world = c.world;
-  const uint32_t epoch = launchEpoch(c, rank);
+  const int world = kOne ? 1 : c.world;
+  uint32_t epoch = 0;
+  if constexpr (kOne) ptx::grid_launch_dependents();
+  else epoch = launchEpoch(c, rank);
   const uint64_t base = c.peerBase[c.rank];
   const uint64_t local = c.peerBase[rank];
   const uint64_t wsOff = reinterpret_cast<uint64_t>(a.workspace) - base;
@@ -124,42 +132,70 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
   if (threadIdx.x < kBatchTokens && tokBegin + static_cast<int>(threadIdx.x) < tokEnd)
     ptx::bulk_prefetch_l2(x + static_cast<size_t>(tokBegin + threadIdx.x) * a.hidden, static_cast<uint32_t>(a.hidden) * 2);
 
-  // ---- A. position of every pair inside its (me, expert) group
-  for (int i = tokBegin * a.topk + threadIdx.x; i < tokEnd * a.topk; i += blockDim.x) {
-    const int e = topkIdx[i];
-    slotMap[i] = (e >= 0 && e < E) ? static_cast<int32_t>(atomicAdd(&ws.cnt[e], 1u)) : -1;
-  }
-  bool healthy = gridBarrier(c, rank, &ctl->gridSync[0], gridDim.x);
-
-  // ---- B. block 0 sends my counts to everybody (its own matrix row included), then re-arms the counters
-  if (blockIdx.x == 0 && healthy) {
-    for (int i = threadIdx.x; i < world * E; i += blockDim.x) {
-      const int p = i / E, e = i % E;
-      uint2* dst = workspaceOf(c, p, wsOff).matrix + rank * kMoeMaxExperts + e;
-      ptx::st_volatile_v2(dst, make_uint2(ws.cnt[e], epoch));
-    }
+  bool healthy = true;
+  if constexpr (kOne) {
+    // ---- A-C. every expert's pairs before this block's share, in it and behind it
+    for (int i = threadIdx.x; i < 3 * kMoeMaxExperts; i += blockDim.x) counts[i / kMoeMaxExperts][i % kMoeMaxExperts] = 0;
+    if (threadIdx.x == 0) overflow = 0;
     __syncthreads();
-    for (int e = threadIdx.x; e < E; e += blockDim.x) ws.cnt[e] = 0;
-  }
-
-  // ---- C. every block collects the whole matrix and derives the first row of each of its groups
-  if (threadIdx.x == 0) overflow = 0;
-  __syncthreads();
-  if (healthy) {
-    for (int i = threadIdx.x; i < world * E; i += blockDim.x) {
-      const int s = i / E, e = i % E;
-      const uint2* src = ws.matrix + s * kMoeMaxExperts + e;
-      SpinGuard g(c.status, c.timeoutNs);
-      uint2 v = ptx::ld_volatile_v2(src);
-      while (v.y != epoch) {
-        if (!g.keepSpinning()) {
-          g.report(kDevTimeoutFlag, rank, 6000 + s, e, epoch, v.y);
-          overflow = 2;
-          break;
-        }
-        v = ptx::ld_volatile_v2(src);
+    ptx::grid_dependency_wait();
+    const int lo = tokBegin * a.topk, hi = tokEnd * a.topk, pairs = a.tokens * a.topk;
+    constexpr int kDepth = 8;
+    for (int i0 = threadIdx.x; i0 - static_cast<int>(threadIdx.x) < pairs; i0 += kDepth * kThreads) {
+      int e[kDepth];
+#pragma unroll
+      for (int k = 0; k < kDepth; k++) {
+        const int i = i0 + k * kThreads;
+        e[k] = i < pairs ? static_cast<int>(ptx::ld_weak_u32(reinterpret_cast<const uint32_t*>(topkIdx) + i)) : -1;
       }
-      counts[s][e] = v.x;
+#pragma unroll
+      for (int k = 0; k < kDepth; k++) {
+        // one addition per expert that a warp meets: a batch that is routed to few experts costs no more than another
+        const int i = i0 + k * kThreads;
+        const bool used = e[k] >= 0 && e[k] < E;
+        const int cell = used ? (static_cast<int>(i >= lo) + static_cast<int>(i >= hi)) * kMoeMaxExperts + e[k] : -1;
+        const uint32_t same = __match_any_sync(0xffffffffu, cell);
+        if (used && (same & ((1u << (threadIdx.x & 31)) - 1u)) == 0) atomicAdd(&counts[cell / kMoeMaxExperts][cell % kMoeMaxExperts], __popc(same));
+      }
+    }
+  } else {
+    // ---- A. position of every pair inside its (me, expert) group
+    for (int i = tokBegin * a.topk + threadIdx.x; i < tokEnd * a.topk; i += blockDim.x) {
+      const int e = topkIdx[i];
+      slotMap[i] = (e >= 0 && e < E) ? static_cast<int32_t>(atomicAdd(&ws.cnt[e], 1u)) : -1;
+    }
+    healthy = gridBarrier(c, rank, &ctl->gridSync[0], gridDim.x);
+
+    // ---- B. block 0 sends my counts to everybody (its own matrix row included), then re-arms the counters
+    if (blockIdx.x == 0 && healthy) {
+      for (int i = threadIdx.x; i < world * E; i += blockDim.x) {
+        const int p = i / E, e = i % E;
+        uint2* dst = workspaceOf(c, p, wsOff).matrix + rank * kMoeMaxExperts + e;
+        ptx::st_volatile_v2(dst, make_uint2(ws.cnt[e], epoch));
+      }
+      __syncthreads();
+      for (int e = threadIdx.x; e < E; e += blockDim.x) ws.cnt[e] = 0;
+    }
+
+    // ---- C. every block collects the whole matrix and derives the first row of each of its groups
+    if (threadIdx.x == 0) overflow = 0;
+    __syncthreads();
+    if (healthy) {
+      for (int i = threadIdx.x; i < world * E; i += blockDim.x) {
+        const int s = i / E, e = i % E;
+        const uint2* src = ws.matrix + s * kMoeMaxExperts + e;
+        SpinGuard g(c.status, c.timeoutNs);
+        uint2 v = ptx::ld_volatile_v2(src);
+        while (v.y != epoch) {
+          if (!g.keepSpinning()) {
+            g.report(kDevTimeoutFlag, rank, 6000 + s, e, epoch, v.y);
+            overflow = 2;
+            break;
+          }
+          v = ptx::ld_volatile_v2(src);
+        }
+        counts[s][e] = v.x;
+      }
     }
   }
   __syncthreads();
@@ -170,10 +206,15 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
     const int e = threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t tot = 0, before = 0;
     if (known && e < E) {
-      for (int s = 0; s < world; s++) {
-        const uint32_t n = counts[s][e];
-        if (s < rank) before += n;
-        tot += n;
+      if constexpr (kOne) {
+        before = counts[0][e];
+        tot = before + counts[1][e] + counts[2][e];
+      } else {
+        for (int s = 0; s < world; s++) {
+          const uint32_t n = counts[s][e];
+          if (s < rank) before += n;
+          tot += n;
+        }
       }
     }
     uint32_t incl = tot;
@@ -219,6 +260,10 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
   const int warps = blockDim.x >> 5;
   const int scalesPerRow = a.hidden / kMoeScaleGroup;
   const bool wide = (recvXOff & 15) == 0;  // the quantised rows may be stored in 16-byte words
+  auto storeWord = [](uint32_t* p, uint32_t v) {
+    if constexpr (kOne) *p = v;
+    else ptx::st_relaxed_sys(p, v);
+  };
   if (send) {
     auto stage = [&](int t0, int n, int buf) {
       const int i = threadIdx.x;
@@ -226,14 +271,17 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
       const int p = t0 * a.topk + i;
       const int e = topkIdx[p];
       uint64_t row = 0, scales = 0;
-      const int r = e >= 0 && e < E ? moeDestinationRow(firstRow[e], slotMap[p], a.capacity) : -1;  // slotMap holds the position in the group
+      int r = -1;
+      if (e >= 0 && e < E) {
+        if constexpr (kOne) r = moeDestinationRow(atomicAdd(&firstRow[e], 1u), 0, a.capacity);
+        else r = moeDestinationRow(firstRow[e], slotMap[p], a.capacity);  // slotMap holds the position in the group
+      }
       slotMap[p] = r;
       if (r >= 0) {
         const uint64_t peer = c.peerBase[e / El];
         row = peer + recvXOff + static_cast<uint64_t>(r) * a.hidden * (a.fp8 ? 1 : 2);
         scales = peer + recvScalesOff + static_cast<uint64_t>(r) * scalesPerRow * 4;
-        ptx::st_relaxed_sys(reinterpret_cast<uint32_t*>(peer + recvSrcOff) + r,
-                            (static_cast<uint32_t>(rank) << 24) | static_cast<uint32_t>(t0 + i / a.topk));
+        storeWord(reinterpret_cast<uint32_t*>(peer + recvSrcOff) + r, (static_cast<uint32_t>(rank) << 24) | static_cast<uint32_t>(t0 + i / a.topk));
       }
       rowAddr[buf][i] = row;
       scaleAddr[buf][i] = scales;
@@ -252,7 +300,7 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
 #pragma unroll
         for (int j = 0; j < kPieceWords; j++) {
           v[j] = make_uint4(0, 0, 0, 0);
-          if (w0 + j * 32 < words) v[j] = ptx::ld_input_v4(src + w0 + j * 32);
+          if (w0 + j * 32 < words) v[j] = kOne ? ptx::ld_weak_v4(src + w0 + j * 32) : ptx::ld_input_v4(src + w0 + j * 32);
         }
       };
       if (warp < units) load(warp, cur);
@@ -311,7 +359,7 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
             }
             const int sw = w0 / 16 + lane;
             if (lane < 2 * kPieceWords && sw < scalesPerRow)
-              ptx::st_relaxed_sys(reinterpret_cast<uint32_t*>(scaleRows[k]) + sw, __float_as_uint(scale));
+              storeWord(reinterpret_cast<uint32_t*>(scaleRows[k]) + sw, __float_as_uint(scale));
           }
         }
 #pragma unroll
@@ -321,20 +369,29 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
   } else {
     for (int i = tokBegin * a.topk + threadIdx.x; i < tokEnd * a.topk; i += blockDim.x) slotMap[i] = -1;
   }
-  // every row of mine is on its way: after this barrier the rows sent TO me have landed
-  if (healthy) rankBarrier(c, rank, 0, blockIdx.x, epoch);
-  finishLaunch(c, rank, epoch);
+  if constexpr (!kOne) {
+    // every row of mine is on its way: after this barrier the rows sent TO me have landed
+    if (healthy) rankBarrier(c, rank, 0, blockIdx.x, epoch);
+    finishLaunch(c, rank, epoch);
+  }
 }
 
 // A unit of the combine is 32 x kWords 16-byte words of one token's result (kFp8: of its quantised rows). A warp takes the
 // units in turn over the whole grid; the rows of kRows experts are requested together (kWords x kRows = 8 loads per lane
 // in flight; launchMoeCombine picks the form), and the expert ids, rows and weights of its next unit while it waits for them (lane k holds the k-th).
-template <int kWords, int kRows, bool kFp8>
+// kOne: one rank. There is nobody to wait for: the launch is not cooperative and overlaps the kernel before it.
+template <int kWords, int kRows, bool kFp8, bool kOne>
 __global__ void __launch_bounds__(kThreads, 1) moeCombineKernel(MoeCombineArgs a) {
   const DeviceComm& c = a.comm;
   const int rank = deviceRank(c);
-  const int world = c.world;
-  const uint32_t epoch = launchEpoch(c, rank);
+  const int world = kOne ? 1 : c.world;
+  uint32_t epoch = 0;
+  if constexpr (kOne) {
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
+  } else {
+    epoch = launchEpoch(c, rank);
+  }
   const uint64_t base = c.peerBase[c.rank];
   const uint64_t local = c.peerBase[rank];
   const int32_t* topkIdx = reinterpret_cast<const int32_t*>(local + (reinterpret_cast<uint64_t>(a.topkIdx) - base));
@@ -351,7 +408,7 @@ __global__ void __launch_bounds__(kThreads, 1) moeCombineKernel(MoeCombineArgs a
   const int64_t units = static_cast<int64_t>(a.tokens) * chunks;
 
   // the peers' expert outputs are final once their kernels run
-  const bool healthy = rankBarrier(c, rank, 0, blockIdx.x, epoch);
+  const bool healthy = kOne || rankBarrier(c, rank, 0, blockIdx.x, epoch);
   const int lane = threadIdx.x & 31;
   const int warpsPerBlock = blockDim.x >> 5;
   const int numWarps = gridDim.x * warpsPerBlock;
@@ -443,9 +500,11 @@ __global__ void __launch_bounds__(kThreads, 1) moeCombineKernel(MoeCombineArgs a
       }
     }
   }
-  // my reads are done: the peers may overwrite their expert outputs after this
-  if (healthy) rankBarrier(c, rank, 1, blockIdx.x, epoch);
-  finishLaunch(c, rank, epoch);
+  if constexpr (!kOne) {
+    // my reads are done: the peers may overwrite their expert outputs after this
+    if (healthy) rankBarrier(c, rank, 1, blockIdx.x, epoch);
+    finishLaunch(c, rank, epoch);
+  }
 }
 
 // One warp per row: the dispatch's quantiser as a stand-alone pass (for expert outputs that are to be combined as fp8).
@@ -489,6 +548,14 @@ cudaError_t launchCoop(Kernel kernel, const Args& args, int nBlocks, int emu, cu
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), grid, block, params, 0, stream);
 }
 
+template <int kWords, int kRows, bool kFp8>
+cudaError_t launchCombine(const MoeCombineArgs& args, int nBlocks, int emu, cudaStream_t stream) {
+  if (args.comm.world > 1) return launchCoop(moeCombineKernel<kWords, kRows, kFp8, false>, args, nBlocks, emu, stream);
+  MoeCombineArgs copy = args;
+  void* params[] = {&copy};
+  return gemm::launchOverlapped(reinterpret_cast<const void*>(moeCombineKernel<kWords, kRows, kFp8, true>), dim3(nBlocks), dim3(kThreads), 0, params, stream);
+}
+
 int defaultBlocks(int emu, int world) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -513,7 +580,10 @@ cudaError_t launchMoeDispatch(const MoeDispatchArgs& args, int nBlocks, cudaStre
   if (args.capacity <= 0 || (args.fp8 && args.recvScales == nullptr)) return cudaErrorInvalidValue;
   if (nBlocks <= 0) nBlocks = defaultBlocks(emu, args.comm.world);
   if (nBlocks > kBarrierSlots) return cudaErrorInvalidValue;
-  return launchCoop(moeDispatchKernel, args, nBlocks, emu, stream);
+  if (!moeCountsAlone(args.comm.world, args.tokens, args.topk)) return launchCoop(moeDispatchKernel<false>, args, nBlocks, emu, stream);
+  MoeDispatchArgs copy = args;
+  void* params[] = {&copy};
+  return gemm::launchOverlapped(reinterpret_cast<const void*>(moeDispatchKernel<true>), dim3(nBlocks), dim3(kThreads), 0, params, stream);
 }
 
 cudaError_t launchMoeQuantizeRows(const __nv_bfloat16* x, void* q, float* scales, int rows, int hidden, cudaStream_t stream) {
@@ -554,16 +624,16 @@ cudaError_t launchMoeCombine(const MoeCombineArgs& args, int nBlocks, cudaStream
   }
   switch (form) {
     case 8:
-      return launchCoop(moeCombineKernel<8, 1, false>, args, nBlocks, emu, stream);
+      return launchCombine<8, 1, false>(args, nBlocks, emu, stream);
     case 4:
-      return args.fp8 ? launchCoop(moeCombineKernel<4, 2, true>, args, nBlocks, emu, stream)
-                      : launchCoop(moeCombineKernel<4, 2, false>, args, nBlocks, emu, stream);
+      return args.fp8 ? launchCombine<4, 2, true>(args, nBlocks, emu, stream)
+                      : launchCombine<4, 2, false>(args, nBlocks, emu, stream);
     case 2:
-      return args.fp8 ? launchCoop(moeCombineKernel<2, 4, true>, args, nBlocks, emu, stream)
-                      : launchCoop(moeCombineKernel<2, 4, false>, args, nBlocks, emu, stream);
+      return args.fp8 ? launchCombine<2, 4, true>(args, nBlocks, emu, stream)
+                      : launchCombine<2, 4, false>(args, nBlocks, emu, stream);
     default:
-      return args.fp8 ? launchCoop(moeCombineKernel<1, 8, true>, args, nBlocks, emu, stream)
-                      : launchCoop(moeCombineKernel<1, 8, false>, args, nBlocks, emu, stream);
+      return args.fp8 ? launchCombine<1, 8, true>(args, nBlocks, emu, stream)
+                      : launchCombine<1, 8, false>(args, nBlocks, emu, stream);
   }
 }
 

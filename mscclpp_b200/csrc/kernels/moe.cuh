@@ -32,6 +32,12 @@ MSCCLPP_HOST_DEVICE_INLINE int moeDestinationRow(uint32_t first, int32_t positio
   return position >= 0 && row < static_cast<uint64_t>(capacity) ? static_cast<int>(row) : -1;
 }
 
+// Whether every block of a dispatch counts all pairs by itself. With one rank that replaces the counters in memory, the grid
+// barrier, the count matrix and the cooperative launch; each block reads all expert ids for it.
+MSCCLPP_HOST_DEVICE_INLINE bool moeCountsAlone(int world, int tokens, int topk) {
+  return world == 1 && static_cast<int64_t>(tokens) * topk <= 16384;
+}
+
 struct MoeDispatchArgs {
   DeviceComm comm;
   int tokens, hidden, topk, numExperts;  // numExperts over all ranks; rank r hosts experts [r * E/world, (r+1) * E/world)
@@ -67,7 +73,8 @@ struct MoeCombineArgs {
 // group / 448. x [rows, hidden] bf16, q [rows, hidden] bytes, scales [rows, hidden / 128]; hidden % 256 == 0.
 cudaError_t launchMoeQuantizeRows(const __nv_bfloat16* x, void* q, float* scales, int rows, int hidden, cudaStream_t stream);
 
-// nBlocks <= 0 picks a default. Both launches are cooperative (grid barriers, and emulated ranks wait on each other).
+// nBlocks <= 0 picks a default. Both launches are cooperative (grid barriers, and emulated ranks wait on each other), except
+// that with one rank the combine, and the dispatch of few pairs (moeCountsAlone), overlap the kernel before them.
 cudaError_t launchMoeDispatch(const MoeDispatchArgs& args, int nBlocks, cudaStream_t stream);
 cudaError_t launchMoeCombine(const MoeCombineArgs& args, int nBlocks, cudaStream_t stream);
 

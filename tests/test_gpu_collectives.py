@@ -650,6 +650,40 @@ def test_moe_one_rank(tokens, hidden, experts, topk, fp8):
     symm.destroy()
 
 
+@pytest.mark.parametrize("tokens,topk,n_blocks", [(4096, 4, 0), (4097, 4, 0), (2, 2, 0), (1000, 8, 7)])
+def test_moe_one_rank_counts(tokens, topk, n_blocks):
+    """Either side of the line up to which every block of a one-rank dispatch counts all pairs; fewer tokens than blocks, few blocks;
+    every token routed to the same experts, and ids that name no expert."""
+    from mscclpp_b200 import SymmetricMemory
+    from mscclpp_b200.parallel.moe import ExpertParallelDispatcher
+
+    hidden, experts = 256, 24
+    symm = SymmetricMemory.emulated(1, nbytes=tokens * topk * hidden * 5 + tokens * hidden * 4 + (64 << 20), timeout_ms=3000)
+    disp = ExpertParallelDispatcher(symm, num_experts=experts, hidden=hidden, max_tokens=tokens, topk=topk, capacity=tokens * topk)
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+    same = (torch.arange(topk, device="cuda", dtype=torch.int32) * 3).expand(tokens, -1).contiguous()
+    holes = same.clone()
+    holes[::3, 0] = -1
+    holes[1::5, -1] = experts
+    for idx in (same, holes):
+        disp.recv_x.zero_()
+        recv, counts, slots = disp.dispatch(x, idx, n_blocks=n_blocks)
+        torch.cuda.synchronize()
+        symm.check()
+        used = (idx >= 0) & (idx < experts)
+        expect = torch.bincount(idx[used].long(), minlength=experts)
+        assert torch.equal(counts.long(), torch.cat([expect, expect.sum(0, keepdim=True)]))
+        assert bool((slots[~used] == -1).all())
+        assert torch.equal(slots[used].sort().values.long(), torch.arange(int(used.sum()), device="cuda"))
+        first = torch.cumsum(expect, 0) - expect
+        e = idx[used].long()
+        assert bool(((slots[used] >= first[e]) & (slots[used] < first[e] + expect[e])).all())
+        token = torch.arange(tokens, device="cuda")[:, None].expand(-1, topk)[used]
+        assert torch.equal(recv[slots[used].long()], x[token])
+    symm.destroy()
+
+
 @pytest.mark.parametrize("offset", [0, 8])
 @pytest.mark.parametrize("tokens,hidden,topk", [(3, 256, 1), (70, 768, 3), (160, 2304, 8)])
 def test_moe_dispatch_fp8_rows_at_eight_byte_offsets(tokens, hidden, topk, offset):
