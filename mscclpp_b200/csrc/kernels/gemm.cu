@@ -65,61 +65,6 @@ __global__ void __launch_bounds__(kNumThreads, 1)
   gemmCtaPair(&tmapA, &tmapB, shape, blockIdx.x / 2, gridDim.x / 2, gate, epi, status, budgetNs, smemRaw);
 }
 
-// Epilogue of a product whose tile rows are the output's columns: D^T tiles in tensor memory, a lane per output column. A warp
-// turns 32 x 32 values at a time around in its staging buffer (bf16, 64 bytes per output row) and stores four lanes to a
-// row's 64 bytes.
-struct StoreTurned {
-  static constexpr bool kNeedsTileBarrier = false;
-  static constexpr bool kBulkStore = false;
-  static constexpr bool kRowEpilogue = true;
-  static constexpr int kBlocks = 1;  // 4 KB of staging per warp
-  __nv_bfloat16* out;
-  int M;  // rows of D
-  int ldd;
-  uint8_t* stage = nullptr;
-  MSCCLPP_DEVICE_INLINE void setup(uint8_t* stage_, uint64_t*, int) { stage = stage_; }
-  MSCCLPP_DEVICE_INLINE void request(int, int, int) const {}
-  template <typename ArriveEmpty>
-  MSCCLPP_DEVICE_INLINE bool tile(uint32_t taddr, int row0, int col0, int, int lane, ArriveEmpty&& arriveEmpty) const {
-    constexpr int kHalves = Config2Turned::kColsPerWarp / 32;
-    __nv_bfloat16* const mine = reinterpret_cast<__nv_bfloat16*>(stage);
-#pragma unroll 1
-    for (int half = 0; half < kHalves; half++) {
-      uint32_t v[32];
-      ptx::tmem_ld_32x32b_x32(taddr + half * 32, v);
-      ptx::tmem_ld_wait();
-      if (half == kHalves - 1) {
-        ptx::tcgen05_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) arriveEmpty();
-      }
-      __syncwarp();  // the buffer's last readers are through
-#pragma unroll
-      for (int i = 0; i < 32; i++) mine[i * 32 + lane] = __float2bfloat16_rn(__uint_as_float(v[i]));
-      __syncwarp();
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int t = j * 8 + (lane >> 2), row = col0 + half * 32 + t;
-        const uint4 word = *reinterpret_cast<const uint4*>(mine + t * 32 + (lane & 3) * 8);
-        if (row < M) *reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * ldd + row0 + (lane & 3) * 8) = word;
-      }
-    }
-    return true;
-  }
-  MSCCLPP_DEVICE_INLINE void drain(int) const {}
-  MSCCLPP_DEVICE_INLINE void warpTileDone(int, int) const {}
-  MSCCLPP_DEVICE_INLINE void warpDrain(int) const {}
-  MSCCLPP_DEVICE_INLINE void auxWarp(int, int) const {}
-};
-
-__global__ void __launch_bounds__(kNumThreads, 1)
-    gemmBf16TurnedKernel(const __grid_constant__ CUtensorMap tmapW, const __grid_constant__ CUtensorMap tmapX, Shape shape, StoreTurned epi,
-                         DeviceStatus* status, uint64_t budgetNs) {
-  extern __shared__ uint8_t smemRaw[];
-  NoGate gate;
-  gemmCtaPair<Config2Turned>(&tmapW, &tmapX, shape, blockIdx.x / 2, gridDim.x / 2, gate, epi, status, budgetNs, smemRaw);
-}
-
 // Tile order of a plain GEMM: bands of `band` row blocks (0 = the default for the tile shape, < 0 = plain column-major walk).
 void setBandOrder(Shape& shape, int numMBlk, int band, int dflt) {
   if (band == 0) band = dflt;
@@ -206,28 +151,6 @@ cudaError_t gemmBf16TwoSm(const void* A, const void* B, void* D, int M, int N, i
   void* params[] = {&ta, &tb, &td, &shape, &status, &budgetNs};
   return launchClusterPair(reinterpret_cast<const void*>(gemmBf16PairKernel), dim3(grid), dim3(kNumThreads), Config2::kSmemBytes, params,
                            false, stream, true);
-}
-
-cudaError_t gemmBf16Turned(const void* A, const void* B, void* D, int M, int N, int K, int ldd, int numCtas, DeviceStatus* status,
-                           cudaStream_t stream, uint64_t budgetNs) {
-  using Cfg = Config2Turned;
-  if (M <= 0 || N <= 0 || K <= 0 || K % kBlockK != 0 || N % Cfg::kPairM != 0 || ldd % 8 != 0) return cudaErrorInvalidValue;
-  if ((reinterpret_cast<uintptr_t>(D) & 15) != 0) return cudaErrorInvalidValue;
-  const int blocks = (M + Cfg::kBlockN - 1) / Cfg::kBlockN;
-  Shape shape{N, blocks * Cfg::kBlockN, K, kBlockM, 1, 0, 0};  // tiles that share weight rows run side by side
-  CUtensorMap tw, tx;
-  cudaError_t e = makeTensorMapBf16(&tw, B, N, K, static_cast<uint64_t>(K) * 2, kBlockM);
-  if (e == cudaSuccess) e = makeTensorMapBf16(&tx, A, M, K, static_cast<uint64_t>(K) * 2, Cfg::kBlockN / 2);  // (rows beyond M read as zeros)
-  const void* kernel = reinterpret_cast<const void*>(gemmBf16TurnedKernel);
-  if (e == cudaSuccess) e = ensureDynamicSmem(kernel, Cfg::kSmemBytes);
-  if (e != cudaSuccess) return e;
-  const int tiles = N / Cfg::kPairM * blocks;
-  int grid = (numCtas > 0 ? numCtas : smCount()) & ~1;
-  if (grid > 2 * tiles) grid = 2 * tiles;
-  if (grid < 2) grid = 2;
-  StoreTurned epi{static_cast<__nv_bfloat16*>(D), M, ldd};
-  void* params[] = {&tw, &tx, &shape, &epi, &status, &budgetNs};
-  return launchClusterPair(kernel, dim3(grid), dim3(kNumThreads), Cfg::kSmemBytes, params, false, stream, true);
 }
 
 int smCount() {

@@ -50,11 +50,6 @@ cudaError_t gemmBf16(const void* A, const void* B, void* D, int M, int N, int K,
 cudaError_t gemmBf16TwoSm(const void* A, const void* B, void* D, int M, int N, int K, int ldd, int numCtas, DeviceStatus* status,
                           cudaStream_t stream, int probe = 0, int band = 0, uint64_t budgetNs = kDefaultBudgetNs);
 
-// Same product with the operands' roles turned around: the rows of B are the tile's rows, 256 x 128 tiles on pairs of SMs, the
-// accumulator is written transposed. For more than one but few 128-row blocks of A (see ops/gemm.py). N % 256 == 0; K % 64 == 0.
-cudaError_t gemmBf16Turned(const void* A, const void* B, void* D, int M, int N, int K, int ldd, int numCtas, DeviceStatus* status,
-                           cudaStream_t stream, uint64_t budgetNs = kDefaultBudgetNs);
-
 // Raises the kernel's dynamic shared-memory limit once per (kernel, device); call before every launch that needs > 48 KB.
 cudaError_t ensureDynamicSmem(const void* kernel, int bytes);
 

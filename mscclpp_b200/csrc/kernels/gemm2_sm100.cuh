@@ -16,15 +16,15 @@
 namespace mscclpp {
 namespace gemm {
 
-template <int kStages_, int kStagingBytes_, int kBarrierBytes_, int kBlockN_ = 256>
+template <int kStages_, int kStagingBytes_, int kBarrierBytes_>
 struct Config2Of {
-  static constexpr int kBlockN = kBlockN_;
+  static constexpr int kBlockN = 256;
   static constexpr int kPairM = 2 * kBlockM;                       // 256 rows per tile
   static constexpr int kStageABytes = kBlockM * kBlockK * 2;       // this CTA's A half: 16 KB
-  static constexpr int kStageBBytes = (kBlockN / 2) * kBlockK * 2;  // this CTA's B half: 16 KB at 256 columns
+  static constexpr int kStageBBytes = (kBlockN / 2) * kBlockK * 2;  // this CTA's B half: 16 KB
   static constexpr int kStageBytes = kStageABytes + kStageBBytes;
   static constexpr int kStages = kStages_;
-  static constexpr int kTmemCols = 2 * kBlockN;  // two accumulator buffers
+  static constexpr int kTmemCols = 2 * kBlockN;  // two accumulator buffers of 256 columns
   static constexpr int kBarrierBytes = kBarrierBytes_;
   static constexpr int kStagingBytes = kStagingBytes_;  // of the epilogue
   static constexpr int kEpiWarps = kNumEpilogueWarps;
@@ -34,11 +34,10 @@ struct Config2Of {
 };
 using Config2 = Config2Of<6, kEpilogueStagingBytes, 256>;
 using Config2Rows = Config2Of<5, 2 * kEpilogueStagingBytes, 512>;  // row epilogues: every block of a warp's tile is staged
-using Config2Turned = Config2Of<8, kEpilogueStagingBytes, 256, 128>;  // 256 weight rows x 128 activation rows (see StoreTurned)
 
-template <typename Cfg>
 MSCCLPP_HOST_DEVICE_INLINE constexpr uint32_t makeInstrDescPair() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(Cfg::kBlockN >> 3) << 17) | (static_cast<uint32_t>(Cfg::kPairM >> 4) << 24);
+  return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(Config2::kBlockN >> 3) << 17) |
+         (static_cast<uint32_t>(Config2::kPairM >> 4) << 24);
 }
 
 // Body of one CTA of a pair. All threads call it; `pairIdx` / `numPairs` index the persistent tile loop.
@@ -144,7 +143,7 @@ MSCCLPP_DEVICE_INLINE void gemmCtaPair(const CUtensorMap* tmapA, const CUtensorM
   } else if (warp == 1) {
     // ===================================================== MMA issuer (one thread of the leader CTA)
     if (leader && ptx::elect_one()) {
-      constexpr uint32_t idesc = makeInstrDescPair<Cfg>();
+      constexpr uint32_t idesc = makeInstrDescPair();
       // one thread feeds the tensor cores of both SMs: descriptors are stepped by adds, waits cost one instruction when
       // the data is already there
       const uint64_t descA0 = makeSmemDesc(ptx::smem_u32(tiles));
