@@ -78,25 +78,20 @@ MSCCLPP_DEVICE_INLINE bool pipeWait(const DeviceComm& c, int rank, int phase, in
   return okSmem[phase] != 0;
 }
 
-// 16-byte units [first, n) from src to dst, kCopyUnroll loads in flight per thread. One side is the user's, src with kUserSrc, else
-// dst: it is read or written once and carries the evict-first policy `once`, so that it does not push the scratch out of L2.
+// 16-byte units [first, n) from src to dst, kCopyUnroll loads in flight per thread.
 constexpr uint32_t kCopyUnroll = 4;
-template <bool kUserSrc>
-MSCCLPP_DEVICE_INLINE void copyUnits(char* dst, const char* src, uint32_t first, uint32_t n, uint64_t once) {
+MSCCLPP_DEVICE_INLINE void copyUnits(char* dst, const char* src, uint32_t first, uint32_t n) {
   for (uint32_t u0 = first + threadIdx.x; u0 < n; u0 += blockDim.x * kCopyUnroll) {
     uint4 v[kCopyUnroll];
 #pragma unroll
     for (uint32_t k = 0; k < kCopyUnroll; k++) {
       const uint32_t u = u0 + k * blockDim.x;  // (loads beyond the end repeat the last unit: no branch around them)
-      const char* from = src + static_cast<uint64_t>(u < n ? u : n - 1) * 16;
-      v[k] = kUserSrc ? ptx::ld_weak_v4_hint(from, once) : ptx::ld_weak_v4(from);
+      v[k] = ptx::ld_weak_v4(src + static_cast<uint64_t>(u < n ? u : n - 1) * 16);
     }
 #pragma unroll
     for (uint32_t k = 0; k < kCopyUnroll; k++) {
       const uint32_t u = u0 + k * blockDim.x;
-      if (u >= n) continue;
-      if constexpr (kUserSrc) ptx::st_weak_v4(dst + static_cast<uint64_t>(u) * 16, v[k]);
-      else ptx::st_weak_v4_hint(dst + static_cast<uint64_t>(u) * 16, v[k], once);
+      if (u < n) ptx::st_weak_v4(dst + static_cast<uint64_t>(u) * 16, v[k]);
     }
   }
 }
@@ -188,14 +183,12 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
   // The part of a slice that this rank reduces is read by nobody else, and nobody else writes its result: with peer loads
   // its whole units skip the scratch both ways (1 / world of the copies).
   const uint32_t ownBegin = static_cast<uint32_t>(rank) * static_cast<uint32_t>(subUnits), ownEnd = ownBegin + static_cast<uint32_t>(subUnits);
-  const uint64_t once = ptx::l2_evict_first();
-  auto copyOthers = [&](char* dst, const char* src, uint32_t whole, auto userSrc) {
-    constexpr bool kUserSrc = decltype(userSrc)::value;
+  auto copyOthers = [&](char* dst, const char* src, uint32_t whole) {
     if constexpr (kNvls) {
-      copyUnits<kUserSrc>(dst, src, 0, whole, once);
+      copyUnits(dst, src, 0, whole);
     } else {
-      copyUnits<kUserSrc>(dst, src, 0, ownBegin < whole ? ownBegin : whole, once);
-      copyUnits<kUserSrc>(dst, src, ownEnd, whole, once);
+      copyUnits(dst, src, 0, ownBegin < whole ? ownBegin : whole);
+      copyUnits(dst, src, ownEnd, whole);
     }
   };
   // 1. copy-in (nothing to do for a slice beyond the end of the message, but the barriers still run: peers may not know)
@@ -203,7 +196,7 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
     const uint32_t have = haveOf(r), tail = tailOf(r, have), whole = have - (tail != 0 ? 1 : 0);
     const char* src = in + firstOf(r) * 16;
     char* dst = reinterpret_cast<char*>(local + inSliceOf(r));
-    copyOthers(dst, src, whole, std::true_type{});
+    copyOthers(dst, src, whole);
     if (tail != 0) copyTail(dst + static_cast<uint64_t>(whole) * 16, src + static_cast<uint64_t>(whole) * 16, tail, 16);
   };
   auto tokenOf = [&](uint64_t r) { return (static_cast<uint64_t>(epoch) << 32) | (r + 1); };
@@ -275,7 +268,7 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
                 const int p = rank + i < world ? rank + i : rank + i - world;
                 ptx::st_weak_v4(reinterpret_cast<void*>(heaps[p] + off), v[k]);
               }
-              ptx::st_weak_v4_hint(reinterpret_cast<void*>(u < direct ? outDirect + static_cast<uint64_t>(u) * 16 : local + off), v[k], once);
+              ptx::st_weak_v4(reinterpret_cast<void*>(u < direct ? outDirect + static_cast<uint64_t>(u) * 16 : local + off), v[k]);
             }
           }
         }
@@ -303,7 +296,7 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
     const uint32_t tail = tailOf(r, have), whole = have - (tail != 0 ? 1 : 0);
     const char* src = reinterpret_cast<const char*>(local + outSlice);
     char* dst = out + firstOf(r) * 16;
-    copyOthers(dst, src, whole, std::false_type{});
+    copyOthers(dst, src, whole);
     if (tail != 0) copyTail(dst + static_cast<uint64_t>(whole) * 16, src + static_cast<uint64_t>(whole) * 16, tail, 0);
   }
   finishLaunch(c, rank, epoch);
