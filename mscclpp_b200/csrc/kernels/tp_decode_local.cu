@@ -108,6 +108,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (a.gamma != nullptr && t == 0) prefetch_l2(a.gamma + col);
   }
   __syncthreads();
+  // both blocks run before one writes into the other's shared memory (below); under the layer before it costs nothing
+  if constexpr (kPair) ptx::cluster_sync_all();
   ptx::grid_dependency_wait();
 
   uint4 residual = make_uint4(0, 0, 0, 0);

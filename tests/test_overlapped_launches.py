@@ -29,3 +29,12 @@ def test_overlapped_kernels_read_nothing_through_the_non_coherent_path():
     for text in parts:
         assert len(text) > 500
         assert not re.search(r"ld_input_v4|__ldg|\.nc\b|__restrict__", text)
+
+
+def test_blocks_of_a_cluster_have_started_before_one_writes_to_another():
+    """Shared memory of another block may be written once that block runs: being scheduled together does not say that it does. The
+    first barrier of the cluster stands before the first such write, where the launch still waits for the kernel before it."""
+    for name, head in (("tp_decode_local.cu", "tpDecodeLocalKernel(const"), ("gemm2_sm100.cuh", "void gemmCtaPair(")):
+        text = _definition(open(os.path.join(KERNELS, name)).read(), head)
+        met, wrote = text.index("cluster_sync_all()"), re.search(r"mapa_shared|shared::cluster", text).start()
+        assert met < text.index("grid_dependency_wait()") and met < wrote, name
