@@ -9,15 +9,16 @@
 //   * the launch overlaps the kernel before it (programmatic dependent launch): as soon as a block of layer n has ended, one of layer
 //     n + 1 takes its place and prefetches its weights, activations and residual into L2. Only then does it wait for
 //     layer n. A prefetch moves data to the point of coherence and shows it to nobody, so it does not matter who writes them;
-//   * weights and activations come as tiles of 64 reduction elements (cp.async.bulk.tensor, 128-byte swizzle), a few dozen requests
-//     per block instead of one per weight row: the copy engine takes about ten cycles per request, 1.4 us for 256 of them;
+//   * weights and activations come as tiles of 128 reduction elements (cp.async.bulk.tensor, 128-byte swizzle, two boxes), a few dozen
+//     requests per block instead of one per weight row: the copy engine takes about ten cycles per request, 1.4 us for 256 of them. The
+//     block waits for the thread that requests them: with one barrier per box instead of one per tile 8 x 5120 x 2560 took 11.6 us, not 10.7;
 //   * the products are warp-level tensor-core instructions with the weights as the 16-row operand and the tokens as the
 //     8-column one, as in tp_decode.cu (a tcgen05 tile starts at 64 rows, and this is a stream); sixteen warps split a block's columns four ways and its tiles four ways;
 //   * the rows' sums of squares need every column. Instead of exchanging them, each block counts itself, and the block (with more
 //     than two tokens: the pair of blocks) that counts last reads all shares and h back and writes `out`.
 //
 // One B200, a chain of layers in a CUDA graph, us per layer before / now (floor: the weights from memory): 1 x 8192 x 1024 11.4 / 7.1
-// (2.6), 8 x 5120 x 2560 17.4 / 11.4 (4.0), 8 x 8192 x 1024 11.6 / 9.3, 5 x 4160 x 3072 19.3 / 11.8, 3 x 1032 x 256 7.2 / 5.1. What
+// (2.6), 8 x 5120 x 2560 17.4 / 10.7 (4.0), 8 x 8192 x 1024 11.6 / 9.3, 5 x 4160 x 3072 19.3 / 11.8, 3 x 1032 x 256 7.2 / 5.1. What
 // bounds it, 1 x 8192 x 1024: 0.7 us from the last store of the layer before to the end of the wait, 0.7 to the first tile,
 // 1.8 for the rest (9.3 TB/s, out of L2), 1.3 for the sums, 0.9 for the count, 1.3 for the last block.
 // Tried instead: splitting K over clusters of four blocks (one more cluster barrier and the partial sums through
@@ -38,10 +39,11 @@ namespace {
 using bf16 = __nv_bfloat16;
 constexpr int kWorkers = 512;              // sixteen warps: four column groups x four tiles at a time
 constexpr int kThreads = kWorkers + 32;    // and the one that requests the tiles
-constexpr int kTileK = 64;                 // reduction elements per tile: 128 bytes
+constexpr int kTileK = 128;                // reduction elements per tile: two boxes of 128 bytes
+constexpr int kBoxK = kTileK / 2;
 constexpr int kMaxCols = 128;              // output columns per block
-constexpr int kMaxTiles = 32;              // in flight
-constexpr int kXBytes = kTpDecodeMaxTokens * kTileK * 2;
+constexpr int kMaxTiles = 16;              // in flight
+constexpr int kXBytes = kTpDecodeMaxTokens * kTileK * 2;  // both boxes
 constexpr int kMaxSmem = 216 * 1024;       // of a block: tiles in flight are worth more than a second block
 
 struct DecodeLocalArgs {
@@ -100,8 +102,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         ptx::mbar_init(&empty[s], 4);  // the four warps that work on a tile
       }
       ptx::fence_mbar_init();
-      for (int k = 0; k < tiles; k++) ptx::tma_prefetch_2d(&tmapW, k * kTileK, col0);
-      for (int k = 0; k < tiles; k++) ptx::tma_prefetch_2d(&tmapX, k * kTileK, 0);
+      for (int k = 0; k < a.K; k += kBoxK) ptx::tma_prefetch_2d(&tmapW, k, col0);
+      for (int k = 0; k < a.K; k += kBoxK) ptx::tma_prefetch_2d(&tmapX, k, 0);
     }
   } else if (mine) {
     if (a.residualIn != nullptr) prefetch_l2(a.residualIn + static_cast<size_t>(t) * N + col);
@@ -122,8 +124,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (k >= a.stages && !mbarWait(&empty[s], phase ^ 1u, a.status, a.budgetNs, 630)) break;
         ptx::mbar_expect_tx(&full[s], static_cast<uint32_t>(a.cols + T) * (kTileK * 2));
         const uint32_t at = tile0 + s * tileBytes;
+        const uint32_t boxBytes = a.cols * (kBoxK * 2), atX = at + 2 * boxBytes;
         ptx::tma_load_2d(at, &tmapW, k * kTileK, col0, &full[s]);
-        ptx::tma_load_2d(at + a.cols * (kTileK * 2), &tmapX, k * kTileK, 0, &full[s]);
+        ptx::tma_load_2d(atX, &tmapX, k * kTileK, 0, &full[s]);
+        ptx::tma_load_2d(at + boxBytes, &tmapW, k * kTileK + kBoxK, col0, &full[s]);
+        ptx::tma_load_2d(atX + kXBytes / 2, &tmapX, k * kTileK + kBoxK, 0, &full[s]);
         if (++s == a.stages) {
           s = 0;
           phase ^= 1u;
@@ -131,14 +136,15 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else {
-    // ---- products. Warp (g, sl): columns [16 g, + 16) and [16 g + 64, + 16) of the slab, tiles sl, sl + 4, ... The rows of
+    // ---- products. Warp (g, sl): columns [16 g, + 16) and [16 g + 64, + 16) of the slab, tiles sl, sl + 4, ...: the
+    // elements [128 sl, + 128) of every 512 of the reduction, the slices of tp_decode.cu, whose sums these are to the bit. The rows of
     // absent columns and tokens hold whatever was there: they reach only their own results, which nobody reads.
     const int g = warp & 3, sl = warp >> 2;
     const int groups = (a.cols + 15) / 16;
     const uint32_t aRow = g * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, aHigh = (lane >> 4) & 1, swz = lane & 7;
     float acc[2][4] = {};
-    // The number of stages is a multiple of four, so that a stage is always this warp's or never: it sees every turn of the
-    // barrier. (A warp that met a barrier only every other turn could take the turn before last for the one it waits for.)
+    // The number of stages is a multiple of four or that of the tiles, so that a stage is always this warp's or never: it
+    // sees every turn of the barrier. (A warp that met a barrier only every other turn could take the turn before last for the one it waits for.)
     int s = sl;
     uint32_t phase = 0;
     bool healthy = true;
@@ -146,18 +152,22 @@ __global__ void __launch_bounds__(kThreads, 1)
       // After a wait that ran out the warp only sees the remaining copies land (bounded): the block must not end before they have.
       const bool ok = mbarWait(&full[s], phase, healthy ? a.status : nullptr, healthy ? a.budgetNs : 2000000ull, 620);
       healthy = __all_sync(0xffffffffu, ok) && healthy;
-      const uint32_t w = tile0 + s * tileBytes, x = w + a.cols * (kTileK * 2);
-      uint32_t b[2][4];
+      const uint32_t boxBytes = a.cols * (kBoxK * 2);
 #pragma unroll
-      for (int half = 0; half < 2; half++) ldmatrix_x4(b[half], x + (lane & 7) * 128 + (((half * 4 + (lane >> 3)) ^ swz) << 4));
+      for (int box = 0; box < 2; box++) {
+        const uint32_t w = tile0 + s * tileBytes + box * boxBytes, x = tile0 + s * tileBytes + 2 * boxBytes + box * (kXBytes / 2);
+        uint32_t b[2][4];
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        if (g + j * 4 < groups) {
+        for (int half = 0; half < 2; half++) ldmatrix_x4(b[half], x + (lane & 7) * 128 + (((half * 4 + (lane >> 3)) ^ swz) << 4));
 #pragma unroll
-          for (int kk = 0; kk < 4; kk++) {
-            uint32_t af[4];
-            ldmatrix_x4(af, w + (aRow + j * 64) * 128 + (((kk * 2 + aHigh) ^ swz) << 4));
-            mma_m16n8k16(acc[j], af, b[kk >> 1][(kk & 1) * 2], b[kk >> 1][(kk & 1) * 2 + 1]);
+        for (int j = 0; j < 2; j++) {
+          if (g + j * 4 < groups) {
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) {
+              uint32_t af[4];
+              ldmatrix_x4(af, w + (aRow + j * 64) * 128 + (((kk * 2 + aHigh) ^ swz) << 4));
+              mma_m16n8k16(acc[j], af, b[kk >> 1][(kk & 1) * 2], b[kk >> 1][(kk & 1) * 2 + 1]);
+            }
           }
         }
       }
@@ -191,7 +201,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int j = 0; j < 8; j++) {
         const float* src = part + t * partRow + ju * 8 + j;
         const int slice = kTpDecodeMaxTokens * partRow;
-        f[j] = (src[0] + src[slice]) + (src[2 * slice] + src[3 * slice]);
+        f[j] = ((src[0] + src[slice]) + src[2 * slice]) + src[3 * slice];  // (in the order of tp_decode.cu)
       }
       // the product rounded to bf16, then the sum with the residual: the roundings of the unfused composition
       uint4 h = Vec16<bf16>::fromFloat(f);
@@ -303,8 +313,8 @@ cudaError_t launchTpDecodeLocal(const TpDecodeArgs& args, void* workspace, cudaS
   const int partBytes = 4 * kTpDecodeMaxTokens * ((a.cols + 15) / 16 * 16) * 4;
   a.stages = static_cast<int>((kMaxSmem - 1024 - partBytes) / tileBytes);
   if (a.stages > kMaxTiles) a.stages = kMaxTiles;
-  if (a.stages > K / kTileK) a.stages = K / kTileK;
-  a.stages &= ~3;  // tile k and the one that comes after it in a stage belong to the same warps (see the kernel)
+  // Tile k and the one that comes after it in a stage belong to the same warps (see the kernel), unless none comes after any.
+  a.stages = a.stages >= K / kTileK ? K / kTileK : a.stages & ~3;
   const bool pair = T > 2;
   if (pair) blocks = (blocks + 1) & ~1;  // (the odd one out has no columns: its weights are out of the map's bounds, read as zeros)
   const void* kernel = pair ? reinterpret_cast<const void*>(tpDecodeLocalKernel<true>) : reinterpret_cast<const void*>(tpDecodeLocalKernel<false>);

@@ -323,6 +323,28 @@ def test_decode_layer_one_gpu(tokens, hidden, k):
     symm.destroy()
 
 
+@pytest.mark.parametrize("tokens,hidden,k", [(1, 8192, 1024), (8, 5120, 2560), (3, 1032, 256), (5, 2048, 768), (2, 18944, 3072)])
+def test_decode_layer_one_gpu_sums_in_the_order_of_the_cooperative_form(tokens, hidden, k):
+    """h = product + residual is the same bits as from the launch that several ranks take (768 and 256: the last tiles leave two of the
+    four slices of the reduction without work)."""
+    from mscclpp_b200 import SymmetricMemory, native
+    from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
+
+    symm = SymmetricMemory.emulated(1, nbytes=64 << 20, timeout_ms=3000)
+    layer = RowParallelLinearNorm(symm, out_features=hidden, k_shard=k, max_tokens=tokens)
+    g = torch.Generator(device="cuda").manual_seed(hidden + k)
+    x = torch.randn((tokens, k), generator=g, device="cuda").to(torch.bfloat16)
+    residual = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+    h = layer.forward_decode(x, residual)[1].clone()
+    native().tp_decode(symm.heap, [x.data_ptr()], [layer.weight.data_ptr()], layer.residual_in.data_ptr(), layer.residual_out.data_ptr(),
+                       layer.out.data_ptr(), layer.gamma.data_ptr(), tokens, hidden, k, layer.eps, False, 0,
+                       torch.cuda.current_stream().cuda_stream, 0, 0)
+    torch.cuda.synchronize()
+    symm.check()
+    assert torch.equal(h, layer.residual_out[:tokens])
+    symm.destroy()
+
+
 @pytest.mark.parametrize("tokens", [1, 8])
 def test_chained_decode_layers_wait_for_one_another(tokens):
     """Decode launches overlap the one before them and prefetch their operands under it: activations that the layer before
