@@ -184,14 +184,9 @@ void registerMoreBindings(py::module_& m) {
         a.emuRanks = heap.emulated() ? heap.world() : 1;
         a.numCtas = numCtas;
         a.stamps = reinterpret_cast<unsigned long long*>(stamps);
-        if (workspace != 0 && heap.world() == 1 && numCtas == 0 && stamps == 0) {
-          const cudaError_t e = launchTpDecodeLocal(a, reinterpret_cast<void*>(workspace), reinterpret_cast<cudaStream_t>(stream));
-          if (e != cudaErrorInvalidValue && e != cudaErrorInvalidConfiguration) {
-            checkCudaMore(e, "tp_decode");
-            return;
-          }
-        }
-        checkCudaMore(launchTpDecode(a, reinterpret_cast<cudaStream_t>(stream)), "tp_decode");
+        void* ws = reinterpret_cast<void*>(workspace);
+        const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+        checkCudaMore(tpDecodeLocalCovers(a, ws) ? launchTpDecodeLocal(a, ws, s) : launchTpDecode(a, s), "tp_decode");
       },
       py::arg("heap"), py::arg("x"), py::arg("w"), py::arg("residual_in"), py::arg("residual_out"), py::arg("out"), py::arg("gamma"),
       py::arg("t"), py::arg("n"), py::arg("k"), py::arg("eps") = 1e-5f, py::arg("nvls") = false, py::arg("num_ctas") = 0, py::arg("stream") = 0,

@@ -296,19 +296,33 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 size_t tpDecodeLocalWorkspaceWords() { return 4 + static_cast<size_t>(kBarrierSlots) * kTpDecodeMaxTokens; }
 
-cudaError_t launchTpDecodeLocal(const TpDecodeArgs& args, void* workspace, cudaStream_t stream) {
+namespace {
+
+int maxBlocks() {
+  const int even = gemm::smCount() & ~1;
+  return even < kBarrierSlots ? even : kBarrierSlots;
+}
+int columnsPerBlock(int N) { return ((N + maxBlocks() - 1) / maxBlocks() + 7) / 8 * 8; }
+
+}  // namespace
+
+bool tpDecodeLocalCovers(const TpDecodeArgs& args, const void* workspace) {
   const int T = args.T, N = args.N, K = args.K;
+  if (workspace == nullptr || args.comm.world != 1 || args.nvls || args.numCtas != 0 || args.stamps != nullptr) return false;
   const uintptr_t aligned = reinterpret_cast<uintptr_t>(args.w[0]) | reinterpret_cast<uintptr_t>(args.x[0]) | reinterpret_cast<uintptr_t>(args.out) |
                             reinterpret_cast<uintptr_t>(args.residualIn) | reinterpret_cast<uintptr_t>(args.residualOut) |
                             reinterpret_cast<uintptr_t>(args.gamma) | reinterpret_cast<uintptr_t>(workspace);
-  if (T < 1 || T > kTpDecodeMaxTokens || N < 8 || N % 8 != 0 || K < 256 || K % 256 != 0 || args.residualOut == nullptr || aligned % 16 != 0) return cudaErrorInvalidValue;
+  if (T < 1 || T > kTpDecodeMaxTokens || N < 8 || N % 8 != 0 || K < 256 || K % 256 != 0 || args.residualOut == nullptr || aligned % 16 != 0) return false;
+  return columnsPerBlock(N) <= kMaxCols;
+}
+
+cudaError_t launchTpDecodeLocal(const TpDecodeArgs& args, void* workspace, cudaStream_t stream) {
+  if (!tpDecodeLocalCovers(args, workspace)) return cudaErrorInvalidValue;
+  const int T = args.T, N = args.N, K = args.K;
   DecodeLocalArgs a{args.residualIn, args.residualOut, args.out, args.gamma, static_cast<float*>(workspace) + 4, static_cast<uint32_t*>(workspace),
                     T, N, K, args.eps, 0, 0, args.comm.status, args.comm.timeoutNs};
-  int blocks = gemm::smCount() & ~1;
-  if (blocks > kBarrierSlots) blocks = kBarrierSlots;
-  a.cols = ((N + blocks - 1) / blocks + 7) / 8 * 8;
-  if (a.cols > kMaxCols) return cudaErrorInvalidConfiguration;
-  blocks = (N + a.cols - 1) / a.cols;
+  a.cols = columnsPerBlock(N);
+  int blocks = (N + a.cols - 1) / a.cols;
   const uint32_t tileBytes = static_cast<uint32_t>(a.cols) * kTileK * 2 + kXBytes;
   const int partBytes = 4 * kTpDecodeMaxTokens * ((a.cols + 15) / 16 * 16) * 4;
   a.stages = static_cast<int>((kMaxSmem - 1024 - partBytes) / tileBytes);

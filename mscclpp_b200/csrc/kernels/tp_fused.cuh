@@ -131,9 +131,10 @@ cudaError_t launchTpDecode(const TpDecodeArgs& args, cudaStream_t stream);
 
 // The same for one rank, with launches that overlap (see tp_decode_local.cu): of `args` it takes the operands, the status and
 // the time limit. workspace: tpDecodeLocalWorkspaceWords() 32-bit words, zero before the first launch; launches that
-// may run at the same time want their own. cudaErrorInvalidValue or cudaErrorInvalidConfiguration, with nothing launched, for what it does
-// not cover: no residualOut, an operand that is not 16-byte aligned, pieces of the weights that do not fit shared memory.
+// may run at the same time want their own. What it does not cover keeps launchTpDecode: several ranks, a request for NVLS, for a number
+// of blocks or for time stamps, no residualOut, an operand that is not 16-byte aligned, slabs of more than 128 columns per SM.
 size_t tpDecodeLocalWorkspaceWords();
+bool tpDecodeLocalCovers(const TpDecodeArgs& args, const void* workspace);
 cudaError_t launchTpDecodeLocal(const TpDecodeArgs& args, void* workspace, cudaStream_t stream);
 
 // Local pass of mode 1: out = h * rinv[row] * gamma.

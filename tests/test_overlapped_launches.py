@@ -38,3 +38,12 @@ def test_blocks_of_a_cluster_have_started_before_one_writes_to_another():
         text = _definition(open(os.path.join(KERNELS, name)).read(), head)
         met, wrote = text.index("cluster_sync_all()"), re.search(r"mapa_shared|shared::cluster", text).start()
         assert met < text.index("grid_dependency_wait()") and met < wrote, name
+
+
+def test_no_binding_goes_on_to_another_kernel_after_an_error():
+    """Which kernel a call takes is asked before the launch (tpDecodeLocalCovers), so that an error of the launch itself reaches the
+    caller: none can be provoked without a fault."""
+    folder = os.path.join(ROOT, "mscclpp_b200", "csrc", "bindings")
+    for name in sorted(os.listdir(folder)):
+        assert not re.search(r"[!=]=\s*cudaError", open(os.path.join(folder, name)).read()), name
+    assert "tpDecodeLocalCovers(" in open(os.path.join(folder, "more.cpp")).read()
