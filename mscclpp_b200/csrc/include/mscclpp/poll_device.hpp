@@ -130,11 +130,14 @@ MSCCLPP_DEVICE_INLINE bool waitGreaterEqualBackoff(const uint32_t* p, uint32_t e
 // Bounded mbarrier wait for the hot loops of a pipeline: the common case (the phase has completed, or completes within
 // the hardware's own try_wait window) costs one instruction and touches nothing else. `abortFlag` (shared memory, may
 // be null) is looked at only while actually waiting. false = gave up or aborted.
+// kTmem: the wait for ptx::mbar_arrive_tmem_read, which orders accesses to tensor memory alone.
+template <bool kTmem = false>
 MSCCLPP_DEVICE_INLINE bool mbarWaitFast(uint64_t* bar, uint32_t parity, DeviceStatus* st, uint64_t budgetNs, uint32_t where,
                                         const volatile uint32_t* abortFlag) {
-  if (ptx::mbar_try_wait(bar, parity)) return true;
+  auto through = [&] { return kTmem ? ptx::mbar_try_wait_tmem(bar, parity) : ptx::mbar_try_wait(bar, parity); };
+  if (through()) return true;
   SpinGuard g(st, budgetNs);
-  while (!ptx::mbar_try_wait(bar, parity)) {
+  while (!through()) {
     if (abortFlag != nullptr && *abortFlag != 0) return false;
     if (!g.keepSpinning()) {
       g.report(kDevTimeoutMbarrier, 0, where, 0, parity, 0);

@@ -47,3 +47,19 @@ def test_no_binding_goes_on_to_another_kernel_after_an_error():
     for name in sorted(os.listdir(folder)):
         assert not re.search(r"[!=]=\s*cudaError", open(os.path.join(folder, name)).read()), name
     assert "tpDecodeLocalCovers(" in open(os.path.join(folder, "more.cpp")).read()
+
+
+def test_signals_between_blocks_of_a_cluster_have_its_scope():
+    """An arrive on another block's barrier without a scope is one at CTA scope, which orders nothing between the two."""
+    include = os.path.join(ROOT, "mscclpp_b200", "csrc", "include", "mscclpp")
+    texts = [open(os.path.join(folder, name)).read() for top in (include, KERNELS) for folder, _, names in os.walk(top) for name in names
+             if name.endswith((".cuh", ".cu", ".hpp"))]
+    arrives = [m for text in texts for m in re.findall(r'"mbarrier\.arrive[^"]*shared::cluster[^"]*"', text)]
+    assert arrives and all(re.search(r"\.(release|relaxed)\.cluster\.", a) for a in arrives), arrives
+    # a relaxed one stands between the two fences of tensor memory
+    core = re.sub(r"//[^\n]*", "", open(os.path.join(KERNELS, "gemm2_sm100.cuh")).read())
+    assert re.search(r"mbarWaitFast<true>\(&st\.tmemEmpty.*?\n\s*if \(!ok\) break;\n\s*ptx::tcgen05_fence_after_sync\(\)", core)
+    for name in ("tp_wave.cu", "tp_fused.cu", "gemm_sm100.cuh"):
+        text = open(os.path.join(KERNELS, name)).read()
+        assert len(re.findall(r"arriveEmpty\(\);", text)) == len(re.findall(
+            r"tcgen05_fence_before_sync\(\);\s*__syncwarp\(\);\s*if \(lane == 0\) arriveEmpty\(\);", text)) > 0, name
