@@ -220,6 +220,7 @@ void registerMoreBindings(py::module_& m) {
       },
       py::arg("heap"), py::arg("a"), py::arg("b"), py::arg("residual"), py::arg("h"), py::arg("out"), py::arg("gamma"), py::arg("parts"),
       py::arg("counters"), py::arg("m"), py::arg("n"), py::arg("k"), py::arg("eps") = 1e-5f, py::arg("stream") = 0);
+  m.def("tp_layer_wave_fits", [](int N) { return tpLayerWaveFits(N); }, py::arg("n"));
   m.def("tp_layer_wave_counter_words", [](int M) { return tpLayerWaveCounterWords(M); }, py::arg("m"));
   m.def(
       "tp_scale_rows_from_sumsq",

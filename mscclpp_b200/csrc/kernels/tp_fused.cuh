@@ -97,6 +97,7 @@ cudaError_t launchTpLocalFused(const void* A, const void* B, const void* residua
 // tp_wave.cu): M >= 256, N % 256 == 0, at most as many 256-column tiles per row as pairs of SMs that run at the same time.
 // parts: M rounded up to 256 rows x N / 128 floats, never cleared; counters: tpLayerWaveCounterWords(M) words, zero before the
 // first launch and left zero by every launch. Launches that may run at the same time want their own of both.
+bool tpLayerWaveFits(int N);  // ... on the current device, with the SMs that this process has
 size_t tpLayerWaveCounterWords(int M);
 cudaError_t launchTpLayerWave(const void* A, const void* B, const void* residual, void* h, void* out, const void* gamma, float* parts,
                               uint32_t* counters, int M, int N, int K, float eps, DeviceStatus* status, uint64_t budgetNs, cudaStream_t stream);

@@ -325,6 +325,8 @@ int residentPairs() {
   std::lock_guard<std::mutex> lock(mu);
   auto it = known.find(dev);
   if (it != known.end()) return it->second;
+  const void* kernel = reinterpret_cast<const void*>(tpLayerWaveKernel);
+  if (gemm::ensureDynamicSmem(kernel, ConfigWave::kSmemBytes) != cudaSuccess) return 0;  // (the query fails without it)
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2);
   cfg.blockDim = dim3(kWaveThreads);
@@ -336,12 +338,14 @@ int residentPairs() {
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, reinterpret_cast<const void*>(tpLayerWaveKernel), &cfg) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) return 0;
   known[dev] = n;
   return n;
 }
 
 }  // namespace
+
+bool tpLayerWaveFits(int N) { return N > 0 && N % ConfigWave::kBlockN == 0 && N / ConfigWave::kBlockN <= residentPairs(); }
 
 size_t tpLayerWaveCounterWords(int M) { return 1 + 2 * static_cast<size_t>((M + ConfigWave::kPairM - 1) / ConfigWave::kPairM); }
 
@@ -361,10 +365,8 @@ cudaError_t launchTpLayerWave(const void* A, const void* B, const void* residual
   if (e == cudaSuccess) e = gemm::ensureDynamicSmem(kernel, ConfigWave::kSmemBytes);
   if (e != cudaSuccess) return e;
   const int tiles = ((M + ConfigWave::kPairM - 1) / ConfigWave::kPairM) * (N / ConfigWave::kBlockN);
+  if (!tpLayerWaveFits(N)) return cudaErrorInvalidValue;  // a row block has to fit two consecutive waves
   int pairs = residentPairs();
-  if (pairs < 1) return cudaErrorCooperativeLaunchTooLarge;
-  if (N / ConfigWave::kBlockN > pairs) return cudaErrorInvalidValue;  // a row block has to fit two consecutive waves
-  if (N / ConfigWave::kBlockN > pairs) return cudaErrorInvalidValue;  // a row block has to fit two consecutive waves
   if (pairs > tiles) pairs = tiles;
   WaveArgs args{static_cast<bf16*>(out), static_cast<const bf16*>(gamma), parts, counters, residual != nullptr, eps, status, budgetNs};
   void* params[] = {&ta, &tb, &tr, &th, &shape, &args};

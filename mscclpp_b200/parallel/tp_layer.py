@@ -190,7 +190,8 @@ class RowParallelLinearNorm:
         # the rows' sums of squares travel in parts ([parts][t] floats, nothing to clear); launches on disjoint row ranges
         # use disjoint pieces of the buffer
         per_row = self.out_features // 64
-        if one_kernel is None and two_sm is None and timeline is None and probe == 0 and self._wave_form(t, self.out_features, self.k_shard):
+        if (one_kernel is None and two_sm is None and timeline is None and probe == 0 and self._wave_form(t, self.out_features, self.k_shard)
+                and n.tp_layer_wave_fits(self.out_features)):
             n.tp_layer_wave(self.symm.heap, x.data_ptr(), self.weight.data_ptr(), self.residual_in[rows].data_ptr(),
                             self.residual_out[rows].data_ptr(), self.out[rows].data_ptr(), self.gamma.data_ptr(),
                             self._parts()[row_offset * per_row:].data_ptr(), self._wave_counters[row_offset:].data_ptr(), t,

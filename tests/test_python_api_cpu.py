@@ -471,6 +471,41 @@ def test_forward_local_forms_by_arguments(monkeypatch):
     assert launched(513, timeline=stamps) == two
 
 
+def test_forward_local_long_prompts_fall_back_to_two_launches(monkeypatch):
+    """Where fewer pairs of SMs run at the same time than a row has tiles (a process that has part of a GPU), the form that holds h
+    on chip cannot run and the two launches are taken."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from mscclpp_b200._core import native as native_module
+    from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
+
+    calls, pairs = [], []
+
+    class FakeNative:
+        def __getattr__(self, name):
+            def call(*args):
+                calls.append(name)
+                return args[0] // 256 <= pairs[-1] if name == "tp_layer_wave_fits" else 1
+            return call
+
+    monkeypatch.setattr(native_module, "load", lambda: FakeNative())
+    layer = object.__new__(RowParallelLinearNorm)
+    layer.symm = SimpleNamespace(world=1, device="cpu", heap=None)
+    t, n, k = 1537, 8192, 1024
+    layer.out_features, layer.k_shard, layer.max_tokens, layer.eps = n, k, t, 1e-5
+    layer.residual_in = layer.residual_out = layer.out = torch.zeros((t, n), dtype=torch.bfloat16)
+    layer.weight, layer.gamma = torch.zeros((n, k), dtype=torch.bfloat16), torch.ones((n,), dtype=torch.bfloat16)
+    layer._local_ws = layer._sumsq_parts = None
+    layer._wave_counters = torch.zeros((t,), dtype=torch.int32)
+    for have, launched in ((74, ["tp_layer_wave"]), (32, ["tp_layer_wave"]), (31, ["gemm_residual_sumsq", "tp_scale_rows_from_sumsq"])):
+        calls.clear()
+        pairs.append(have)
+        layer.forward_local(torch.zeros((t, k), dtype=torch.bfloat16), stream=SimpleNamespace(cuda_stream=0))
+        assert [name for name in calls if name != "tp_layer_wave_fits"] == launched
+
+
 def test_forward_local_long_prompts_by_size():
     """The line between two launches and the one-launch form for long prompts: 222 tiles of 256 x 256 and 1024 reduction elements."""
     from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
