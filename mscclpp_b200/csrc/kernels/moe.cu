@@ -16,7 +16,7 @@
 //   No staging buffer and no second pass. With fp8 = 1 the expert outputs are e4m3 with 1 x 128 scales (quantised by
 //   the expert GEMM's epilogue or by launchMoeQuantizeRows), half the bytes over NVLink.
 // With one rank there is nobody to exchange counts with or to wait for: neither launch is cooperative, both overlap the kernel
-// before them, and every block of the dispatch counts all pairs by itself (up to 16384 of them). Dispatch and combine together
+// before them, and every block of the dispatch counts all pairs by itself (up to 8192 of them). Dispatch and combine together
 // on one B200, before / now: 4096 tokens x 4096 bf16, top-2 of 64 experts 51 / 42 us (201 MB, 4.8 TB/s), 777 tokens x 7168
 // fp8, top-8 of 256 experts 39 / 33 us.
 // With several ranks both end with a cross-rank barrier: after dispatch returns every row sent to this rank has landed; after combine

@@ -410,6 +410,12 @@ TEST(RangeAllocator, FirstFitReleaseAndCoalescing) {
   EXPECT_EQ(r.allocate(0), RangeAllocator::npos);
 }
 
+// From 12288 pairs on, counting them in every block takes longer than the exchange that it replaces.
+TEST(MoeDispatch, BlocksCountFewPairsOfOneRankAlone) {
+  EXPECT_EQ(moeCountsAlone(1, 1024, 8) && moeCountsAlone(1, 4096, 2) && moeCountsAlone(1, 0, 8), true);
+  EXPECT_EQ(moeCountsAlone(1, 1025, 8) || moeCountsAlone(1, 2048, 8) || moeCountsAlone(2, 4, 2) || moeCountsAlone(1, (1 << 24) - 1, 32), false);
+}
+
 // A dispatch block that gives up marks its own tokens as not sent while other blocks, which got through, read the positions of
 // theirs: the blocks' shares of the tokens cover each one once, and a position that marks "not sent" leads to no row.
 TEST(MoeDispatch, BlocksShareNoTokenAndRowsStayInTheBuffer) {

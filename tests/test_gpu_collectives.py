@@ -650,7 +650,7 @@ def test_moe_one_rank(tokens, hidden, experts, topk, fp8):
     symm.destroy()
 
 
-@pytest.mark.parametrize("tokens,topk,n_blocks", [(4096, 4, 0), (4097, 4, 0), (2, 2, 0), (1000, 8, 7)])
+@pytest.mark.parametrize("tokens,topk,n_blocks", [(4096, 4, 0), (4097, 4, 0), (2048, 4, 0), (2049, 4, 0), (2, 2, 0), (1000, 8, 7)])
 def test_moe_one_rank_counts(tokens, topk, n_blocks):
     """Either side of the line up to which every block of a one-rank dispatch counts all pairs; fewer tokens than blocks, few blocks;
     every token routed to the same experts, and ids that name no expert."""
