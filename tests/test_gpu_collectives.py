@@ -684,6 +684,66 @@ def test_moe_one_rank_counts(tokens, topk, n_blocks):
     symm.destroy()
 
 
+@pytest.mark.parametrize("tokens,topk", [(3, 2), (1000, 8), (4096, 2), (1100, 8)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_moe_one_rank_chain(tokens, topk, fp8):
+    """Dispatch and combine of one batch right behind those of another: each launch overlaps the one before it, which may still read or
+    write the received rows, the slots and the counts. Without waiting, eagerly and from a graph, the same bits as one by one. (1100 x 8:
+    the dispatch that does not overlap, between combines that do.)"""
+    from mscclpp_b200 import SymmetricMemory
+    from mscclpp_b200.parallel.moe import ExpertParallelDispatcher
+
+    hidden, experts = 2048, 64
+    symm = SymmetricMemory.emulated(1, nbytes=tokens * topk * hidden * 8 + tokens * hidden * 12 + (64 << 20), timeout_ms=3000)
+    disp = ExpertParallelDispatcher(symm, num_experts=experts, hidden=hidden, max_tokens=tokens, topk=topk, capacity=tokens * topk, fp8=fp8, fp8_combine=fp8)
+    if fp8:
+        disp.expert_out_q, disp.expert_out_scales = disp.recv_x, disp.recv_scales
+    else:
+        disp.expert_out = disp.recv_x
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    batches = []
+    for _ in range(3):
+        x = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+        idx = torch.rand((tokens, experts), generator=g, device="cuda").topk(topk, dim=1).indices.to(torch.int32)
+        batches.append((x, idx, torch.rand((tokens, topk), generator=g, device="cuda"), symm.tensor((tokens, hidden), torch.bfloat16)))
+
+    def run(each=lambda: None):
+        for x, idx, weights, y in batches:
+            slots = disp.dispatch(x, idx)[2]
+            each()
+            disp.combine(idx, weights, slots, out=y)
+            each()
+
+    def results():
+        torch.cuda.synchronize()
+        symm.check()
+        got = [y.clone() for *_, y in batches] + [disp.recv_counts.clone()]
+        for *_, y in batches:
+            y.fill_(float("nan"))
+        disp.recv_counts.zero_()
+        torch.cuda.synchronize()
+        return got
+
+    run(torch.cuda.synchronize)
+    expect = results()
+    assert all(bool(torch.isfinite(e).all()) for e in expect)
+    for _ in range(5):
+        run()
+        assert all(torch.equal(a, b) for a, b in zip(results(), expect))
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        with torch.cuda.graph(graph, stream=side):
+            run()
+    torch.cuda.current_stream().wait_stream(side)
+    for _ in range(5):
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(results(), expect))
+    del graph
+    symm.destroy()
+
+
 @pytest.mark.parametrize("offset", [0, 8])
 @pytest.mark.parametrize("tokens,hidden,topk", [(3, 256, 1), (70, 768, 3), (160, 2304, 8)])
 def test_moe_dispatch_fp8_rows_at_eight_byte_offsets(tokens, hidden, topk, offset):
