@@ -217,7 +217,7 @@ struct LayerRows {
           published++;
           continue;
         }
-        if (published > it && ptx::ld_acquire_gpu(counters + mBlk) >= static_cast<uint32_t>(perRow)) break;
+        if (published > it && static_cast<int32_t>(ptx::ld_acquire_gpu(counters + mBlk)) >= perRow) break;
         if (!guard.keepSpinning()) {
           guard.report(kDevTimeoutFlag, 0, 470, mBlk, perRow, published);
           return;  // the scale warps' wait for this tile runs out too

@@ -170,6 +170,110 @@ def test_single_gpu_layer_in_waves(tokens, hidden, k):
     symm.destroy()
 
 
+def test_single_gpu_layer_default_forms_in_a_chain():
+    """forward_local as it is called, no form forced: long prompts in one launch between shorter ones in two, all reading what the
+    launch before wrote; pieces of the rows with an offset; without waiting the same bits as one by one. Against fp64 at the end."""
+    from mscclpp_b200 import SymmetricMemory, native
+    from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
+
+    size, short, long = 2048, 1280, 28 * 256 + 37  # 8 tiles a row block: 40 tiles, 232 tiles
+    total = short + long
+    assert native().tp_layer_wave_fits(8192) and not RowParallelLinearNorm._wave_form(short, size, size)
+    assert RowParallelLinearNorm._wave_form(long, size, size) and RowParallelLinearNorm._wave_form(total, size, size)
+    symm = SymmetricMemory.emulated(1, nbytes=3 * total * size * 8 + (64 << 20), timeout_ms=3000)
+    layers = [RowParallelLinearNorm(symm, out_features=size, k_shard=size, max_tokens=total, seed=i) for i in range(3)]
+    g = torch.Generator(device="cuda").manual_seed(11)
+    for layer in layers:
+        layer.out.zero_()
+        layer.residual_out.zero_()
+        layer.residual_in.copy_(torch.randn((total, size), generator=g, device="cuda"))
+    layers[1].residual_in, layers[2].residual_in = layers[0].residual_out, layers[1].residual_out
+    x = torch.randn((total, size), generator=g, device="cuda").to(torch.bfloat16)
+
+    def step(i, rows, src):
+        return lambda: layers[i].forward_local(src[rows], row_offset=rows.start)
+
+    first, rest, every = slice(0, short), slice(short, total), slice(0, total)
+    chain = [step(0, first, x), step(0, rest, x), step(1, every, layers[0].out), step(2, rest, layers[1].out), step(2, first, layers[1].out)]
+    _same_without_waiting(chain, [t for layer in layers for t in (layer.out, layer.residual_out)])
+    symm.check()
+    assert not any(bool(layer._wave_counters.any()) for layer in layers)
+    for launch in chain:
+        launch()
+    torch.cuda.synchronize()
+    rows = torch.randint(0, total, (300,), generator=g, device="cuda")
+    src, residual = x, layers[0].residual_in
+    for layer in layers:
+        p = src[rows].double() @ layer.weight.double().t()
+        h, got = p + residual[rows].double(), layer.residual_out[rows].double()
+        slack = (src[rows].double().abs() @ layer.weight.double().abs().t()) * size * 2.0 ** -24 + p.abs() * 2.0 ** -8 + h.abs() * 2.0 ** -8
+        assert bool(((got - h).abs() <= slack).all())
+        y = got * torch.rsqrt(got.square().mean(-1, keepdim=True) + layer.eps)
+        assert bool(((layer.out[rows].double() - y).abs() <= y.abs() * 2.0 ** -8).all())
+        src, residual = layer.out, layer.residual_out
+    symm.destroy()
+
+
+def test_single_gpu_layer_in_waves_from_host_memory():
+    """forward_from_host in pieces that are long prompts themselves (row offsets into the parts and the counters)."""
+    from mscclpp_b200 import SymmetricMemory
+    from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
+
+    tokens, hidden, k = 2 * 1792 + 5, 8192, 1024  # 7 row blocks x 32 tiles in each of two pieces, a piece of five rows behind them
+    assert RowParallelLinearNorm._wave_form(1792, hidden, k)
+    symm = SymmetricMemory.emulated(1, nbytes=tokens * hidden * 8 + (64 << 20), timeout_ms=3000)
+    layer = RowParallelLinearNorm(symm, out_features=hidden, k_shard=k, max_tokens=tokens)
+    layer.residual_in.normal_()
+    x = torch.randn((tokens, k)).to(torch.bfloat16).pin_memory()
+    layer.forward_from_host(x, chunks=3)
+    torch.cuda.synchronize()
+    got = layer.out.clone(), layer.residual_out.clone()
+    layer.out.zero_()
+    layer.residual_out.zero_()
+    layer.forward_local(x.cuda(), one_kernel=False)
+    torch.cuda.synchronize()
+    symm.check()
+    assert torch.equal(got[1], layer.residual_out)
+    # two orders of the rows' sums: 1/rms to fp32 rounding, `out` to one bf16 rounding
+    assert bool(((got[0].double() - layer.out.double()).abs() <= layer.out.double().abs() * 2.0 ** -7).all())
+    symm.destroy()
+
+
+def test_single_gpu_layer_in_waves_gives_up():
+    """A row block that is never complete (its counter starts below zero): the waits for it run out, the launch ends, the status says
+    so, the counters are zero again and the next launch is right. One tile per pair of SMs, so that nothing is in flight when
+    the waits run out."""
+    from mscclpp_b200 import SymmetricMemory, native
+
+    n = native()
+    tokens, hidden, k = 1024, 1024, 128
+    x, w, r = (torch.randn(s, device="cuda").to(torch.bfloat16) for s in ((tokens, k), (hidden, k), (tokens, hidden)))
+    parts = torch.empty((tokens * hidden // 128,), device="cuda")
+    counters = torch.zeros((n.tp_layer_wave_counter_words(tokens),), dtype=torch.int32, device="cuda")
+
+    def launch(symm):
+        out, h = torch.zeros_like(r), torch.zeros_like(r)
+        n.tp_layer_wave(symm.heap, x.data_ptr(), w.data_ptr(), r.data_ptr(), h.data_ptr(), out.data_ptr(), 0, parts.data_ptr(), counters.data_ptr(),
+                        tokens, hidden, k, 1e-5, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        return out, h
+
+    symm = SymmetricMemory.emulated(1, nbytes=64 << 20, timeout_ms=50)
+    counters[1 + 3] = -1  # 128-row block 3
+    launch(symm)
+    with pytest.raises(Exception):
+        symm.check()
+    assert not bool(counters.any())
+    symm.destroy()
+    symm = SymmetricMemory.emulated(1, nbytes=64 << 20, timeout_ms=3000)
+    out, h = launch(symm)
+    symm.check()
+    p = x.double() @ w.double().t()
+    assert bool(((h.double() - p - r.double()).abs() <= (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24 + p.abs() * 2.0 ** -8 + h.double().abs() * 2.0 ** -7).all())
+    assert bool(torch.isfinite(out).all())
+    symm.destroy()
+
+
 @pytest.mark.parametrize("rows,n,parts", [(1, 8, 1), (3, 72, 2), (445, 1000, 5), (444 * 32 + 7, 256, 4), (900, 8192, 64), (37, 16392, 128)])
 def test_scale_pass_sizes(rows, n, parts):
     """out = h * rsqrt(sum of the row's parts / n + eps) * gamma at the edges of the pass: rows of less than a warp's words,
