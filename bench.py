@@ -142,7 +142,7 @@ def main():
     import torch
     import torch.distributed as dist
 
-    from mscclpp_b200 import SymmetricMemory
+    from mscclpp_b200 import SymmetricMemory, native
     from mscclpp_b200.ops import all_reduce
     from mscclpp_b200.ops.gemm import pick_block_n
     from mscclpp_b200.parallel.tp_layer import RowParallelLinearNorm
@@ -213,8 +213,8 @@ def main():
         return time_steps(graph.replay, 5, 2) / reps
 
     # ------------------------------------------------------------------ values first: the layer against an fp32 PyTorch reference
-    def verify(t_check, fn, label):
-        """fn() runs the layer on xs_check; every rank compares the result with the fp32 composition of ALL ranks' shards."""
+    def verify(t_check, fn, label, x_check):
+        """fn() runs the layer on x_check; every rank compares the result with the fp32 composition of ALL ranks' shards."""
         out, res = fn()
         torch.cuda.synchronize()
         symm.check()
@@ -242,6 +242,8 @@ def main():
     # ------------------------------------------------------------------ pick the fused variant (untimed)
     # variant = (mode, nvls, reducer CTAs, GEMM core): core 1 = one-SM tiles, 2 = 256 x 256 tiles on SM pairs (cta_group::2)
     def fused(t, mode, nvls, reducers, core=1):
+        if mode == -5:  # one GPU: the form that the layer picks itself
+            return lambda: layer.forward_local(xs[t])
         if mode == -4:  # up to 8 tokens: weight-streaming slabs + one-shot packet allreduce + residual + norm, one launch
             return lambda: layer.forward_decode(xs[t], nvls=nvls)
         if mode in (-2, -3):  # one GPU: GEMM whose epilogue adds the residual and sums the squares; the normalisation as a
@@ -265,7 +267,8 @@ def main():
     if world > 4 and symm.nvls:  # plain peer loads/stores for comparison
         variants += [(m, False, r, 2) for m in (1, 3) for r in (32, 64)]
     if world == 1:
-        variants = [(1, False, 64, 1), (-1, False, 0, 1), (-2, False, 0, 1), (-2, False, 0, 2), (-3, False, 0, 1), (-3, False, 0, 2)]
+        variants = [(1, False, 64, 1), (-1, False, 0, 1), (-2, False, 0, 1), (-2, False, 0, 2), (-3, False, 0, 1), (-3, False, 0, 2),
+                    (-5, False, 0, 1)]
     best = {}
     tune_scores = {}
     for t in TOKEN_SIZES:
@@ -287,6 +290,8 @@ def main():
         mode, nvls, reducers, core = v
         if mode == -4:
             return layer.forward_decode(x, nvls=nvls)
+        if mode == -5:
+            return layer.forward_local(x)
         if mode in (-2, -3):
             return layer.forward_local(x, two_sm=(core == 2 and x.shape[0] >= 256), one_kernel=(mode == -3))
         if mode < 0:
@@ -294,10 +299,12 @@ def main():
         return layer.forward_fused(x, mode=mode, nvls=nvls, num_reducers=reducers,
                                    block_n=-1 if (core == 2 and x.shape[0] >= 256) else pick_block_n(x.shape[0], HIDDEN))
 
-    value_check["headline_variant_T256"] = verify(T_CHECK, lambda: run_variant(x_check, best[HEADLINE_T]), "the headline variant")
+    value_check["headline_variant_T256"] = verify(T_CHECK, lambda: run_variant(x_check, best[HEADLINE_T]), "the headline variant", x_check)
+    if best[HEADLINE_T][0] == -5:  # (which takes another form for long prompts)
+        value_check["headline_variant_T2048"] = verify(2048, lambda: layer.forward_local(xs[2048]), "the headline variant", xs[2048])
     value_check["end_to_end_path_T256"] = verify(
         T_CHECK, lambda: layer.forward_from_host(x_check.cpu().pin_memory(), chunks=1, **fused_kwargs(best[HEADLINE_T], T_CHECK)),
-        "the end-to-end path")
+        "the end-to-end path", x_check)
 
     # ------------------------------------------------------------------ headline: fused TP layer at T = 8192
     sampler = ClockSampler(local_rank if "CUDA_VISIBLE_DEVICES" not in os.environ else
@@ -309,7 +316,8 @@ def main():
     ms_per_step = time_steps(head_fn, args.steps, max(args.warmup, 3))
     # kernels of this library per step: the one-kernel paths (fused modes 0 and 3, the single-GPU layer) launch 1, fused mode 1
     # adds its local scale pass, the unfused path is GEMM + allreduce/norm kernel
-    launches = args.steps * (1 if head_mode in (0, 3, -3) else 2)
+    waves = head_mode == -5 and layer._wave_form(HEADLINE_T, HIDDEN, K_SHARD) and native().tp_layer_wave_fits(HIDDEN)
+    launches = args.steps * (1 if head_mode in (0, 3, -3) or waves else 2)
 
     # ------------------------------------------------------------------ per-T table: eager launches and CUDA-graph replay
     tp_us, tp_graph_us, tp_unfused_us, tp_baseline_us = {}, {}, {}, {}
@@ -456,9 +464,10 @@ def main():
             "tokens_per_s": round(HEADLINE_T / (ms_per_step * 1e-3), 1),
             "aggregate_tflops": round(flops / (ms_per_step * 1e-3) / 1e12, 1),
             "variant": {"mode": head_mode, "nvls": head_nvls, "reducer_ctas": head_reducers,
-                        "gemm_core": "two-SM 256x256 (cta_group::2)" if head_core == 2 else "one-SM 128x256",
-                        "kernel": ("gemmResidualSumsqKernel (tcgen05 GEMM, epilogue adds residual + row sums of squares) then scale pass"
-                                   if head_mode == -2 else
+                        "gemm_core": "two-SM 256x256 (cta_group::2)" if head_core == 2 or waves else "one-SM 128x256",
+                        "kernel": ("tpLayerWaveKernel (tcgen05 GEMM + residual + RMSNorm in one launch, h held on chip)" if waves else
+                                   "gemmResidualSumsqKernel (tcgen05 GEMM, epilogue adds residual + row sums of squares) then scale pass"
+                                   if head_mode in (-2, -5) else
                                    "tpLocalFusedKernel (tcgen05 GEMM + residual + RMSNorm in one launch)" if head_mode == -3 else
                                    "gemmBf16Kernel (tcgen05) then twoShot/LL allreduce+residual+RMSNorm kernel" if head_mode < 0 else
                                    "tpFusedKernel (tcgen05 GEMM + multimem/peer reduce + residual + RMSNorm in one launch)" +
