@@ -1,4 +1,4 @@
-// Packed bf16 arithmetic shared by the kernels of the single-GPU layer.
+// Packed bf16 arithmetic shared by the kernels of the single-GPU layer, and the products of the decode kernels.
 #pragma once
 
 #include <cstdint>
@@ -67,6 +67,17 @@ MSCCLPP_DEVICE_INLINE uint64_t fmaPair(uint64_t a, uint64_t b, uint64_t c) {
 MSCCLPP_DEVICE_INLINE uint32_t packPair(uint64_t p) {
   const float2 f = valuesOf(p);
   return asWord(__floats2bfloat162_rn(f.x, f.y));
+}
+
+// Warp-level tensor-core products of the decode kernels: four 8 x 8 matrices out of shared memory, and
+// D[16 x 8] += A[16 x 16] (row-major) * B[16 x 8] (column-major), bf16 operands, fp32 accumulation.
+MSCCLPP_DEVICE_INLINE void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+MSCCLPP_DEVICE_INLINE void mma_m16n8k16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 }  // namespace mscclpp

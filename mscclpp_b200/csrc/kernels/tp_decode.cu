@@ -32,6 +32,7 @@
 #include <mscclpp/gpu_data_types.hpp>
 #include <mscclpp/packet_device.hpp>
 
+#include "bf16x8.cuh"
 #include "gemm.cuh"
 
 namespace mscclpp {
@@ -51,18 +52,6 @@ constexpr int kSlices = 4;              // warps that share a column group, each
 // {share of the row's sum of squares, epoch} words of the thread blocks: [gridDim.x][kTpDecodeMaxTokens]
 MSCCLPP_DEVICE_INLINE uint2* shareTable(const DeviceComm& c, int rank) {
   return reinterpret_cast<uint2*>(c.peerBase[rank] + c.auxFlagsOff + kTpDecodeAuxOffset);
-}
-
-MSCCLPP_DEVICE_INLINE void ldmatrix_x4(uint32_t (&r)[4], const void* smemRow) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(ptx::smem_u32(smemRow)));
-}
-// D[16 x 8] += A[16 x 16] (row-major) * B[16 x 8] (column-major), bf16 operands, fp32 accumulation
-MSCCLPP_DEVICE_INLINE void mma_m16n8k16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 template <bool kNvls>
@@ -178,7 +167,7 @@ __global__ void __launch_bounds__(kThreads, 1) tpDecodeKernel(TpDecodeArgs a) {
         for (int kk = 0; kk < kChunkK / kSlices; kk += 16) {
           if (k0 + kk < len) {
             uint32_t af[4];
-            ldmatrix_x4(af, rowBase + (k0 + kk + aKoff) * 2);
+            ldmatrix_x4(af, ptx::smem_u32(rowBase + (k0 + kk + aKoff) * 2));
             const bf16* xb = xLane + ch * kChunkK + k0 + kk;
             mma_m16n8k16(acc, af, *reinterpret_cast<const uint32_t*>(xb), *reinterpret_cast<const uint32_t*>(xb + 8));
           }

@@ -45,10 +45,11 @@ class RowParallelLinearNorm:
         self.rinv = symm.tensor((max_tokens,), torch.float32)
         self._local_ws = None  # workspace of the one-kernel single-GPU path, made on first use
         self._sumsq_parts = None  # parts of the rows' sums of squares on their way from the GEMM's epilogue to the norm
-        # counters of the long-prompt form of forward_local: zero before and after every launch (so made here, where no graph is being
-        # captured); a launch on rows [r, r + t) uses words from r on
+        # One rank: words that are zero before and after every launch, so made here, where no graph is being captured. The count and the
+        # rows' shares of forward_decode, and the counters of forward_local's long-prompt form (a launch on rows [r, r + t) uses words
+        # from r on).
         self._decode_ws = torch.zeros((native.load().tp_decode_workspace_words(),), dtype=torch.int32, device=dev) if symm.world == 1 else None
-        self._wave_counters = torch.zeros((max_tokens,), dtype=torch.int32, device=dev)
+        self._wave_counters = torch.zeros((max_tokens,), dtype=torch.int32, device=dev) if symm.world == 1 else None
         self.launches_per_forward = 1  # forward_fused, mode 0
 
     def forward(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None, algo: Optional[str] = None,
@@ -160,7 +161,10 @@ class RowParallelLinearNorm:
         of its 256 x 256 tiles ends in an exchange, which only the matrix products of the next wave hide. B200, graph replay, time
         of two launches / of this form by waves of 74 tiles, widths 1024 to 8192: K = 2048 up to 1.5 waves 0.69-1.11, 2-2.7
         0.95-1.08, 3.2-5.4 1.02-1.14, 6.9 and more 1.06-1.19; K = 1024 likewise 0.72-1.12, 0.94-1.08, 1.08-1.20, 1.13-1.25; K = 512
-        0.69-1.08, 0.82-1.00, 0.91-1.10, 0.97-1.05; K = 256 0.71-1.07, 0.79-1.01, 0.89-1.09, 1.01-1.14."""
+        0.69-1.08, 0.82-1.00, 0.91-1.10, 0.97-1.05; K = 256 0.71-1.07, 0.79-1.01, 0.89-1.09, 1.01-1.14. The line in K lies where three
+        waves are even: 2048 x 8192 with K = 768 41.2 us against 41.4, with 896 44.8 against 42.7. It gives away 1.06-1.18 of larger prompts
+        with K from 640 on (8192 x 8192 x 768 141 against 125). Widths above 8192: 10240 and 12288 1.03-1.18, but 16384 0.93-1.00 and 18432
+        0.95, where a row's tiles fill most of a wave and every tile waits for all of it."""
         return t >= 256 and n % 256 == 0 and n <= 8192 and k >= 1024 and (t + 255) // 256 * (n // 256) >= 222
 
     def forward_local(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None, two_sm: Optional[bool] = None,
