@@ -413,6 +413,25 @@ PYBIND11_MODULE(_native, m) {
       py::arg("block_n") = 256, py::arg("num_ctas") = 0, py::arg("status") = 0, py::arg("stream") = 0, py::arg("probe") = 0,
       py::arg("band") = 0);
 
+  // The product in the form that planForm picks (pair_m < 0), or in the one given.
+  m.def(
+      "gemm_bf16_form",
+      [](uintptr_t A, uintptr_t B, uintptr_t D, int M, int N, int K, int ldd, uintptr_t stream, int pairM, int blockN, int split) {
+        const gemm::Form form = pairM < 0 ? gemm::planForm(M, N, K) : gemm::Form{pairM, blockN, split};
+        checkCuda(gemm::gemmBf16Form(reinterpret_cast<const void*>(A), reinterpret_cast<const void*>(B), reinterpret_cast<void*>(D), M, N, K, ldd, form,
+                                     nullptr, reinterpret_cast<cudaStream_t>(stream)),
+                  "gemm_bf16_form");
+      },
+      py::arg("a"), py::arg("b"), py::arg("d"), py::arg("m"), py::arg("n"), py::arg("k"), py::arg("ldd"), py::arg("stream") = 0,
+      py::arg("pair_m") = -1, py::arg("block_n") = 0, py::arg("split") = 1);
+  m.def(
+      "gemm_plan_form",
+      [](int M, int N, int K) {
+        const gemm::Form f = gemm::planForm(M, N, K);
+        return py::make_tuple(f.pairM, f.blockN, f.split);
+      },
+      py::arg("m"), py::arg("n"), py::arg("k"));
+
   m.def(
       "gemm_bf16_two_sm",
       [](uintptr_t A, uintptr_t B, uintptr_t D, int M, int N, int K, int ldd, int numCtas, uintptr_t status, uintptr_t stream, int probe, int band) {

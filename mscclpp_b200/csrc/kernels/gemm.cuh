@@ -50,11 +50,25 @@ cudaError_t gemmBf16(const void* A, const void* B, void* D, int M, int N, int K,
 cudaError_t gemmBf16TwoSm(const void* A, const void* B, void* D, int M, int N, int K, int ldd, int numCtas, DeviceStatus* status,
                           cudaStream_t stream, int probe = 0, int band = 0, uint64_t budgetNs = kDefaultBudgetNs);
 
+// How a product is cut up. pairM = 0: tiles of 128 rows x blockN columns on one SM; split = 4 (tiles of 64 columns): shared by a cluster of
+// four CTAs, each with its part of K (at least 256). pairM = 128 or 256: tiles of that many rows on pairs of SMs (256 x 256, 128 x 256 or
+// 128 x 128).
+struct Form {
+  int pairM, blockN, split;
+};
+// The form that gemm_bf16 takes where the caller asks for none, and the product in a given one. N % 64 == 0, K % 64 == 0. N need not be a
+// multiple of the tile.
+Form planForm(int M, int N, int K);
+cudaError_t gemmBf16Form(const void* A, const void* B, void* D, int M, int N, int K, int ldd, Form form, DeviceStatus* status, cudaStream_t stream,
+                         uint64_t budgetNs = kDefaultBudgetNs);
+
 // Raises the kernel's dynamic shared-memory limit once per (kernel, device); call before every launch that needs > 48 KB.
 cudaError_t ensureDynamicSmem(const void* kernel, int bytes);
 
-// Launch helper for kernels built on the two-SM core: clusters of two CTAs along x, optionally cooperative. overlapped: see
-// launchOverlapped (not for cooperative launches).
+// Launch helpers for kernels of clusters of `ctas` CTAs (two) along x, optionally cooperative. overlapped: see launchOverlapped
+// (not for cooperative launches).
+cudaError_t launchClusters(const void* kernel, int ctas, dim3 grid, dim3 block, size_t smemBytes, void** params, bool cooperative,
+                           cudaStream_t stream, bool overlapped = false);
 cudaError_t launchClusterPair(const void* kernel, dim3 grid, dim3 block, size_t smemBytes, void** params, bool cooperative,
                               cudaStream_t stream, bool overlapped = false);
 

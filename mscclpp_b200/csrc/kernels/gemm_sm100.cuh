@@ -45,20 +45,34 @@ constexpr int kNumEpilogueThreads = kNumEpilogueWarps * 32;
 constexpr int kNumThreads = 64 + kNumEpilogueThreads;  // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2-9: epilogue
 constexpr int kStagingBytesPerWarp = 32 * 128;  // 32 rows x 64 bf16 columns
 constexpr int kEpilogueStagingBytes = kNumEpilogueWarps * kStagingBytesPerWarp;
+constexpr int kPartBytes = 32 * 64 * 4;  // a 32-row x 64-column block of the accumulator on its way to the CTA that finishes it
 
-template <int kBlockN>
+// kSplit > 1: a cluster of kSplit CTAs shares one tile, each with its part of the reduction (see splitEpilogueTile).
+template <int kBlockN, int kSplit = 1>
 struct Config {
+  // k blocks per stage. The two threads that feed the tensor core spend 135 ns on a stage even without its loads and products, however many
+  // stages there are. Two k blocks instead of one: 128 x 4096 in tiles of 64 columns 186 -> 146 ns per k block. Wider tiles are left
+  // with too few stages: 128 columns 184 -> 173 ns with few SMs busy, but 266 -> 281 with all of them.
+  static constexpr int kKb = kBlockN == 64 ? 2 : 1;
   static_assert(kBlockN == 64 || kBlockN == 128 || kBlockN == 256, "unsupported N tile");
   static constexpr int kStageABytes = kBlockM * kBlockK * 2;
   static constexpr int kStageBBytes = kBlockN * kBlockK * 2;
-  static constexpr int kStageBytes = kStageABytes + kStageBBytes;
-  static constexpr int kStages = kBlockN == 256 ? 4 : (kBlockN == 128 ? 6 : 8);
-  static constexpr int kTmemCols = 2 * kBlockN;  // two accumulator buffers (power of two >= 32)
+  static constexpr int kStageBytes = kKb * (kStageABytes + kStageBBytes);  // A blocks, then B blocks
+  // 32-row x 64-column blocks of the tile, how many of them a CTA of the cluster finishes, and what its peers send it for them
+  static constexpr int kBlocks = 4 * kBlockN / 64;
+  static_assert(kBlocks % kSplit == 0 && (kSplit == 1 || kBlockN == 64), "a CTA finishes whole blocks, a warp sends or finishes one");
+  static constexpr int kOwnBlocks = kBlocks / kSplit;
+  static constexpr int kRecvBytes = (kSplit - 1) * kOwnBlocks * kPartBytes;
+  static constexpr int kStages = (kBlockN == 256 ? 4 : (kBlockN == 128 ? 6 : 8)) / kKb;
+  static constexpr int kTmemCols = (kSplit > 1 ? 1 : 2) * kBlockN;  // two accumulator buffers (power of two >= 32); one tile needs one
   static constexpr int kBarrierBytes = 256;
   // epilogue warps that take part: every warp owns 32 rows (its TMEM lane quarter) x a multiple of 64 columns
   static constexpr int kEpiWarps = kBlockN >= 128 ? kNumEpilogueWarps : 4;
   static constexpr int kColsPerWarp = kBlockN / (kEpiWarps / 4);
-  static constexpr int kSmemBytes = kStages * kStageBytes + kEpilogueStagingBytes + kBarrierBytes + 1024;  // +1024: manual alignment
+  // (where the reduction is split, a CTA has one tile: its blocks are staged in the operand stages, which are done with by then)
+  static constexpr int kStagingBytes = kSplit > 1 ? 0 : kEpilogueStagingBytes;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kRecvBytes + kStagingBytes + kBarrierBytes + 1024;  // +1024: manual alignment
+  static_assert(kSmemBytes <= 227 * 1024 && kEpilogueStagingBytes + kNumEpilogueWarps * kPartBytes <= kStages * kStageBytes, "shared memory of one CTA");
 };
 
 MSCCLPP_DEVICE_INLINE void tileCoord(const Shape& s, int tile, int numMBlk, int numNBlk, int& mBlk, int& nBlk) {
@@ -171,6 +185,30 @@ struct IsRowEpilogue : std::false_type {};
 template <typename E>
 struct IsRowEpilogue<E, std::void_t<decltype(E::kRowEpilogue)>> : std::bool_constant<E::kRowEpilogue> {};
 
+// A warp's 32 x 64 block of the accumulator, packed, into its staging buffer.
+template <typename Epilogue>
+MSCCLPP_DEVICE_INLINE void stageBlock(uint32_t (&v0)[32], uint32_t (&v1)[32], uint8_t* stage, int lane) {
+  // the buffer is free once the bulk store of the previous block has read it (or block() has ended)
+  if constexpr (Epilogue::kBulkStore) {
+    if (lane == 0) ptx::bulk_wait_read<0>();
+  }
+  __syncwarp();
+  if constexpr (IsGatedEpilogue<Epilogue>::value) {
+#pragma unroll
+    for (int i = 0; i < 32; i++) v0[i] = __float_as_uint(Epilogue::gatePair(__uint_as_float(v0[i]), __uint_as_float(v1[i])));
+#pragma unroll
+    for (int c = 0; c < 4; c++) *reinterpret_cast<uint4*>(stage + stagedOffset(lane, c)) = packChunk<Epilogue>(v0, c);
+  } else {
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      *reinterpret_cast<uint4*>(stage + stagedOffset(lane, c)) = packChunk<Epilogue>(v0, c);
+      *reinterpret_cast<uint4*>(stage + stagedOffset(lane, c + 4)) = packChunk<Epilogue>(v1, c);
+    }
+  }
+  if constexpr (Epilogue::kBulkStore) ptx::fence_proxy_async_smem();
+  __syncwarp();
+}
+
 // One epilogue warp, one tile: `taddr` is the TMEM address of the warp's lane quarter at its first column,
 // (row0, col0) the global coordinates of that corner. Calls arriveEmpty() as soon as the warp's last accumulator
 // read has completed, i.e. before the last block is written out.
@@ -197,43 +235,77 @@ MSCCLPP_DEVICE_INLINE void stagedEpilogueTile(Epilogue& epi, uint32_t taddr, uin
       __syncwarp();
       if (lane == 0) arriveEmpty();
     }
-    // the buffer is free once the bulk store of the previous block has read it (or block() has ended)
-    if constexpr (Epilogue::kBulkStore) {
-      if (lane == 0) ptx::bulk_wait_read<0>();
-    }
-    __syncwarp();
-    if constexpr (IsGatedEpilogue<Epilogue>::value) {
-#pragma unroll
-      for (int i = 0; i < 32; i++) v0[i] = __float_as_uint(Epilogue::gatePair(__uint_as_float(v0[i]), __uint_as_float(v1[i])));
-#pragma unroll
-      for (int c = 0; c < 4; c++) *reinterpret_cast<uint4*>(stage + stagedOffset(lane, c)) = packChunk<Epilogue>(v0, c);
-    } else {
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        *reinterpret_cast<uint4*>(stage + stagedOffset(lane, c)) = packChunk<Epilogue>(v0, c);
-        *reinterpret_cast<uint4*>(stage + stagedOffset(lane, c + 4)) = packChunk<Epilogue>(v1, c);
-      }
-    }
-    if constexpr (Epilogue::kBulkStore) ptx::fence_proxy_async_smem();
-    __syncwarp();
+    stageBlock<Epilogue>(v0, v1, stage, lane);
     if (!drop) epi.block(stage, row0, col0 + b * 64, lane, b);
   }
 }
 
-// Body of a GEMM CTA. All 192 threads call it. `ctaIdx`/`numCtas` index the persistent tile loop.
-template <int kBlockN, typename AGate, typename Epilogue>
+// One epilogue warp of a CTA whose cluster shares one tile: every CTA holds the products of its part of the reduction, and each
+// finishes kOwnBlocks of the tile's 32 x 64 blocks. A warp has one block. It either copies it into the shared memory of the CTA that finishes
+// it (fp32, a float4 of every lane next to one another: no bank conflicts on either side; a bulk copy, whose bytes count on the
+// block's barrier there - plain stores to the other CTA and a release took 0.3-0.7 us longer), or it adds what comes for it to its
+// accumulator, in the order of the ranks, and finishes it like any other. Returns false if a part did not come.
+template <int kBlockN, int kSplit, typename Epilogue>
+MSCCLPP_DEVICE_INLINE bool splitEpilogueTile(Epilogue& epi, uint32_t taddr, uint8_t* recv, uint64_t* got, uint8_t* send, uint8_t* stage, int row0,
+                                             int col0, int quarter, int part, int lane, DeviceStatus* status, uint64_t budgetNs) {
+  using Cfg = Config<kBlockN, kSplit>;
+  const int rank = static_cast<int>(ptx::cluster_ctarank());
+  const int block = part * 4 + quarter, owner = block / Cfg::kOwnBlocks, slot = block % Cfg::kOwnBlocks;
+  uint32_t v0[32], v1[32];
+  ptx::tmem_ld_32x32b_x32(taddr + part * 64, v0);
+  ptx::tmem_ld_32x32b_x32(taddr + part * 64 + 32, v1);
+  ptx::tmem_ld_wait();
+  if (owner != rank) {
+    uint4* out = reinterpret_cast<uint4*>(send) + lane;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      out[j * 32] = make_uint4(v0[4 * j], v0[4 * j + 1], v0[4 * j + 2], v0[4 * j + 3]);
+      out[(j + 8) * 32] = make_uint4(v1[4 * j], v1[4 * j + 1], v1[4 * j + 2], v1[4 * j + 3]);
+    }
+    ptx::fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      ptx::bulk_s2cluster(ptx::mapa_shared(ptx::smem_u32(recv) + (slot * (kSplit - 1) + (rank < owner ? rank : rank - 1)) * kPartBytes, owner), send,
+                          kPartBytes, ptx::mapa_shared(ptx::smem_u32(&got[slot]), owner));
+    }
+    return true;
+  }
+  const bool ok = __all_sync(0xffffffffu, mbarWait(&got[slot], 0, status, budgetNs, 460 + slot));
+  if (!ok) return false;
+  const float4* in = reinterpret_cast<const float4*>(recv + slot * (kSplit - 1) * kPartBytes) + lane;
+#pragma unroll
+  for (int s = 0; s < kSplit - 1; s++) {
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      uint32_t* v = j < 8 ? &v0[4 * j] : &v1[4 * j - 32];
+      const float4 p = in[s * (kPartBytes / 16) + j * 32];
+      v[0] = __float_as_uint(__uint_as_float(v[0]) + p.x);
+      v[1] = __float_as_uint(__uint_as_float(v[1]) + p.y);
+      v[2] = __float_as_uint(__uint_as_float(v[2]) + p.z);
+      v[3] = __float_as_uint(__uint_as_float(v[3]) + p.w);
+    }
+  }
+  stageBlock<Epilogue>(v0, v1, stage, lane);
+  epi.block(stage, row0, col0 + part * 64, lane, 0);
+  return true;
+}
+
+// Body of a GEMM CTA. All 192 threads call it. `ctaIdx`/`numCtas` index the persistent tile loop. kSplit > 1: they index clusters of
+// kSplit CTAs, as many as there are tiles.
+template <int kBlockN, typename AGate, typename Epilogue, int kSplit = 1>
 MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* tmapB, Shape shape, int ctaIdx,
                                    int numCtas, AGate& gate, Epilogue& epi, DeviceStatus* status, uint64_t budgetNs,
                                    uint8_t* smemRaw) {
-  using Cfg = Config<kBlockN>;
+  using Cfg = Config<kBlockN, kSplit>;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
   // ---- carve shared memory (tiles need 1024-byte alignment for the 128B swizzle)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
   uint8_t* tiles = smem;
-  uint8_t* staging = smem + Cfg::kStages * Cfg::kStageBytes;  // 1024-byte aligned: every stage is a multiple of 1024 bytes
-  uint64_t* bars = reinterpret_cast<uint64_t*>(staging + kEpilogueStagingBytes);
+  [[maybe_unused]] uint8_t* recv = smem + Cfg::kStages * Cfg::kStageBytes;
+  uint8_t* staging = kSplit > 1 ? tiles : recv;  // 1024-byte aligned: every stage is a multiple of 1024 bytes
+  uint64_t* bars = reinterpret_cast<uint64_t*>(recv + Cfg::kRecvBytes + Cfg::kStagingBytes);
   SharedState st;
   st.full = bars;
   st.empty = bars + Cfg::kStages;
@@ -242,11 +314,17 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
   st.tmemBase = reinterpret_cast<uint32_t*>(bars + 2 * Cfg::kStages + 4);
   st.abortFlag = reinterpret_cast<volatile uint32_t*>(st.tmemBase + 1);
   st.epiArrivals = reinterpret_cast<volatile uint32_t*>(st.tmemBase + 2);
+  [[maybe_unused]] uint64_t* got = bars + 2 * Cfg::kStages + 6;  // [kOwnBlocks] the peers' parts of a block have come
+  static_assert(kSplit == 1 || (2 * Cfg::kStages + 6 + Cfg::kOwnBlocks) * 8 <= Cfg::kBarrierBytes, "barriers");
+  static_assert(kSplit == 1 || (!Epilogue::kNeedsTileBarrier && !IsGatedEpilogue<Epilogue>::value), "the split form finishes single blocks");
 
   const int numMBlk = (shape.M + kBlockM - 1) / kBlockM;
-  const int numNBlk = shape.N / kBlockN;
+  const int numNBlk = (shape.N + kBlockN - 1) / kBlockN;  // (the last tile may reach beyond N: see StoreBf16)
   const int numTiles = numMBlk * numNBlk;
-  const int numKBlk = shape.K / kBlockK;
+  const int numKBlkAll = shape.K / kBlockK;
+  const int split = kSplit > 1 ? static_cast<int>(ptx::cluster_ctarank()) : 0;
+  const int kBlk0 = kSplit > 1 ? numKBlkAll * split / kSplit : 0;  // this CTA's part of the reduction
+  const int kBlkEnd = kSplit > 1 ? numKBlkAll * (split + 1) / kSplit : numKBlkAll;
   unsigned long long* tl = shape.stamps != nullptr ? shape.stamps + static_cast<size_t>(blockIdx.x) * kStampWords : nullptr;
   if (tl != nullptr && threadIdx.x == 0) tl[0] = ptx::globaltimer();
 
@@ -258,6 +336,12 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
     for (int s = 0; s < 2; s++) {
       ptx::mbar_init(&st.tmemFull[s], 1);
       ptx::mbar_init(&st.tmemEmpty[s], Cfg::kEpiWarps);  // one arrival per epilogue warp that takes part
+    }
+    if constexpr (kSplit > 1) {
+      for (int s = 0; s < Cfg::kOwnBlocks; s++) {
+        ptx::mbar_init(&got[s], 1);
+        ptx::mbar_expect_tx(&got[s], (kSplit - 1) * kPartBytes);
+      }
     }
     *st.abortFlag = 0;
     *st.epiArrivals = 0;
@@ -271,6 +355,8 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
   }
   ptx::tcgen05_fence_before_sync();
   __syncthreads();
+  // every CTA of the cluster runs and its barriers exist before a peer writes into its shared memory
+  if constexpr (kSplit > 1) ptx::cluster_sync_all();
   ptx::tcgen05_fence_after_sync();
   const uint32_t tmemBase = *st.tmemBase;
   // everything up to here is this CTA's own: with a programmatic dependent launch it ran under the kernel before
@@ -295,7 +381,7 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
         ok = gate.waitRowBlock(mBlk);
         int aRow;
         const CUtensorMap* tmapARows = gate.tmapA(mBlk, tmapA, aRow);
-        for (int kb = 0; kb < numKBlk && ok; kb++) {
+        for (int kb = kBlk0; kb < kBlkEnd && ok; kb += Cfg::kKb) {
           if (tl != nullptr) {
             const unsigned long long t0 = ptx::globaltimer();
             ok = mbarWaitFast(&st.empty[stage], phase ^ 1u, status, budgetNs, 100 + stage, st.abortFlag);
@@ -305,13 +391,18 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
           }
           if (!ok) break;
           uint8_t* sa = tiles + stage * Cfg::kStageBytes;
-          uint8_t* sb = sa + Cfg::kStageABytes;
+          uint8_t* sb = sa + Cfg::kKb * Cfg::kStageABytes;
           if (shape.probe & 1) {
             ptx::mbar_arrive(&st.full[stage]);
           } else {
-            ptx::mbar_expect_tx(&st.full[stage], shape.aBoxRows * kBlockK * 2 + Cfg::kStageBBytes);
-            ptx::tma_load_2d(sa, tmapARows, kb * kBlockK, aRow, &st.full[stage]);
-            ptx::tma_load_2d(sb, tmapB, kb * kBlockK, nBlk * kBlockN, &st.full[stage]);
+            const int blocks = Cfg::kKb == 1 || kBlkEnd - kb > Cfg::kKb ? Cfg::kKb : kBlkEnd - kb;  // (the last stage may not be full)
+            ptx::mbar_expect_tx(&st.full[stage], blocks * (shape.aBoxRows * kBlockK * 2 + Cfg::kStageBBytes));
+#pragma unroll
+            for (int j = 0; j < Cfg::kKb; j++) {
+              if (j >= blocks) break;
+              ptx::tma_load_2d(sa + j * Cfg::kStageABytes, tmapARows, (kb + j) * kBlockK, aRow, &st.full[stage]);
+              ptx::tma_load_2d(sb + j * Cfg::kStageBBytes, tmapB, (kb + j) * kBlockK, nBlk * kBlockN, &st.full[stage]);
+            }
           }
           armed |= 1u << stage;
           armedParity = (armedParity & ~(1u << stage)) | (phase << stage);
@@ -336,7 +427,7 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
       // The issue loop is ONE thread feeding the tensor core: every instruction in it is on the critical path of the
       // whole SM. Descriptors are formed once and stepped by adds; the common case of each wait is one instruction.
       const uint64_t descA0 = makeSmemDesc(ptx::smem_u32(tiles));
-      const uint64_t descB0 = makeSmemDesc(ptx::smem_u32(tiles) + Cfg::kStageABytes);
+      const uint64_t descB0 = makeSmemDesc(ptx::smem_u32(tiles) + Cfg::kKb * Cfg::kStageABytes);
       constexpr uint64_t kStageStep = Cfg::kStageBytes >> 4;  // a stage, in the descriptor's 16-byte address units
       const bool issue = (shape.probe & 2) == 0;
       int stage = 0;
@@ -356,7 +447,7 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
         if (!ok) break;
         ptx::tcgen05_fence_after_sync();
         const uint32_t tmemD = tmemBase + acc * kBlockN;
-        for (int kb = 0; kb < numKBlk; kb++) {
+        for (int kb = kBlk0; kb < kBlkEnd; kb += Cfg::kKb) {
           if (tl != nullptr) {
             const unsigned long long t0 = ptx::globaltimer();
             ok = mbarWaitFast(&st.full[stage], phase, status, budgetNs, 300 + stage, st.abortFlag);
@@ -370,9 +461,16 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
           const uint64_t descB = descB0 + stage * kStageStep;
           if (issue) {
             // advancing K by 16 elements = 32 bytes inside the 128-byte swizzle row: +2 in the (>>4) address field
-            ptx::tcgen05_mma_f16(tmemD, descA, descB, idesc, kb != 0 ? 1u : 0u);
+            ptx::tcgen05_mma_f16(tmemD, descA, descB, idesc, kb != kBlk0 ? 1u : 0u);
 #pragma unroll
             for (int k = 1; k < kBlockK / kUmmaK; k++) ptx::tcgen05_mma_f16_acc(tmemD, descA + 2 * k, descB + 2 * k, idesc);
+#pragma unroll
+            for (int j = 1; j < Cfg::kKb; j++) {
+              if (kb + j >= kBlkEnd) break;
+#pragma unroll
+              for (int k = 0; k < kBlockK / kUmmaK; k++)
+                ptx::tcgen05_mma_f16_acc(tmemD, descA + j * (Cfg::kStageABytes >> 4) + 2 * k, descB + j * (Cfg::kStageBBytes >> 4) + 2 * k, idesc);
+            }
           }
           ptx::tcgen05_commit(&st.empty[stage]);  // frees the smem stage once these MMAs retire
           if (++stage == Cfg::kStages) {
@@ -400,7 +498,11 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
       const int row0 = mBlk * kBlockM + quarter * 32;
       const int col0 = nBlk * kBlockN + part * Cfg::kColsPerWarp;
       // lets the epilogue put loads it will need (a residual, a bias) in flight while the MMAs of this tile still run
-      epi.tileBegin(row0, col0, lane);
+      if constexpr (kSplit > 1) {
+        if ((part * 4 + quarter) / Cfg::kOwnBlocks == split) epi.tileBegin(row0, col0, lane);
+      } else {
+        epi.tileBegin(row0, col0, lane);
+      }
       const bool stampIt = tl != nullptr && warp == 2 && lane == 0;
       unsigned long long tw0 = 0;
       if (stampIt) tw0 = ptx::globaltimer();
@@ -413,6 +515,11 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
         tw0 = now;
       }
       ptx::tcgen05_fence_after_sync();
+      if constexpr (kSplit > 1) {
+        ok = splitEpilogueTile<kBlockN, kSplit>(epi, tmemBase + (static_cast<uint32_t>(quarter * 32) << 16), recv, got, staging + kEpilogueStagingBytes + (warp - 2) * kPartBytes, stage, row0, nBlk * kBlockN,
+                                                quarter, part, lane, status, budgetNs);
+        break;
+      }
       const uint32_t taddr = tmemBase + (static_cast<uint32_t>(quarter * 32) << 16) + acc * kBlockN + part * Cfg::kColsPerWarp;
       // the accumulator buffer can be overwritten by the MMA warp as soon as every warp has read its part
       stagedEpilogueTile<Cfg::kColsPerWarp>(epi, taddr, stage, row0, col0, lane, [&] { ptx::mbar_arrive(&st.tmemEmpty[acc]); }, shape.probe);
@@ -465,21 +572,24 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
   // ---- teardown: everybody meets, then the allocating warp frees TMEM
   ptx::tcgen05_fence_before_sync();
   __syncthreads();
+  // (a peer may still write into this CTA's shared memory, or this one into a peer's)
+  if constexpr (kSplit > 1) ptx::cluster_sync_all();
   ptx::tcgen05_fence_after_sync();
   if (warp == 1) ptx::tmem_dealloc(tmemBase, Cfg::kTmemCols);
 }
 
 // Plain epilogue: every staged 32 x 64 block leaves with one tiled bulk store (rows beyond M are clipped by the
-// tensor map, whose box is 64 columns x 32 rows with the 128-byte swizzle of the staging layout).
+// tensor map, whose box is 64 columns x 32 rows with the 128-byte swizzle of the staging layout). N is a multiple of 64, not
+// necessarily of the tile: rows of B beyond N are read as zeros, blocks beyond it stay where they are.
 struct StoreBf16 {
   static constexpr bool kNeedsTileBarrier = false;
   static constexpr bool kBulkStore = true;
   const CUtensorMap* tmapD;
-  int M;
+  int M, N;
   MSCCLPP_DEVICE_INLINE static float convert(float x) { return x; }
   MSCCLPP_DEVICE_INLINE void tileBegin(int, int, int) const {}
   MSCCLPP_DEVICE_INLINE void block(const uint8_t* stage, int row0, int col0, int lane, int /*b*/) const {
-    if (lane == 0 && row0 < M) {
+    if (lane == 0 && row0 < M && col0 < N) {
       ptx::tma_store_2d(tmapD, stage, col0, row0);
       ptx::bulk_commit();
     }

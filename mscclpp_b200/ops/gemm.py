@@ -24,8 +24,10 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = No
               stream: Optional[torch.cuda.Stream] = None, two_sm: Optional[bool] = None, probe: int = 0, band: int = 0) -> torch.Tensor:
     """out[M, N] = a[M, K] @ w[N, K]^T  (w in nn.Linear layout: out_features x in_features).
 
-    two_sm: run 256 x 256 tiles on pairs of SMs (tcgen05 cta_group::2); None picks it when the problem has enough
-    such tiles to fill the GPU and no N tile was asked for.
+    Without any of the options below the shape decides how the product is cut up: tiles on single SMs or on pairs of them, of 128 or 256
+    rows, with the reduction split over a cluster of SMs where there are few tiles (gemm::planForm).
+    two_sm: run 256 x 256 tiles on pairs of SMs (tcgen05 cta_group::2); None with another option picks it when the problem has
+    enough such tiles to fill the GPU and no N tile was asked for.
     band: row blocks per band of the tile order (0 = default for the tile shape, -1 = plain column-major walk).
     probe: diagnostics only (the result is then garbage): bit 0 drops the operand loads, bit 1 the MMAs, bit 2 the
     epilogue's stores; timing each shows which of the kernel's three pipelines bounds a shape."""
@@ -38,6 +40,11 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = No
         out = torch.empty((m, nn), dtype=torch.bfloat16, device=a.device)
     assert out.is_contiguous() and out.shape == (m, nn)
     s = (stream or torch.cuda.current_stream()).cuda_stream
+    if two_sm is None and block_n == 0 and num_ctas == 0 and probe == 0 and band == 0:
+        if nn % 64 != 0:
+            raise ValueError("N must be a multiple of 64")
+        n.gemm_bf16_form(a.data_ptr(), w.data_ptr(), out.data_ptr(), m, nn, k, nn, s)
+        return out
     if two_sm is None:
         two_sm = block_n == 0 and nn % 256 == 0 and ((m + 255) // 256) * (nn // 256) >= 74
     if two_sm:

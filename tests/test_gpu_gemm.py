@@ -58,6 +58,40 @@ def test_gemm_two_sm_tiles(m, n, k):
     assert (out.float() - ref).abs().max().item() <= 1e-2 * ref.abs().max().item() + 1e-2
 
 
+# (rows per pair of SMs or 0, columns, CTAs that share a tile)
+FORMS = [(0, 64, 1), (0, 64, 4), (0, 128, 1), (0, 256, 1), (256, 256, 1), (128, 256, 1), (128, 128, 1)]
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("m,n,k", [
+    (1, 64, 256),        # one row, one block of columns
+    (129, 320, 320),     # one row and one block of columns more than tiles have; an odd number of k blocks
+    (77, 192, 576),      # (and of parts of the reduction)
+    (128, 256, 4096),    # the ring of stages many times round
+    (2000, 4160, 192),   # several tiles per SM or pair
+])
+def test_gemm_forms(form, m, n, k):
+    from mscclpp_b200 import native
+
+    if k // 64 < form[2]:
+        pytest.skip("more parts than k blocks")
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randn((m, k), generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn((n, k), generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    buf = torch.full((m * n + 4096,), 7.0, device="cuda", dtype=torch.bfloat16)  # what lies behind the result stays as it is
+    out = buf[:m * n].view(m, n)
+    ref = a.double() @ w.double().t()
+    # one rounding to bf16 (eight significant bits: half a unit in the last place is at most 2^-8 of the value) of an fp32 sum,
+    # whose own error is at most K roundings of the sum of the products' magnitudes
+    bound = ref.abs() * 2.0 ** -8 * 1.01 + (a.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24
+    for rep in range(2):
+        out.fill_(float("nan"))
+        native().gemm_bf16_form(a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, n, torch.cuda.current_stream().cuda_stream, *form)
+        torch.cuda.synchronize()
+        assert bool(((out.double() - ref).abs() <= bound).all())
+    assert bool((buf[m * n:] == 7.0).all())
+
+
 @pytest.mark.parametrize("one_kernel", [True, False])
 @pytest.mark.parametrize("tokens,hidden,k,two_sm", [(200, 1024, 256, False), (1024, 2048, 512, True), (777, 512, 128, False),
                                                     (1, 8192, 1024, False), (2048, 8192, 1024, True), (1333, 2048, 256, True)])

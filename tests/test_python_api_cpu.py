@@ -514,3 +514,21 @@ def test_forward_local_long_prompts_by_size():
     assert wave(1537, 8192, 1024) and wave(8192, 8192, 1024) and wave(14337, 1024, 2048)
     assert not wave(1536, 8192, 1024)  # 192 tiles
     assert not wave(8192, 8192, 960) and not wave(8192, 8200, 1024) and not wave(8192, 8448, 1024) and not wave(255, 8192, 1024)
+
+
+def test_gemm_form_fits_the_shape():
+    """Every shape that gemm_bf16 takes gets a form that exists and that the shape can be cut into."""
+    import random
+
+    import mscclpp_b200
+
+    n = mscclpp_b200.native()
+    forms = {(0, 64, 1), (0, 64, 4), (0, 128, 1), (0, 256, 1), (256, 256, 1), (128, 256, 1), (128, 128, 1)}
+    rng = random.Random(3)
+    picked = set()
+    for _ in range(3000):
+        m, nn, k = round(2 ** rng.uniform(0, 15)), 64 * round(2 ** rng.uniform(0, 10)), 64 * round(2 ** rng.uniform(0, 10))
+        form = n.gemm_plan_form(m, nn, k)
+        assert form in forms and form[2] <= k // 64
+        picked.add(form)
+    assert picked == forms  # none of them is there for nothing
