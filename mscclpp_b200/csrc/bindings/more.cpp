@@ -145,16 +145,21 @@ void registerMoreBindings(py::module_& m) {
   m.def(
       "gemm_residual_sumsq",
       [](uintptr_t a, uintptr_t b, uintptr_t residual, uintptr_t h, uintptr_t sumsq, int M, int N, int K, int blockN, bool twoSm,
-         uintptr_t stream) {
+         uintptr_t stream, int pairM) {
+        // block_n = 0: the form that suits the shape; pair_m >= 0: tiles of pair_m x block_n; else as two_sm and block_n say
+        const gemm::Form form = pairM >= 0 ? gemm::Form{pairM, blockN, 1}
+                                : twoSm    ? gemm::Form{256, 256, 1}
+                                : blockN != 0 ? gemm::Form{0, blockN, 1}
+                                              : gemm::planLayerForm(M, N, K);
         checkCudaMore(launchGemmResidualSumsq(reinterpret_cast<const void*>(a), reinterpret_cast<const void*>(b),
                                               reinterpret_cast<const void*>(residual), reinterpret_cast<void*>(h),
-                                              reinterpret_cast<float*>(sumsq), M, N, K, blockN, twoSm, nullptr,
+                                              reinterpret_cast<float*>(sumsq), M, N, K, form, nullptr,
                                               reinterpret_cast<cudaStream_t>(stream)),
                       "gemm_residual_sumsq");
-        return tpSumsqParts(N, blockN, twoSm);  // parts per row written to sumsq[part][row]
+        return tpSumsqParts(N, form);  // parts per row written to sumsq[part][row]
       },
       py::arg("a"), py::arg("b"), py::arg("residual"), py::arg("h"), py::arg("sumsq"), py::arg("m"), py::arg("n"), py::arg("k"),
-      py::arg("block_n") = 256, py::arg("two_sm") = false, py::arg("stream") = 0);
+      py::arg("block_n") = 256, py::arg("two_sm") = false, py::arg("stream") = 0, py::arg("pair_m") = -1);
   m.def(
       "tp_decode",
       [](SymmetricHeap& heap, std::vector<uintptr_t> x, std::vector<uintptr_t> w, uintptr_t residualIn, uintptr_t residualOut, uintptr_t out,

@@ -59,6 +59,8 @@ struct Form {
 // The form that gemm_bf16 takes where the caller asks for none, and the product in a given one. N % 64 == 0, K % 64 == 0. N need not be a
 // multiple of the tile.
 Form planForm(int M, int N, int K);
+// The same for the product whose epilogue adds a residual (launchGemmResidualSumsq), of whose tiles N is a multiple.
+Form planLayerForm(int M, int N, int K);
 cudaError_t gemmBf16Form(const void* A, const void* B, void* D, int M, int N, int K, int ldd, Form form, DeviceStatus* status, cudaStream_t stream,
                          uint64_t budgetNs = kDefaultBudgetNs);
 

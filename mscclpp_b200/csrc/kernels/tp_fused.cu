@@ -927,14 +927,15 @@ __global__ void __launch_bounds__(gemm::kNumThreads, 1)
 // tiled bulk store takes it. The boxes of a tile need twice the staging memory, which takes one of the six operand stages.
 // One B200, 8192 x 8192 x 1024 with residual: 131 -> 111 us (the plain product 97 us); 2048 rows 38 -> 31 us. Requesting the
 // residual further ahead in the epilogue above changed nothing there.
+template <typename Cfg>
 struct ResidualSumsqRows {
   static constexpr bool kNeedsTileBarrier = false;
   static constexpr bool kBulkStore = true;
   static constexpr bool kRowEpilogue = true;
-  static constexpr int kBlocks = gemm::Config2Rows::kColsPerWarp / 64;
+  static constexpr int kBlocks = Cfg::kColsPerWarp / 64;
   const CUtensorMap* tmapResidual;  // boxes of 64 columns x 32 rows; null = no residual
   const CUtensorMap* tmapH;
-  float* sumsq;  // [N / 128][M]
+  float* sumsq;  // [N / kColsPerWarp][M]
   int M;
   DeviceStatus* status;
   uint64_t budgetNs;
@@ -990,7 +991,7 @@ struct ResidualSumsqRows {
 #pragma unroll
       for (int c = 0; c < 8; c++) {
         uint4* word = reinterpret_cast<uint4*>(box + gemm::stagedOffset(lane, c));
-        uint4 x = c < 4 ? gemm::packChunk<ResidualSumsqRows>(v0, c & 3) : gemm::packChunk<ResidualSumsqRows>(v1, c & 3);
+        uint4 x = c < 4 ? gemm::packChunk<ResidualSumsqRows<Cfg>>(v0, c & 3) : gemm::packChunk<ResidualSumsqRows<Cfg>>(v1, c & 3);
         if (tmapResidual != nullptr) x = addBf16x8(x, *word);
         ss[c & 1] += sumSquaresBf16x8(x);
         *word = x;
@@ -1015,14 +1016,15 @@ struct ResidualSumsqRows {
   MSCCLPP_DEVICE_INLINE void auxWarp(int, int) const {}
 };
 
+template <typename Cfg>
 __global__ void __launch_bounds__(gemm::kNumThreads, 1)
     gemmResidualSumsqPairKernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
                                 const __grid_constant__ CUtensorMap tmapResidual, const __grid_constant__ CUtensorMap tmapH, gemm::Shape shape,
                                 int hasResidual, float* sumsq, DeviceStatus* status, uint64_t budgetNs) {
   extern __shared__ uint8_t smemRaw[];
   gemm::NoGate gate;
-  ResidualSumsqRows epi{hasResidual ? &tmapResidual : nullptr, &tmapH, sumsq, shape.M, status, budgetNs};
-  gemm::gemmCtaPair<gemm::Config2Rows>(&tmapA, &tmapB, shape, blockIdx.x / 2, gridDim.x / 2, gate, epi, status, budgetNs, smemRaw);
+  ResidualSumsqRows<Cfg> epi{hasResidual ? &tmapResidual : nullptr, &tmapH, sumsq, shape.M, status, budgetNs};
+  gemm::gemmCtaPair<Cfg>(&tmapA, &tmapB, shape, blockIdx.x / 2, gridDim.x / 2, gate, epi, status, budgetNs, smemRaw);
 }
 
 // out[row] = h[row] * rsqrt(sum of the row's parts / N + eps) * gamma. A block takes kScaleRows (or fewer) consecutive rows:
@@ -1295,79 +1297,88 @@ cudaError_t launchTpReduceNorm(const TpFusedArgs& argsIn, int numCtas, cudaStrea
   return cudaGetLastError();
 }
 
-template <int kBlockN>
-cudaError_t launchLocalTyped(const CUtensorMap& ta, const CUtensorMap& tb, gemm::Shape shape, ResidualSumsqStore epi, DeviceStatus* status,
-                             cudaStream_t stream) {
-  using Cfg = SmemOf<kBlockN>;
-  auto kernel = gemmResidualSumsqKernel<kBlockN>;
-  cudaError_t e = gemm::ensureDynamicSmem(reinterpret_cast<const void*>(kernel), Cfg::kSmemBytes);
-  if (e != cudaSuccess) return e;
-  uint64_t budget = 2000000000ull;
-  const int tiles = ((shape.M + gemm::kBlockM - 1) / gemm::kBlockM) * (shape.N / kBlockN);
-  int grid = gemm::smCount();
-  if (grid > tiles) grid = tiles;
-  void* params[] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), &shape, &epi, &status, &budget};
-  return gemm::launchOverlapped(reinterpret_cast<const void*>(kernel), dim3(grid), dim3(gemm::kNumThreads), Cfg::kSmemBytes, params, stream);
-}
-
-static cudaError_t launchLocalPair(const CUtensorMap& ta, const CUtensorMap& tb, gemm::Shape shape, const void* residual, void* h, float* sumsq,
-                                   DeviceStatus* status, cudaStream_t stream) {
-  CUtensorMap tr, th;
-  cudaError_t e = gemm::makeTensorMapBf16(&th, h, shape.M, shape.N, static_cast<uint64_t>(shape.N) * 2, 32);
-  if (e == cudaSuccess) e = gemm::makeTensorMapBf16(&tr, residual != nullptr ? residual : h, shape.M, shape.N, static_cast<uint64_t>(shape.N) * 2, 32);
-  const void* kernel = reinterpret_cast<const void*>(gemmResidualSumsqPairKernel);
-  if (e == cudaSuccess) e = gemm::ensureDynamicSmem(kernel, gemm::Config2Rows::kSmemBytes);
-  if (e != cudaSuccess) return e;
-  const int tiles = ((shape.M + gemm::Config2::kPairM - 1) / gemm::Config2::kPairM) * (shape.N / gemm::Config2::kBlockN);
-  int grid = gemm::smCount() & ~1;
-  if (grid > 2 * tiles) grid = 2 * tiles;
-  int hasResidual = residual != nullptr;
-  uint64_t budget = 2000000000ull;
-  void* params[] = {const_cast<CUtensorMap*>(&ta), const_cast<CUtensorMap*>(&tb), &tr, &th, &shape, &hasResidual, &sumsq, &status, &budget};
-  return gemm::launchClusterPair(kernel, dim3(grid), dim3(gemm::kNumThreads), gemm::Config2Rows::kSmemBytes, params, false, stream, true);
-}
-
-int tpSumsqParts(int N, int blockN, bool twoSm) {
-  const int blocksPerWarp = twoSm ? gemm::Config2::kColsPerWarp / 64 : (blockN >= 128 ? blockN / 128 : 1);
-  return N / (64 * blocksPerWarp);
-}
-
-cudaError_t launchGemmResidualSumsq(const void* A, const void* B, const void* residual, void* h, float* sumsq, int M, int N, int K,
-                                    int blockN, bool twoSm, DeviceStatus* status, cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || K <= 0 || K % gemm::kBlockK != 0 || N % 8 != 0) return cudaErrorInvalidValue;
-  if (twoSm && (M < gemm::Config2::kPairM || N % gemm::Config2::kBlockN != 0)) return cudaErrorInvalidValue;
-  if (!twoSm && (blockN != 64 && blockN != 128 && blockN != 256)) return cudaErrorInvalidValue;
-  if (!twoSm && N % blockN != 0) return cudaErrorInvalidValue;
-  cudaError_t e = cudaSuccess;
-  gemm::Shape shape{M, N, K, M < gemm::kBlockM ? M : gemm::kBlockM, 0, 0, 0};
-  if (twoSm) shape.aBoxRows = gemm::kBlockM;
-  // bands of 2048 rows, the order of a plain GEMM of this size: a wave re-reads its operands from L2, and the rows that are
-  // finished last are complete and still in L2 when the scale pass starts with them
-  const int band = 2048 / (twoSm ? gemm::Config2::kPairM : gemm::kBlockM);
-  if ((M + (twoSm ? gemm::Config2::kPairM : gemm::kBlockM) - 1) / (twoSm ? gemm::Config2::kPairM : gemm::kBlockM) > band) {
+// bands of 2048 rows, the order of a plain GEMM of this size: a wave re-reads its operands from L2, and the rows that are
+// finished last are complete and still in L2 when the scale pass starts with them
+static gemm::Shape localShape(int M, int N, int K, int aBoxRows, int tileM) {
+  gemm::Shape shape{M, N, K, aBoxRows, 0, 0, 0};
+  if ((M + tileM - 1) / tileM > 2048 / tileM) {
     shape.mOrder = 3;
-    shape.mOrderParam = band;
+    shape.mOrderParam = 2048 / tileM;
   }
+  return shape;
+}
+
+template <int kBlockN>
+cudaError_t launchLocalOne(const void* A, const void* B, const void* residual, void* h, float* sumsq, int M, int N, int K, DeviceStatus* status,
+                           cudaStream_t stream) {
+  using Cfg = gemm::Config<kBlockN>;
+  const void* kernel = reinterpret_cast<const void*>(gemmResidualSumsqKernel<kBlockN>);
+  gemm::Shape shape = localShape(M, N, K, M < gemm::kBlockM ? M : gemm::kBlockM, gemm::kBlockM);
   CUtensorMap ta, tb;
-  e = gemm::makeTensorMapBf16(&ta, A, M, K, static_cast<uint64_t>(K) * 2, shape.aBoxRows);
+  cudaError_t e = gemm::makeTensorMapBf16(&ta, A, M, K, static_cast<uint64_t>(K) * 2, shape.aBoxRows);
+  if (e == cudaSuccess) e = gemm::makeTensorMapBf16(&tb, B, N, K, static_cast<uint64_t>(K) * 2, kBlockN);
+  if (e == cudaSuccess) e = gemm::ensureDynamicSmem(kernel, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
-  e = gemm::makeTensorMapBf16(&tb, B, N, K, static_cast<uint64_t>(K) * 2, twoSm ? gemm::Config2::kBlockN / 2 : blockN);
-  if (e != cudaSuccess) return e;
-  if (twoSm) return launchLocalPair(ta, tb, shape, residual, h, sumsq, status, stream);
   ResidualSumsqStore epi{};
   epi.residual = static_cast<const bf16*>(residual);
   epi.h = static_cast<bf16*>(h);
   epi.sumsq = sumsq;
   epi.M = M;
   epi.N = N;
-  epi.blocksPerWarp = blockN >= 128 ? blockN / 128 : 1;
-  switch (blockN) {
-    case 64:
-      return launchLocalTyped<64>(ta, tb, shape, epi, status, stream);
-    case 128:
-      return launchLocalTyped<128>(ta, tb, shape, epi, status, stream);
+  epi.blocksPerWarp = kBlockN >= 128 ? kBlockN / 128 : 1;
+  uint64_t budget = 2000000000ull;
+  const int tiles = ((M + gemm::kBlockM - 1) / gemm::kBlockM) * (N / kBlockN);
+  void* params[] = {&ta, &tb, &shape, &epi, &status, &budget};
+  const int grid = gemm::smCount() < tiles ? gemm::smCount() : tiles;
+  return gemm::launchOverlapped(kernel, dim3(grid), dim3(gemm::kNumThreads), Cfg::kSmemBytes, params, stream);
+}
+
+template <typename Cfg>
+cudaError_t launchLocalPair(const void* A, const void* B, const void* residual, void* h, float* sumsq, int M, int N, int K, DeviceStatus* status,
+                            cudaStream_t stream) {
+  gemm::Shape shape = localShape(M, N, K, Cfg::kRows, Cfg::kPairM);
+  CUtensorMap ta, tb, tr, th;
+  cudaError_t e = gemm::makeTensorMapBf16(&ta, A, M, K, static_cast<uint64_t>(K) * 2, Cfg::kRows);
+  if (e == cudaSuccess) e = gemm::makeTensorMapBf16(&tb, B, N, K, static_cast<uint64_t>(K) * 2, Cfg::kBlockN / 2);
+  if (e == cudaSuccess) e = gemm::makeTensorMapBf16(&th, h, M, N, static_cast<uint64_t>(N) * 2, 32);
+  if (e == cudaSuccess) e = gemm::makeTensorMapBf16(&tr, residual != nullptr ? residual : h, M, N, static_cast<uint64_t>(N) * 2, 32);
+  const void* kernel = reinterpret_cast<const void*>(gemmResidualSumsqPairKernel<Cfg>);
+  if (e == cudaSuccess) e = gemm::ensureDynamicSmem(kernel, Cfg::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  const int tiles = ((M + Cfg::kPairM - 1) / Cfg::kPairM) * (N / Cfg::kBlockN);
+  int grid = gemm::smCount() & ~1;
+  if (grid > 2 * tiles) grid = 2 * tiles;
+  int hasResidual = residual != nullptr;
+  uint64_t budget = 2000000000ull;
+  void* params[] = {&ta, &tb, &tr, &th, &shape, &hasResidual, &sumsq, &status, &budget};
+  return gemm::launchClusterPair(kernel, dim3(grid), dim3(gemm::kNumThreads), Cfg::kSmemBytes, params, false, stream, true);
+}
+
+int tpSumsqParts(int N, gemm::Form form) {
+  // columns that one warp of the epilogue sums up
+  const int cols = form.pairM != 0 ? (form.pairM == 256 ? 128 : 64) : (form.blockN == 256 ? 128 : 64);
+  return N / cols;
+}
+
+cudaError_t launchGemmResidualSumsq(const void* A, const void* B, const void* residual, void* h, float* sumsq, int M, int N, int K,
+                                    gemm::Form form, DeviceStatus* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || K % gemm::kBlockK != 0 || N % 8 != 0) return cudaErrorInvalidValue;
+  if (form.blockN <= 0 || N % form.blockN != 0 || (form.pairM == 256 && M < form.pairM)) return cudaErrorInvalidValue;
+  switch (form.pairM * 1000000 + form.blockN * 1000 + form.split) {
+    case 64001:
+      return launchLocalOne<64>(A, B, residual, h, sumsq, M, N, K, status, stream);
+    case 128001:
+      return launchLocalOne<128>(A, B, residual, h, sumsq, M, N, K, status, stream);
+    case 256001:
+      return launchLocalOne<256>(A, B, residual, h, sumsq, M, N, K, status, stream);
+    case 256256001:
+      return launchLocalPair<gemm::Config2Rows>(A, B, residual, h, sumsq, M, N, K, status, stream);
+    case 128256001:
+      return launchLocalPair<gemm::Config2Flat256>(A, B, residual, h, sumsq, M, N, K, status, stream);
+    case 128128001:
+      return launchLocalPair<gemm::Config2Flat128>(A, B, residual, h, sumsq, M, N, K, status, stream);
     default:
-      return launchLocalTyped<256>(ta, tb, shape, epi, status, stream);
+      return cudaErrorInvalidValue;
   }
 }
 

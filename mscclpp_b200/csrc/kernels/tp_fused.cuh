@@ -74,12 +74,12 @@ cudaError_t launchTpFused(const TpFusedArgs& args, const void* const* A, const v
 cudaError_t launchTpReduceNorm(const TpFusedArgs& args, int numCtas, cudaStream_t stream);
 
 // One GPU, no collective: h = bf16(A * B^T) + residual written by the GEMM epilogue, which also writes every row's
-// sum of squares in parts: sumsq[part][row], tpSumsqParts(N, blockN, twoSm) parts of M floats each, every word written
+// sum of squares in parts: sumsq[part][row], tpSumsqParts(N, form) parts of M floats each, every word written
 // exactly once (no clearing, no atomics); launchTpScaleRowsFromSumsq adds the parts up and produces the RMSNorm.
-// twoSm selects the 256 x 256 pair tiles (M >= 256, N % 256 == 0), else one-SM tiles of blockN columns.
-int tpSumsqParts(int N, int blockN, bool twoSm);
+// N % form.blockN == 0, and M >= 256 for tiles of 256 rows.
+int tpSumsqParts(int N, gemm::Form form);
 cudaError_t launchGemmResidualSumsq(const void* A, const void* B, const void* residual, void* h, float* sumsq, int M, int N, int K,
-                                    int blockN, bool twoSm, DeviceStatus* status, cudaStream_t stream);
+                                    gemm::Form form, DeviceStatus* status, cudaStream_t stream);
 // out = h * rsqrt(sum_p sumsqParts[p][row] / N + eps) * gamma
 cudaError_t launchTpScaleRowsFromSumsq(const void* h, const float* sumsqParts, int numParts, const void* gamma, void* out, int M, int N,
                                        float eps, cudaStream_t stream);

@@ -177,7 +177,8 @@ class RowParallelLinearNorm:
         counters first, and its few extra warps wait out a loaded L2 for every row (B200, graph replay, hidden 8192, K
         1024: 128 tokens 13.0 us against 35, 2048 tokens 46 against 74, 8192 tokens 160 against 190). By default (both None) it
         is taken up to a few thousand tokens; longer prompts take a third form, one launch whose extra warps hold h on chip
-        until its rows are complete (2048 tokens 43 us, 8192 139; see _wave_form).
+        until its rows are complete (2048 tokens 43 us, 8192 139; see _wave_form). two_sm: 256 x 256 tiles on pairs of SMs, or tiles on
+        single ones; without it the two launches take the tiles that suit the shape, and the one-kernel path pairs from 1024 tokens on.
         timeline (one-kernel path, one-SM tiles): zeroed int64 CUDA tensor [148, 16] that receives per-CTA time stamps in ns
         (start, last MMA issued, MMA waits, epilogue waits and work, drain, first extra warp's rows / waits / work). Only the
         one-kernel form has it and `probe`; given either of them, one_kernel=None is that form up to 512 tokens."""
@@ -203,15 +204,9 @@ class RowParallelLinearNorm:
             return self.out[rows], self.residual_out[rows]
         if one_kernel is None:
             one_kernel = t <= 512 and (timeline is not None or probe != 0)
-        if two_sm is None:
-            # From 1024 tokens on, and for shorter prompts that fill at least 64 pairs of SMs. Two launches, graph replay, weights
-            # from HBM, K = 1024, us on one-SM / two-SM tiles by pairs: 16 (512 x 2048) 11.5 / 14.4, 32 (512 x 4096) 13.1 / 15.8,
-            # 48 (512 x 6144) 18.7 / 17.5, 63 (768 x 5376) 20.5 / 17.5, 64 (512 x 8192) 21.2 / 18.1, 96 (700 x 8192) 28.3 / 22.8,
-            # 128 (1023 x 8192) 30.5 / 25.2; K = 256 and 2048 alike. The forms cross where the one-SM tiles no longer fit one
-            # wave, between 32 and 48 pairs; up to 63 the one-SM form is kept.
-            pairs = (t + 255) // 256 * (self.out_features // 256)
-            two_sm = self.out_features % 256 == 0 and (t >= 1024 or (t >= 256 and pairs >= 64 and not one_kernel))
         if one_kernel:
+            if two_sm is None:
+                two_sm = self.out_features % 256 == 0 and t >= 1024
             ws_bytes = (n.tp_local_fused_workspace_bytes(self.max_tokens, self.out_features) + 255) // 256 * 256
             if self._local_ws is None:  # one workspace per 256-row-aligned launch that may be in flight: indexed by row offset
                 self._local_ws = torch.empty((8, ws_bytes // 4), dtype=torch.float32, device=self.symm.device)
@@ -220,9 +215,13 @@ class RowParallelLinearNorm:
                              self.out[rows].data_ptr(), self.gamma.data_ptr(), ws.data_ptr(), t, self.out_features, self.k_shard,
                              self.eps, pick_block_n(t, self.out_features), two_sm, 0, s, probe, 0 if timeline is None else timeline.data_ptr())
             return self.out[rows], self.residual_out[rows]
+        if self.out_features % 64 != 0:
+            raise ValueError("N must be a multiple of 64")
         parts_buf = self._parts()[row_offset * per_row:]
+        # (0: the tiles that suit the shape, gemm::planLayerForm)
+        block_n = 0 if two_sm is None else pick_block_n(t, self.out_features)
         parts = n.gemm_residual_sumsq(x.data_ptr(), self.weight.data_ptr(), self.residual_in[rows].data_ptr(), self.residual_out[rows].data_ptr(),
-                                      parts_buf.data_ptr(), t, self.out_features, self.k_shard, pick_block_n(t, self.out_features), two_sm, s)
+                                      parts_buf.data_ptr(), t, self.out_features, self.k_shard, block_n, bool(two_sm), s)
         n.tp_scale_rows_from_sumsq(self.residual_out[rows].data_ptr(), parts_buf.data_ptr(), parts, self.gamma.data_ptr(),
                                    self.out[rows].data_ptr(), t, self.out_features, self.eps, s)
         return self.out[rows], self.residual_out[rows]

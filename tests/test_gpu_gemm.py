@@ -120,6 +120,42 @@ def test_single_gpu_layer_gemm_epilogue_residual_sumsq(tokens, hidden, k, two_sm
     symm.destroy()
 
 
+@pytest.mark.parametrize("tokens", [1, 63, 129, 700])
+@pytest.mark.parametrize("hidden,k,tile", [
+    (1024, 320, (128, 128)),   # (an odd number of k blocks)
+    (1024, 320, (128, 256)),
+    (5120, 256, (128, 256)),   # several tiles per pair of SMs
+    (1152, 576, (0, 0)),       # the tile that the shape gets: N is a multiple of 128 only
+    (1088, 320, (0, 0)),       # ... of 64 only
+])
+def test_single_gpu_layer_gemm_tiles_of_128_rows(tokens, hidden, k, tile):
+    """The product with its epilogue in tiles of 128 rows on pairs of SMs, and where the width leaves no choice: h, and the sums of
+    squares that the scale pass makes 1/rms of."""
+    from mscclpp_b200 import native
+
+    g = torch.Generator(device="cuda").manual_seed(tokens + hidden)
+    x = torch.randn((tokens, k), generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn((hidden, k), generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    residual = torch.randn((tokens, hidden), generator=g, device="cuda").to(torch.bfloat16)
+    buf = torch.full((tokens * hidden + 4096,), 7.0, device="cuda", dtype=torch.bfloat16)
+    h = buf[:tokens * hidden].view(tokens, hidden)
+    sums = torch.full((hidden // 64 * tokens + 64,), -1.0, device="cuda")
+    product = x.double() @ w.double().t()
+    ref = product + residual.double()
+    # the product is rounded to bf16 and the sum again: 2^-8 of either value; the fp32 sum's own error as in test_gemm_forms
+    bound = (product.abs() + ref.abs()) * 2.0 ** -8 * 1.01 + (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24
+    for _ in range(2):
+        h.fill_(float("nan"))
+        parts = native().gemm_residual_sumsq(x.data_ptr(), w.data_ptr(), residual.data_ptr(), h.data_ptr(), sums.data_ptr(), tokens, hidden, k,
+                                             tile[1], False, torch.cuda.current_stream().cuda_stream, tile[0] or -1)
+        torch.cuda.synchronize()
+        assert bool(((h.double() - ref).abs() <= bound).all())
+        total = sums[:parts * tokens].view(parts, tokens).double().sum(0)
+        want = h.double().square().sum(1)
+        assert bool(((total - want).abs() <= want * hidden * 2.0 ** -24).all())
+    assert bool((buf[tokens * hidden:] == 7.0).all()) and bool((sums[parts * tokens:] == -1.0).all())
+
+
 @pytest.mark.parametrize("tokens,hidden,k", [
     (256, 256, 64),      # one tile, one block of the reduction
     (257, 2048, 192),    # a row block with one row, warps without rows
