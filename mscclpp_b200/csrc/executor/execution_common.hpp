@@ -153,6 +153,7 @@ struct ExecArgs {
   uint64_t scratchOff;   // heap offset of the scratch buffer (first half when double buffered)
   uint64_t scratchHalf;  // bytes of one scratch half (0 = no double buffering)
   int emuRanks;
+  int team;              // CTAs of a cluster that share a plan thread block (1, 2, 4 or 8; see executionKernel)
   int packetLL8;         // packet ops use 8-byte LL8 packets instead of 16-byte LL16 ones
   int portContext;       // index of this plan context in the host proxy's table
   FifoDeviceHandle portFifo;  // request queue of the executor's host proxy (triggers == nullptr: the plan has no port ops)

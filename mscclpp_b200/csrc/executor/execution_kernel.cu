@@ -1,4 +1,4 @@
-// Plan interpreter for sm_100a: one CUDA block per plan thread block walks its op list. Semantics of
+// Plan interpreter for sm_100a: one CUDA block (or a cluster of them, see executionKernel) per plan thread block walks its op list. Semantics of
 // the 30 opcodes follow the execution-plan contract (reference handlers:
 // src/core/include/execution_kernel.hpp:75-685), re-implemented on the symmetric heap:
 //   * operands are (rank, heap offset) pairs resolved by the host; peer memory is peerBase[rank] + offset;
@@ -14,11 +14,16 @@
 //     reference silently skips them on CUDA).
 #include "execution_kernel.hpp"
 
+#include <map>
+#include <mutex>
+#include <tuple>
 #include <type_traits>
 
 #include <mscclpp/copy_device.hpp>
 #include <mscclpp/npkit/npkit.hpp>
 #include <mscclpp/packet_device.hpp>
+
+#include "../kernels/gemm.cuh"
 
 namespace mscclpp {
 
@@ -52,8 +57,34 @@ struct Ctx {
   uint64_t pipeOff;   // byte offset of the current pipeline iteration inside each operand
   uint64_t pipeUnit;  // bytes per pipeline iteration (0 = not in a pipeline)
   uint32_t* barrierPasses;  // shared memory: grid barriers this block has passed in this launch, per barrier id
-  bool healthy;  // the same in every thread of the block: operations run as a whole block or not at all
+  bool healthy;  // the same in every thread of the block (of the team): operations run as a whole or not at all
+  int* ok;       // shared memory, 1 until a wait of this thread block has run out
+  int team, member;        // CTAs that share the plan thread block, and which of them this one is
+  uint32_t tid, threads;  // this thread among those of all of them
 };
+
+// The plan thread block's barrier: among the threads of the CTA, or of all CTAs of its team. What one of them has read or written is
+// ordered before what another one does behind it.
+MSCCLPP_DEVICE_INLINE void teamSync(const Ctx& x) {
+  if (x.team == 1) {
+    __syncthreads();
+  } else {
+    __syncwarp();
+    ptx::cluster_sync_all();
+  }
+}
+// A wait of the first CTA's has run out: its team hears of it at the barrier that ends the operation. (The others are there: they cannot
+// have gone before that barrier.)
+MSCCLPP_DEVICE_INLINE void teamGivesUp(const Ctx& x) {
+  *x.ok = 0;
+  for (int m = 1; m < x.team; m++)
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(ptx::mapa_shared(ptx::smem_u32(x.ok), m)), "r"(0) : "memory");
+}
+// End of an operation in which threads of the first CTA have waited. It began with a teamSync: by then everybody had read `ok`.
+MSCCLPP_DEVICE_INLINE void teamVerdict(Ctx& x) {
+  teamSync(x);
+  if (*x.ok == 0) x.healthy = false;
+}
 
 // End of an operation whose threads wait on their own (packets: a thread without one has nothing to miss): the block agrees on
 // whether all of them got what they waited for. Without the vote the threads that gave up leave the operation loop alone, and
@@ -115,7 +146,7 @@ MSCCLPP_DEVICE_INLINE void writeWords(Pkt* pk, int words, uint4 v, uint32_t epoc
 
 MSCCLPP_DEVICE_INLINE void signalChannels(const Ctx& x, const DevOp& op, bool relaxed) {
   const int t = threadIdx.x;
-  if (t < op.nIds) {
+  if (t < op.nIds && x.member == 0) {
     const DevChannel ch = x.plan->channels[op.channelType][op.ids[t]];
     ExecState* peer = reinterpret_cast<ExecState*>(x.c->peerBase[ch.peer] + x.a->stateOff);
     if (relaxed) {
@@ -128,21 +159,18 @@ MSCCLPP_DEVICE_INLINE void signalChannels(const Ctx& x, const DevOp& op, bool re
 }
 
 MSCCLPP_DEVICE_INLINE void waitChannels(Ctx& x, const DevOp& op, bool relaxed) {
-  __shared__ int waitOk;
-  if (threadIdx.x == 0) waitOk = 1;
-  __syncthreads();
+  teamSync(x);
   const int t = threadIdx.x;
-  if (t < op.nIds) {
+  if (t < op.nIds && x.member == 0) {
     const int cid = op.ids[t];
     const uint64_t expect = ++x.state->expected[op.channelType][cid];
     if (!waitGreaterEqual(&x.state->inbound[op.channelType][cid], expect, x.c->status, x.c->timeoutNs, kDevTimeoutSemaphore,
                           x.rank, 500 + cid, x.plan->channels[op.channelType][cid].peer)) {
-      waitOk = 0;
+      teamGivesUp(x);
     }
     (void)relaxed;  // acquire is used in both cases: a relaxed wait is a pure optimisation hint
   }
-  __syncthreads();
-  if (!waitOk) x.healthy = false;
+  teamVerdict(x);
 }
 
 // Port-channel operations: thread 0 queues one request per destination for the host proxy. kind: data and/or signal
@@ -150,10 +178,9 @@ MSCCLPP_DEVICE_INLINE void waitChannels(Ctx& x, const DevOp& op, bool relaxed) {
 // after its copy stream has drained.
 // packetSpace: both ends are packet-format scratch ranges (the bytes moved are the packets themselves, twice the payload).
 MSCCLPP_DEVICE_INLINE void portRequests(Ctx& x, const DevOp& op, uint32_t kind, bool packetSpace = false) {
-  __shared__ int portOk;
-  __syncthreads();  // data this block produced for the put is complete
-  if (threadIdx.x == 0) {
-    portOk = 1;
+  teamSync(x);  // data this thread block produced for the put is complete
+  if (threadIdx.x == 0 && x.member == 0) {
+    int portOk = 1;
     __threadfence_system();  // ... and visible to the copy engines
     FifoDeviceHandle fifo = x.a->portFifo;
     uint64_t last = UINT64_MAX;
@@ -192,17 +219,44 @@ MSCCLPP_DEVICE_INLINE void portRequests(Ctx& x, const DevOp& op, uint32_t kind, 
     if ((kind & kPortSync) && portOk && last != UINT64_MAX) {
       if (!fifo.sync(last, x.c->status, x.c->timeoutNs)) portOk = 0;
     }
+    if (!portOk) teamGivesUp(x);
   }
-  __syncthreads();
-  if (!portOk) x.healthy = false;
+  teamVerdict(x);
 }
 
 // The vector body of a reduction, a function of its own: inlined into the interpreter it has to share 64 registers with
 // every other operation's state, and the loads in flight are what gets spilled.
 template <typename T>
-__noinline__ __device__ void reduceWords(char* const* src, int nSrc, char* const* dst, int nDst, uint64_t nvec) {
+__noinline__ __device__ void reduceWords(char* const* src, int nSrc, char* const* dst, int nDst, uint64_t nvec, uint32_t tid, uint32_t threads) {
+  uint64_t i = tid;
+  // two sources: four words at a time, so that there are eight loads in flight (reduce-scatter of 16 MB over two ranks, 16 blocks: 70 -> 52 us)
+  if (nSrc == 2) {
+    const char *s0 = src[0], *s1 = src[1];
 #pragma unroll 1
-  for (uint64_t i = threadIdx.x; i < nvec; i += blockDim.x) {
+    for (; i + 3ull * threads < nvec; i += 4ull * threads) {
+      uint4 v[4], w[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        v[k] = ptx::ld_weak_v4(s0 + (i + static_cast<uint64_t>(k) * threads) * 16);
+        w[k] = ptx::ld_weak_v4(s1 + (i + static_cast<uint64_t>(k) * threads) * 16);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        ExecAccum<T> acc;
+        acc.init(v[k]);
+        acc.add(w[k]);
+        v[k] = acc.result();
+      }
+#pragma unroll 1
+      for (int d = 0; d < nDst; d++) {
+        char* to = dst[d] + i * 16;
+#pragma unroll
+        for (int k = 0; k < 4; k++) ptx::st_weak_v4(to + static_cast<uint64_t>(k) * threads * 16, v[k]);
+      }
+    }
+  }
+#pragma unroll 1
+  for (; i < nvec; i += threads) {
     ExecAccum<T> acc;
     auto batch = [&](int s, auto count) {
       constexpr int kCount = decltype(count)::value;
@@ -244,10 +298,10 @@ MSCCLPP_DEVICE_INLINE void reduceOp(const Ctx& x, const DevOp& op) {
   if (threadIdx.x < static_cast<uint32_t>(nSrc)) srcAddr[threadIdx.x] = plainAddr(x, op.src[threadIdx.x], skip);
   if (threadIdx.x >= 32 - static_cast<uint32_t>(nDst) && threadIdx.x < 32) dstAddr[31 - threadIdx.x] = plainAddr(x, op.dst[31 - threadIdx.x], skip);
   __syncthreads();
-  reduceWords<T>(srcAddr, nSrc, dstAddr, nDst, nvec);
+  reduceWords<T>(srcAddr, nSrc, dstAddr, nDst, nvec, x.tid, x.threads);
   // tail shorter than one vector (only with alignment < 16): element-wise through a zero-padded word
   const uint64_t tail = bytes - nvec * 16;
-  if (tail != 0 && threadIdx.x == 0) {
+  if (tail != 0 && x.tid == 0) {
     auto load = [&](const DevOperand& o) {
       uint32_t w[4] = {0, 0, 0, 0};
       const char* p = plainAddr(x, o, skip) + nvec * 16;
@@ -347,6 +401,38 @@ MSCCLPP_DEVICE_INLINE void switchStore(const Ctx& x, const DevOperand& o, uint64
     ptx::st_na_v4(reinterpret_cast<void*>(x.c->peerBase[g.ranks[i]] + o.offset + (o.isScratch ? x.half : 0) + byteOff), v);
 }
 
+// 16-byte words of a large copy, four loads in flight per thread: one at a time (copyBytes) is 16 KB per block of 1024 threads and round trip to
+// memory. A function of its own like reduceWords. All-gather of 16 MB over eight ranks, 64 blocks: 88 -> 63 us.
+__noinline__ __device__ void copyWords(char* dst, const char* src, uint64_t words, uint32_t tid, uint32_t threads) {
+  uint64_t i = tid;
+#pragma unroll 1
+  for (; i + 3ull * threads < words; i += 4ull * threads) {
+    uint4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = ptx::ld_nc_na_v4(src + (i + static_cast<uint64_t>(k) * threads) * 16);
+#pragma unroll
+    for (int k = 0; k < 4; k++) ptx::st_na_v4(dst + (i + static_cast<uint64_t>(k) * threads) * 16, v[k]);
+  }
+#pragma unroll 1
+  for (; i < words; i += threads) ptx::st_na_v4(dst + i * 16, ptx::ld_nc_na_v4(src + i * 16));
+}
+constexpr uint64_t kCopyWordsMin = 64 << 10;  // bytes: every thread of a block has its four
+
+// src[k] -> dst[k] of a put, get or copy.
+MSCCLPP_DEVICE_INLINE void copyOp(const Ctx& x, const DevOp& op) {
+  uint64_t skip = 0;
+  for (int i = 0; i < op.nDst; i++) {
+    const uint64_t n = sliced(x, op, op.src[i], skip);
+    char* dst = plainAddr(x, op.dst[i], skip);
+    const char* src = plainAddr(x, op.src[i], skip);
+    if (n >= kCopyWordsMin && ((reinterpret_cast<uint64_t>(dst) | reinterpret_cast<uint64_t>(src) | n) & 15) == 0) {
+      copyWords(dst, src, n / 16, x.tid, x.threads);
+    } else {
+      copyBytes(dst, src, n, x.tid, x.threads);
+    }
+  }
+}
+
 template <typename T, typename Pkt>
 MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
   using Payload = typename Pkt::Payload;
@@ -354,13 +440,11 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
   uint64_t skip = 0;
   switch (type) {
     case OpType::NOP:
-      __syncthreads();
+      teamSync(x);
       break;
     case OpType::BARRIER: {
-      __shared__ int barOk;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        barOk = 1;
+      teamSync(x);
+      if (threadIdx.x == 0 && x.member == 0) {
         const uint32_t target = (++x.barrierPasses[op.arg1]) * op.arg0;
         uint32_t* counter = &x.state->barriers[op.arg1];
         ptx::fence_acq_rel_gpu();
@@ -370,13 +454,12 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
         while (static_cast<int32_t>((v = ptx::ld_acquire_gpu(counter)) - target) < 0) {
           if (!g.keepSpinning()) {
             g.report(kDevTimeoutBarrier, x.rank, 600 + op.arg1, 0, target, v);
-            barOk = 0;
+            teamGivesUp(x);
             break;
           }
         }
       }
-      __syncthreads();
-      if (!barOk) x.healthy = false;
+      teamVerdict(x);
       break;
     }
     case OpType::SIGNAL:
@@ -404,21 +487,15 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
         portRequests(x, op, kPortData | (type != OpType::PUT ? kPortSignal : 0u) | (type == OpType::PUT_WITH_SIGNAL_AND_FLUSH ? kPortSync : 0u));
         break;
       }
-      for (int i = 0; i < op.nDst; i++) {
-        const uint64_t n = sliced(x, op, op.src[i], skip);
-        copyBytes(plainAddr(x, op.dst[i], skip), plainAddr(x, op.src[i], skip), n, threadIdx.x, blockDim.x);
-      }
+      copyOp(x, op);
       if (type != OpType::PUT) {
-        __syncthreads();
+        teamSync(x);
         signalChannels(x, op, false);
       }
       break;
     case OpType::GET:
     case OpType::COPY:
-      for (int i = 0; i < op.nDst; i++) {
-        const uint64_t n = sliced(x, op, op.src[i], skip);
-        copyBytes(plainAddr(x, op.dst[i], skip), plainAddr(x, op.src[i], skip), n, threadIdx.x, blockDim.x);
-      }
+      copyOp(x, op);
       break;
     case OpType::REDUCE:
     case OpType::REDUCE_SEND:
@@ -483,7 +560,7 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
       break;
     case OpType::GROUP_LOAD_REDUCE_STORE: {
       const uint64_t n = sliced(x, op, op.src[0], skip) / 16;
-      for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) {
+      for (uint64_t i = x.tid; i < n; i += x.threads) {
         const uint4 v = switchLoadReduce<T>(x, op.src[0], skip + i * 16);
         switchStore(x, op.dst[0], skip + i * 16, v);
       }
@@ -491,7 +568,7 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
     }
     case OpType::GROUP_STORE: {
       const uint64_t n = sliced(x, op, op.src[0], skip) / 16;
-      for (uint64_t i = threadIdx.x; i < n; i += blockDim.x)
+      for (uint64_t i = x.tid; i < n; i += x.threads)
         switchStore(x, op.dst[0], skip + i * 16, *reinterpret_cast<const uint4*>(plainAddr(x, op.src[0], skip) + i * 16));
       break;
     }
@@ -521,13 +598,11 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
     }
     case OpType::SEM_ACQUIRE:
     case OpType::SEM_RELEASE: {
-      __shared__ int semOk;
-      if (threadIdx.x == 0) semOk = 1;
-      __syncthreads();
-      if (threadIdx.x < op.nIds) {
+      teamSync(x);
+      if (threadIdx.x < op.nIds && x.member == 0) {
         // semaphores are re-armed by block 0 at the start of every launch: wait for that first
         if (!waitGreaterEqual(&x.state->semInit, x.epoch, x.c->status, x.c->timeoutNs, kDevTimeoutSemaphore, x.rank, 700, 0)) {
-          semOk = 0;
+          teamGivesUp(x);
         } else {
           int* sem = &x.state->semaphores[op.ids[threadIdx.x]];
           if (type == OpType::SEM_RELEASE) {
@@ -543,15 +618,14 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
               }
               if (!g.keepSpinning()) {
                 g.report(kDevTimeoutSemaphore, x.rank, 701, 0, 1, static_cast<uint64_t>(cur));
-                semOk = 0;
+                teamGivesUp(x);
                 break;
               }
             }
           }
         }
       }
-      __syncthreads();
-      if (!semOk) x.healthy = false;
+      teamVerdict(x);
       break;
     }
     default:
@@ -562,7 +636,7 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
 // One operation with its entry/exit trace events (thread 0; the cost is one predictable branch when tracing is off).
 template <typename T, typename Pkt>
 MSCCLPP_DEVICE_INLINE void tracedOp(Ctx& x, const DevOp& op) {
-  NpKitEventCollectContext* trace = x.a->npkit;
+  NpKitEventCollectContext* trace = x.member == 0 ? x.a->npkit : nullptr;
   if (trace != nullptr && threadIdx.x == 0)
     npkitCollectGpuEvent(trace, NPKIT_EVENT_EXECUTOR_OP_BASE_ENTRY + op.type, static_cast<uint32_t>(op.nSrc ? op.src[0].size : 0), x.rank);
   execOp<T, Pkt>(x, op);
@@ -573,7 +647,15 @@ MSCCLPP_DEVICE_INLINE void tracedOp(Ctx& x, const DevOp& op) {
   }
 }
 
-template <typename T, typename Pkt>
+// A plan's thread blocks are few (its author counts on one SM for each), and one SM keeps neither memory nor a fast link busy: a thread
+// block may be run by a team of CTAs, a cluster that shares the words of every copy and reduction like the threads of one CTA, and whose
+// first CTA does whatever a thread block does once: signals, waits, barriers, semaphores, requests to the proxy.
+// One B200, all ranks on it, us with one CTA each / teams (ranks x instances, bytes of the full-size buffer): reduce-scatter 2 x 1, 2 MB 50 /
+// 24, 8 x 2, 8 MB 86 / 39, 8 x 8, 16 MB 48 / 41 (128 SMs, 3.6 TB/s); all-gather 2 x 1, 2 MB 60 / 25, 8 x 8, 16 MB 63 / 50; all-to-all 8 x 2,
+// 8 MB 105 / 46. (Of which 15 are the launch and the signals.) Tried instead: one CTA with 192 KB of bulk copies in flight, requested by a
+// warp of its own: 48 -> 78 us, 0.25-0.5 us per piece in the requesting warp.
+// kTeams is a template parameter for the launches that have none: with the branches in one kernel, plans of a few KB took 0.3-1.6 us longer.
+template <typename T, typename Pkt, bool kTeams>
 __global__ void __launch_bounds__(1024, 1) executionKernel(ExecArgs a) {
   const DeviceComm& c = a.comm;
   const int rank = deviceRank(c);
@@ -582,7 +664,9 @@ __global__ void __launch_bounds__(1024, 1) executionKernel(ExecArgs a) {
   ExecState* state = reinterpret_cast<ExecState*>(c.peerBase[rank] + a.stateOff);
 
   __shared__ uint32_t barrierPasses[kExecMaxBarriers];
+  __shared__ int ok;
   if (threadIdx.x < kExecMaxBarriers) barrierPasses[threadIdx.x] = 0;
+  if (threadIdx.x == 0) ok = 1;
   __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     for (uint32_t i = 0; i < plan->nSemaphores; i++) state->semaphores[i] = plan->semInit[i];
@@ -590,7 +674,8 @@ __global__ void __launch_bounds__(1024, 1) executionKernel(ExecArgs a) {
     ptx::st_release_sys(&state->semInit, epoch);
   }
 
-  if (blockIdx.x < plan->nThreadBlocks) {
+  const uint32_t planBlock = kTeams ? blockIdx.x / a.team : blockIdx.x;
+  if (planBlock < plan->nThreadBlocks) {
     Ctx x;
     x.c = &c;
     x.a = &a;
@@ -603,7 +688,12 @@ __global__ void __launch_bounds__(1024, 1) executionKernel(ExecArgs a) {
     x.pipeUnit = 0;
     x.barrierPasses = barrierPasses;
     x.healthy = true;
-    const DevThreadBlock tb = plan->tbs[blockIdx.x];
+    x.ok = &ok;
+    x.team = kTeams ? a.team : 1;
+    x.member = kTeams ? static_cast<int>(blockIdx.x - planBlock * a.team) : 0;
+    x.tid = kTeams ? static_cast<uint32_t>(x.member) * blockDim.x + threadIdx.x : threadIdx.x;
+    x.threads = kTeams ? static_cast<uint32_t>(a.team) * blockDim.x : blockDim.x;
+    const DevThreadBlock tb = plan->tbs[planBlock];
     const DevOp* ops = plan->ops;
     uint32_t i = tb.opBegin;
     while (i < tb.opEnd && x.healthy) {
@@ -641,22 +731,57 @@ __global__ void __launch_bounds__(1024, 1) executionKernel(ExecArgs a) {
   }
 }
 
+// Clusters of `team` CTAs of `nThreads` threads that the current device can run at the same time.
+int residentTeams(const void* kernel, int team, int nThreads) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void*, int, int, int>, int> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  const std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_tuple(kernel, dev, team, nThreads);
+  const auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(team);
+  cfg.blockDim = dim3(nThreads);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(team);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    n = 0;
+  }
+  known[key] = n;
+  return n;
+}
+
 template <typename T>
 cudaError_t launchTyped(const ExecArgs& args, int nBlocks, int nThreads, cudaStream_t stream) {
-  dim3 grid(nBlocks, args.emuRanks > 1 ? args.emuRanks : 1, 1);
+  const int emu = args.emuRanks > 1 ? args.emuRanks : 1;
   dim3 block(nThreads, 1, 1);
   // thread blocks of a plan wait on one another (barriers, semaphores) and on peers: co-residency is required
   ExecArgs copy = args;
   void* params[] = {&copy};
-  const void* kernel = args.packetLL8 ? reinterpret_cast<const void*>(executionKernel<T, LL8Packet>)
-                                      : reinterpret_cast<const void*>(executionKernel<T, LL16Packet>);
+  const void* kernel = args.packetLL8 ? reinterpret_cast<const void*>(executionKernel<T, LL8Packet, false>)
+                                      : reinterpret_cast<const void*>(executionKernel<T, LL16Packet, false>);
+  const void* teams = reinterpret_cast<const void*>(executionKernel<T, LL16Packet, true>);  // (of plans without packets)
   // every block of the launch has to be resident at once: say so here, with numbers, instead of leaving it to the launch
   int perSm = 0, sms = 0, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, nThreads, 0) == cudaSuccess) {
-    if (static_cast<long long>(perSm) * sms < static_cast<long long>(grid.x) * grid.y) return cudaErrorCooperativeLaunchTooLarge;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, nThreads, 0) != cudaSuccess) {
+    perSm = sms = 0;
+  } else if (static_cast<long long>(perSm) * sms < static_cast<long long>(nBlocks) * emu) {
+    return cudaErrorCooperativeLaunchTooLarge;
   }
-  return cudaLaunchCooperativeKernel(kernel, grid, block, params, 0, stream);
+  // teams only of SMs that nobody else of the launch needs
+  if (nThreads % 32 != 0) copy.team = 1;
+  while (copy.team > 1 && (nBlocks * emu * copy.team > sms || nBlocks * emu > residentTeams(teams, copy.team, nThreads))) copy.team /= 2;
+  if (copy.team > 1) return gemm::launchClusters(teams, copy.team, dim3(nBlocks * copy.team, emu), block, 0, params, true, stream);
+  return cudaLaunchCooperativeKernel(kernel, dim3(nBlocks, emu), block, params, 0, stream);
 }
 
 }  // namespace

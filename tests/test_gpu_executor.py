@@ -242,6 +242,61 @@ def test_reductions_of_every_number_of_sources(world):
         _run_both(single_node.build("reducescatter_allpairs", world).to_json(), world, world * per, per, np.int32, inplace=False)
 
 
+# elements of a chunk, fp16: thread blocks of 128 KB, 256 KB and 512 KB are run by 2, 4 and 8 CTAs; the words do not divide by their threads
+@pytest.mark.parametrize("world,instances,per", [(2, 1, 32768 + 8), (2, 1, 65536 + 24), (2, 1, 131072 + 1032), (3, 2, 262144 + 16), (8, 2, 131072 + 16),
+                                                 (8, 8, 65536 + 64)])
+def test_thread_blocks_of_several_ctas(world, instances, per):
+    from mscclpp_b200.default_algos import single_node
+
+    build = lambda name: single_node.build(name, world, instances=instances, in_place=False).to_json()
+    _run_both(build("reducescatter_allpairs"), world, world * per, per, np.float16, inplace=False)
+    _run_both(build("alltoall_allpairs"), world, world * per, world * per, np.float16, inplace=False)
+    _run_both(build("allgather_allpairs"), world, per, world * per, np.float16, inplace=False)
+    _run_both(single_node.build("allreduce_nvls", world, instances=instances).to_json(), world, world * per, world * per, np.float16, inplace=True)
+
+
+def test_a_wait_that_runs_out_ends_every_cta_of_a_thread_block():
+    """The signals that the first wait is for are left out of the plan. The error is reported, nobody has reduced anything, and the
+    complete plan works afterwards."""
+    from mscclpp_b200 import SymmetricMemory, native
+    from mscclpp_b200.default_algos import single_node
+
+    n = native()
+    plan = json.loads(single_node.build("reducescatter_allpairs", 2, in_place=False).to_json())
+    complete = n.ExecutionPlan.from_string(json.dumps(plan), 0)
+    plan["name"] += "_without_signals"
+    for gpu in plan["gpus"]:
+        for tb in gpu["threadblocks"]:
+            assert tb["ops"][0]["name"] == "rlxsignal"
+            tb["ops"] = tb["ops"][1:]
+    lacking = n.ExecutionPlan.from_string(json.dumps(plan), 0)
+    symm = SymmetricMemory.emulated(2, nbytes=64 << 20, timeout_ms=300)
+    per = 1 << 18  # two sources of 1 MB: eight CTAs
+    t_in, t_out = symm.tensor((2 * per,), torch.float32), symm.tensor((per,), torch.float32)
+    ins = [torch.arange(2 * per, device="cuda", dtype=torch.float32) * (r + 1) for r in range(2)]
+    for r in range(2):
+        symm.rank_view(t_in, r).copy_(ins[r])
+        symm.rank_view(t_out, r).fill_(-1.0)
+    executor = n.Executor(symm.heap)
+
+    def run(loaded):
+        executor.execute(0, t_in.data_ptr(), t_out.data_ptr(), 8 * per, 4 * per, n.DataType.float32, loaded, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+
+    run(lacking)
+    with pytest.raises(Exception, match="gave up"):
+        symm.check()
+    for r in range(2):
+        assert bool((symm.rank_view(t_out, r) == -1.0).all())
+    symm.heap.reset_status()
+    run(complete)
+    symm.check()
+    for r in range(2):
+        assert torch.equal(symm.rank_view(t_out, r), (ins[0] + ins[1])[r * per:(r + 1) * per])
+    executor.reset()
+    symm.destroy()
+
+
 def _packets_then_reduction(kind):
     """Two ranks, one thread block each: a packet operation of fewer packets than threads, then a reduction of other
     chunks, which the DSL puts directly behind it (their chunks do not overlap)."""
