@@ -17,8 +17,8 @@
 //   the expert GEMM's epilogue or by launchMoeQuantizeRows), half the bytes over NVLink.
 // With one rank there is nobody to exchange counts with or to wait for: neither launch is cooperative, both overlap the kernel
 // before them, and every block of the dispatch counts all pairs by itself (up to 8192 of them). Dispatch and combine together
-// on one B200, before / now: 4096 tokens x 4096 bf16, top-2 of 64 experts 51 / 42 us (201 MB, 4.8 TB/s), 777 tokens x 7168
-// fp8, top-8 of 256 experts 39 / 33 us.
+// on one B200, with the cooperative dispatch / now: 4096 tokens x 4096 bf16, top-2 of 64 experts 51 / 37 us (201 MB, 5.4 TB/s), 777
+// tokens x 7168 fp8, top-8 of 256 experts 39 / 27 us.
 // With several ranks both end with a cross-rank barrier: after dispatch returns every row sent to this rank has landed; after combine
 // returns the peers are done reading this rank's expert outputs.
 //
@@ -140,22 +140,34 @@ __global__ void __launch_bounds__(kThreads, 1) moeDispatchKernel(MoeDispatchArgs
     __syncthreads();
     ptx::grid_dependency_wait();
     const int lo = tokBegin * a.topk, hi = tokEnd * a.topk, pairs = a.tokens * a.topk;
-    constexpr int kDepth = 8;
-    for (int i0 = threadIdx.x; i0 - static_cast<int>(threadIdx.x) < pairs; i0 += kDepth * kThreads) {
-      int e[kDepth];
+    // All expert ids are requested at once, sixteen per thread, and counted one by one: additions to one word of shared memory take turns, but
+    // finding the ids that a warp's lanes have in common first (__match_any_sync) took 7 us for 8192 pairs.
+    auto count = [&](int i, int e) {
+      if (e >= 0 && e < E) atomicAdd(&counts[static_cast<int>(i >= lo) + static_cast<int>(i >= hi)][e], 1u);
+    };
+    const bool vectors = (reinterpret_cast<uintptr_t>(topkIdx) & 15) == 0;
+    constexpr int kDepth = 4;
+    for (int v0 = threadIdx.x; 4 * (v0 - static_cast<int>(threadIdx.x)) < pairs; v0 += kDepth * kThreads) {
+      int e[kDepth][4];
 #pragma unroll
       for (int k = 0; k < kDepth; k++) {
-        const int i = i0 + k * kThreads;
-        e[k] = i < pairs ? static_cast<int>(ptx::ld_weak_u32(reinterpret_cast<const uint32_t*>(topkIdx) + i)) : -1;
+        const int i = 4 * (v0 + k * kThreads);
+        const uint32_t* at = reinterpret_cast<const uint32_t*>(topkIdx) + i;
+        if (vectors && i + 3 < pairs) {
+          const uint4 v = ptx::ld_weak_v4(at);
+          e[k][0] = static_cast<int>(v.x);
+          e[k][1] = static_cast<int>(v.y);
+          e[k][2] = static_cast<int>(v.z);
+          e[k][3] = static_cast<int>(v.w);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; j++) e[k][j] = i + j < pairs ? static_cast<int>(ptx::ld_weak_u32(at + j)) : -1;
+        }
       }
 #pragma unroll
       for (int k = 0; k < kDepth; k++) {
-        // one addition per expert that a warp meets: a batch that is routed to few experts costs no more than another
-        const int i = i0 + k * kThreads;
-        const bool used = e[k] >= 0 && e[k] < E;
-        const int cell = used ? (static_cast<int>(i >= lo) + static_cast<int>(i >= hi)) * kMoeMaxExperts + e[k] : -1;
-        const uint32_t same = __match_any_sync(0xffffffffu, cell);
-        if (used && (same & ((1u << (threadIdx.x & 31)) - 1u)) == 0) atomicAdd(&counts[cell / kMoeMaxExperts][cell % kMoeMaxExperts], __popc(same));
+#pragma unroll
+        for (int j = 0; j < 4; j++) count(4 * (v0 + k * kThreads) + j, e[k][j]);
       }
     }
   } else {
@@ -424,7 +436,11 @@ __global__ void __launch_bounds__(kThreads, 1) moeCombineKernel(MoeCombineArgs a
         wgt = weights[p];
       }
     };
-    int64_t u = blockIdx.x * warpsPerBlock + (threadIdx.x >> 5);
+    // With few rounds the units go round the blocks first: those of the last round, when not every warp has one, are spread over all SMs (777
+    // tokens x 7168 fp8, top-8, 2.3 rounds: dispatch and combine 27.6 -> 26.9 us). With more, neighbouring warps take neighbouring pieces
+    // of a row (4096 x 4096 bf16, top-2, 3.5 rounds: 37.2 us against 38.8).
+    const int warp = threadIdx.x >> 5;
+    int64_t u = units < 3 * static_cast<int64_t>(numWarps) ? static_cast<int64_t>(warp) * gridDim.x + blockIdx.x : static_cast<int64_t>(blockIdx.x) * warpsPerBlock + warp;
     fetch(u);
     for (; u < units; u += numWarps) {
       const int t = static_cast<int>(u / chunks);
