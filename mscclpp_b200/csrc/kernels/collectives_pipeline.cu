@@ -6,19 +6,23 @@
 //
 //   1. copy-in     user input  -> its slice of the local scratch-in            (local stores)
 //   2. barrier A   with the blocks of the same index on every rank            (all slices of this index are staged)
-//   3. reduce      this rank's 1/world of the slice: multimem.ld_reduce through the NVSwitch (or peer loads with an fp32
-//                  accumulator), result to EVERY rank's scratch-out            (multimem.st or peer stores)
-//   4. barrier B   (every rank's part of my scratch-out slice has landed)
-//   5. copy-out    scratch-out -> user output                                  (local loads, L1 bypassed)
+//   3. reduce      this rank's 1/world of the slice: multimem.ld_reduce through the NVSwitch, result to EVERY rank's scratch-out
+//                  (multimem.st), or peer loads with an fp32 accumulator, result to its OWN scratch-out (of two ranks, the other one's)
+//   4. barrier B   (every rank's part of the slice is reduced)
+//   5. copy-out    scratch-out -> user output: the local one, or each part from the rank that has reduced it
 //
 // The barriers are split into a signal and a wait, and the copy-in of round r + 1 (with its signal) sits between round r's
 // reduction and its wait for barrier B, so a block copies while its peers reduce. Blocks never wait for other blocks of
 // their own rank, so while one block sits in a barrier the others copy and reduce as well: with a few blocks per SM the
 // NVLink transfers, the local copies and the barrier latencies overlap. Scratch is double buffered per block (round
 // parity), which is what makes two barriers per round enough.
-// Four ranks on one B200 (one HBM; 32 MB bf16 each): 102 us, 121 us when a rank's own part went through the scratch as well;
-// 629 us with one copy load in flight per thread, system-scope accesses, the barriers unsplit and 16 blocks per rank
-// instead of the 74 that fit.
+// What bounds it with all ranks on one GPU: the bytes stored, of which an SM gets rid of 25-30 GB/s (a plain fill of 16 MB or 256 MB alike: 3.2-3.9
+// TB/s), and a round's waits and round trips, 9 us whatever it moves. Four ranks on one B200 (32 MB bf16 each), us: reduced parts stored
+// to every peer's scratch 110, to the own one and fetched from there (2 S of stores per rank instead of 2.5 S) 100, in 5
+// rounds instead of 7 91 (on two other boxes, both together, 106 -> 99 and 107 -> 102); 121 when a rank's own part went through the scratch as well; 629 with one copy load in flight per
+// thread, system-scope accesses, the barriers unsplit and 16 blocks per rank instead of the 74 that fit. Tried instead: a
+// warp for each copy and the others reducing, with three flags a round, 139; all three legs in one step with a single barrier
+// 119; evict-first and evict-last accesses, which take a third of the DRAM writes away (265 -> 182 MB), 1 %.
 // One round that covers the whole message is the un-pipelined "reduce-scatter + all-gather through scratch" form.
 //
 // Role of the reference's allreduce_nvls_block_pipeline.cu:16-147 / allreduce_nvls_warp_pipeline.cu:14-112 (NVLS) and
@@ -199,6 +203,9 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
     copyOthers(dst, src, whole);
     if (tail != 0) copyTail(dst + static_cast<uint64_t>(whole) * 16, src + static_cast<uint64_t>(whole) * 16, tail, 16);
   };
+  // Where the sums of my part go: with two ranks to the other one's scratch, of which there is only one, with more to the own
+  [[maybe_unused]] const bool pull = world > 2;
+  [[maybe_unused]] const uint64_t reducedTo = world == 2 ? c.peerBase[1 - rank] : local;
   auto tokenOf = [&](uint64_t r) { return (static_cast<uint64_t>(epoch) << 32) | (r + 1); };
 
   bool healthy = true;
@@ -263,12 +270,9 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
             if constexpr (kNvls) {
               ptx::multimem_st_v4(reinterpret_cast<void*>(c.mcBase + off), v[k]);
             } else {
-#pragma unroll 1
-              for (int i = 1; i < world; i++) {
-                const int p = rank + i < world ? rank + i : rank + i - world;
-                ptx::st_weak_v4(reinterpret_cast<void*>(heaps[p] + off), v[k]);
-              }
-              ptx::st_weak_v4(reinterpret_cast<void*>(u < direct ? outDirect + static_cast<uint64_t>(u) * 16 : local + off), v[k]);
+              ptx::st_weak_v4(reinterpret_cast<void*>(reducedTo + off), v[k]);
+              if (u < direct) ptx::st_weak_v4(reinterpret_cast<void*>(outDirect + static_cast<uint64_t>(u) * 16), v[k]);
+              else ptx::st_weak_v4(reinterpret_cast<void*>(local + off), v[k]);
             }
           }
         }
@@ -294,10 +298,31 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
     if (!healthy) break;
     // 5. copy-out
     const uint32_t tail = tailOf(r, have), whole = have - (tail != 0 ? 1 : 0);
-    const char* src = reinterpret_cast<const char*>(local + outSlice);
     char* dst = out + firstOf(r) * 16;
-    copyOthers(dst, src, whole);
-    if (tail != 0) copyTail(dst + static_cast<uint64_t>(whole) * 16, src + static_cast<uint64_t>(whole) * 16, tail, 0);
+    if constexpr (kNvls) {
+      copyUnits(dst, reinterpret_cast<const char*>(local + outSlice), 0, whole);
+    } else {
+      const uint32_t sub = static_cast<uint32_t>(subUnits), mineBegin = ownBegin < whole ? ownBegin : whole, mineEnd = ownEnd < whole ? ownEnd : whole;
+      const uint32_t n = whole - (mineEnd - mineBegin);
+      for (uint32_t i0 = threadIdx.x; i0 < n; i0 += blockDim.x * kCopyUnroll) {
+        uint4 v[kCopyUnroll];
+        uint32_t at[kCopyUnroll];
+#pragma unroll
+        for (uint32_t k = 0; k < kCopyUnroll; k++) {
+          uint32_t u = i0 + k * blockDim.x < n ? i0 + k * blockDim.x : n - 1;
+          if (u >= mineBegin) u += mineEnd - mineBegin;
+          at[k] = u;
+          v[k] = ptx::ld_weak_v4(reinterpret_cast<const void*>((pull ? heaps[u / sub] : local) + outSlice + static_cast<uint64_t>(u) * 16));
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kCopyUnroll; k++)
+          if (i0 + k * blockDim.x < n) ptx::st_weak_v4(dst + static_cast<uint64_t>(at[k]) * 16, v[k]);
+      }
+    }
+    if (tail != 0) {
+      const uint64_t from = kNvls || !pull ? local : heaps[whole / static_cast<uint32_t>(subUnits)];
+      copyTail(dst + static_cast<uint64_t>(whole) * 16, reinterpret_cast<const char*>(from + outSlice) + static_cast<uint64_t>(whole) * 16, tail, 0);
+    }
   }
   finishLaunch(c, rank, epoch);
 }

@@ -63,3 +63,19 @@ def test_grids_are_sized_for_one_block_per_sm():
             for n in (1 << 10, 1 << 20, 64 << 20):
                 blocks, threads = C._grid_for(n, algo, world)
                 assert 1 <= blocks <= 148 and 32 <= threads <= 1024
+
+
+def test_pipeline_slices_cover_the_message_in_equal_rounds():
+    """Whatever the message and the number of blocks: the slices fit the scratch, cover the message, and none of the rounds is empty."""
+    from types import SimpleNamespace
+
+    for world in (2, 3, 4, 8):
+        symm = SimpleNamespace(world=world)
+        scratch = 4 * C.PIPELINE_MAX_BLOCKS * C._pipeline_slice(symm)
+        for blocks in (1, 7, 37, 74, 128):
+            for nbytes in (1, 16 * world, 65536, 65537, 1 << 20, (32 << 20) + 16, 300 << 20):
+                slice_bytes = C._pipeline_slice_for(symm, nbytes, blocks, scratch)
+                rounds = -(-nbytes // (blocks * slice_bytes))
+                assert slice_bytes % (16 * world) == 0 and 4 * blocks * slice_bytes <= scratch
+                assert (rounds - 1) * blocks * slice_bytes < nbytes <= rounds * blocks * slice_bytes
+                assert rounds <= -(-nbytes // (blocks * (scratch // (4 * blocks) // (16 * world) * 16 * world)))
