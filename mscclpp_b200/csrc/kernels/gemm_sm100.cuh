@@ -316,7 +316,7 @@ MSCCLPP_DEVICE_INLINE void gemmCta(const CUtensorMap* tmapA, const CUtensorMap* 
   st.epiArrivals = reinterpret_cast<volatile uint32_t*>(st.tmemBase + 2);
   [[maybe_unused]] uint64_t* got = bars + 2 * Cfg::kStages + 6;  // [kOwnBlocks] the peers' parts of a block have come
   static_assert(kSplit == 1 || (2 * Cfg::kStages + 6 + Cfg::kOwnBlocks) * 8 <= Cfg::kBarrierBytes, "barriers");
-  static_assert(kSplit == 1 || (!Epilogue::kNeedsTileBarrier && !IsGatedEpilogue<Epilogue>::value), "the split form finishes single blocks");
+  static_assert(kSplit == 1 || !Epilogue::kNeedsTileBarrier, "the split form finishes single blocks");
 
   const int numMBlk = (shape.M + kBlockM - 1) / kBlockM;
   const int numNBlk = (shape.N + kBlockN - 1) / kBlockN;  // (the last tile may reach beyond N: see StoreBf16)

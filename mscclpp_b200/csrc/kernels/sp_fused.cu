@@ -83,7 +83,7 @@ struct StoreAct {
   static constexpr bool kNeedsTileBarrier = false;
   static constexpr bool kBulkStore = true;
   const CUtensorMap* tmapD;
-  int M;
+  int M, N;  // (tiles of one rank's form may reach beyond N)
   MSCCLPP_DEVICE_INLINE static float convert(float x) {
     if constexpr (kAct == 1) {
       // 0.5 x (1 + tanh(u)) = x sigmoid(2 u)
@@ -96,7 +96,7 @@ struct StoreAct {
   }
   MSCCLPP_DEVICE_INLINE void tileBegin(int, int, int) const {}
   MSCCLPP_DEVICE_INLINE void block(const uint8_t* stage, int row0, int col0, int lane, int /*b*/) const {
-    if (lane == 0 && row0 < M) {
+    if (lane == 0 && row0 < M && col0 < N) {
       ptx::tma_store_2d(tmapD, stage, col0, row0);
       ptx::bulk_commit();
     }
@@ -125,7 +125,7 @@ struct StoreGated {
     for (int i = 0; i < 4; i++) {
       const int r = 8 * i + (lane >> 2), ch = lane & 3;
       const int row = row0 + r;
-      if (row < M) {
+      if (row < M && col0 / 2 < halfN) {
         *reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * halfN + col0 / 2 + ch * 8) =
             *reinterpret_cast<const uint4*>(stage + gemm::stagedOffset(r, ch));
       }
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(gemm::kNumThreads, 1)
         const uint64_t dOff = reinterpret_cast<uint64_t>(a.D) - c.peerBase[c.rank];
         return StoreGated{reinterpret_cast<__nv_bfloat16*>(c.peerBase[rank] + dOff), a.shape.M, a.shape.N / 2};
       } else {
-        return StoreAct<kAct>{&maps.d[blockIdx.y], a.shape.M};
+        return StoreAct<kAct>{&maps.d[blockIdx.y], a.shape.M, a.shape.N};
       }
     };
     auto epi = makeEpilogue();
@@ -307,6 +307,91 @@ cudaError_t launchAct(const AgTmaps& maps, const AgGemmArgs& args, int grid, cud
   }
 }
 
+// One rank: there is nothing to gather, so the product with its activation is a plain GEMM launch - not cooperative, over the
+// kernel before it, in whatever tiles suit the shape (gemm::planForm).
+template <int kAct>
+MSCCLPP_DEVICE_INLINE auto localEpilogue(const CUtensorMap* tmapD, bf16* out, const gemm::Shape& shape) {
+  if constexpr (kAct == 3) return StoreGated{out, shape.M, shape.N / 2};
+  else return StoreAct<kAct>{tmapD, shape.M, shape.N};
+}
+template <int kBlockN, int kSplit, int kAct>
+__global__ void __launch_bounds__(gemm::kNumThreads, 1)
+    actGemmKernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const __grid_constant__ CUtensorMap tmapD,
+                  bf16* out, gemm::Shape shape, DeviceStatus* status, uint64_t budgetNs) {
+  extern __shared__ uint8_t smemRaw[];
+  gemm::NoGate gate;
+  auto epi = localEpilogue<kAct>(&tmapD, out, shape);
+  gemm::gemmCta<kBlockN, gemm::NoGate, decltype(epi), kSplit>(&tmapA, &tmapB, shape, blockIdx.x / kSplit, gridDim.x / kSplit, gate, epi, status, budgetNs,
+                                                              smemRaw);
+}
+template <typename Cfg, int kAct>
+__global__ void __launch_bounds__(gemm::kNumThreads, 1)
+    actGemmPairKernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const __grid_constant__ CUtensorMap tmapD,
+                      bf16* out, gemm::Shape shape, DeviceStatus* status, uint64_t budgetNs) {
+  extern __shared__ uint8_t smemRaw[];
+  gemm::NoGate gate;
+  auto epi = localEpilogue<kAct>(&tmapD, out, shape);
+  gemm::gemmCtaPair<Cfg>(&tmapA, &tmapB, shape, blockIdx.x / 2, gridDim.x / 2, gate, epi, status, budgetNs, smemRaw);
+}
+
+// tileM x tileN tiles, `boxM` rows of A and `boxN` of B in a CTA's operand tiles, clusters of `ctas` CTAs per tile, persistent or not
+cudaError_t launchActGemm(const void* kernel, const AgGemmArgs& a, const void* B, int tileM, int tileN, int boxM, int boxN, int ctas, bool persistent,
+                          int smemBytes, cudaStream_t stream) {
+  const int M = a.shape.M, N = a.shape.N, K = a.shape.K, dCols = a.activation == 3 ? N / 2 : N;
+  gemm::Shape shape{M, N, K, boxM, 0, 0, 0};
+  const int rowBlocks = (M + tileM - 1) / tileM;
+  if (rowBlocks > 2048 / tileM) {  // bands of 2048 rows, the order of a plain GEMM
+    shape.mOrder = 3;
+    shape.mOrderParam = 2048 / tileM;
+  }
+  CUtensorMap ta, tb, td;
+  cudaError_t e = gemm::makeTensorMapBf16(&ta, a.aLocal, M, K, static_cast<uint64_t>(K) * 2, boxM);
+  if (e == cudaSuccess) e = gemm::makeTensorMapBf16(&tb, B, N, K, static_cast<uint64_t>(K) * 2, boxN);
+  if (e == cudaSuccess) e = gemm::makeTensorMapBf16(&td, a.D, M, dCols, static_cast<uint64_t>(dCols) * 2, 32);  // (the gated epilogue stores without it)
+  if (e == cudaSuccess) e = gemm::ensureDynamicSmem(kernel, smemBytes);
+  if (e != cudaSuccess) return e;
+  const int tiles = rowBlocks * ((N + tileN - 1) / tileN), resident = gemm::smCount() / ctas;
+  const int grid = (persistent && tiles > resident ? resident : tiles) * ctas;
+  bf16* out = static_cast<bf16*>(a.D);
+  DeviceStatus* status = a.comm.status;
+  uint64_t budget = a.comm.timeoutNs;
+  void* params[] = {&ta, &tb, &td, &out, &shape, &status, &budget};
+  if (ctas > 1) return gemm::launchClusters(kernel, ctas, dim3(grid), dim3(gemm::kNumThreads), smemBytes, params, false, stream, true);
+  return gemm::launchOverlapped(kernel, dim3(grid), dim3(gemm::kNumThreads), smemBytes, params, stream);
+}
+template <int kBlockN, int kSplit, int kAct>
+cudaError_t launchActOne(const AgGemmArgs& a, const void* B, cudaStream_t stream) {
+  return launchActGemm(reinterpret_cast<const void*>(actGemmKernel<kBlockN, kSplit, kAct>), a, B, gemm::kBlockM, kBlockN, gemm::kBlockM, kBlockN, kSplit,
+                       kSplit == 1, gemm::Config<kBlockN, kSplit>::kSmemBytes, stream);
+}
+template <typename Cfg, int kAct>
+cudaError_t launchActPair(const AgGemmArgs& a, const void* B, cudaStream_t stream) {
+  return launchActGemm(reinterpret_cast<const void*>(actGemmPairKernel<Cfg, kAct>), a, B, Cfg::kPairM, Cfg::kBlockN, Cfg::kRows, Cfg::kBlockN / 2, 2, true,
+                       Cfg::kSmemBytes, stream);
+}
+template <int kAct>
+cudaError_t launchActForm(const AgGemmArgs& a, const void* B, cudaStream_t stream) {
+  const gemm::Form form = gemm::planForm(a.shape.M, a.shape.N, a.shape.K);
+  switch (form.pairM * 1000000 + form.blockN * 1000 + form.split) {
+    case 64001:
+      return launchActOne<64, 1, kAct>(a, B, stream);
+    case 64004:
+      return launchActOne<64, 4, kAct>(a, B, stream);
+    case 128001:
+      return launchActOne<128, 1, kAct>(a, B, stream);
+    case 256001:
+      return launchActOne<256, 1, kAct>(a, B, stream);
+    case 256256001:
+      return launchActPair<gemm::Config2, kAct>(a, B, stream);
+    case 128256001:
+      return launchActPair<gemm::Config2Flat256, kAct>(a, B, stream);
+    case 128128001:
+      return launchActPair<gemm::Config2Flat128, kAct>(a, B, stream);
+    default:
+      return cudaErrorInvalidValue;
+  }
+}
+
 }  // namespace
 
 cudaError_t launchAllGatherGemm(const AgGemmArgs& argsIn, const void* const* B, int numCopiers, cudaStream_t stream) {
@@ -314,6 +399,23 @@ cudaError_t launchAllGatherGemm(const AgGemmArgs& argsIn, const void* const* B, 
   const int M = args.shape.M, N = args.shape.N, K = args.shape.K;
   const int world = args.comm.world;
   if (M <= 0 || world < 1 || world > 8 || M % (world * gemm::kBlockM) != 0) return cudaErrorInvalidValue;
+  if (world == 1 && args.blockN < 0 && args.numGemmCtas <= 0 && numCopiers <= 0) {
+    if (N % 128 != 0 || K % 128 != 0 || M / gemm::kBlockM > kAgMaxMBlk) return cudaErrorInvalidValue;
+    switch (args.activation) {
+      case 0:
+        return launchActForm<0>(args, B[0], stream);
+      case 1:
+        return launchActForm<1>(args, B[0], stream);
+      case 2:
+        return launchActForm<2>(args, B[0], stream);
+      case 3:
+        return launchActForm<3>(args, B[0], stream);
+      default:
+        return cudaErrorInvalidValue;
+    }
+  }
+  if (args.blockN < 0)
+    args.blockN = M % (world * gemm::Config2::kPairM) == 0 && N % gemm::Config2::kBlockN == 0 ? 0 : (N % 256 == 0 ? 256 : 128);
   const bool twoSm = args.blockN == 0;  // block_n 0 = 256 x 256 tiles on SM pairs
   const int tileN = twoSm ? gemm::Config2::kBlockN : args.blockN;
   if (N % tileN != 0 || K % 128 != 0) return cudaErrorInvalidValue;

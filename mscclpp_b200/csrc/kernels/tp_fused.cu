@@ -1189,9 +1189,11 @@ cudaError_t launchTpFused(const TpFusedArgs& argsIn, const void* const* A, const
   TpFusedArgs args = argsIn;
   const int M = args.shape.M, N = args.shape.N, K = args.shape.K;
   const int world = args.comm.world;
+  const bool anyTile = args.mode == 2 && args.blockN < 0;  // the widest that divides the problem, or on one rank what suits its shape
+  if (anyTile) args.blockN = M % (world * gemm::Config2::kPairM) == 0 && N % gemm::Config2::kBlockN == 0 ? 0 : (N % 256 == 0 ? 256 : 128);
   const bool twoSm = args.blockN == 0;  // block_n 0 = 256 x 256 tiles on SM pairs
   const int tileN = twoSm ? gemm::Config2::kBlockN : args.blockN;
-  if (M <= 0 || N % tileN != 0 || K % gemm::kBlockK != 0) return cudaErrorInvalidValue;
+  if (M <= 0 || tileN <= 0 || N % tileN != 0 || K % gemm::kBlockK != 0) return cudaErrorInvalidValue;
   if (twoSm && M < gemm::Config2::kPairM) return cudaErrorInvalidValue;
   if (N / tileN > kMaxNBlk || world > 8) return cudaErrorInvalidValue;
   if (N * 2 / 16 > kWordsPerThread * kGroupThreads) return cudaErrorInvalidValue;
@@ -1215,6 +1217,7 @@ cudaError_t launchTpFused(const TpFusedArgs& argsIn, const void* const* A, const
       // one rank: the product is the result, and the plain GEMM writes it where it belongs. Through `partial` and the
       // reducers the same bits cost a second pass over it; a caller that asks for reducers gets them.
       const uint64_t budget = args.comm.timeoutNs;
+      if (anyTile && args.numGemmCtas <= 0) return gemm::gemmBf16Form(A[0], B[0], args.out, M, N, K, N, gemm::planForm(M, N, K), args.comm.status, stream, budget);
       return twoSm ? gemm::gemmBf16TwoSm(A[0], B[0], args.out, M, N, K, N, args.numGemmCtas, args.comm.status, stream, 0, 0, budget)
                    : gemm::gemmBf16(A[0], B[0], args.out, M, N, K, N, args.blockN, args.numGemmCtas, args.comm.status, stream, 0, 0, budget);
     }

@@ -40,8 +40,8 @@ def all_gather_gemm(symm: SymmetricMemory, a_local: torch.Tensor, a_full: torch.
     weights = weight if isinstance(weight, (list, tuple)) else [weight]
     n_cols = weights[0].shape[0]
     assert a_local.shape == (s_rows // symm.world, k) and out.shape == (s_rows, n_cols // 2 if activation == "swiglu" else n_cols)
-    if block_n < 0:  # 0 = two-SM tiles (256 x 256 on SM pairs) when the shape allows, else one-SM 256- or 128-wide tiles
-        block_n = 0 if (s_rows % (symm.world * 256) == 0 and n_cols % 256 == 0) else (256 if n_cols % 256 == 0 else 128)
+    # (block_n < 0: two-SM tiles, 256 x 256 on SM pairs, when the shape allows, else one-SM 256- or 128-wide tiles; on one rank, which has
+    # nothing to gather, a plain product in the tiles that suit the shape)
     assert all(w.shape == (n_cols, k) and w.is_contiguous() and w.dtype == torch.bfloat16 for w in weights)
     st = (stream or torch.cuda.current_stream()).cuda_stream
     n.all_gather_gemm(symm.heap, a_local.data_ptr(), a_full.data_ptr(), [w.data_ptr() for w in weights], out.data_ptr(), s_rows, n_cols, k,
@@ -62,10 +62,9 @@ def gemm_reduce_scatter(symm: SymmetricMemory, a, weight, partial: torch.Tensor,
     s_rows, k = a_list[0].shape
     n_cols = w_list[0].shape[0]
     assert partial.shape == (s_rows, n_cols) and out.shape == (s_rows // symm.world, n_cols)
-    if block_n < 0:
-        block_n = 0 if (s_rows % (symm.world * 256) == 0 and n_cols % 256 == 0) else (256 if n_cols % 256 == 0 else 128)
     nvls = symm.nvls if nvls is None else nvls
     st = (stream or torch.cuda.current_stream()).cuda_stream
+    # (block_n < 0: as in all_gather_gemm)
     n.tp_fused(symm.heap, [x.data_ptr() for x in a_list], [w.data_ptr() for w in w_list], partial.data_ptr(), 0, 0, out.data_ptr(), 0, 0,
                s_rows, n_cols, k, 0.0, block_n, num_gemm_ctas, num_reducers, 0, 2, nvls, st)
     return out

@@ -391,6 +391,50 @@ def test_all_gather_gemm_one_kernel(world, rows_per_rank, k, n_cols, act):
     symm.destroy()
 
 
+# a shape for every form that one rank's product may take (gemm_plan_form), of widths that are no multiple of its tiles where it can be
+@pytest.mark.parametrize("act", ["none", "gelu", "silu", "swiglu"])
+@pytest.mark.parametrize("m,n,k,form", [(128, 1152, 256, (0, 64, 1)), (128, 640, 4096, (0, 64, 4)), (512, 3456, 256, (0, 128, 1)),
+                                        (1408, 2944, 384, (0, 256, 1)), (640, 4224, 1280, (256, 256, 1)), (384, 3200, 1280, (128, 256, 1)),
+                                        (256, 2688, 1536, (128, 128, 1))])
+def test_all_gather_gemm_of_one_rank(act, m, n, k, form):
+    """Nothing to gather: a plain product with its activation, against 64 bits. Activations of values up to +-100 and more, where the exponential
+    overflows on one side."""
+    from mscclpp_b200 import SymmetricMemory, native
+    from mscclpp_b200.parallel.sp_layer import all_gather_gemm, interleave_gate_up
+
+    assert native().gemm_plan_form(m, n, k) == form
+    symm = SymmetricMemory.emulated(1, nbytes=256 << 20, timeout_ms=3000)
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    x, full = symm.tensor((m, k), torch.bfloat16), symm.tensor((m, k), torch.bfloat16)
+    out = symm.tensor((m, n // 2 if act == "swiglu" else n), torch.bfloat16)
+    x.copy_(torch.randn((m, k), generator=g, device="cuda"))
+    w = (torch.randn((n, k), generator=g, device="cuda") * (30 / k ** 0.5)).to(torch.bfloat16)
+    p = x.double() @ w.double().t()
+    d = (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24  # of the fp32 sum: at most K roundings of the products' magnitudes
+    eps = 16 * 2.0 ** -23  # of the activation itself in fp32: exponential, reciprocal and products, a few units each
+    if act == "none":
+        ref, bound = p, d
+    elif act == "silu":  # (its slope and GELU's are at most 1.13; an exponential's relative error grows with its argument)
+        ref = torch.nn.functional.silu(p)
+        bound = 1.13 * d + eps * (1 + p.abs()) * ref.abs()
+    elif act == "gelu":
+        ref = torch.nn.functional.gelu(p, approximate="tanh")
+        bound = 1.13 * d + eps * (1 + p.abs() + p.abs() ** 3) * ref.abs()
+    else:
+        gate, up, dg, du = p[:, :n // 2], p[:, n // 2:], d[:, :n // 2], d[:, n // 2:]
+        ref = torch.nn.functional.silu(gate) * up
+        bound = 1.13 * dg * (up.abs() + du) + torch.nn.functional.silu(gate).abs() * du + eps * (1 + gate.abs()) * ref.abs()
+        w = interleave_gate_up(w[:n // 2], w[n // 2:])
+    bound = bound + ref.abs() * 2.0 ** -8 * 1.01 + 1e-37  # one rounding to bf16 (eight significant bits), or to zero below its range
+    for _ in range(2):
+        out.fill_(float("nan"))
+        all_gather_gemm(symm, x, full, w, out, activation=act)
+        torch.cuda.synchronize()
+        symm.check()
+        assert bool(((out.double() - ref).abs() <= bound).all())
+    symm.destroy()
+
+
 @pytest.mark.parametrize("world,rows_per_rank,k,ffn,block_n", [(2, 256, 256, 256, 256), (4, 128, 512, 128, 128), (2, 256, 128, 384, -1)])
 def test_all_gather_gemm_swiglu(world, rows_per_rank, k, ffn, block_n):
     """All-gather -> GEMM over interleaved gate / up weights with the gated epilogue: out = silu(x Wg^T) * (x Wu^T), one
