@@ -20,6 +20,8 @@
 //  residual-add and norm are one kernel.
 #include "collectives.cuh"
 
+#include "gemm.cuh"
+
 #include <type_traits>
 
 #include <mscclpp/packet_device.hpp>
@@ -138,6 +140,10 @@ __global__ void __launch_bounds__(kNorm ? 1024 : 512, 1) allreduceLLKernel(CollA
   const uint64_t emu = static_cast<uint64_t>(blockIdx.y) * a.emuStride;
   const char* in = reinterpret_cast<const char*>(a.in) + emu;
   char* out = reinterpret_cast<char*>(a.out) + emu;
+  if constexpr (!kNorm) {  // the launch may overlap the kernel before it
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
+  }
   const uint32_t flag = launchEpoch(c, rank);
   const uint64_t bufOff = c.llScratchOff + static_cast<uint64_t>(flag & 1u) * (static_cast<uint64_t>(world) * c.llSlotBytes);
   const uint64_t bytes = a.bytes;
@@ -631,14 +637,13 @@ __global__ void __launch_bounds__(512, 1) twoShotKernel(CollArgs a) {
 
 // --------------------------------------------------------------------------------------------
 template <typename KernelT>
-cudaError_t launchMaybeCooperative(KernelT kernel, const CollArgs& args, int nBlocks, int nThreads, cudaStream_t stream) {
+cudaError_t launchMaybeCooperative(KernelT kernel, const CollArgs& args, int nBlocks, int nThreads, cudaStream_t stream, bool overlapped = false) {
   dim3 grid(nBlocks, args.emuRanks > 1 ? args.emuRanks : 1, 1);
   dim3 block(nThreads, 1, 1);
   if (args.emuRanks > 1) {
-    // emulated ranks wait on one another inside one grid: it has to be co-resident
     CollArgs copy = args;
     void* params[] = {&copy};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), grid, block, params, 0, stream);
+    return launchEmulatedRanks(reinterpret_cast<const void*>(kernel), grid, block, params, 1, stream, overlapped);
   }
   kernel<<<grid, block, 0, stream>>>(args);
   return cudaGetLastError();
@@ -657,10 +662,10 @@ cudaError_t launchLLTyped(const CollArgs& a, int nBlocks, int nThreads, cudaStre
   }
   if (a.ll8) {
     if (a.nvls) return cudaErrorInvalidValue;
-    return launchMaybeCooperative(allreduceLLKernel<T, Op, false, false, true>, a, nBlocks, nThreads, s);
+    return launchMaybeCooperative(allreduceLLKernel<T, Op, false, false, true>, a, nBlocks, nThreads, s, true);
   }
-  return a.nvls ? launchMaybeCooperative(allreduceLLKernel<T, Op, true, false>, a, nBlocks, nThreads, s)
-                : launchMaybeCooperative(allreduceLLKernel<T, Op, false, false>, a, nBlocks, nThreads, s);
+  return a.nvls ? launchMaybeCooperative(allreduceLLKernel<T, Op, true, false>, a, nBlocks, nThreads, s, true)
+                : launchMaybeCooperative(allreduceLLKernel<T, Op, false, false>, a, nBlocks, nThreads, s, true);
 }
 
 template <typename T, ReduceOp Op>
@@ -712,6 +717,24 @@ cudaError_t launchTwoShotTyped(const CollArgs& a, int nBlocks, int nThreads, cud
   } while (0)
 
 }  // namespace
+
+cudaError_t launchEmulatedRanks(const void* kernel, dim3 grid, dim3 block, void** params, int blocksPerSm, cudaStream_t stream, bool overlapped) {
+  if (grid.y > 8 || 2 * static_cast<int>(grid.x * grid.y) > blocksPerSm * gemm::smCount())
+    return cudaLaunchCooperativeKernel(kernel, grid, block, params, 0, stream);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = stream;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = attrs[0].val.clusterDim.z = 1;
+  attrs[0].val.clusterDim.y = grid.y;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = overlapped ? 2 : 1;
+  return cudaLaunchKernelExC(&cfg, kernel, params);
+}
 
 cudaError_t launchAllreduceLL(const CollArgs& args, DataType dtype, ReduceOp op, int nBlocks, int nThreads,
                               cudaStream_t stream) {

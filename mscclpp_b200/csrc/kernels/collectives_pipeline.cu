@@ -343,7 +343,7 @@ cudaError_t launchPipeTyped(const PipeArgs& a, int nBlocks, int nThreads, cudaSt
   }
   PipeArgs copy = a;
   void* params[] = {&copy};
-  if (a.emuRanks > 1) return cudaLaunchCooperativeKernel(kernel, grid, block, params, 0, stream);
+  if (a.emuRanks > 1) return launchEmulatedRanks(kernel, grid, block, params, 2, stream);
   return cudaLaunchKernel(kernel, grid, block, params, 0, stream);
 }
 

@@ -30,6 +30,8 @@ def test_overlapped_kernels_read_nothing_through_the_non_coherent_path():
     # (the several-rank forms of the same source are launched after what they read: `kOne ? overlapped : not` is the one place they differ in)
     parts += [_definition(moe, head).replace("kOne ? ptx::ld_weak_v4(src + w0 + j * 32) : ptx::ld_input_v4(src + w0 + j * 32)", "")
               for head in ("moeDispatchKernel(MoeDispatchArgs a)", "moeCombineKernel(MoeCombineArgs a)")]
+    parts.append(_definition(open(os.path.join(KERNELS, "collectives.cu")).read(), "allreduceLLKernel(CollArgs a)"))
+    parts.append(_definition(open(os.path.join(KERNELS, "sp_fused.cu")).read(), "struct StoreGated {"))
     for text in parts:
         assert len(text) > 500
         assert not re.search(r"ld_input_v4|__ldg|\.nc\b|__restrict__", text)
