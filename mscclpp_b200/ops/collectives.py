@@ -19,7 +19,7 @@ from typing import Optional
 import torch
 
 from .._core import native
-from .._core.symm import SymmetricMemory, torch_dtype_to_native
+from .._core.symm import SymmetricMemory, stream_handle, torch_dtype_to_native
 
 MODE_ALLREDUCE, MODE_REDUCE_SCATTER, MODE_ALLGATHER, MODE_BROADCAST, MODE_ALLTOALL = 0, 1, 2, 3, 4
 
@@ -27,17 +27,15 @@ MODE_ALLREDUCE, MODE_REDUCE_SCATTER, MODE_ALLGATHER, MODE_BROADCAST, MODE_ALLTOA
 LL_MAX_BYTES = 512 << 10
 
 
-def _stream(stream: Optional[torch.cuda.Stream]) -> int:
-    return (stream or torch.cuda.current_stream()).cuda_stream
-
-
 def _nbytes(t: torch.Tensor) -> int:
     return t.numel() * t.element_size()
 
 
 def _op(op: str):
+    if op not in ("sum", "min"):
+        raise KeyError(op)
     n = native.load()
-    return {"sum": n.ReduceOp.SUM, "min": n.ReduceOp.MIN}[op]
+    return n.ReduceOp.SUM if op == "sum" else n.ReduceOp.MIN
 
 
 def ll_max_bytes(world: int) -> int:
@@ -121,12 +119,13 @@ def _ll128_scratch(symm: SymmetricMemory):
 
 
 def _ll_capacity(symm: SymmetricMemory) -> int:
-    import struct
+    cap = symm.__dict__.get("_ll_capacity")
+    if cap is None:  # fixed when the heap is made
+        import struct
 
-    raw = symm.heap.device_comm_bytes()
-    # DeviceComm: 16 x u64 peerBase, mcBase, heapBytes, llScratchOff, llSlotBytes, ...
-    ll_slot = struct.unpack_from("<Q", raw, 8 * 19)[0]
-    return ll_slot // 2
+        # DeviceComm: 16 x u64 peerBase, mcBase, heapBytes, llScratchOff, llSlotBytes, ...
+        cap = symm.__dict__["_ll_capacity"] = struct.unpack_from("<Q", symm.heap.device_comm_bytes(), 8 * 19)[0] // 2
+    return cap
 
 
 def _grid_for(nbytes: int, algo: str, world: int) -> tuple[int, int]:
@@ -175,7 +174,7 @@ def all_reduce(symm: SymmetricMemory, inp: torch.Tensor, out: Optional[torch.Ten
         if not n_blocks:
             slice_bytes = _pipeline_slice_for(symm, nbytes, blocks, scratch.numel())
         n.pipeline_allreduce(symm.heap, inp.data_ptr(), out.data_ptr(), nbytes, torch_dtype_to_native(inp.dtype), _op(op), scratch.data_ptr(),
-                             slice_bytes, blocks, n_threads or 512, _stream(stream), algo == "nvls_block_pipeline", emu_stride)
+                             slice_bytes, blocks, n_threads or 512, stream_handle(stream), algo == "nvls_block_pipeline", emu_stride)
         return out
     blocks, threads = _grid_for(nbytes, algo, symm.world)
     blocks = n_blocks or blocks
@@ -184,7 +183,7 @@ def all_reduce(symm: SymmetricMemory, inp: torch.Tensor, out: Optional[torch.Ten
     if algo in ("packet", "nvls_packet", "allpair_packet"):
         if symm.emulated_mode and not symmetric:
             raise ValueError("emulated ranks need heap tensors")
-        n.allreduce_ll(symm.heap, inp.data_ptr(), out.data_ptr(), nbytes, dt, _op(op), blocks, threads, _stream(stream),
+        n.allreduce_ll(symm.heap, inp.data_ptr(), out.data_ptr(), nbytes, dt, _op(op), blocks, threads, stream_handle(stream),
                        algo == "nvls_packet", algo == "allpair_packet")
     elif algo == "packet128":
         if nbytes > ll128_max_bytes(symm.world):
@@ -195,12 +194,12 @@ def all_reduce(symm: SymmetricMemory, inp: torch.Tensor, out: Optional[torch.Ten
         lines = (nbytes + 119) // 120
         blocks = n_blocks or max(1, min(64, (lines * 8 + 511) // 512))
         n.allreduce_ll128(symm.heap, inp.data_ptr(), out.data_ptr(), nbytes, dt, _op(op), scratch.data_ptr(), slot, blocks, n_threads or 512,
-                          _stream(stream))
+                          stream_handle(stream))
     elif algo in ("rsag_zero_copy", "nvls_zero_copy"):
         if not symmetric:
             raise ValueError(f"{algo} needs tensors from symm.tensor()")
         n.two_shot(symm.heap, inp.data_ptr(), out.data_ptr(), nbytes, dt, _op(op), MODE_ALLREDUCE, blocks, threads,
-                   _stream(stream), algo == "nvls_zero_copy")
+                   stream_handle(stream), algo == "nvls_zero_copy")
     else:
         raise ValueError(f"unknown allreduce algorithm {algo}")
     return out
@@ -214,7 +213,7 @@ def reduce_scatter(symm: SymmetricMemory, inp: torch.Tensor, out: torch.Tensor, 
     assert _nbytes(inp) == _nbytes(out) * symm.world
     blocks, threads = _grid_for(_nbytes(inp), "nvls_zero_copy" if nvls else "rsag_zero_copy", symm.world)
     n.two_shot(symm.heap, inp.data_ptr(), out.data_ptr(), _nbytes(inp), torch_dtype_to_native(inp.dtype), _op(op),
-               MODE_REDUCE_SCATTER, n_blocks or blocks, threads, _stream(stream), nvls)
+               MODE_REDUCE_SCATTER, n_blocks or blocks, threads, stream_handle(stream), nvls)
     return out
 
 
@@ -226,7 +225,7 @@ def all_gather(symm: SymmetricMemory, inp: torch.Tensor, out: torch.Tensor, nvls
     assert _nbytes(out) == _nbytes(inp) * symm.world
     blocks, threads = _grid_for(_nbytes(out), "nvls_zero_copy" if nvls else "rsag_zero_copy", symm.world)
     n.two_shot(symm.heap, inp.data_ptr(), out.data_ptr(), _nbytes(out), torch_dtype_to_native(inp.dtype), _op("sum"),
-               MODE_ALLGATHER, n_blocks or blocks, threads, _stream(stream), nvls)
+               MODE_ALLGATHER, n_blocks or blocks, threads, stream_handle(stream), nvls)
     return out
 
 
@@ -239,7 +238,7 @@ def broadcast(symm: SymmetricMemory, inp: torch.Tensor, out: torch.Tensor, root:
     assert _nbytes(inp) == _nbytes(out) and 0 <= root < symm.world
     blocks, threads = _grid_for(_nbytes(out), "nvls_zero_copy" if nvls else "rsag_zero_copy", symm.world)
     n.two_shot(symm.heap, inp.data_ptr(), out.data_ptr(), _nbytes(out), n.DataType.uint32, _op("sum"), MODE_BROADCAST, n_blocks or blocks,
-               threads, _stream(stream), nvls, root)
+               threads, stream_handle(stream), nvls, root)
     return out
 
 
@@ -250,7 +249,7 @@ def all_to_all(symm: SymmetricMemory, inp: torch.Tensor, out: torch.Tensor, stre
     assert _nbytes(inp) == _nbytes(out) and _nbytes(inp) % (16 * symm.world) == 0 and inp.data_ptr() != out.data_ptr()
     blocks, threads = _grid_for(_nbytes(out), "rsag_zero_copy", symm.world)
     n.two_shot(symm.heap, inp.data_ptr(), out.data_ptr(), _nbytes(out), n.DataType.uint32, _op("sum"), MODE_ALLTOALL, n_blocks or blocks,
-               threads, _stream(stream), False, 0)
+               threads, stream_handle(stream), False, 0)
     return out
 
 
@@ -294,20 +293,20 @@ def all_reduce_rmsnorm(symm: SymmetricMemory, inp: torch.Tensor, out: torch.Tens
         rinv = _rinv_buffer(symm, rows) if mode == 1 else None
         nvls = symm.nvls and algo == "rows"
         n.tp_reduce_norm(symm.heap, inp.data_ptr(), ptr(residual_in), ptr(residual_out), out.data_ptr(), ptr(gamma), ptr(rinv), rows, hidden,
-                         eps, n_blocks, 0, mode, nvls, _stream(stream))
+                         eps, n_blocks, 0, mode, nvls, stream_handle(stream))
         if mode == 1:
-            n.tp_scale_rows(residual_out.data_ptr(), rinv.data_ptr(), ptr(gamma), out.data_ptr(), rows, hidden, _stream(stream))
+            n.tp_scale_rows(residual_out.data_ptr(), rinv.data_ptr(), ptr(gamma), out.data_ptr(), rows, hidden, stream_handle(stream))
         return out
     if algo in ("packet", "nvls_packet"):
         blocks = n_blocks or max(1, min(rows, 64))
         threads = 1024 if hidden * inp.element_size() // 16 >= 1024 else 512
         n.allreduce_ll_rmsnorm(symm.heap, inp.data_ptr(), out.data_ptr(), rows, hidden, dt, eps, ptr(residual_in),
-                               ptr(residual_out), ptr(gamma), blocks, threads, _stream(stream), algo == "nvls_packet")
+                               ptr(residual_out), ptr(gamma), blocks, threads, stream_handle(stream), algo == "nvls_packet")
     else:
         if not symmetric:
             raise ValueError(f"{algo} needs tensors from symm.tensor()")
         own_rows = (rows + symm.world - 1) // symm.world
         blocks = n_blocks or max(1, min(own_rows, 128))
         n.two_shot_rmsnorm(symm.heap, inp.data_ptr(), out.data_ptr(), rows, hidden, dt, eps, ptr(residual_in),
-                           ptr(residual_out), ptr(gamma), True, blocks, 512, _stream(stream), algo == "nvls_zero_copy")
+                           ptr(residual_out), ptr(gamma), True, blocks, 512, stream_handle(stream), algo == "nvls_zero_copy")
     return out

@@ -6,6 +6,7 @@ from typing import Optional
 import torch
 
 from .._core import native
+from .._core.symm import stream_handle
 
 
 def pick_block_n(m: int, n: int) -> int:
@@ -39,7 +40,7 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = No
     if out is None:
         out = torch.empty((m, nn), dtype=torch.bfloat16, device=a.device)
     assert out.is_contiguous() and out.shape == (m, nn)
-    s = (stream or torch.cuda.current_stream()).cuda_stream
+    s = stream_handle(stream)
     if two_sm is None and block_n == 0 and num_ctas == 0 and probe == 0 and band == 0:
         if nn % 64 != 0:
             raise ValueError("N must be a multiple of 64")

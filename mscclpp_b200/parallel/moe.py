@@ -19,7 +19,7 @@ from typing import Optional, Tuple
 import torch
 
 from .._core import native
-from .._core.symm import SymmetricMemory
+from .._core.symm import SymmetricMemory, stream_handle
 
 
 class ExpertParallelDispatcher:
@@ -59,7 +59,7 @@ class ExpertParallelDispatcher:
         t = x.shape[0]
         assert t <= self.max_tokens and x.shape[1] == self.hidden and topk_idx.shape == (t, self.topk)
         assert x.dtype == torch.bfloat16 and topk_idx.dtype == torch.int32 and x.is_contiguous() and topk_idx.is_contiguous()
-        st = (stream or torch.cuda.current_stream()).cuda_stream
+        st = stream_handle(stream)
         n.moe_dispatch(self.symm.heap, x.data_ptr(), topk_idx.data_ptr(), self.slot_map.data_ptr(), self.recv_x.data_ptr(),
                        self.recv_scales.data_ptr() if self.fp8 else 0, self.recv_src.data_ptr(), self.recv_counts.data_ptr(),
                        self.workspace.data_ptr(), t, self.hidden, self.topk, self.num_experts, self.capacity, self.fp8, n_blocks, st)
@@ -70,7 +70,7 @@ class ExpertParallelDispatcher:
         rank: which emulated rank's buffers (emulated heaps only)."""
         assert self.fp8_combine, "construct the dispatcher with fp8_combine=True"
         view = (lambda ten: self.symm.rank_view(ten, rank)) if (self.symm.emulated_mode and rank is not None) else (lambda ten: ten)
-        st = (stream or torch.cuda.current_stream()).cuda_stream
+        st = stream_handle(stream)
         native.load().moe_quantize_rows(view(self.expert_out).data_ptr(), view(self.expert_out_q).data_ptr(), view(self.expert_out_scales).data_ptr(),
                                         rows, self.hidden, st)
 
@@ -89,7 +89,7 @@ class ExpertParallelDispatcher:
             expert_out = self.expert_out if expert_out is None else expert_out
         out = self.y[:t] if out is None else out
         assert topk_weights.dtype == torch.float32 and topk_weights.shape == (t, self.topk) and slot_map.shape == (t, self.topk)
-        st = (stream or torch.cuda.current_stream()).cuda_stream
+        st = stream_handle(stream)
         n.moe_combine(self.symm.heap, topk_idx.data_ptr(), topk_weights.data_ptr(), slot_map.data_ptr(), expert_out.data_ptr(), out.data_ptr(),
                       t, self.hidden, self.topk, self.num_experts, n_blocks, st, self.expert_out_scales.data_ptr() if fp8 else 0)
         return out

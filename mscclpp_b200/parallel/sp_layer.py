@@ -15,7 +15,7 @@ from typing import Optional
 import torch
 
 from .._core import native
-from .._core.symm import SymmetricMemory
+from .._core.symm import SymmetricMemory, stream_handle
 
 ACTIVATIONS = {"none": 0, "gelu": 1, "silu": 2, "swiglu": 3}
 
@@ -43,7 +43,7 @@ def all_gather_gemm(symm: SymmetricMemory, a_local: torch.Tensor, a_full: torch.
     # (block_n < 0: two-SM tiles, 256 x 256 on SM pairs, when the shape allows, else one-SM 256- or 128-wide tiles; on one rank, which has
     # nothing to gather, a plain product in the tiles that suit the shape)
     assert all(w.shape == (n_cols, k) and w.is_contiguous() and w.dtype == torch.bfloat16 for w in weights)
-    st = (stream or torch.cuda.current_stream()).cuda_stream
+    st = stream_handle(stream)
     n.all_gather_gemm(symm.heap, a_local.data_ptr(), a_full.data_ptr(), [w.data_ptr() for w in weights], out.data_ptr(), s_rows, n_cols, k,
                       block_n, num_gemm_ctas, num_copiers, ACTIVATIONS[activation], st)
     return out
@@ -63,7 +63,7 @@ def gemm_reduce_scatter(symm: SymmetricMemory, a, weight, partial: torch.Tensor,
     n_cols = w_list[0].shape[0]
     assert partial.shape == (s_rows, n_cols) and out.shape == (s_rows // symm.world, n_cols)
     nvls = symm.nvls if nvls is None else nvls
-    st = (stream or torch.cuda.current_stream()).cuda_stream
+    st = stream_handle(stream)
     # (block_n < 0: as in all_gather_gemm)
     n.tp_fused(symm.heap, [x.data_ptr() for x in a_list], [w.data_ptr() for w in w_list], partial.data_ptr(), 0, 0, out.data_ptr(), 0, 0,
                s_rows, n_cols, k, 0.0, block_n, num_gemm_ctas, num_reducers, 0, 2, nvls, st)

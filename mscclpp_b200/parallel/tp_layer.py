@@ -15,7 +15,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from .._core.symm import SymmetricMemory
+from .._core.symm import SymmetricMemory, stream_handle
 from ..ops.collectives import all_reduce_rmsnorm
 from ..ops.gemm import gemm_bf16, pick_block_n
 
@@ -103,7 +103,7 @@ class RowParallelLinearNorm:
             bn = 0  # 256 x 256 tiles on pairs of SMs (tcgen05 cta_group::2)
         else:
             bn = block_n or pick_block_n(t, self.out_features)
-        s = (stream or torch.cuda.current_stream()).cuda_stream
+        s = stream_handle(stream)
         if emulated_inputs is not None:
             a_ptrs = [xi.data_ptr() for xi, _ in emulated_inputs]
             b_ptrs = [wi.data_ptr() for _, wi in emulated_inputs]
@@ -143,7 +143,7 @@ class RowParallelLinearNorm:
             self.residual_in[:t].copy_(residual)
         if nvls is None:
             nvls = bool(self.symm.nvls) and self.symm.world > 2
-        s = (stream or torch.cuda.current_stream()).cuda_stream
+        s = stream_handle(stream)
         if emulated_inputs is not None:
             xp = [xi.data_ptr() for xi, _ in emulated_inputs]
             wp = [wi.data_ptr() for _, wi in emulated_inputs]
@@ -191,7 +191,7 @@ class RowParallelLinearNorm:
         rows = slice(row_offset, row_offset + t)
         if residual is not None:
             self.residual_in[rows].copy_(residual)
-        s = (stream or torch.cuda.current_stream()).cuda_stream
+        s = stream_handle(stream)
         # the rows' sums of squares travel in parts ([parts][t] floats, nothing to clear); launches on disjoint row ranges
         # use disjoint pieces of the buffer
         per_row = self.out_features // 64
