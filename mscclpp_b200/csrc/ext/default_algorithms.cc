@@ -195,6 +195,7 @@ std::shared_ptr<Algorithm> makePipeline(const std::string& name, std::shared_ptr
         a.out = out;
         a.bytes = inBytes;
         a.scratch = scratch->base;
+        a.scratchBytes = scratch->bytes;
         a.sliceBytes = slice;
         a.emuRanks = 1;
         a.nvls = nvls ? 1 : 0;

@@ -74,10 +74,13 @@ struct PipeArgs {
   void* out;
   uint64_t bytes;      // any size (a tail shorter than 16 bytes is zero-padded inside the scratch)
   void* scratch;
+  uint64_t scratchBytes;  // what there is of it, the same number in all launches that use it: fixes where its two halves meet. 0: not known,
+                          // the launch is as large as its slices need and ends with a barrier
   uint64_t sliceBytes;
   uint64_t emuStride;
   int emuRanks;
   int nvls;
+  uint64_t outOffset;     // set by launchPipelineAllreduce: scratch-out begins here
 };
 size_t pipelineScratchBytes(int nBlocks, uint64_t sliceBytes);
 cudaError_t launchPipelineAllreduce(const PipeArgs& args, DataType dtype, ReduceOp op, int nBlocks, int nThreads, cudaStream_t stream);

@@ -166,7 +166,9 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
   const uint64_t subUnits = sliceUnits / world;
   const uint64_t roundUnits = sliceUnits * gridDim.x;
   const uint64_t rounds = (nunits + roundUnits - 1) / roundUnits;
-  // scratch (heap offset, equal on every rank): [parity][in | out][slot][sliceBytes]
+  // scratch (heap offset, equal on every rank): [in | out][parity][slot][sliceBytes]. A rank that is through with a launch may copy in
+  // for its next one, with other slices, while its peers still fetch reduced parts of this one from it, so where `out` begins
+  // must not change from launch to launch.
   const uint64_t scratchOff = reinterpret_cast<uint64_t>(a.scratch) - c.peerBase[c.rank];
   const uint64_t local = c.peerBase[rank];
   __shared__ int okSmem[2];
@@ -175,9 +177,9 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
   if (threadIdx.x < 2) okSmem[threadIdx.x] = 1;
   __syncthreads();
 
-  const uint64_t roundBytes = 2ull * gridDim.x * a.sliceBytes;  // scratch of one parity
+  const uint64_t parityBytes = static_cast<uint64_t>(gridDim.x) * a.sliceBytes;
   const uint32_t tailBytes = static_cast<uint32_t>(bytes & 15);   // of the message's last unit, 0 = it is whole
-  auto inSliceOf = [&](uint64_t r) { return scratchOff + (r & 1) * roundBytes + static_cast<uint64_t>(slot) * a.sliceBytes; };
+  auto inSliceOf = [&](uint64_t r) { return scratchOff + (r & 1) * parityBytes + static_cast<uint64_t>(slot) * a.sliceBytes; };
   auto firstOf = [&](uint64_t r) { return r * roundUnits + static_cast<uint64_t>(slot) * sliceUnits; };  // first global unit of my slice
   auto haveOf = [&](uint64_t r) {  // units of my slice that exist, the last of them possibly not whole
     const uint64_t first = firstOf(r);
@@ -216,7 +218,7 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
 #pragma unroll 1
   for (uint64_t r = 0; r < rounds; r++) {
     const uint64_t inSlice = inSliceOf(r);
-    const uint64_t outSlice = inSlice + static_cast<uint64_t>(gridDim.x) * a.sliceBytes;
+    const uint64_t outSlice = inSlice + a.outOffset;
     const uint32_t have = haveOf(r);
     // 2. every rank has staged its slice of this index
     healthy = pipeWait(c, rank, 0, slot, tokenOf(r), okSmem);
@@ -324,6 +326,12 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
       copyTail(dst + static_cast<uint64_t>(whole) * 16, reinterpret_cast<const char*>(from + outSlice) + static_cast<uint64_t>(whole) * 16, tail, 0);
     }
   }
+  if constexpr (!kNvls) {  // the next launch may have its halves elsewhere: nobody goes on while a peer fetches
+    if (pull && a.scratchBytes == 0 && healthy) {
+      pipeSignal(c, rank, 1, slot, tokenOf(rounds));
+      pipeWait(c, rank, 1, slot, tokenOf(rounds), okSmem);
+    }
+  }
   finishLaunch(c, rank, epoch);
 }
 
@@ -342,6 +350,7 @@ cudaError_t launchPipeTyped(const PipeArgs& a, int nBlocks, int nThreads, cudaSt
     kernel = reinterpret_cast<const void*>(pipelineAllreduceKernel<T, Op, false>);
   }
   PipeArgs copy = a;
+  copy.outOffset = a.scratchBytes != 0 ? a.scratchBytes / 32 * 16 : pipelineScratchBytes(nBlocks, a.sliceBytes) / 2;
   void* params[] = {&copy};
   if (a.emuRanks > 1) return launchEmulatedRanks(kernel, grid, block, params, 2, stream);
   return cudaLaunchKernel(kernel, grid, block, params, 0, stream);
@@ -356,6 +365,7 @@ cudaError_t launchPipelineAllreduce(const PipeArgs& args, DataType dtype, Reduce
   if (args.bytes == 0 || world < 1 || world > 8) return cudaErrorInvalidValue;
   if (nBlocks < 1 || nBlocks > kBarrierSlots || nThreads < 32 || nThreads > 512 || nThreads < world) return cudaErrorInvalidValue;
   if (args.sliceBytes == 0 || args.sliceBytes % (16ull * world) != 0) return cudaErrorInvalidValue;
+  if (args.scratchBytes != 0 && args.scratchBytes < pipelineScratchBytes(nBlocks, args.sliceBytes)) return cudaErrorInvalidValue;
   if (args.scratch == nullptr || (reinterpret_cast<uintptr_t>(args.scratch) & 15) != 0) return cudaErrorInvalidValue;
   if (args.nvls && args.comm.mcBase == 0) return cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(args.in) & 15) != 0 || (reinterpret_cast<uintptr_t>(args.out) & 15) != 0) return cudaErrorInvalidValue;

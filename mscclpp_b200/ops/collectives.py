@@ -171,10 +171,11 @@ def all_reduce(symm: SymmetricMemory, inp: torch.Tensor, out: Optional[torch.Ten
             if not n_blocks:
                 blocks = min(PIPELINE_MAX_BLOCKS, -(-nbytes * symm.world // (2 * PIPELINE_SLICE_BYTES)))
             blocks = max(1, min(blocks, 2 * sms // symm.world))
-        if not n_blocks:
+        if not n_blocks or blocks > PIPELINE_MAX_BLOCKS:
             slice_bytes = _pipeline_slice_for(symm, nbytes, blocks, scratch.numel())
         n.pipeline_allreduce(symm.heap, inp.data_ptr(), out.data_ptr(), nbytes, torch_dtype_to_native(inp.dtype), _op(op), scratch.data_ptr(),
-                             slice_bytes, blocks, n_threads or 512, stream_handle(stream), algo == "nvls_block_pipeline", emu_stride)
+                             slice_bytes, blocks, n_threads or 512, stream_handle(stream), algo == "nvls_block_pipeline", emu_stride,
+                             scratch.numel())
         return out
     blocks, threads = _grid_for(nbytes, algo, symm.world)
     blocks = n_blocks or blocks

@@ -108,6 +108,41 @@ def test_allreduce_pipeline_ragged(world, numel, n_blocks, dtype):
     symm.destroy()
 
 
+def test_allreduce_pipeline_scratch_halves_stay_apart():
+    """Peers may still fetch reduced parts of a launch when a rank copies in for the next one, which has other slices: what is
+    copied in stays in the scratch's first half and what is reduced in its second, whatever the slices. A launch that is not told
+    the scratch's size ends with a barrier instead."""
+    from mscclpp_b200 import native
+    from mscclpp_b200.ops import all_reduce
+    from mscclpp_b200.ops import collectives as C
+
+    world = 4
+    symm = _symm(world)
+    scratch = C._pipeline_scratch(symm)
+    halves = [symm.rank_view(scratch, r).view(torch.float32).chunk(2) for r in range(world)]
+    for first, second in halves:
+        first.zero_(), second.zero_()
+    for numel, n_blocks in ((37 << 10, 0), (8 << 20, 0), (1 << 20, 3), (3 << 20, 7), (5000, 0)):
+        x = torch.ones(world, numel, device="cuda")
+        out = torch.empty_like(x)
+        all_reduce(symm, x, out, algo="rsag_pipeline", n_blocks=n_blocks)
+        assert bool((out == world).all())
+        for first, second in halves:
+            assert bool((first == 1).any()) and not bool((first == world).any())
+            assert bool((second == world).any()) and not bool((second == 1).any())
+    n = native()
+    for blocks, slice_bytes in ((5, 4096), (16, 64 << 10)):
+        out.zero_()
+        n.pipeline_allreduce(symm.heap, x.data_ptr(), out.data_ptr(), numel * 4, n.DataType.float32, n.ReduceOp.SUM, scratch.data_ptr(),
+                             slice_bytes, blocks, 512, torch.cuda.current_stream().cuda_stream, False, numel * 4)
+        assert bool((out == world).all())
+    with pytest.raises(Exception):
+        n.pipeline_allreduce(symm.heap, x.data_ptr(), out.data_ptr(), numel * 4, n.DataType.float32, n.ReduceOp.SUM, scratch.data_ptr(),
+                             64 << 10, 16, 512, torch.cuda.current_stream().cuda_stream, False, numel * 4, 1 << 20)
+    symm.check()
+    symm.destroy()
+
+
 @pytest.mark.parametrize("world", [2, 8])
 def test_allreduce_ll_int_and_min(world):
     from mscclpp_b200.ops import all_reduce
