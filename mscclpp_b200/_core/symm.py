@@ -96,7 +96,7 @@ class SymmetricMemory:
     @classmethod
     def emulated(cls, world: int, nbytes: int = 256 << 20, ll_slot_bytes: int = 0, timeout_ms: int = 2000,
                  device: Optional[torch.device] = None) -> "SymmetricMemory":
-        """`world` heaps on one GPU; collective kernels run all ranks in one cooperative launch."""
+        """`world` heaps on one GPU; collective kernels run all ranks in one launch."""
         n = native.load()
         device = device or torch.device("cuda", torch.cuda.current_device())
         with torch.cuda.device(device):

@@ -7,7 +7,7 @@
 // each heap hold a SymmControl block: launch epoch, cross-rank barrier flags and LL packet scratch.
 //
 // Kernels can also run several "emulated" ranks inside ONE launch on ONE GPU (gridDim.y = world,
-// rank = comm.rank + blockIdx.y, cooperative launch). That is how multi-rank protocols are tested
+// rank = comm.rank + blockIdx.y, a cooperative launch or clusters of the ranks). That is how multi-rank protocols are tested
 // when fewer GPUs than ranks are available: separate launches that wait on one another are never
 // used, because nothing guarantees that they are co-resident.
 #pragma once

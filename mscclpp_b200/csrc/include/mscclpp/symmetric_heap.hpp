@@ -10,7 +10,7 @@
 // src/core/switch_channel.cc:174-191; its API is kept in core.hpp for code that wants it.)
 //
 // An "emulated" heap places `world` heaps of one process on ONE device, for running multi-rank
-// kernels as a single cooperative launch when fewer GPUs than ranks are available.
+// kernels as a single launch when fewer GPUs than ranks are available.
 #pragma once
 
 #include <cstddef>

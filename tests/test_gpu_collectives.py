@@ -1,6 +1,6 @@
 """Native collective kernels against a plain PyTorch fp32 reference.
 
-All ranks are emulated on ONE GPU: the kernels run every rank inside one cooperative launch
+All ranks are emulated on ONE GPU: the kernels run every rank inside one launch
 (gridDim.y = world), which exercises exactly the device code that runs across GPUs, minus NVLS.
 """
 import pytest
