@@ -57,9 +57,6 @@ cudaError_t launchAllreduceLL128(const CollArgs& args, DataType dtype, ReduceOp 
 cudaError_t launchTwoShot(const CollArgs& args, DataType dtype, ReduceOp op, int nBlocks, int nThreads,
                           cudaStream_t stream);
 
-// Allreduce of buffers outside the symmetric heap through heap scratch, pipelined inside one kernel (see
-// collectives_pipeline.cu). `scratch`: pipelineScratchBytes(nBlocks, sliceBytes) bytes of symmetric-heap memory at the
-// same offset on every rank. sliceBytes: a multiple of 16 * world; one round moves nBlocks * sliceBytes of the message.
 // Launch of emulated ranks (grid.y of them), for kernels whose blocks only ever wait for the blocks of the same index on the other
 // ranks: they have to run at the same time. A cluster of them does, without what a cooperative launch costs the host and the device
 // (packet allreduce of two ranks, called eagerly, 11.7 -> 8.0 us with the launch over the kernel before it). Clusters may not leave their
@@ -68,6 +65,9 @@ cudaError_t launchTwoShot(const CollArgs& args, DataType dtype, ReduceOp op, int
 // groups hold at least that. overlapped: the kernel waits for the one before it by itself (ptx::grid_dependency_wait).
 cudaError_t launchEmulatedRanks(const void* kernel, dim3 grid, dim3 block, void** params, int blocksPerSm, cudaStream_t stream, bool overlapped = false);
 
+// Allreduce of buffers outside the symmetric heap through heap scratch, pipelined inside one kernel (see
+// collectives_pipeline.cu). `scratch`: pipelineScratchBytes(nBlocks, sliceBytes) bytes of symmetric-heap memory at the
+// same offset on every rank. sliceBytes: a multiple of 16 * world; one round moves nBlocks * sliceBytes of the message.
 struct PipeArgs {
   DeviceComm comm;
   const void* in;      // local buffer, anywhere in device memory, 16-byte aligned; emulated rank e uses in + e * emuStride
