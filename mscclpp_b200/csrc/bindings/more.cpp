@@ -46,6 +46,7 @@ void registerMoreBindings(py::module_& m) {
           py::arg("dtype"), py::arg("plan"), py::arg("stream") = 0, py::arg("packet_type") = PacketType::LL16)
       .def("reset", &Executor::reset)
       .def("zero_copy_launches", &Executor::zeroCopyLaunches)
+      .def("last_team", &Executor::lastTeam)
       .def("check_canaries", &Executor::checkCanaries)
       .def("canary_regions", [](const Executor& self) {
         std::vector<std::tuple<std::string, uint64_t, size_t>> out;

@@ -760,12 +760,11 @@ int residentTeams(const void* kernel, int team, int nThreads) {
 }
 
 template <typename T>
-cudaError_t launchTyped(const ExecArgs& args, int nBlocks, int nThreads, cudaStream_t stream) {
+cudaError_t launchTyped(ExecArgs& args, int nBlocks, int nThreads, cudaStream_t stream) {
   const int emu = args.emuRanks > 1 ? args.emuRanks : 1;
   dim3 block(nThreads, 1, 1);
   // thread blocks of a plan wait on one another (barriers, semaphores) and on peers: co-residency is required
-  ExecArgs copy = args;
-  void* params[] = {&copy};
+  void* params[] = {&args};
   const void* kernel = args.packetLL8 ? reinterpret_cast<const void*>(executionKernel<T, LL8Packet, false>)
                                       : reinterpret_cast<const void*>(executionKernel<T, LL16Packet, false>);
   const void* teams = reinterpret_cast<const void*>(executionKernel<T, LL16Packet, true>);  // (of plans without packets)
@@ -778,15 +777,15 @@ cudaError_t launchTyped(const ExecArgs& args, int nBlocks, int nThreads, cudaStr
     return cudaErrorCooperativeLaunchTooLarge;
   }
   // teams only of SMs that nobody else of the launch needs
-  if (nThreads % 32 != 0) copy.team = 1;
-  while (copy.team > 1 && (nBlocks * emu * copy.team > sms || nBlocks * emu > residentTeams(teams, copy.team, nThreads))) copy.team /= 2;
-  if (copy.team > 1) return gemm::launchClusters(teams, copy.team, dim3(nBlocks * copy.team, emu), block, 0, params, true, stream);
+  if (nThreads % 32 != 0) args.team = 1;
+  while (args.team > 1 && (nBlocks * emu * args.team > sms || nBlocks * emu > residentTeams(teams, args.team, nThreads))) args.team /= 2;
+  if (args.team > 1) return gemm::launchClusters(teams, args.team, dim3(nBlocks * args.team, emu), block, 0, params, true, stream);
   return cudaLaunchCooperativeKernel(kernel, dim3(nBlocks, emu), block, params, 0, stream);
 }
 
 }  // namespace
 
-cudaError_t launchExecutionKernel(const ExecArgs& args, DataType dtype, int nBlocks, int nThreads, cudaStream_t stream) {
+cudaError_t launchExecutionKernel(ExecArgs& args, DataType dtype, int nBlocks, int nThreads, cudaStream_t stream) {
   if (nBlocks < 1 || nThreads < 32 || nThreads > 1024) return cudaErrorInvalidValue;
   switch (dtype) {
     case DataType::FLOAT16:

@@ -455,6 +455,7 @@ struct Executor::Impl {
   std::shared_ptr<mscclpp::Context> regContext;
   std::map<std::pair<uintptr_t, size_t>, MappedBuffer> mapped;
   uint64_t zeroCopyLaunches = 0;
+  int lastTeam = 0;
 
   // ---- guard bands around the executor's own heap buffers (MSCCLPP_EXECUTOR_CANARY=1). The reference has no such
   // check; its plans are trusted. Here a plan's operands are range-checked when they are resolved, and the bands catch
@@ -762,6 +763,7 @@ Executor::~Executor() {
 
 std::shared_ptr<SymmetricHeap> Executor::heap() const { return impl_->heap; }
 uint64_t Executor::zeroCopyLaunches() const { return impl_->zeroCopyLaunches; }
+int Executor::lastTeam() const { return impl_->lastTeam; }
 std::vector<Executor::CanaryRegion> Executor::canaryRegions() const { return impl_->canaryRegions(); }
 size_t Executor::checkCanaries() { return impl_->checkCanaries(); }
 
@@ -1003,6 +1005,7 @@ void Executor::execute(int rank, void* sendbuff, void* recvbuff, size_t sendBuff
   args.npkit = NpKit::GetGpuEventCollectContexts();
   if (ctx.maxThreadBlocks > 0) {
     cudaError_t e = launchExecutionKernel(args, dataType, ctx.maxThreadBlocks, p.nThreadsPerBlock, stream);
+    impl_->lastTeam = args.team;
     if (e == cudaErrorCooperativeLaunchTooLarge) {
       (void)cudaGetLastError();
       throw Error("plan '" + p.name + "' needs " + std::to_string(ctx.maxThreadBlocks) + " thread blocks of " + std::to_string(p.nThreadsPerBlock) +

@@ -61,6 +61,8 @@ class Executor {
   std::shared_ptr<SymmetricHeap> heap() const;
   // How many execute() calls so far ran directly on buffers outside the heap (mapped on every rank) instead of staging them.
   uint64_t zeroCopyLaunches() const;
+  // How many CTAs shared each thread block of the plan in the latest launch (1: one each; 0: nothing has been launched).
+  int lastTeam() const;
 
   // Debugging aid, switched on with MSCCLPP_EXECUTOR_CANARY=1 when the executor is created: every buffer the executor
   // allocates for a plan (scratch, staging) gets a guard band of 256 bytes of 0xA5 on both sides. checkCanaries()

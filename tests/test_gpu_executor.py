@@ -48,8 +48,10 @@ def _run_both(plan_json, world, in_elems, out_elems, np_dtype, inplace, launches
             else:
                 np.testing.assert_allclose(got.astype(np.float32), expect[r].astype(np.float32), rtol=2e-3, atol=2e-3,
                                            err_msg=f"rank {r} of {world}, launch {launch}, {in_elems} elements, packets {packet_type}")
+    team = executor.last_team()
     executor.reset()
     symm.destroy()
+    return team
 
 
 @pytest.mark.parametrize("world", [2, 4, 8])
@@ -249,10 +251,67 @@ def test_thread_blocks_of_several_ctas(world, instances, per):
     from mscclpp_b200.default_algos import single_node
 
     build = lambda name: single_node.build(name, world, instances=instances, in_place=False).to_json()
-    _run_both(build("reducescatter_allpairs"), world, world * per, per, np.float16, inplace=False)
-    _run_both(build("alltoall_allpairs"), world, world * per, world * per, np.float16, inplace=False)
-    _run_both(build("allgather_allpairs"), world, per, world * per, np.float16, inplace=False)
-    _run_both(single_node.build("allreduce_nvls", world, instances=instances).to_json(), world, world * per, world * per, np.float16, inplace=True)
+    teams = [_run_both(build("reducescatter_allpairs"), world, world * per, per, np.float16, inplace=False),
+             _run_both(build("alltoall_allpairs"), world, world * per, world * per, np.float16, inplace=False),
+             _run_both(build("allgather_allpairs"), world, per, world * per, np.float16, inplace=False),
+             _run_both(single_node.build("allreduce_nvls", world, instances=instances).to_json(), world, world * per, world * per, np.float16, inplace=True)]
+    assert all(t in (1, 2, 4, 8) for t in teams) and teams[0] > 1
+
+
+def _plan_of_large_operations(kind):
+    """Two ranks: what a thread block does once (barrier, semaphore, request to the host proxy) between the operations that its CTAs
+    share, a pipeline, and sizes that leave a part of a word."""
+    from mscclpp_b200.default_algos.single_node import make_spec
+    from mscclpp_b200.language.channel import MemoryChannel, PortChannel
+    from mscclpp_b200.language.collectives import AllReduce
+    from mscclpp_b200.language.loop import LoopIterationContext
+    from mscclpp_b200.language.program import CollectiveProgram
+    from mscclpp_b200.language.rank import Buffer, Rank, Semaphore
+
+    prog = CollectiveProgram.from_spec(make_spec(f"large_{kind}", AllReduce(2, 2, True), 2, buffer_alignment=4 if kind == "tail" else 16))
+    with prog:
+        scratch = [Buffer(r, 2) for r in range(2)]
+        inputs = [Rank(r).get_input_buffer() for r in range(2)]
+        if kind in ("port", "tail"):
+            chan = [(PortChannel if kind == "port" else MemoryChannel)(1 - r, r) for r in range(2)]
+            for r in range(2):
+                chan[r].put(scratch[1 - r][0:1], inputs[r][0:1], tb=0)
+                chan[r].signal(tb=0)
+            for r in range(2):
+                chan[r].wait(tb=0)
+                Rank(r).reduce(scratch[r][0:1], [inputs[r][0:1]], tb=0)
+            for r in range(2):
+                Rank(r).copy(inputs[r][0:1], scratch[r][0:1], tb=0)
+            return prog.to_json()
+        for r in range(2):
+            rank, inp, s = Rank(r), inputs[r], scratch[r]
+            if kind == "barrier":
+                for tb in range(2):
+                    rank.copy(s[tb:tb + 1], inp[tb:tb + 1], tb=tb)
+                rank.barrier([0, 1])
+                for tb in range(2):
+                    rank.reduce(inp[2 + tb:3 + tb], [s[1 - tb:2 - tb]], tb=tb)
+                rank.barrier([0, 1])
+                for tb in range(2):
+                    rank.copy(inp[tb:tb + 1], inp[3 - tb:4 - tb], tb=tb)
+            else:
+                sem = Semaphore(r, 0)
+                loop = LoopIterationContext(unit=512 << 10, num_chunks=1) if kind == "pipeline" else None
+                if loop is not None:
+                    loop.__enter__()
+                rank.copy(s[0:1], inp[0:1], tb=0)
+                sem.release(tb=0)
+                sem.acquire(tb=1)
+                rank.reduce(inp[2:3], [s[0:1]], tb=1)
+                if loop is not None:
+                    loop.__exit__(None, None, None)
+    return prog.to_json()
+
+
+@pytest.mark.parametrize("kind,per", [("barrier", (512 << 10) + 48), ("semaphore", (512 << 10) + 48), ("pipeline", (1536 << 10) + 80), ("port", (512 << 10) + 48),
+                                      ("tail", (512 << 10) + 4)])
+def test_what_a_thread_block_of_several_ctas_does_once(kind, per):
+    assert _run_both(_plan_of_large_operations(kind), 2, per, per, np.int32, inplace=True, launches=3) == 8  # (four chunks of `per` bytes, int32)
 
 
 def test_a_wait_that_runs_out_ends_every_cta_of_a_thread_block():
@@ -284,6 +343,7 @@ def test_a_wait_that_runs_out_ends_every_cta_of_a_thread_block():
         torch.cuda.synchronize()
 
     run(lacking)
+    assert executor.last_team() == 8
     with pytest.raises(Exception, match="gave up"):
         symm.check()
     for r in range(2):
