@@ -58,32 +58,51 @@ struct Ctx {
   uint64_t pipeUnit;  // bytes per pipeline iteration (0 = not in a pipeline)
   uint32_t* barrierPasses;  // shared memory: grid barriers this block has passed in this launch, per barrier id
   bool healthy;  // the same in every thread of the block (of the team): operations run as a whole or not at all
-  int* ok;       // shared memory, 1 until a wait of this thread block has run out
-  int team, member;        // CTAs that share the plan thread block, and which of them this one is
-  uint32_t tid, threads;  // this thread among those of all of them
 };
+// What a team of CTAs needs (kTeams), and what is left of it where the thread block is a CTA. Nothing of it is kept in a register: with these as
+// members of Ctx, and a reduction with eight loads in flight, the kernel without teams spilled half as much again (64 puts of 4 KB with signal
+// and wait 422 us before there were teams, 455 so, 430 now).
+template <bool kTeams>
+struct TeamCtx : Ctx {
+  // CTAs that share the plan thread block, and which of them this one is
+  MSCCLPP_DEVICE_INLINE int team() const { return kTeams ? a->team : 1; }
+  MSCCLPP_DEVICE_INLINE int member() const { return kTeams ? static_cast<int>(ptx::cluster_ctarank()) : 0; }
+  // this thread among those of all of them
+  MSCCLPP_DEVICE_INLINE uint32_t tid() const { return kTeams ? static_cast<uint32_t>(member()) * blockDim.x + threadIdx.x : threadIdx.x; }
+  MSCCLPP_DEVICE_INLINE uint32_t threads() const { return kTeams ? static_cast<uint32_t>(team()) * blockDim.x : blockDim.x; }
+};
+// 1 until a wait of this thread block has run out.
+MSCCLPP_DEVICE_INLINE int& teamOk() {
+  __shared__ int ok;
+  return ok;
+}
 
 // The plan thread block's barrier: among the threads of the CTA, or of all CTAs of its team. What one of them has read or written is
 // ordered before what another one does behind it.
-MSCCLPP_DEVICE_INLINE void teamSync(const Ctx& x) {
-  if (x.team == 1) {
-    __syncthreads();
-  } else {
+template <bool kTeams>
+MSCCLPP_DEVICE_INLINE void teamSync(const TeamCtx<kTeams>&) {
+  if constexpr (kTeams) {
     __syncwarp();
     ptx::cluster_sync_all();
+  } else {
+    __syncthreads();
   }
 }
 // A wait of the first CTA's has run out: its team hears of it at the barrier that ends the operation. (The others are there: they cannot
 // have gone before that barrier.)
-MSCCLPP_DEVICE_INLINE void teamGivesUp(const Ctx& x) {
-  *x.ok = 0;
-  for (int m = 1; m < x.team; m++)
-    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(ptx::mapa_shared(ptx::smem_u32(x.ok), m)), "r"(0) : "memory");
+template <bool kTeams>
+MSCCLPP_DEVICE_INLINE void teamGivesUp(const TeamCtx<kTeams>& x) {
+  teamOk() = 0;
+  if constexpr (kTeams) {
+    for (int m = 1; m < x.team(); m++)
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(ptx::mapa_shared(ptx::smem_u32(&teamOk()), m)), "r"(0) : "memory");
+  }
 }
 // End of an operation in which threads of the first CTA have waited. It began with a teamSync: by then everybody had read `ok`.
-MSCCLPP_DEVICE_INLINE void teamVerdict(Ctx& x) {
+template <bool kTeams>
+MSCCLPP_DEVICE_INLINE void teamVerdict(TeamCtx<kTeams>& x) {
   teamSync(x);
-  if (*x.ok == 0) x.healthy = false;
+  if (teamOk() == 0) x.healthy = false;
 }
 
 // End of an operation whose threads wait on their own (packets: a thread without one has nothing to miss): the block agrees on
@@ -144,9 +163,10 @@ MSCCLPP_DEVICE_INLINE void writeWords(Pkt* pk, int words, uint4 v, uint32_t epoc
   }
 }
 
-MSCCLPP_DEVICE_INLINE void signalChannels(const Ctx& x, const DevOp& op, bool relaxed) {
+template <bool kTeams>
+MSCCLPP_DEVICE_INLINE void signalChannels(const TeamCtx<kTeams>& x, const DevOp& op, bool relaxed) {
   const int t = threadIdx.x;
-  if (t < op.nIds && x.member == 0) {
+  if (t < op.nIds && x.member() == 0) {
     const DevChannel ch = x.plan->channels[op.channelType][op.ids[t]];
     ExecState* peer = reinterpret_cast<ExecState*>(x.c->peerBase[ch.peer] + x.a->stateOff);
     if (relaxed) {
@@ -158,10 +178,11 @@ MSCCLPP_DEVICE_INLINE void signalChannels(const Ctx& x, const DevOp& op, bool re
   }
 }
 
-MSCCLPP_DEVICE_INLINE void waitChannels(Ctx& x, const DevOp& op, bool relaxed) {
+template <bool kTeams>
+MSCCLPP_DEVICE_INLINE void waitChannels(TeamCtx<kTeams>& x, const DevOp& op, bool relaxed) {
   teamSync(x);
   const int t = threadIdx.x;
-  if (t < op.nIds && x.member == 0) {
+  if (t < op.nIds && x.member() == 0) {
     const int cid = op.ids[t];
     const uint64_t expect = ++x.state->expected[op.channelType][cid];
     if (!waitGreaterEqual(&x.state->inbound[op.channelType][cid], expect, x.c->status, x.c->timeoutNs, kDevTimeoutSemaphore,
@@ -177,9 +198,10 @@ MSCCLPP_DEVICE_INLINE void waitChannels(Ctx& x, const DevOp& op, bool relaxed) {
 // and/or sync; with sync the thread also waits (bounded) until the proxy has consumed the request, which it does only
 // after its copy stream has drained.
 // packetSpace: both ends are packet-format scratch ranges (the bytes moved are the packets themselves, twice the payload).
-MSCCLPP_DEVICE_INLINE void portRequests(Ctx& x, const DevOp& op, uint32_t kind, bool packetSpace = false) {
+template <bool kTeams>
+MSCCLPP_DEVICE_INLINE void portRequests(TeamCtx<kTeams>& x, const DevOp& op, uint32_t kind, bool packetSpace = false) {
   teamSync(x);  // data this thread block produced for the put is complete
-  if (threadIdx.x == 0 && x.member == 0) {
+  if (threadIdx.x == 0 && x.member() == 0) {
     int portOk = 1;
     __threadfence_system();  // ... and visible to the copy engines
     FifoDeviceHandle fifo = x.a->portFifo;
@@ -226,22 +248,25 @@ MSCCLPP_DEVICE_INLINE void portRequests(Ctx& x, const DevOp& op, uint32_t kind, 
 
 // The vector body of a reduction, a function of its own: inlined into the interpreter it has to share 64 registers with
 // every other operation's state, and the loads in flight are what gets spilled.
-template <typename T>
+template <typename T, bool kTeams>
 __noinline__ __device__ void reduceWords(char* const* src, int nSrc, char* const* dst, int nDst, uint64_t nvec, uint32_t tid, uint32_t threads) {
   uint64_t i = tid;
-  // two sources: four words at a time, so that there are eight loads in flight (reduce-scatter of 16 MB over two ranks, 16 blocks: 70 -> 52 us)
+  // Two sources: several words at a time, so that there are more than two loads in flight. Four words where a team of CTAs has much to reduce
+  // (reduce-scatter of 16 MB over two ranks, 16 blocks of 8 CTAs: 31.7 us with two, 28.9 with four); in the kernel without teams two, since four
+  // make every operation slower (64 puts of 4 KB with signal and wait 432 us with one or two, 455 with four).
+  constexpr int kWords = kTeams ? 4 : 2;
   if (nSrc == 2) {
     const char *s0 = src[0], *s1 = src[1];
 #pragma unroll 1
-    for (; i + 3ull * threads < nvec; i += 4ull * threads) {
-      uint4 v[4], w[4];
+    for (; i + (kWords - 1ull) * threads < nvec; i += static_cast<uint64_t>(kWords) * threads) {
+      uint4 v[kWords], w[kWords];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
+      for (int k = 0; k < kWords; k++) {
         v[k] = ptx::ld_weak_v4(s0 + (i + static_cast<uint64_t>(k) * threads) * 16);
         w[k] = ptx::ld_weak_v4(s1 + (i + static_cast<uint64_t>(k) * threads) * 16);
       }
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
+      for (int k = 0; k < kWords; k++) {
         ExecAccum<T> acc;
         acc.init(v[k]);
         acc.add(w[k]);
@@ -251,7 +276,7 @@ __noinline__ __device__ void reduceWords(char* const* src, int nSrc, char* const
       for (int d = 0; d < nDst; d++) {
         char* to = dst[d] + i * 16;
 #pragma unroll
-        for (int k = 0; k < 4; k++) ptx::st_weak_v4(to + static_cast<uint64_t>(k) * threads * 16, v[k]);
+        for (int k = 0; k < kWords; k++) ptx::st_weak_v4(to + static_cast<uint64_t>(k) * threads * 16, v[k]);
       }
     }
   }
@@ -283,8 +308,8 @@ __noinline__ __device__ void reduceWords(char* const* src, int nSrc, char* const
 }
 
 // dst[k] (all of them) = sum over src[*]. Sizes are multiples of 16 bytes (plans align chunks to 16).
-template <typename T>
-MSCCLPP_DEVICE_INLINE void reduceOp(const Ctx& x, const DevOp& op) {
+template <typename T, bool kTeams>
+MSCCLPP_DEVICE_INLINE void reduceOp(const TeamCtx<kTeams>& x, const DevOp& op) {
   uint64_t skip;
   const uint64_t bytes = sliced(x, op, op.src[0], skip);
   const uint64_t nvec = bytes / 16;
@@ -298,10 +323,10 @@ MSCCLPP_DEVICE_INLINE void reduceOp(const Ctx& x, const DevOp& op) {
   if (threadIdx.x < static_cast<uint32_t>(nSrc)) srcAddr[threadIdx.x] = plainAddr(x, op.src[threadIdx.x], skip);
   if (threadIdx.x >= 32 - static_cast<uint32_t>(nDst) && threadIdx.x < 32) dstAddr[31 - threadIdx.x] = plainAddr(x, op.dst[31 - threadIdx.x], skip);
   __syncthreads();
-  reduceWords<T>(srcAddr, nSrc, dstAddr, nDst, nvec, x.tid, x.threads);
+  reduceWords<T, kTeams>(srcAddr, nSrc, dstAddr, nDst, nvec, x.tid(), x.threads());
   // tail shorter than one vector (only with alignment < 16): element-wise through a zero-padded word
   const uint64_t tail = bytes - nvec * 16;
-  if (tail != 0 && x.tid == 0) {
+  if (tail != 0 && x.tid() == 0) {
     auto load = [&](const DevOperand& o) {
       uint32_t w[4] = {0, 0, 0, 0};
       const char* p = plainAddr(x, o, skip) + nvec * 16;
@@ -419,22 +444,23 @@ __noinline__ __device__ void copyWords(char* dst, const char* src, uint64_t word
 constexpr uint64_t kCopyWordsMin = 64 << 10;  // bytes: every thread of a block has its four
 
 // src[k] -> dst[k] of a put, get or copy.
-MSCCLPP_DEVICE_INLINE void copyOp(const Ctx& x, const DevOp& op) {
+template <bool kTeams>
+MSCCLPP_DEVICE_INLINE void copyOp(const TeamCtx<kTeams>& x, const DevOp& op) {
   uint64_t skip = 0;
   for (int i = 0; i < op.nDst; i++) {
     const uint64_t n = sliced(x, op, op.src[i], skip);
     char* dst = plainAddr(x, op.dst[i], skip);
     const char* src = plainAddr(x, op.src[i], skip);
     if (n >= kCopyWordsMin && ((reinterpret_cast<uint64_t>(dst) | reinterpret_cast<uint64_t>(src) | n) & 15) == 0) {
-      copyWords(dst, src, n / 16, x.tid, x.threads);
+      copyWords(dst, src, n / 16, x.tid(), x.threads());
     } else {
-      copyBytes(dst, src, n, x.tid, x.threads);
+      copyBytes(dst, src, n, x.tid(), x.threads());
     }
   }
 }
 
-template <typename T, typename Pkt>
-MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
+template <typename T, typename Pkt, bool kTeams>
+MSCCLPP_DEVICE_INLINE void execOp(TeamCtx<kTeams>& x, const DevOp& op) {
   using Payload = typename Pkt::Payload;
   const OpType type = static_cast<OpType>(op.type);
   uint64_t skip = 0;
@@ -444,7 +470,7 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
       break;
     case OpType::BARRIER: {
       teamSync(x);
-      if (threadIdx.x == 0 && x.member == 0) {
+      if (threadIdx.x == 0 && x.member() == 0) {
         const uint32_t target = (++x.barrierPasses[op.arg1]) * op.arg0;
         uint32_t* counter = &x.state->barriers[op.arg1];
         ptx::fence_acq_rel_gpu();
@@ -560,7 +586,7 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
       break;
     case OpType::GROUP_LOAD_REDUCE_STORE: {
       const uint64_t n = sliced(x, op, op.src[0], skip) / 16;
-      for (uint64_t i = x.tid; i < n; i += x.threads) {
+      for (uint64_t i = x.tid(); i < n; i += x.threads()) {
         const uint4 v = switchLoadReduce<T>(x, op.src[0], skip + i * 16);
         switchStore(x, op.dst[0], skip + i * 16, v);
       }
@@ -568,7 +594,7 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
     }
     case OpType::GROUP_STORE: {
       const uint64_t n = sliced(x, op, op.src[0], skip) / 16;
-      for (uint64_t i = x.tid; i < n; i += x.threads)
+      for (uint64_t i = x.tid(); i < n; i += x.threads())
         switchStore(x, op.dst[0], skip + i * 16, *reinterpret_cast<const uint4*>(plainAddr(x, op.src[0], skip) + i * 16));
       break;
     }
@@ -599,7 +625,7 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
     case OpType::SEM_ACQUIRE:
     case OpType::SEM_RELEASE: {
       teamSync(x);
-      if (threadIdx.x < op.nIds && x.member == 0) {
+      if (threadIdx.x < op.nIds && x.member() == 0) {
         // semaphores are re-armed by block 0 at the start of every launch: wait for that first
         if (!waitGreaterEqual(&x.state->semInit, x.epoch, x.c->status, x.c->timeoutNs, kDevTimeoutSemaphore, x.rank, 700, 0)) {
           teamGivesUp(x);
@@ -634,9 +660,9 @@ MSCCLPP_DEVICE_INLINE void execOp(Ctx& x, const DevOp& op) {
 }
 
 // One operation with its entry/exit trace events (thread 0; the cost is one predictable branch when tracing is off).
-template <typename T, typename Pkt>
-MSCCLPP_DEVICE_INLINE void tracedOp(Ctx& x, const DevOp& op) {
-  NpKitEventCollectContext* trace = x.member == 0 ? x.a->npkit : nullptr;
+template <typename T, typename Pkt, bool kTeams>
+MSCCLPP_DEVICE_INLINE void tracedOp(TeamCtx<kTeams>& x, const DevOp& op) {
+  NpKitEventCollectContext* trace = x.member() == 0 ? x.a->npkit : nullptr;
   if (trace != nullptr && threadIdx.x == 0)
     npkitCollectGpuEvent(trace, NPKIT_EVENT_EXECUTOR_OP_BASE_ENTRY + op.type, static_cast<uint32_t>(op.nSrc ? op.src[0].size : 0), x.rank);
   execOp<T, Pkt>(x, op);
@@ -664,9 +690,8 @@ __global__ void __launch_bounds__(1024, 1) executionKernel(ExecArgs a) {
   ExecState* state = reinterpret_cast<ExecState*>(c.peerBase[rank] + a.stateOff);
 
   __shared__ uint32_t barrierPasses[kExecMaxBarriers];
-  __shared__ int ok;
   if (threadIdx.x < kExecMaxBarriers) barrierPasses[threadIdx.x] = 0;
-  if (threadIdx.x == 0) ok = 1;
+  if (threadIdx.x == 0) teamOk() = 1;
   __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     for (uint32_t i = 0; i < plan->nSemaphores; i++) state->semaphores[i] = plan->semInit[i];
@@ -676,7 +701,7 @@ __global__ void __launch_bounds__(1024, 1) executionKernel(ExecArgs a) {
 
   const uint32_t planBlock = kTeams ? blockIdx.x / a.team : blockIdx.x;
   if (planBlock < plan->nThreadBlocks) {
-    Ctx x;
+    TeamCtx<kTeams> x;
     x.c = &c;
     x.a = &a;
     x.plan = plan;
@@ -688,11 +713,6 @@ __global__ void __launch_bounds__(1024, 1) executionKernel(ExecArgs a) {
     x.pipeUnit = 0;
     x.barrierPasses = barrierPasses;
     x.healthy = true;
-    x.ok = &ok;
-    x.team = kTeams ? a.team : 1;
-    x.member = kTeams ? static_cast<int>(blockIdx.x - planBlock * a.team) : 0;
-    x.tid = kTeams ? static_cast<uint32_t>(x.member) * blockDim.x + threadIdx.x : threadIdx.x;
-    x.threads = kTeams ? static_cast<uint32_t>(a.team) * blockDim.x : blockDim.x;
     const DevThreadBlock tb = plan->tbs[planBlock];
     const DevOp* ops = plan->ops;
     uint32_t i = tb.opBegin;
