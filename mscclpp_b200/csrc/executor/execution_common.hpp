@@ -2,6 +2,7 @@
 // and the interpreter kernel consumes.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 
 #include <mscclpp/device/symm.cuh>
@@ -146,6 +147,96 @@ MSCCLPP_HOST_DEVICE_INLINE PortRequest decodePortRequest(const ProxyTrigger& t) 
   return r;
 }
 
+// What a thread block's operations take, in us, on `team` CTAs of nThreads threads (see executionKernel): only as much of it as depends on the
+// team. It shares the words of one source of one operation at a time - in a pipeline, of one iteration - so a source with few of them keeps
+// few CTAs busy; and wherever a thread block meets, the barrier is one of the cluster. What the host proxy moves is shared by nobody. < 0: the
+// block has packet operations, whose CTAs would all wait by themselves.
+// The rates are those of one CTA of 1024 threads and the 0.55 us those of a cluster's barrier, one B200, all ranks on it. Plans of one thread
+// block per rank, us on 1 / 2 / 4 / 8 CTAs: all-gather over eight ranks (seven puts), 32 KB each 24.4 / 26.9 / 26.9 / 26.8, 64 KB 28.9 / 28.9 / 26.8 / 26.8,
+// 512 KB 104 / 66 / 44 / 35; reduce-scatter over two ranks, 128 KB 19.5 / 22.2 / 20.8 / 20.8, 512 KB 31.6 / 27.4 / 23.1 / 21.7; 64 puts of 128 KB with
+// signal and wait 612 / 715 / 687 / 666, 8 of 256 KB 104 / 105 / 95 / 91. (By the bytes of all its operations together, whatever they are, the
+// first and the last two of these got eight CTAs each, and 64 puts of 4 KB 574 us instead of 372.)
+inline float execBlockUs(const DevOp* ops, size_t nOps, int nThreads, int team) {
+  float us = 0.f, iterations = 1.f;
+  uint64_t unit = 0;
+  for (size_t i = 0; i < nOps; i++) {
+    const DevOp& op = ops[i];
+    const bool port = op.channelType == 1;
+    float rate = 48.f;  // KB per us and CTA: copies
+    int syncs = 0;
+    switch (static_cast<OpType>(op.type)) {
+      case OpType::PIPELINE_BEGIN:
+        iterations = static_cast<float>(op.arg0);
+        unit = op.arg1;
+        continue;
+      case OpType::PIPELINE_END:
+        iterations = 1.f;
+        unit = 0;
+        continue;
+      case OpType::NOP:
+        syncs = 1;
+        break;
+      case OpType::BARRIER:
+      case OpType::WAIT:
+      case OpType::RELAXED_WAIT:
+      case OpType::SEM_ACQUIRE:
+      case OpType::SEM_RELEASE:
+        syncs = 2;
+        break;
+      case OpType::SIGNAL:
+      case OpType::RELAXED_SIGNAL:
+      case OpType::FLUSH:
+        syncs = port ? 2 : 0;
+        break;
+      case OpType::PUT:
+        syncs = port ? 2 : 0;
+        break;
+      case OpType::PUT_WITH_SIGNAL:
+      case OpType::PUT_WITH_SIGNAL_AND_FLUSH:
+        syncs = port ? 2 : 1;
+        break;
+      case OpType::GET:
+      case OpType::COPY:
+        break;
+      case OpType::REDUCE:
+      case OpType::REDUCE_SEND:
+      case OpType::READ_REDUCE:
+      case OpType::READ_REDUCE_SEND:
+        rate = op.nSrc > 2 ? 80.f : 64.f;
+        break;
+      case OpType::GROUP_LOAD_REDUCE_STORE:
+      case OpType::GROUP_STORE:
+        break;
+      default:
+        return -1.f;
+    }
+    if (team > 1) us += 0.55f * iterations * static_cast<float>(syncs);
+    if (port) continue;
+    for (int k = 0; k < op.nSrc; k++) {
+      const uint64_t size = op.src[k].size, atOnce = unit != 0 && op.inPipeline && size > unit ? unit : size;
+      const float busy = static_cast<float>(atOnce) / 16.f / static_cast<float>(nThreads);  // CTAs whose threads have a word each
+      const float ctas = busy < 1.f ? 1.f : busy < static_cast<float>(team) ? busy : static_cast<float>(team);
+      us += static_cast<float>(size) / 1000.f / (rate * static_cast<float>(nThreads) / 1024.f * ctas);
+    }
+  }
+  return us;
+}
+
+// The CTAs per thread block that pay: at most and at least (1 and 1: none do), from blocksUs[k], the longest of the plan's thread blocks on 2^k of
+// them. The launch takes as many of these as there are SMs for.
+struct ExecTeam {
+  int most = 1, least = 1;
+};
+inline ExecTeam execTeam(const float (&blocksUs)[4]) {
+  ExecTeam t;
+  for (int k = 1; k < 4; k++) {
+    if (blocksUs[k] + 0.5f >= blocksUs[0]) continue;  // (half a microsecond: what the model is off by)
+    if (t.most == 1) t.least = 1 << k;
+    if (t.most == 1 || blocksUs[k] + 0.05f < blocksUs[k - 1]) t.most = 1 << k;
+  }
+  return t;
+}
+
 struct ExecArgs {
   DeviceComm comm;
   const DevPlan* plans[kMaxRanks];  // [emulated rank]; real mode uses entry 0
@@ -154,6 +245,7 @@ struct ExecArgs {
   uint64_t scratchHalf;  // bytes of one scratch half (0 = no double buffering)
   int emuRanks;
   int team;              // CTAs of a cluster that share a plan thread block (1, 2, 4 or 8; see executionKernel)
+  int leastTeam;         // host: the fewest that pay (see execTeam)
   int packetLL8;         // packet ops use 8-byte LL8 packets instead of 16-byte LL16 ones
   int portContext;       // index of this plan context in the host proxy's table
   FifoDeviceHandle portFifo;  // request queue of the executor's host proxy (triggers == nullptr: the plan has no port ops)

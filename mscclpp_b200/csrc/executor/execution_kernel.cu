@@ -798,7 +798,8 @@ cudaError_t launchTyped(ExecArgs& args, int nBlocks, int nThreads, cudaStream_t 
   }
   // teams only of SMs that nobody else of the launch needs
   if (nThreads % 32 != 0) args.team = 1;
-  while (args.team > 1 && (nBlocks * emu * args.team > sms || nBlocks * emu > residentTeams(teams, args.team, nThreads))) args.team /= 2;
+  while (args.team > 1 && (nBlocks * emu * args.team > sms || nBlocks * emu > residentTeams(teams, args.team, nThreads)))
+    args.team = args.team > args.leastTeam ? args.team / 2 : 1;
   if (args.team > 1) return gemm::launchClusters(teams, args.team, dim3(nBlocks * args.team, emu), block, 0, params, true, stream);
   return cudaLaunchCooperativeKernel(kernel, dim3(nBlocks, emu), block, params, 0, stream);
 }

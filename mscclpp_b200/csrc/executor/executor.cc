@@ -172,21 +172,6 @@ int ExecutionPlan::nThreadsPerBlock() const { return impl_->nThreadsPerBlock; }
 // ------------------------------------------------------------------------------------------ plan -> DevPlan
 namespace {
 
-bool isPacketOp(OpType t) {
-  return t == OpType::PUT_PACKETS || t == OpType::READ_PUT_PACKETS || t == OpType::COPY_PACKETS || t == OpType::UNPACK_PACKETS ||
-         t == OpType::REDUCE_PACKETS || t == OpType::REDUCE_SEND_PACKETS || t == OpType::REDUCE_COPY_PACKETS ||
-         t == OpType::REDUCE_COPY_SEND_PACKETS || t == OpType::GROUP_STORE_PACKETS;
-}
-
-// CTAs for a thread block that moves so many bytes (see executionKernel; the launch takes fewer where there are no SMs for them). Packet
-// operations, whose CTAs would all wait by themselves, keep one.
-int teamOf(uint64_t bytes) {
-  constexpr uint64_t kPerCta = 64 << 10;  // (from 32 to 128 KB alike; 16 KB: four ranks, 256 KB 19.1 -> 23.3 us)
-  int team = 1;
-  while (team < 8 && bytes >= 2 * static_cast<uint64_t>(team) * kPerCta) team *= 2;
-  return team;
-}
-
 struct Resolved {
   std::vector<DevOp> ops;
   DevPlan plan{};
@@ -432,7 +417,7 @@ struct Executor::Impl {
     std::vector<DevOp*> devOps;
     std::vector<DevPlan*> devPlans;
     int maxThreadBlocks = 0;
-    uint64_t blockBytes = 0;  // most bytes that a thread block copies or reduces, 0 where the plan has packet operations
+    ExecTeam team;            // CTAs per thread block that the plan's operations are worth
     // port channels: what the host proxy needs to carry out a request of this context
     bool usesPort = false;
     int portIndex = -1;                                    // slot in Impl::portTable
@@ -946,7 +931,7 @@ void Executor::execute(int rank, void* sendbuff, void* recvbuff, size_t sendBuff
     impl_->freeDevPlans(ctx);
     const int nPlans = heap.emulated() ? heap.world() : 1;
     ctx.maxThreadBlocks = 0;
-    ctx.blockBytes = 0;
+    float blocksUs[4] = {};
     bool packets = false;
     ctx.usesPort = false;
     ctx.portChannels.assign(nPlans, {});
@@ -965,15 +950,15 @@ void Executor::execute(int rank, void* sendbuff, void* recvbuff, size_t sendBuff
       ctx.devPlans.push_back(dplan);
       ctx.maxThreadBlocks = std::max<int>(ctx.maxThreadBlocks, static_cast<int>(res.plan.nThreadBlocks));
       for (uint32_t b = 0; b < res.plan.nThreadBlocks; b++) {
-        uint64_t bytes = 0;
-        for (uint32_t i = res.plan.tbs[b].opBegin; i < res.plan.tbs[b].opEnd; i++) {
-          packets = packets || isPacketOp(static_cast<OpType>(res.ops[i].type));
-          for (int k = 0; k < res.ops[i].nSrc; k++) bytes += res.ops[i].src[k].size;
+        const DevThreadBlock& tb = res.plan.tbs[b];
+        for (int k = 0; k < 4; k++) {
+          const float us = execBlockUs(res.ops.data() + tb.opBegin, tb.opEnd - tb.opBegin, p.nThreadsPerBlock, 1 << k);
+          packets = packets || us < 0.f;
+          blocksUs[k] = std::max(blocksUs[k], us);
         }
-        ctx.blockBytes = std::max(ctx.blockBytes, bytes);
       }
     }
-    if (packets) ctx.blockBytes = 0;
+    ctx.team = packets ? ExecTeam{} : execTeam(blocksUs);
     ctx.S = layout.S;
     ctx.placement = placement;
   }
@@ -985,7 +970,8 @@ void Executor::execute(int rank, void* sendbuff, void* recvbuff, size_t sendBuff
   args.scratchOff = layout.scratchOff;
   args.scratchHalf = p.doubleScratch ? half : 0;
   args.emuRanks = heap.emulated() ? heap.world() : 1;
-  args.team = teamOf(ctx.blockBytes);
+  args.team = ctx.team.most;
+  args.leastTeam = ctx.team.least;
   args.packetLL8 = packetType == PacketType::LL8 ? 1 : 0;
   if (ctx.usesPort) {
     impl_->ensureProxy();

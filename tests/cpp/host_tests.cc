@@ -28,6 +28,7 @@
 #include "core/range_allocator.hpp"
 #include "core/socket.hpp"
 #include "core/unix_socket.hpp"
+#include "executor/execution_common.hpp"
 #include "kernels/moe.cuh"
 #include <mscclpp/ext/collectives/algorithm_collection_builder.hpp>
 
@@ -408,6 +409,64 @@ TEST(RangeAllocator, FirstFitReleaseAndCoalescing) {
   }
   EXPECT_THROW(r.release(12345), std::invalid_argument);
   EXPECT_EQ(r.allocate(0), RangeAllocator::npos);
+}
+
+// A team of CTAs pays where the words that it shares outweigh the barriers that it meets at: many small operations are no reason for one, nor
+// is what the host proxy moves.
+TEST(PlanTeams, SharedWordsAgainstBarriers) {
+  const uint64_t kb = 1 << 10;
+  auto op = [](OpType type, uint64_t bytes = 0, int sources = 1) {
+    DevOp d{};
+    d.type = static_cast<uint8_t>(type);
+    d.nSrc = static_cast<uint8_t>(bytes != 0 ? sources : 0);
+    for (int k = 0; k < d.nSrc; k++) d.src[k].size = bytes;
+    return d;
+  };
+  auto team = [](const std::vector<DevOp>& ops, int nThreads = 1024) {
+    float us[4];
+    for (int k = 0; k < 4; k++) us[k] = execBlockUs(ops.data(), ops.size(), nThreads, 1 << k);
+    if (us[0] < 0.f) return -1;
+    const ExecTeam t = execTeam(us);
+    EXPECT_TRUE(t.least <= t.most && (t.least == 1) == (t.most == 1));
+    return t.most;
+  };
+  // `ops` between signals and waits, as the library's plans have them
+  auto plan = [&](const std::vector<DevOp>& ops) {
+    std::vector<DevOp> all = {op(OpType::RELAXED_SIGNAL), op(OpType::RELAXED_WAIT), op(OpType::NOP)};
+    all.insert(all.end(), ops.begin(), ops.end());
+    for (OpType t : {OpType::NOP, OpType::SIGNAL, OpType::WAIT, OpType::NOP}) all.push_back(op(t));
+    return all;
+  };
+  auto repeated = [](std::vector<DevOp> ops, int n) {
+    std::vector<DevOp> all;
+    for (int i = 0; i < n; i++) all.insert(all.end(), ops.begin(), ops.end());
+    return all;
+  };
+  EXPECT_EQ(team({}), 1);
+  EXPECT_EQ(team(plan({op(OpType::COPY, 128 * kb)})), 1);
+  EXPECT_EQ(team(plan({op(OpType::COPY, 512 * kb)})), 8);
+  EXPECT_EQ(team(plan({op(OpType::READ_REDUCE, 128 * kb, 2)})), 1);
+  EXPECT_EQ(team(plan({op(OpType::READ_REDUCE, 256 * kb, 8)})), 8);
+  EXPECT_EQ(team(plan(repeated({op(OpType::PUT, 32 * kb)}, 7))), 1);
+  EXPECT_EQ(team(plan(repeated({op(OpType::PUT, 64 * kb)}, 7))), 4);  // (no words for more)
+  const std::vector<OpType> around = {OpType::NOP, OpType::SIGNAL, OpType::NOP, OpType::WAIT, OpType::NOP};
+  for (uint64_t each : {4 * kb, 64 * kb, 128 * kb, 256 * kb}) {
+    std::vector<DevOp> one = {op(OpType::PUT, each)};
+    for (OpType t : around) one.push_back(op(t));
+    EXPECT_EQ(team(repeated(one, 64)), each >= 256 * kb ? 8 : 1);
+  }
+  DevOp port = op(OpType::PUT_WITH_SIGNAL_AND_FLUSH, 64 << 20);
+  port.channelType = 1;
+  EXPECT_EQ(team(plan({port})), 1);
+  EXPECT_EQ(team(plan({port, op(OpType::COPY, 1024 * kb)})), 8);
+  EXPECT_EQ(team(plan({op(OpType::COPY, 64 << 20), op(OpType::COPY_PACKETS, 16)})), -1);
+  DevOp begin = op(OpType::PIPELINE_BEGIN), inside = op(OpType::COPY, 8 << 20);
+  inside.inPipeline = 1;
+  for (uint64_t unit : {16 * kb, 64 * kb, 1024 * kb}) {
+    begin.arg0 = static_cast<uint32_t>((8 << 20) / unit);
+    begin.arg1 = static_cast<uint32_t>(unit);
+    EXPECT_EQ(team({begin, inside, op(OpType::NOP), op(OpType::SEM_RELEASE), op(OpType::NOP), op(OpType::PIPELINE_END)}), unit >= 1024 * kb ? 8 : 1);
+  }
 }
 
 // From 12288 pairs on, counting them in every block takes longer than the exchange that it replaces.

@@ -244,10 +244,11 @@ def test_reductions_of_every_number_of_sources(world):
         _run_both(single_node.build("reducescatter_allpairs", world).to_json(), world, world * per, per, np.int32, inplace=False)
 
 
-# elements of a chunk, fp16: thread blocks of 128 KB, 256 KB and 512 KB are run by 2, 4 and 8 CTAs; the words do not divide by their threads
-@pytest.mark.parametrize("world,instances,per", [(2, 1, 32768 + 8), (2, 1, 65536 + 24), (2, 1, 131072 + 1032), (3, 2, 262144 + 16), (8, 2, 131072 + 16),
-                                                 (8, 8, 65536 + 64)])
-def test_thread_blocks_of_several_ctas(world, instances, per):
+# elements of a chunk, fp16; the words do not divide by their threads. team: the CTAs that run each thread block of the reduction
+@pytest.mark.parametrize("world,instances,per,team", [(2, 1, 32768 + 8, 1), (2, 1, 65536 + 24, 1), (2, 1, 131072 + 1032, 8), (2, 1, 262144 + 1032, 8),
+                                                      (3, 2, 262144 + 16, 8), (4, 5, 5 * 131072 + 80, 4), (8, 1, 65536 + 16, 8), (8, 8, 65536 + 64, 1),
+                                                      (8, 8, 524288 + 64, 2)])
+def test_thread_blocks_of_several_ctas(world, instances, per, team):
     from mscclpp_b200.default_algos import single_node
 
     build = lambda name: single_node.build(name, world, instances=instances, in_place=False).to_json()
@@ -255,7 +256,7 @@ def test_thread_blocks_of_several_ctas(world, instances, per):
              _run_both(build("alltoall_allpairs"), world, world * per, world * per, np.float16, inplace=False),
              _run_both(build("allgather_allpairs"), world, per, world * per, np.float16, inplace=False),
              _run_both(single_node.build("allreduce_nvls", world, instances=instances).to_json(), world, world * per, world * per, np.float16, inplace=True)]
-    assert all(t in (1, 2, 4, 8) for t in teams) and teams[0] > 1
+    assert teams[0] == team
 
 
 def _plan_of_large_operations(kind):
