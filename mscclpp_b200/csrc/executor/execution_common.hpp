@@ -4,6 +4,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <cstdlib>
 
 #include <mscclpp/device/symm.cuh>
 #include <mscclpp/fifo_device.hpp>
@@ -227,14 +228,28 @@ inline float execBlockUs(const DevOp* ops, size_t nOps, int nThreads, int team) 
 struct ExecTeam {
   int most = 1, least = 1;
 };
-inline ExecTeam execTeam(const float (&blocksUs)[4]) {
+inline ExecTeam execTeam(const float (&blocksUs)[4], int allowed = 8) {
   ExecTeam t;
-  for (int k = 1; k < 4; k++) {
+  for (int k = 1; k < 4 && (1 << k) <= allowed; k++) {
     if (blocksUs[k] + 0.5f >= blocksUs[0]) continue;  // (half a microsecond: what the model is off by)
     if (t.most == 1) t.least = 1 << k;
     if (t.most == 1 || blocksUs[k] + 0.05f < blocksUs[k - 1]) t.most = 1 << k;
   }
   return t;
+}
+
+// How many CTAs an executor allows per thread block: what MSCCLPP_EXECUTOR_TEAM says (`setting`, null or empty where it is not set; rounded down to a
+// power of two), else eight where all ranks are in the launch, and one where there are others. A plan's author counts on one SM for each
+// thread block. Launches of ranks on several GPUs wait for one another: two plans on two streams that fit a GPU side by side finish in
+// whatever order the ranks start them, but where a team of the one has taken the SMs of the other, ranks that start them in different
+// orders wait until their time limit. Nor does a plan of few blocks leave SMs to the kernel that it is to run beside.
+inline int execAllowedTeam(const char* setting, bool allRanksHere) {
+  const int byDefault = allRanksHere ? 8 : 1;
+  if (setting == nullptr || setting[0] == '\0') return byDefault;
+  const int wanted = std::atoi(setting);
+  int team = wanted < 1 ? 0 : 1;
+  while (team != 0 && team < 8 && 2 * team <= wanted) team *= 2;
+  return team != 0 ? team : byDefault;
 }
 
 struct ExecArgs {

@@ -440,7 +440,7 @@ struct Executor::Impl {
   std::shared_ptr<mscclpp::Context> regContext;
   std::map<std::pair<uintptr_t, size_t>, MappedBuffer> mapped;
   uint64_t zeroCopyLaunches = 0;
-  int lastTeam = 0;
+  int allowedTeam = 1, lastTeam = 0;
 
   // ---- guard bands around the executor's own heap buffers (MSCCLPP_EXECUTOR_CANARY=1). The reference has no such
   // check; its plans are trusted. Here a plan's operands are range-checked when they are resolved, and the bands catch
@@ -718,11 +718,13 @@ bool canariesWanted() {
   const char* e = std::getenv("MSCCLPP_EXECUTOR_CANARY");
   return e != nullptr && e[0] != '\0' && e[0] != '0';
 }
+int allowedTeam(const SymmetricHeap& heap) { return execAllowedTeam(std::getenv("MSCCLPP_EXECUTOR_TEAM"), heap.emulated() || heap.world() == 1); }
 }  // namespace
 
 Executor::Executor(std::shared_ptr<SymmetricHeap> heap) : impl_(std::make_unique<Impl>()) {
   impl_->heap = std::move(heap);
   impl_->canaries = canariesWanted();
+  impl_->allowedTeam = allowedTeam(*impl_->heap);
   startTracing(*impl_->heap);
 }
 
@@ -731,6 +733,7 @@ Executor::Executor(std::shared_ptr<Communicator> comm, std::shared_ptr<char>) : 
   SymmetricHeap::Options opt;
   impl_->heap = SymmetricHeap::create(comm->bootstrap(), opt);
   impl_->canaries = canariesWanted();
+  impl_->allowedTeam = allowedTeam(*impl_->heap);
   startTracing(*impl_->heap);
 }
 
@@ -958,7 +961,7 @@ void Executor::execute(int rank, void* sendbuff, void* recvbuff, size_t sendBuff
         }
       }
     }
-    ctx.team = packets ? ExecTeam{} : execTeam(blocksUs);
+    ctx.team = packets ? ExecTeam{} : execTeam(blocksUs, impl_->allowedTeam);
     ctx.S = layout.S;
     ctx.placement = placement;
   }

@@ -61,7 +61,9 @@ class Executor {
   std::shared_ptr<SymmetricHeap> heap() const;
   // How many execute() calls so far ran directly on buffers outside the heap (mapped on every rank) instead of staging them.
   uint64_t zeroCopyLaunches() const;
-  // How many CTAs shared each thread block of the plan in the latest launch (1: one each; 0: nothing has been launched).
+  // How many CTAs shared each thread block of the plan in the latest launch (1: one each; 0: nothing has been launched). Plans of large copies and
+  // reductions get up to eight where all ranks are emulated on one GPU, and elsewhere as many as MSCCLPP_EXECUTOR_TEAM allowed when the
+  // executor was created (1, 2, 4 or 8; unset: 1, a plan takes one SM per thread block).
   int lastTeam() const;
 
   // Debugging aid, switched on with MSCCLPP_EXECUTOR_CANARY=1 when the executor is created: every buffer the executor

@@ -469,6 +469,22 @@ TEST(PlanTeams, SharedWordsAgainstBarriers) {
   }
 }
 
+// Ranks on other GPUs: a plan takes the SMs that it names, unless the user allows more.
+TEST(PlanTeams, OnlyWhereNobodyElseIsWaitedForOrOnRequest) {
+  for (const char* unset : {static_cast<const char*>(nullptr), "", "0", "-3", "many"}) {
+    EXPECT_EQ(execAllowedTeam(unset, true), 8);
+    EXPECT_EQ(execAllowedTeam(unset, false), 1);
+  }
+  for (bool here : {false, true}) {
+    EXPECT_EQ(execAllowedTeam("1", here), 1);
+    EXPECT_EQ(execAllowedTeam("2", here), 2);
+    EXPECT_EQ(execAllowedTeam("7", here), 4);
+    EXPECT_EQ(execAllowedTeam("64", here), 8);
+  }
+  const float us[4] = {100.f, 60.f, 35.f, 20.f};
+  for (int allowed : {1, 2, 4, 8}) EXPECT_EQ(execTeam(us, allowed).most, allowed);
+}
+
 // From 12288 pairs on, counting them in every block takes longer than the exchange that it replaces.
 TEST(MoeDispatch, BlocksCountFewPairsOfOneRankAlone) {
   EXPECT_EQ(moeCountsAlone(1, 1024, 8) && moeCountsAlone(1, 4096, 2) && moeCountsAlone(1, 0, 8), true);

@@ -315,6 +315,15 @@ def test_what_a_thread_block_of_several_ctas_does_once(kind, per):
     assert _run_both(_plan_of_large_operations(kind), 2, per, per, np.int32, inplace=True, launches=3) == 8  # (four chunks of `per` bytes, int32)
 
 
+@pytest.mark.parametrize("setting,team", [("1", 1), ("2", 2), ("", 8)])
+def test_how_many_ctas_share_a_thread_block_can_be_limited(monkeypatch, setting, team):
+    from mscclpp_b200.default_algos import single_node
+
+    monkeypatch.setenv("MSCCLPP_EXECUTOR_TEAM", setting)
+    per = 262144 + 1032
+    assert _run_both(single_node.build("reducescatter_allpairs", 2, in_place=False).to_json(), 2, 2 * per, per, np.float16, inplace=False) == team
+
+
 def test_a_wait_that_runs_out_ends_every_cta_of_a_thread_block():
     """The signals that the first wait is for are left out of the plan. The error is reported, nobody has reduced anything, and the
     complete plan works afterwards."""
