@@ -441,7 +441,6 @@ __noinline__ __device__ void copyWords(char* dst, const char* src, uint64_t word
 #pragma unroll 1
   for (; i < words; i += threads) ptx::st_na_v4(dst + i * 16, ptx::ld_nc_na_v4(src + i * 16));
 }
-constexpr uint64_t kCopyWordsMin = 64 << 10;  // bytes: every thread of a block has its four
 
 // src[k] -> dst[k] of a put, get or copy.
 template <bool kTeams>
@@ -451,7 +450,8 @@ MSCCLPP_DEVICE_INLINE void copyOp(const TeamCtx<kTeams>& x, const DevOp& op) {
     const uint64_t n = sliced(x, op, op.src[i], skip);
     char* dst = plainAddr(x, op.dst[i], skip);
     const char* src = plainAddr(x, op.src[i], skip);
-    if (n >= kCopyWordsMin && ((reinterpret_cast<uint64_t>(dst) | reinterpret_cast<uint64_t>(src) | n) & 15) == 0) {
+    // (from four words per thread on: 64 KB for 1024 threads, 512 KB for a team of eight such CTAs)
+    if (n / 64 >= x.threads() && ((reinterpret_cast<uint64_t>(dst) | reinterpret_cast<uint64_t>(src) | n) & 15) == 0) {
       copyWords(dst, src, n / 16, x.tid(), x.threads());
     } else {
       copyBytes(dst, src, n, x.tid(), x.threads());
