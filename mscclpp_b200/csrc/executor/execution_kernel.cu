@@ -662,14 +662,18 @@ MSCCLPP_DEVICE_INLINE void execOp(TeamCtx<kTeams>& x, const DevOp& op) {
 // One operation with its entry/exit trace events (thread 0; the cost is one predictable branch when tracing is off).
 template <typename T, typename Pkt, bool kTeams>
 MSCCLPP_DEVICE_INLINE void tracedOp(TeamCtx<kTeams>& x, const DevOp& op) {
-  NpKitEventCollectContext* trace = x.member() == 0 ? x.a->npkit : nullptr;
-  if (trace != nullptr && threadIdx.x == 0)
-    npkitCollectGpuEvent(trace, NPKIT_EVENT_EXECUTOR_OP_BASE_ENTRY + op.type, static_cast<uint32_t>(op.nSrc ? op.src[0].size : 0), x.rank);
+  NpKitEventCollectContext* trace = x.a->npkit;
+  // the buffer of the plan's thread block, whoever runs it
+  auto collect = [&](int event) {
+    if (threadIdx.x == 0 && x.member() == 0)
+      npkitCollectGpuEventIn(trace, (blockIdx.x + static_cast<uint64_t>(gridDim.x) * blockIdx.y) / x.team(), static_cast<uint8_t>(event + op.type),
+                             static_cast<uint32_t>(op.nSrc ? op.src[0].size : 0), x.rank);
+  };
+  if (trace != nullptr) collect(NPKIT_EVENT_EXECUTOR_OP_BASE_ENTRY);
   execOp<T, Pkt>(x, op);
   if (trace != nullptr) {
     __syncthreads();  // the exit stamp is taken when the whole block is done with the operation
-    if (threadIdx.x == 0)
-      npkitCollectGpuEvent(trace, NPKIT_EVENT_EXECUTOR_OP_BASE_EXIT + op.type, static_cast<uint32_t>(op.nSrc ? op.src[0].size : 0), x.rank);
+    collect(NPKIT_EVENT_EXECUTOR_OP_BASE_EXIT);
   }
 }
 

@@ -21,7 +21,8 @@
 
 class NpKit {
  public:
-  static constexpr uint64_t kNumGpuEventBuffers = 256;          // traced thread blocks (blockIdx.x + gridDim.x * blockIdx.y)
+  static constexpr uint64_t kNumGpuEventBuffers = 256;          // traced thread blocks (blockIdx.x + gridDim.x * blockIdx.y; of the plan
+                                                                // interpreter: thread block of the plan + their number * emulated rank)
   static constexpr uint64_t kNumCpuEventBuffers = 64;           // host channels
   static constexpr uint64_t kMaxNumGpuEventsPerBuffer = 1ull << 14;  // 256 * 16 Ki * 16 B = 64 MiB of device memory
   static constexpr uint64_t kMaxNumCpuEventsPerBuffer = 1ull << 16;
@@ -38,11 +39,9 @@ class NpKit {
 };
 
 #if defined(__CUDACC__)
-// One thread per block calls this (the caller picks the thread). Events beyond the buffer capacity are dropped.
-__device__ __forceinline__ void npkitCollectGpuEvent(NpKitEventCollectContext* contexts, uint8_t type, uint32_t size, uint32_t rsvd) {
-  if (contexts == nullptr) return;
-  const uint64_t buf = blockIdx.x + static_cast<uint64_t>(gridDim.x) * blockIdx.y;
-  if (buf >= NpKit::kNumGpuEventBuffers) return;
+// An event of buffer `buf`, which only the calling thread writes to during the launch. Events beyond the buffer capacity are dropped.
+__device__ __forceinline__ void npkitCollectGpuEventIn(NpKitEventCollectContext* contexts, uint64_t buf, uint8_t type, uint32_t size, uint32_t rsvd) {
+  if (contexts == nullptr || buf >= NpKit::kNumGpuEventBuffers) return;
   NpKitEventCollectContext& ctx = contexts[buf];
   const uint64_t head = ctx.event_buffer_head;
   if (head >= NpKit::kMaxNumGpuEventsPerBuffer) return;
@@ -51,5 +50,9 @@ __device__ __forceinline__ void npkitCollectGpuEvent(NpKitEventCollectContext* c
   e.bits[1] = mscclpp::ptx::globaltimer();
   ctx.event_buffer[head] = e;
   ctx.event_buffer_head = head + 1;
+}
+// One thread per block calls this (the caller picks the thread).
+__device__ __forceinline__ void npkitCollectGpuEvent(NpKitEventCollectContext* contexts, uint8_t type, uint32_t size, uint32_t rsvd) {
+  npkitCollectGpuEventIn(contexts, blockIdx.x + static_cast<uint64_t>(gridDim.x) * blockIdx.y, type, size, rsvd);
 }
 #endif

@@ -190,6 +190,41 @@ def test_tracer_records_executor_operations(tmp_path):
     symm.destroy()
 
 
+def test_tracer_names_thread_blocks_that_several_ctas_run(tmp_path):
+    """Two thread blocks on each of two ranks, run by four CTAs each or more: a buffer per thread block of the plan, each with all of its operations,
+    one after the other."""
+    from mscclpp_b200 import SymmetricMemory, native
+    from mscclpp_b200.utils.npkit_trace import convert_npkit_dump_to_trace
+
+    n = native()
+    plan_json = _plan_of_large_operations("barrier")
+    names = [[op["name"] for op in tb["ops"]] for gpu in json.loads(plan_json)["gpus"] for tb in gpu["threadblocks"]]
+    assert len(names) == 4
+    symm = SymmetricMemory.emulated(2, nbytes=64 << 20, timeout_ms=3000)
+    t = symm.tensor((1 << 19,), torch.float32, zero=True)
+    executor = n.Executor(symm.heap)
+    plan = n.ExecutionPlan.from_string(plan_json, 0)
+    n.npkit.init(0)
+    try:
+        executor.execute(0, t.data_ptr(), t.data_ptr(), t.numel() * 4, t.numel() * 4, n.DataType.float32, plan, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        symm.check()
+        assert executor.last_team() >= 4
+        n.npkit.dump(str(tmp_path))
+    finally:
+        n.npkit.shutdown()
+    prefix = "gpu_events_rank_0_buf_"
+    written = {int(f[len(prefix):]) for f in os.listdir(tmp_path) if f.startswith(prefix) and os.path.getsize(tmp_path / f) > 0}
+    assert written == {0, 1, 2, 3}
+    for b in range(4):
+        events = np.fromfile(tmp_path / f"{prefix}{b}", dtype=np.uint64).reshape(-1, 2)
+        assert len(events) == 2 * len(names[b]) and (np.diff(events[:, 1].astype(np.int64)) >= 0).all()
+    trace = json.loads(open(convert_npkit_dump_to_trace(str(tmp_path), str(tmp_path / "out"))).read())["traceEvents"]
+    assert sum(e["ph"] == "X" for e in trace) == sum(len(ops) for ops in names)
+    executor.reset()
+    symm.destroy()
+
+
 def test_guard_bands_around_executor_buffers(monkeypatch):
     """With MSCCLPP_EXECUTOR_CANARY=1 the executor's scratch sits between two bands of 0xA5 on every rank. A correct plan
     leaves them alone (a packet plan writes its scratch from every peer, up to the last byte); a byte written just past
