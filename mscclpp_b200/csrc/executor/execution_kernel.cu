@@ -672,7 +672,7 @@ MSCCLPP_DEVICE_INLINE void tracedOp(TeamCtx<kTeams>& x, const DevOp& op) {
   if (trace != nullptr) collect(NPKIT_EVENT_EXECUTOR_OP_BASE_ENTRY);
   execOp<T, Pkt>(x, op);
   if (trace != nullptr) {
-    __syncthreads();  // the exit stamp is taken when the whole block is done with the operation
+    teamSync(x);  // the exit stamp is taken when the whole thread block is done with the operation, all CTAs of it
     collect(NPKIT_EVENT_EXECUTOR_OP_BASE_EXIT);
   }
 }

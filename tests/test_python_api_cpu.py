@@ -148,6 +148,20 @@ def test_nccl_shim_host_calls():
         assert hasattr(lib, sym), sym
 
 
+def test_exit_stamps_wait_for_every_cta_of_a_thread_block():
+    """The plan interpreter stamps the end of an operation behind the barrier of all CTAs that share the thread block, and all of them get there."""
+    import os
+
+    import mscclpp_b200
+
+    source = open(os.path.join(os.path.dirname(mscclpp_b200.__file__), "csrc", "executor", "execution_kernel.cu")).read()
+    body = source[source.index("void tracedOp("):]
+    body = body[body.index("execOp<T, Pkt>(x, op);"):body.index("\n}\n")]
+    assert body.index("if (trace != nullptr) {") < body.index("teamSync(x);") < body.index("collect(NPKIT_EVENT_EXECUTOR_OP_BASE_EXIT);")
+    assert "__syncthreads" not in body
+    assert "NpKitEventCollectContext* trace = x.a->npkit;" in source  # (not the first CTA's alone)
+
+
 def test_npkit_trace_generator(tmp_path):
     """The converter pairs ENTRY/EXIT events of a synthetic dump and places GPU events on the host time line."""
     from mscclpp_b200.utils.npkit_trace import convert_npkit_dump_to_trace, parse_event_header
