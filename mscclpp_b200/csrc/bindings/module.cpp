@@ -361,7 +361,7 @@ PYBIND11_MODULE(_native, m) {
   m.def(
       "pipeline_allreduce",
       [](SymmetricHeap& heap, uintptr_t in, uintptr_t out, uint64_t bytes, DataType dtype, ReduceOp op, uintptr_t scratch, uint64_t sliceBytes,
-         int nBlocks, int nThreads, uintptr_t stream, bool nvls, uint64_t emuStride, uint64_t scratchBytes) {
+         int nBlocks, int nThreads, uintptr_t stream, bool nvls, uint64_t emuStride, uint64_t scratchBytes, int fetch) {
         if (nvls && !heap.nvls()) throw Error("NVLS requested but the heap has no multicast mapping", ErrorCode::InvalidUsage);
         if (!heap.contains(reinterpret_cast<const void*>(scratch), std::max<uint64_t>(scratchBytes, pipelineScratchBytes(nBlocks, sliceBytes))))
           throw Error("pipeline_allreduce: the scratch must be symmetric-heap memory of pipeline_scratch_bytes(n_blocks, slice_bytes)",
@@ -373,6 +373,7 @@ PYBIND11_MODULE(_native, m) {
         a.bytes = bytes;
         a.scratch = reinterpret_cast<void*>(scratch);
         a.scratchBytes = scratchBytes;
+        a.fetch = fetch;
         a.sliceBytes = sliceBytes;
         a.emuRanks = heap.emulated() ? heap.world() : 1;
         a.emuStride = heap.emulated() ? emuStride : 0;
@@ -381,7 +382,7 @@ PYBIND11_MODULE(_native, m) {
       },
       py::arg("heap"), py::arg("input"), py::arg("output"), py::arg("bytes"), py::arg("dtype"), py::arg("op") = SUM, py::arg("scratch"),
       py::arg("slice_bytes"), py::arg("n_blocks") = 64, py::arg("n_threads") = 512, py::arg("stream") = 0, py::arg("nvls") = false,
-      py::arg("emu_stride") = 0, py::arg("scratch_bytes") = 0);
+      py::arg("emu_stride") = 0, py::arg("scratch_bytes") = 0, py::arg("fetch") = -1);
   m.def("pipeline_scratch_bytes", [](int nBlocks, uint64_t sliceBytes) { return pipelineScratchBytes(nBlocks, sliceBytes); },
         py::arg("n_blocks"), py::arg("slice_bytes"));
   m.def(

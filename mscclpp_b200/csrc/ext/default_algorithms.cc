@@ -199,6 +199,7 @@ std::shared_ptr<Algorithm> makePipeline(const std::string& name, std::shared_ptr
         a.sliceBytes = slice;
         a.emuRanks = 1;
         a.nvls = nvls ? 1 : 0;
+        a.fetch = -1;
         return toResult(launchPipelineAllreduce(a, dtype, op, nBlocks, nThreads, stream));
       },
       0, maxBytes, CollectiveBufferMode::Any);

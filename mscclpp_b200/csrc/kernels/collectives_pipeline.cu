@@ -7,7 +7,8 @@
 //   1. copy-in     user input  -> its slice of the local scratch-in            (local stores)
 //   2. barrier A   with the blocks of the same index on every rank            (all slices of this index are staged)
 //   3. reduce      this rank's 1/world of the slice: multimem.ld_reduce through the NVSwitch, result to EVERY rank's scratch-out
-//                  (multimem.st), or peer loads with an fp32 accumulator, result to its OWN scratch-out (of two ranks, the other one's)
+//                  (multimem.st), or peer loads with an fp32 accumulator, result to every rank's scratch-out (peer stores) or, see
+//                  pipelineFetches, to its own
 //   4. barrier B   (every rank's part of the slice is reduced)
 //   5. copy-out    scratch-out -> user output: the local one, or each part from the rank that has reduced it
 //
@@ -150,7 +151,8 @@ struct PipeAccum<T, Op, false> {
   MSCCLPP_DEVICE_INLINE uint4 result() const { return acc; }
 };
 
-template <typename T, ReduceOp Op, bool kNvls>
+// kFetch (peer loads): a rank's sums stay in its own scratch, from which the peers fetch them, instead of going to every peer's
+template <typename T, ReduceOp Op, bool kNvls, bool kFetch>
 __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
   const DeviceComm& c = a.comm;
   const int rank = deviceRank(c);
@@ -205,9 +207,6 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
     copyOthers(dst, src, whole);
     if (tail != 0) copyTail(dst + static_cast<uint64_t>(whole) * 16, src + static_cast<uint64_t>(whole) * 16, tail, 16);
   };
-  // Where the sums of my part go: with two ranks to the other one's scratch, of which there is only one, with more to the own
-  [[maybe_unused]] const bool pull = world > 2;
-  [[maybe_unused]] const uint64_t reducedTo = world == 2 ? c.peerBase[1 - rank] : local;
   auto tokenOf = [&](uint64_t r) { return (static_cast<uint64_t>(epoch) << 32) | (r + 1); };
 
   bool healthy = true;
@@ -272,9 +271,17 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
             if constexpr (kNvls) {
               ptx::multimem_st_v4(reinterpret_cast<void*>(c.mcBase + off), v[k]);
             } else {
-              ptx::st_weak_v4(reinterpret_cast<void*>(reducedTo + off), v[k]);
-              if (u < direct) ptx::st_weak_v4(reinterpret_cast<void*>(outDirect + static_cast<uint64_t>(u) * 16), v[k]);
-              else ptx::st_weak_v4(reinterpret_cast<void*>(local + off), v[k]);
+              if constexpr (!kFetch) {
+#pragma unroll 1
+                for (int i = 1; i < world; i++) {
+                  const int p = rank + i < world ? rank + i : rank + i - world;
+                  ptx::st_weak_v4(reinterpret_cast<void*>(heaps[p] + off), v[k]);
+                }
+                ptx::st_weak_v4(reinterpret_cast<void*>(u < direct ? outDirect + static_cast<uint64_t>(u) * 16 : local + off), v[k]);
+              } else {
+                ptx::st_weak_v4(reinterpret_cast<void*>(local + off), v[k]);
+                if (u < direct) ptx::st_weak_v4(reinterpret_cast<void*>(outDirect + static_cast<uint64_t>(u) * 16), v[k]);
+              }
             }
           }
         }
@@ -301,8 +308,8 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
     // 5. copy-out
     const uint32_t tail = tailOf(r, have), whole = have - (tail != 0 ? 1 : 0);
     char* dst = out + firstOf(r) * 16;
-    if constexpr (kNvls) {
-      copyUnits(dst, reinterpret_cast<const char*>(local + outSlice), 0, whole);
+    if constexpr (!kFetch) {
+      copyOthers(dst, reinterpret_cast<const char*>(local + outSlice), whole);
     } else {
       const uint32_t sub = static_cast<uint32_t>(subUnits), mineBegin = ownBegin < whole ? ownBegin : whole, mineEnd = ownEnd < whole ? ownEnd : whole;
       const uint32_t n = whole - (mineEnd - mineBegin);
@@ -314,7 +321,7 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
           uint32_t u = i0 + k * blockDim.x < n ? i0 + k * blockDim.x : n - 1;
           if (u >= mineBegin) u += mineEnd - mineBegin;
           at[k] = u;
-          v[k] = ptx::ld_weak_v4(reinterpret_cast<const void*>((pull ? heaps[u / sub] : local) + outSlice + static_cast<uint64_t>(u) * 16));
+          v[k] = ptx::ld_weak_v4(reinterpret_cast<const void*>(heaps[u / sub] + outSlice + static_cast<uint64_t>(u) * 16));
         }
 #pragma unroll
         for (uint32_t k = 0; k < kCopyUnroll; k++)
@@ -322,12 +329,12 @@ __global__ void __launch_bounds__(512, 2) pipelineAllreduceKernel(PipeArgs a) {
       }
     }
     if (tail != 0) {
-      const uint64_t from = kNvls || !pull ? local : heaps[whole / static_cast<uint32_t>(subUnits)];
+      const uint64_t from = !kFetch ? local : heaps[whole / static_cast<uint32_t>(subUnits)];
       copyTail(dst + static_cast<uint64_t>(whole) * 16, reinterpret_cast<const char*>(from + outSlice) + static_cast<uint64_t>(whole) * 16, tail, 0);
     }
   }
-  if constexpr (!kNvls) {  // the next launch may have its halves elsewhere: nobody goes on while a peer fetches
-    if (pull && a.scratchBytes == 0 && healthy) {
+  if constexpr (kFetch) {  // the next launch may have its halves elsewhere: nobody goes on while a peer fetches
+    if (a.scratchBytes == 0 && healthy) {
       pipeSignal(c, rank, 1, slot, tokenOf(rounds));
       pipeWait(c, rank, 1, slot, tokenOf(rounds), okSmem);
     }
@@ -339,15 +346,10 @@ template <typename T, ReduceOp Op>
 cudaError_t launchPipeTyped(const PipeArgs& a, int nBlocks, int nThreads, cudaStream_t stream) {
   dim3 grid(nBlocks, a.emuRanks > 1 ? a.emuRanks : 1, 1);
   dim3 block(nThreads, 1, 1);
-  const void* kernel;
-  if (a.nvls) {
-    if constexpr (switchReducible<T, Op>()) {
-      kernel = reinterpret_cast<const void*>(pipelineAllreduceKernel<T, Op, true>);
-    } else {
-      kernel = reinterpret_cast<const void*>(pipelineAllreduceKernel<T, Op, false>);  // the switch cannot reduce this type: peer loads
-    }
-  } else {
-    kernel = reinterpret_cast<const void*>(pipelineAllreduceKernel<T, Op, false>);
+  const void* kernel = pipelineFetches(a.fetch, a.comm.world, a.emuRanks) ? reinterpret_cast<const void*>(pipelineAllreduceKernel<T, Op, false, true>)
+                                                                          : reinterpret_cast<const void*>(pipelineAllreduceKernel<T, Op, false, false>);
+  if constexpr (switchReducible<T, Op>()) {  // (other types: peer loads)
+    if (a.nvls) kernel = reinterpret_cast<const void*>(pipelineAllreduceKernel<T, Op, true, false>);
   }
   PipeArgs copy = a;
   copy.outOffset = a.scratchBytes != 0 ? a.scratchBytes / 32 * 16 : pipelineScratchBytes(nBlocks, a.sliceBytes) / 2;

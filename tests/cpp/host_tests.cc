@@ -29,6 +29,7 @@
 #include "core/socket.hpp"
 #include "core/unix_socket.hpp"
 #include "executor/execution_common.hpp"
+#include "kernels/collectives.cuh"
 #include "kernels/moe.cuh"
 #include <mscclpp/ext/collectives/algorithm_collection_builder.hpp>
 
@@ -409,6 +410,18 @@ TEST(RangeAllocator, FirstFitReleaseAndCoalescing) {
   }
   EXPECT_THROW(r.release(12345), std::invalid_argument);
   EXPECT_EQ(r.allocate(0), RangeAllocator::npos);
+}
+
+// Ranks on several GPUs store their reduced parts to one another unless the caller asks for the other form; that one is for ranks on one GPU.
+TEST(PipelineAllreduce, PartsAreFetchedWhereAllRanksShareOneGpu) {
+  for (int world = 1; world <= 8; world++) {
+    EXPECT_EQ(pipelineFetches(-1, world, 1), false);
+    EXPECT_EQ(pipelineFetches(-1, world, world), world > 2);
+    for (int emu : {1, world}) {
+      EXPECT_EQ(pipelineFetches(0, world, emu), false);
+      EXPECT_EQ(pipelineFetches(1, world, emu), world > 2);
+    }
+  }
 }
 
 // A team of CTAs pays where the words that it shares outweigh the barriers that it meets at: many small operations are no reason for one, nor

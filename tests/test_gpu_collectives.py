@@ -108,6 +108,30 @@ def test_allreduce_pipeline_ragged(world, numel, n_blocks, dtype):
     symm.destroy()
 
 
+@pytest.mark.parametrize("world", [2, 3, 4, 8])
+@pytest.mark.parametrize("numel", [5, 4099, (1 << 18) + 3])
+def test_allreduce_pipeline_parts_stored_or_fetched(world, numel):
+    """Both ways for a reduced part to reach the other ranks, in turn on the same scratch, with slices that leave a part of a unit. (Whole numbers that
+    fp32 sums exactly.)"""
+    from mscclpp_b200 import native
+    from mscclpp_b200.ops import collectives as C
+
+    n = native()
+    symm = _symm(world)
+    scratch = C._pipeline_scratch(symm)
+    x = torch.randint(-1000, 1000, (world, numel + (-numel) % 4), device="cuda").float()  # (rows begin at 16-byte boundaries)
+    out = torch.empty_like(x)
+    nbytes = numel * 4
+    for fetch in (0, 1, -1, 0, 1):
+        for blocks, slice_bytes in ((3, 32 * world), (8, 16 * world * 100)):
+            out.fill_(-1.0)
+            n.pipeline_allreduce(symm.heap, x.data_ptr(), out.data_ptr(), nbytes, n.DataType.float32, n.ReduceOp.SUM, scratch.data_ptr(), slice_bytes, blocks,
+                                 512, torch.cuda.current_stream().cuda_stream, False, x.shape[1] * 4, scratch.numel(), fetch)
+            symm.check()
+            assert torch.equal(out[:, :numel], x.sum(0)[:numel].expand(world, -1)) and bool((out[:, numel:] == -1.0).all())
+    symm.destroy()
+
+
 def test_allreduce_pipeline_scratch_halves_stay_apart():
     """Peers may still fetch reduced parts of a launch when a rank copies in for the next one, which has other slices: what is
     copied in stays in the scratch's first half and what is reduced in its second, whatever the slices. A launch that is not told
