@@ -15,6 +15,7 @@
 
 #include <mscclpp/gpu_data_types.hpp>
 
+#include "activation.cuh"
 #include "gemm2_sm100.cuh"
 #include "gemm_sm100.cuh"
 
@@ -67,16 +68,6 @@ struct GatherGate {
   }
 };
 
-// x * sigmoid(y) in fp32. Of the two a division is the larger: with x / (1 + exp(-x)) as it stands an epilogue took longer than the products
-// in front of it (1664 x 2176 x 1024 SiLU 30.9 us, without activation 10.0; with the reciprocal 11.8; GELU
-// with tanhf 13.6, SwiGLU 19.7, now 12.3 and 10.3). Same distance from the 64-bit results. rcp.approx keeps
-// subnormal results, so that large negative values end as they do in the division.
-MSCCLPP_DEVICE_INLINE float timesSigmoid(float x, float y) {
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-y)));
-  return x * r;
-}
-
 // Activation in fp32 on the accumulator, then one tiled bulk store per staged 32 x 64 block.
 template <int kAct>
 struct StoreAct {
@@ -86,10 +77,9 @@ struct StoreAct {
   int M, N;  // (tiles of one rank's form may reach beyond N)
   MSCCLPP_DEVICE_INLINE static float convert(float x) {
     if constexpr (kAct == 1) {
-      // 0.5 x (1 + tanh(u)) = x sigmoid(2 u)
-      return timesSigmoid(x, 1.5957691216057308f * (x + 0.044715f * x * x * x));
+      return geluTanh(x);
     } else if constexpr (kAct == 2) {
-      return timesSigmoid(x, x);
+      return silu(x);
     } else {
       return x;
     }
@@ -117,7 +107,7 @@ struct StoreGated {
   __nv_bfloat16* out;  // [M, N / 2]
   int M, halfN;
   MSCCLPP_DEVICE_INLINE static float convert(float x) { return x; }
-  MSCCLPP_DEVICE_INLINE static float gatePair(float g, float u) { return timesSigmoid(g, g) * u; }
+  MSCCLPP_DEVICE_INLINE static float gatePair(float g, float u) { return silu(g) * u; }
   MSCCLPP_DEVICE_INLINE void tileBegin(int, int, int) const {}
   MSCCLPP_DEVICE_INLINE void block(const uint8_t* stage, int row0, int col0, int lane, int /*b*/) const {
     // four lanes per row (chunks 0-3), eight rows per step

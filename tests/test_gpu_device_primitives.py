@@ -28,6 +28,45 @@ def _offsets(fmt):
     return offs
 
 
+@pytest.mark.parametrize("kind", ["silu", "gelu"])
+@pytest.mark.parametrize("values", ["normal", "wide", "positive", "negative", "far negative"])
+def test_activations_are_as_exact_as_with_a_division(kind, values):
+    """Relative error against 64 bits: rms and largest no larger than of x / (1 + exp(-x)) and 0.5 x (1 + tanh(u)) in fp32."""
+    from mscclpp_b200.utils import KernelBuilder
+
+    k = KernelBuilder("activations.cu", "activations", file_dir=KDIR).get_compiled_kernel()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    u = torch.rand(1 << 20, generator=g, device="cuda", dtype=torch.float64)
+    x = {"normal": torch.randn(1 << 20, generator=g, device="cuda"), "wide": 4 * torch.randn(1 << 20, generator=g, device="cuda"),
+         "positive": torch.exp(-9.2 + 13.8 * u), "negative": -torch.exp(-9.2 + 10.8 * u), "far negative": -5 - 75 * u}[values].float()
+
+    def run(x, which):
+        out = torch.full_like(x, 7.0)
+        k.launch_kernel(struct.pack("PPii", x.data_ptr(), out.data_ptr(), x.numel(), which), 64, 256, stream=torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        return out
+
+    d = x.double()
+    ref = torch.nn.functional.silu(d) if kind == "silu" else d * torch.sigmoid(1.5957691216057308 * (d + 0.044715 * d ** 3))
+    sized = ref.abs() > 1e-36  # (below, fp32 has not all of its bits)
+
+    def errors(out):
+        e = ((out.double() - ref) / ref)[sized]
+        return e.square().mean().sqrt().item(), e.abs().max().item()
+
+    which = 0 if kind == "silu" else 1
+    (rms, largest), (rms0, largest0) = errors(run(x, which)), errors(run(x, which + 2))
+    assert rms <= 1.005 * rms0 and largest <= 1.02 * largest0, (rms, rms0, largest, largest0)  # (a sample's scatter)
+    ends = torch.tensor([float("inf"), -float("inf"), float("nan"), 0.0, -0.0, 1e30, -1e30, 3e38, -3e38, -88.0, -88.7, -89.0, -103.0, 88.0, 1e-38, -1e-38, 1e-42],
+                        device="cuda")
+    got, want = run(ends, which), run(ends, which + 2)
+    if kind == "silu":  # GELU by tanhf is 0 from -6 on
+        assert torch.allclose(got, want, rtol=1e-5, atol=0.0, equal_nan=True), (got, want)
+    else:
+        big = ends.abs() > 80
+        assert torch.equal(got[big & ~got.isnan()], want[big & ~got.isnan()]) and torch.equal(got.isnan(), want.isnan())
+
+
 @pytest.mark.parametrize("kind,nbytes", [(8, 4096), (16, 4096), (16, 1 << 20)])
 def test_packets_cross_block(kind, nbytes):
     k = _kernel("packetPingPong")
