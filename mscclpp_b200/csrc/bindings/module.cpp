@@ -428,11 +428,11 @@ PYBIND11_MODULE(_native, m) {
       py::arg("pair_m") = -1, py::arg("block_n") = 0, py::arg("split") = 1);
   m.def(
       "gemm_plan_form",
-      [](int M, int N, int K) {
-        const gemm::Form f = gemm::planForm(M, N, K);
+      [](int M, int N, int K, int sms, int fours) {
+        const gemm::Form f = gemm::planForm(M, N, K, sms, fours);
         return py::make_tuple(f.pairM, f.blockN, f.split);
       },
-      py::arg("m"), py::arg("n"), py::arg("k"));
+      py::arg("m"), py::arg("n"), py::arg("k"), py::arg("sms") = 0, py::arg("fours") = 0);
 
   m.def(
       "gemm_bf16_two_sm",

@@ -14,9 +14,6 @@
 //     reference silently skips them on CUDA).
 #include "execution_kernel.hpp"
 
-#include <map>
-#include <mutex>
-#include <tuple>
 #include <type_traits>
 
 #include <mscclpp/copy_device.hpp>
@@ -755,34 +752,6 @@ __global__ void __launch_bounds__(1024, 1) executionKernel(ExecArgs a) {
   }
 }
 
-// Clusters of `team` CTAs of `nThreads` threads that the current device can run at the same time.
-int residentTeams(const void* kernel, int team, int nThreads) {
-  static std::mutex mu;
-  static std::map<std::tuple<const void*, int, int, int>, int> known;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  const std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_tuple(kernel, dev, team, nThreads);
-  const auto it = known.find(key);
-  if (it != known.end()) return it->second;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(team);
-  cfg.blockDim = dim3(nThreads);
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = static_cast<unsigned>(team);
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
-    (void)cudaGetLastError();
-    n = 0;
-  }
-  known[key] = n;
-  return n;
-}
-
 template <typename T>
 cudaError_t launchTyped(ExecArgs& args, int nBlocks, int nThreads, cudaStream_t stream) {
   const int emu = args.emuRanks > 1 ? args.emuRanks : 1;
@@ -802,7 +771,7 @@ cudaError_t launchTyped(ExecArgs& args, int nBlocks, int nThreads, cudaStream_t 
   }
   // teams only of SMs that nobody else of the launch needs
   if (nThreads % 32 != 0) args.team = 1;
-  while (args.team > 1 && (nBlocks * emu * args.team > sms || nBlocks * emu > residentTeams(teams, args.team, nThreads)))
+  while (args.team > 1 && (nBlocks * emu * args.team > sms || nBlocks * emu > gemm::residentClusters(teams, args.team, nThreads, 0)))
     args.team = args.team > args.leastTeam ? args.team / 2 : 1;
   if (args.team > 1) return gemm::launchClusters(teams, args.team, dim3(nBlocks * args.team, emu), block, 0, params, true, stream);
   return cudaLaunchCooperativeKernel(kernel, dim3(nBlocks, emu), block, params, 0, stream);

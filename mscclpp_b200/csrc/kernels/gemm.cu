@@ -1,9 +1,12 @@
 // Plain bf16 GEMM on tcgen05/TMEM (see gemm_sm100.cuh for the kernel body) and tensor-map helpers.
 #include "gemm.cuh"
 
+#include <atomic>
 #include <cmath>
+#include <map>
 #include <mutex>
 #include <set>
+#include <tuple>
 #include <utility>
 
 #include "gemm2_sm100.cuh"
@@ -92,6 +95,34 @@ cudaError_t ensureDynamicSmem(const void* kernel, int bytes) {
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e == cudaSuccess) done.insert({kernel, dev});
   return e;
+}
+
+int residentClusters(const void* kernel, int ctas, int nThreads, int smemBytes) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void*, int, int, int, int>, int> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  const std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_tuple(kernel, dev, ctas, nThreads, smemBytes);
+  const auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(nThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(smemBytes);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(ctas);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  known[key] = n;
+  return n;
 }
 
 cudaError_t launchClusters(const void* kernel, int ctas, dim3 grid, dim3 block, size_t smemBytes, void** params, bool cooperative,
@@ -246,11 +277,29 @@ struct Rates {
   float sm, all, memory;  // KB per us into one SM and into all of them, and TB/s of the memory
 };
 
-float timeOf(const Cost& c, const Rates& rates, int M, int N, int K) {
-  const int sms = smCount();
+// Clusters of four of the split form that run at the same time: they leave SMs over in the groups that they may not leave (34 of 148 SMs on a
+// B200, where 37 would have them).
+int clustersOfFour() {
+  static std::atomic<int> known[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return smCount() / 4 - 3;
+  int n = known[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    const void* kernel = reinterpret_cast<const void*>(gemmBf16Kernel<64, 4>);
+    constexpr int kSmemBytes = Config<64, 4>::kSmemBytes;
+    if (ensureDynamicSmem(kernel, kSmemBytes) != cudaSuccess) return 0;
+    n = residentClusters(kernel, 4, kNumThreads, kSmemBytes);
+    known[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// 0: nothing of this form fits the device.
+float timeOf(const Cost& c, const Rates& rates, int M, int N, int K, int sms, int fours) {
   const int tileM = c.form.pairM != 0 ? c.form.pairM : kBlockM, ctas = c.form.pairM != 0 ? 2 : c.form.split;
   const int64_t tiles = static_cast<int64_t>((M + tileM - 1) / tileM) * ((N + c.form.blockN - 1) / c.form.blockN);
-  const int slots = ctas == 4 ? sms / 4 - 3 : sms / ctas;  // (clusters of four leave SMs over in the groups that they may not leave)
+  const int slots = ctas == 4 ? fours : sms / ctas;
+  if (slots < 1) return 0.f;
   const int64_t waves = (tiles + slots - 1) / slots;
   const float active = static_cast<float>((tiles < slots ? tiles : slots) * ctas);
   const float kb = static_cast<float>((M < tileM ? M : tileM) + c.form.blockN) * (2 * kBlockK) / 1000.f / (c.form.pairM != 0 ? 2 : 1);
@@ -270,7 +319,7 @@ float timeOf(const Cost& c, const Rates& rates, int M, int N, int K) {
 // gemm_bf16, us before / now: 80 x 1408 x 4992 17.4 / 8.5, 645 x 704 x 6144 21.1 / 12.0, 840 x 5696 x 1600 27.9 / 20.5, 333 x 6144 x 4096
 // 23.7 / 22.0, 5510 x 1728 x 640 23.4 / 15.6, 2233 x 6592 x 4160 184 / 107; shapes of up to 8.4 us wait for the host either way.
 // Split over clusters of two, tiles of 128 or 256 columns split over 2, 4 or 8: never more than 3 % ahead.
-Form planForm(int M, int N, int K) {
+Form planForm(int M, int N, int K, int sms, int fours) {
   static constexpr Cost kCosts[] = {
       {{256, 256, 1}, 3.99f, 0.299f, 1.05f}, {{128, 256, 1}, 3.54f, 0.154f, 0.84f}, {{128, 128, 1}, 3.00f, 0.093f, 0.60f}, {{0, 64, 1}, 2.65f, 0.145f, 0.25f},
       {{0, 128, 1}, 2.94f, 0.182f, 0.62f},   {{0, 256, 1}, 3.65f, 0.274f, 1.50f},   {{0, 64, 4}, 4.34f, 0.134f, 4.70f},
@@ -278,11 +327,13 @@ Form planForm(int M, int N, int K) {
   static constexpr Rates kRates = {147.f, 21100.f, 5.4f};
   const float memory = 2e-6f / kRates.memory * (static_cast<float>(M) * K + static_cast<float>(N) * K + static_cast<float>(M) * N);
   const float memory2 = memory * memory;
+  if (sms <= 0) sms = smCount(), fours = clustersOfFour();
   Form best{0, 64, 1};
   float least = 0.f;
   for (const Cost& c : kCosts) {
     if (K / kBlockK < c.form.split) continue;
-    const float loop = timeOf(c, kRates, M, N, K), loop2 = loop * loop;
+    const float loop = timeOf(c, kRates, M, N, K, sms, fours), loop2 = loop * loop;
+    if (loop == 0.f) continue;
     const float t = c.fixed + sqrtf(sqrtf(loop2 * loop2 + memory2 * memory2));
     if (least == 0.f || t < least) {
       least = t;
@@ -296,15 +347,17 @@ Form planForm(int M, int N, int K) {
 // 9-8192, N 1024-8192, K 256-2048 (with the scale pass behind them): within 3.8 %, the pick 0.1 % slower than the best form, at worst
 // 4 %. Both launches, us by the rule before (one-SM tiles below 64 pairs or 256 rows) / now: 61 x 7680 x 1536 11.3 / 10.0,
 // 66 x 4352 x 1024 9.3 / 8.0, 128 x 8192 x 1024 11.5 / 10.3, 185 x 6144 x 1600 17.0 / 13.1, 596 x 2816 x 320 11.9 / 9.5.
-Form planLayerForm(int M, int N, int K) {
+Form planLayerForm(int M, int N, int K, int sms) {
   static constexpr Cost kCosts[] = {{{256, 256, 1}, 4.2f, 0.31f, 0.05f}, {{128, 256, 1}, 3.65f, 0.092f, 1.f}, {{128, 128, 1}, 3.2f, 0.07f, 1.f}};
   static constexpr Rates kRates = {162.f, 24000.f, 7.8f};
   const float memory = 2e-6f / kRates.memory * (static_cast<float>(M) * K + static_cast<float>(N) * K + 2.f * static_cast<float>(M) * N);
+  if (sms <= 0) sms = smCount();
   Form best{0, 64, 1};  // where N is no multiple of 128
   float least = 0.f;
   for (const Cost& c : kCosts) {
     if (N % c.form.blockN != 0 || (c.form.pairM == 256 && M < 256)) continue;
-    const float loop = timeOf(c, kRates, M, N, K);
+    const float loop = timeOf(c, kRates, M, N, K, sms, 0);
+    if (loop == 0.f) continue;
     const float t = c.fixed + sqrtf(loop * loop + memory * memory);
     if (least == 0.f || t < least) {
       least = t;

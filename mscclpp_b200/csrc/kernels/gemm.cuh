@@ -58,11 +58,15 @@ struct Form {
 };
 // The form that gemm_bf16 takes where the caller asks for none, and the product in a given one. N % 64 == 0, K % 64 == 0. N need not be a
 // multiple of the tile.
-Form planForm(int M, int N, int K);
+// sms, fours: the SMs and the clusters of four that run at the same time; 0: what the current device has.
+Form planForm(int M, int N, int K, int sms = 0, int fours = 0);
 // The same for the product whose epilogue adds a residual (launchGemmResidualSumsq), of whose tiles N is a multiple.
-Form planLayerForm(int M, int N, int K);
+Form planLayerForm(int M, int N, int K, int sms = 0);
 cudaError_t gemmBf16Form(const void* A, const void* B, void* D, int M, int N, int K, int ldd, Form form, DeviceStatus* status, cudaStream_t stream,
                          uint64_t budgetNs = kDefaultBudgetNs);
+
+// Clusters of `ctas` CTAs of a kernel (along x) that the current device can run at the same time, 0 where it does not say.
+int residentClusters(const void* kernel, int ctas, int nThreads, int smemBytes);
 
 // Raises the kernel's dynamic shared-memory limit once per (kernel, device); call before every launch that needs > 48 KB.
 cudaError_t ensureDynamicSmem(const void* kernel, int bytes);

@@ -58,6 +58,19 @@ def test_gemm_two_sm_tiles(m, n, k):
     assert (out.float() - ref).abs().max().item() <= 1e-2 * ref.abs().max().item() + 1e-2
 
 
+def test_gemm_form_on_this_gpu():
+    """The device says how many clusters of four it holds; a whole B200 holds as many as the costs were fitted with."""
+    from mscclpp_b200 import native
+
+    n = native()
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("not a whole B200")
+    for m in (9, 33, 80, 200, 645, 1500):
+        for nn in (512, 704, 1408, 2048, 4096):
+            for k in (512, 2048, 4992, 8192):
+                assert n.gemm_plan_form(m, nn, k) == n.gemm_plan_form(m, nn, k, 148, 34)
+
+
 # (rows per pair of SMs or 0, columns, CTAs that share a tile)
 FORMS = [(0, 64, 1), (0, 64, 4), (0, 128, 1), (0, 256, 1), (256, 256, 1), (128, 256, 1), (128, 128, 1)]
 

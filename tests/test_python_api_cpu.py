@@ -546,3 +546,22 @@ def test_gemm_form_fits_the_shape():
         assert form in forms and form[2] <= k // 64
         picked.add(form)
     assert picked == forms  # none of them is there for nothing
+
+
+def test_gemm_form_fits_a_small_gpu():
+    """A part of a GPU: no form whose clusters do not fit, and none that looks cheap because of it. (Fewer SMs than one cluster of four and its like
+    divided by zero.)"""
+    import random
+
+    import mscclpp_b200
+
+    n = mscclpp_b200.native()
+    rng = random.Random(4)
+    for sms in (1, 2, 3, 4, 7, 12, 13, 15, 16, 19, 36, 74, 148):
+        for fours in {0, max(0, sms // 4 - 3), sms // 4}:
+            for _ in range(100):
+                m, nn, k = round(2 ** rng.uniform(0, 13)), 64 * round(2 ** rng.uniform(0, 8)), 64 * round(2 ** rng.uniform(0, 8))
+                pair_m, block_n, split = n.gemm_plan_form(m, nn, k, sms, fours)
+                assert (pair_m == 0 or sms >= 2) and (split == 1 or fours >= 1) and block_n in (64, 128, 256)
+    for m, nn, k in ((80, 1408, 4992), (333, 6144, 4096), (2233, 6592, 4160), (16, 512, 8192)):
+        assert n.gemm_plan_form(m, nn, k) == n.gemm_plan_form(m, nn, k, 148, 34)  # (without a device: a B200)
