@@ -20,10 +20,21 @@ from . import native
 _DTYPE_MAP = None
 
 
+def _current_stream_finder():
+    """torch.cuda.current_stream() finds the current stream by way of a dozen Python functions and a Stream object, 2 of the 8 to 12 us that a
+    call of a small operation takes on the host. What it calls underneath is taken where this build of torch has it."""
+    device, raw_stream = getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if device is None or raw_stream is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw_stream(device())
+
+
+_current_stream = _current_stream_finder()
+
+
 def stream_handle(stream: Optional[torch.cuda.Stream] = None) -> int:
-    """The cudaStream_t of `stream`, or of the current stream of the current device. torch.cuda.current_stream() finds the latter by way of
-    a dozen Python functions and a Stream object, 2 of the 8 to 12 us that a call of a small operation takes on the host."""
-    return stream.cuda_stream if stream is not None else torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    """The cudaStream_t of `stream`, or of the current stream of the current device."""
+    return stream.cuda_stream if stream is not None else _current_stream()
 
 
 def torch_dtype_to_native(dtype: torch.dtype):

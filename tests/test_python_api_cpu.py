@@ -548,6 +548,23 @@ def test_gemm_form_fits_the_shape():
     assert picked == forms  # none of them is there for nothing
 
 
+def test_current_stream_with_another_build_of_torch(monkeypatch):
+    """Without the functions underneath torch.cuda.current_stream(), that one is asked."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from mscclpp_b200._core import symm
+
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 3, raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 40 + device, raising=False)
+    assert symm._current_stream_finder()() == 43
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: SimpleNamespace(cuda_stream=77))
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+    monkeypatch.setattr(symm, "_current_stream", symm._current_stream_finder())
+    assert symm.stream_handle() == 77 and symm.stream_handle(SimpleNamespace(cuda_stream=5)) == 5
+
+
 def test_gemm_form_fits_a_small_gpu():
     """A part of a GPU: no form whose clusters do not fit, and none that looks cheap because of it. (Fewer SMs than one cluster of four and its like
     divided by zero.)"""
