@@ -436,11 +436,7 @@ __global__ void __launch_bounds__(kThreads, 1) moeCombineKernel(MoeCombineArgs a
         wgt = weights[p];
       }
     };
-    // With few rounds the units go round the blocks first: those of the last round, when not every warp has one, are spread over all SMs (777
-    // tokens x 7168 fp8, top-8, 2.3 rounds: dispatch and combine 27.6 -> 26.9 us). With more, neighbouring warps take neighbouring pieces
-    // of a row (4096 x 4096 bf16, top-2, 3.5 rounds: 37.2 us against 38.8).
-    const int warp = threadIdx.x >> 5;
-    int64_t u = units < 3 * static_cast<int64_t>(numWarps) ? static_cast<int64_t>(warp) * gridDim.x + blockIdx.x : static_cast<int64_t>(blockIdx.x) * warpsPerBlock + warp;
+    int64_t u = static_cast<int>(blockIdx.x) * a.blockStep + static_cast<int>(threadIdx.x >> 5) * a.warpStep;
     fetch(u);
     for (; u < units; u += numWarps) {
       const int t = static_cast<int>(u / chunks);
@@ -566,8 +562,19 @@ cudaError_t launchCoop(Kernel kernel, const Args& args, int nBlocks, int emu, cu
 
 template <int kWords, int kRows, bool kFp8>
 cudaError_t launchCombine(const MoeCombineArgs& args, int nBlocks, int emu, cudaStream_t stream) {
-  if (args.comm.world > 1) return launchCoop(moeCombineKernel<kWords, kRows, kFp8, false>, args, nBlocks, emu, stream);
   MoeCombineArgs copy = args;
+  const int words = args.hidden / (kFp8 ? 16 : 8);
+  const int64_t units = static_cast<int64_t>(args.tokens) * ((words + 32 * kWords - 1) / (32 * kWords)), warps = static_cast<int64_t>(nBlocks) * (kThreads / 32);
+  // With few rounds the units go round the blocks first: those of the last round, when not every warp has one, are spread over all SMs. With
+  // more, neighbouring warps take neighbouring pieces of a row. One B200, dispatch and combine, us in neighbouring pieces / round the
+  // blocks: 4096 bf16, top-2 (long pieces), 1.7 rounds 17.8 / 17.2, 2.0 23.1 / 22.4, 2.2 24.2 / 23.3, 2.4 25.7 / 26.0, 2.6 27.7 / 28.8, 2.8 29.6 / 30.8;
+  // 8192 bf16, top-2, and 4096, top-1, cross at the same place: two or fewer rows leave little else to do than to read pieces in order.
+  // 7168 fp8, top-8, 2.2 rounds 25.8 / 24.5, 2.6 27.5 / 27.1, 3.0 63.2 / 63.1, 3.5 46.9 / 46.9; top-4 2.8 rounds 20.1 / 18.9; 4096 bf16, top-4, 2.6
+  // rounds 55.1 / 54.5, top-8 93.0 / 91.8; eight emulated ranks within 1 % but for 4096 fp8, top-8, 2.1 rounds 42.7 / 40.7.
+  const bool roundTheBlocks = kWords == 8 && args.topk <= 2 ? 3 * units < 7 * warps : units < 3 * warps;
+  copy.blockStep = roundTheBlocks ? 1 : kThreads / 32;
+  copy.warpStep = roundTheBlocks ? nBlocks : 1;
+  if (args.comm.world > 1) return launchCoop(moeCombineKernel<kWords, kRows, kFp8, false>, copy, nBlocks, emu, stream);
   void* params[] = {&copy};
   return gemm::launchOverlapped(reinterpret_cast<const void*>(moeCombineKernel<kWords, kRows, kFp8, true>), dim3(nBlocks), dim3(kThreads), 0, params, stream);
 }
