@@ -249,8 +249,9 @@ template <typename T, bool kTeams>
 __noinline__ __device__ void reduceWords(char* const* src, int nSrc, char* const* dst, int nDst, uint64_t nvec, uint32_t tid, uint32_t threads) {
   uint64_t i = tid;
   // Two sources: several words at a time, so that there are more than two loads in flight. Four words where a team of CTAs has much to reduce
-  // (reduce-scatter of 16 MB over two ranks, 16 blocks of 8 CTAs: 31.7 us with two, 28.9 with four); in the kernel without teams two, since four
-  // make every operation slower (64 puts of 4 KB with signal and wait 432 us with one or two, 455 with four).
+  // (reduce-scatter of 16 MB over two ranks, 16 blocks of 8 CTAs: 31.7 us with two, 28.9 with four); in the kernel without teams two (the same on
+  // one CTA each 70 us with one, 45 with two), since four make every operation slower there (64 puts of 4 KB with signal and wait 432 us with
+  // one or two, 455 with four).
   constexpr int kWords = kTeams ? 4 : 2;
   if (nSrc == 2) {
     const char *s0 = src[0], *s1 = src[1];
@@ -674,12 +675,12 @@ MSCCLPP_DEVICE_INLINE void tracedOp(TeamCtx<kTeams>& x, const DevOp& op) {
   }
 }
 
-// A plan's thread blocks are few (its author counts on one SM for each), and one SM keeps neither memory nor a fast link busy: a thread
-// block may be run by a team of CTAs, a cluster that shares the words of every copy and reduction like the threads of one CTA, and whose
-// first CTA does whatever a thread block does once: signals, waits, barriers, semaphores, requests to the proxy.
-// One B200, all ranks on it, us with one CTA each / teams (ranks x instances, bytes of the full-size buffer): reduce-scatter 2 x 1, 2 MB 50 /
-// 24, 8 x 2, 8 MB 86 / 39, 8 x 8, 16 MB 48 / 41 (128 SMs, 3.6 TB/s); all-gather 2 x 1, 2 MB 60 / 25, 8 x 8, 16 MB 63 / 50; all-to-all 8 x 2,
-// 8 MB 105 / 46. (Of which 15 are the launch and the signals.) Tried instead: one CTA with 192 KB of bulk copies in flight, requested by a
+// A plan's thread blocks are few, and one SM keeps neither memory nor a fast link busy: a thread block may be run by a team of CTAs, a cluster
+// that shares the words of every copy and reduction like the threads of one CTA, and whose first CTA does whatever a thread block does
+// once: signals, waits, barriers, semaphores, requests to the proxy. (Whether it is: execBlockUs, execAllowedTeam.)
+// One B200, all ranks on it, us with one CTA each / teams (ranks x instances, bytes of the full-size buffer): reduce-scatter 2 x 1, 2 MB 43 /
+// 24, 8 x 2, 8 MB 92 / 40, 8 x 8, 16 MB 46 / 40 (128 SMs, 3.6 TB/s); all-gather 2 x 1, 2 MB 60 / 26, 8 x 8, 16 MB 62 / 49; all-to-all 8 x 2,
+// 8 MB 104 / 46. (Of which 15 are the launch and the signals.) Tried instead: one CTA with 192 KB of bulk copies in flight, requested by a
 // warp of its own: 48 -> 78 us, 0.25-0.5 us per piece in the requesting warp.
 // kTeams is a template parameter for the launches that have none: with the branches in one kernel, plans of a few KB took 0.3-1.6 us longer.
 template <typename T, typename Pkt, bool kTeams>

@@ -17,13 +17,15 @@
 // their own rank, so while one block sits in a barrier the others copy and reduce as well: with a few blocks per SM the
 // NVLink transfers, the local copies and the barrier latencies overlap. Scratch is double buffered per block (round
 // parity), which is what makes two barriers per round enough.
-// What bounds it with all ranks on one GPU: the bytes stored, of which an SM gets rid of 25-30 GB/s (a plain fill of 16 MB or 256 MB alike: 3.2-3.9
-// TB/s), and a round's waits and round trips, 9 us whatever it moves. Four ranks on one B200 (32 MB bf16 each), us: reduced parts stored
-// to every peer's scratch 110, to the own one and fetched from there (2 S of stores per rank instead of 2.5 S) 100, in 5
-// rounds instead of 7 91 (on two other boxes, both together, 106 -> 99 and 107 -> 102); 121 when a rank's own part went through the scratch as well; 629 with one copy load in flight per
-// thread, system-scope accesses, the barriers unsplit and 16 blocks per rank instead of the 74 that fit. Tried instead: a
-// warp for each copy and the others reducing, with three flags a round, 139; all three legs in one step with a single barrier
-// 119; evict-first and evict-last accesses, which take a third of the DRAM writes away (265 -> 182 MB), 1 %.
+// With all ranks on one GPU (four ranks, 32 MB bf16 each, one B200): 256 MB are stored and 320 MB read, the detour included, in 97-118 us on different
+// boxes, 4.9-5.9 TB/s together; a plain copy reads and writes 8.1 TB/s of 32 MB (inside L2) and 6.4 of 256 MB. A round costs 9-10 us however
+// little it moves - slices of 32 KB, 14 rounds 177 us, 48 KB, 10 rounds 138, 64 KB, 7 rounds 111, 96 KB, 5 rounds 106 on one box: its two waits and the
+// round trips on either side of them, which only the SM's other block covers. So with slices that fill the scratch neither the bytes nor
+// the waits alone bound it. On one box each, us: reduced parts stored to every peer's scratch 110, to the own one and fetched from there 100; both
+// changes together, with 5 rounds instead of 7, 106 -> 99 and 107 -> 102; a rank's own part through the scratch as well 121; one copy load in
+// flight per thread, system-scope accesses, the barriers unsplit and 16 blocks per rank instead of the 74 that fit 629. Tried instead: a warp
+// for each copy and the others reducing, with three flags a round, 139; all three legs in one step with a single barrier 119; evict-first and
+// evict-last accesses, which take a third of the DRAM writes away (265 -> 182 MB), 1 %.
 // One round that covers the whole message is the un-pipelined "reduce-scatter + all-gather through scratch" form.
 //
 // Role of the reference's allreduce_nvls_block_pipeline.cu:16-147 / allreduce_nvls_warp_pipeline.cu:14-112 (NVLS) and

@@ -36,7 +36,8 @@ MSCCLPP_HOST_DEVICE_INLINE int moeDestinationRow(uint32_t first, int32_t positio
 // barrier, the count matrix and the cooperative launch; each block reads all expert ids for it. Dispatch and combine on one B200, us with
 // the exchange / with this: 2048 pairs 20.1-20.7 / 19.4-19.8; 8192 pairs, 1024 tokens x 4096 bf16, top-8 of 64 32.6 / 24.8; 16384 pairs, 2048 x
 // 4096 bf16, top-8 62.8 / 52.9, 2048 x 2048 fp8, top-8 of 256 28.4 / 19.8; 32768 pairs 122 / 111 and 49 / 40; 65536 pairs, 8192 x 2048
-// fp8, top-8 93 / 81. The line is from before, when counting 8192 pairs took 7 us; it would now pay to move it.
+// fp8, top-8 93 / 81. The line is from when counting 8192 pairs took 7 us and lost from 12288 on. It no longer lies where the two cross, which is
+// above 65536: larger batches of one rank leave a tenth to a third of their time here.
 MSCCLPP_HOST_DEVICE_INLINE bool moeCountsAlone(int world, int tokens, int topk) {
   return world == 1 && static_cast<int64_t>(tokens) * topk <= 8192;
 }

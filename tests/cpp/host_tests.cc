@@ -498,7 +498,7 @@ TEST(PlanTeams, OnlyWhereNobodyElseIsWaitedForOrOnRequest) {
   for (int allowed : {1, 2, 4, 8}) EXPECT_EQ(execTeam(us, allowed).most, allowed);
 }
 
-// From 12288 pairs on, counting them in every block takes longer than the exchange that it replaces.
+// The line as it stands: up to 8192 pairs of one rank. (Counting in every block has since become ahead beyond it, see moeCountsAlone.)
 TEST(MoeDispatch, BlocksCountFewPairsOfOneRankAlone) {
   EXPECT_EQ(moeCountsAlone(1, 1024, 8) && moeCountsAlone(1, 4096, 2) && moeCountsAlone(1, 0, 8), true);
   EXPECT_EQ(moeCountsAlone(1, 1025, 8) || moeCountsAlone(1, 2048, 8) || moeCountsAlone(2, 4, 2) || moeCountsAlone(1, (1 << 24) - 1, 32), false);
