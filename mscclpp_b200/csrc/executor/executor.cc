@@ -207,7 +207,7 @@ class Resolver {
     for (size_t t = 0; t < tbs.size(); t++) {
       tb_ = &tbs.at(t);
       out.plan.tbs[t].opBegin = static_cast<uint32_t>(out.ops.size());
-      emitOps(tb_->at("ops"), out.ops, false);
+      emitOps(tb_->at("ops"), out.ops, 0);
       out.plan.tbs[t].opEnd = static_cast<uint32_t>(out.ops.size());
     }
     out.plan.nOps = static_cast<uint32_t>(out.ops.size());
@@ -315,7 +315,31 @@ class Resolver {
     return d;
   }
 
-  void emitOps(const json::Value& ops, std::vector<DevOp>& out, bool inPipeline) {
+  // Reductions and the switch's operations go by 16-byte words: an operand that does not begin at one is an error here and not on the GPU. (A
+  // range shorter than a word is handled byte by byte, wherever it begins.)
+  void checkWords(const DevOp& op, const std::string& name, uint64_t unit) const {
+    const OpType t = static_cast<OpType>(op.type);
+    const bool packets = t == OpType::REDUCE_PACKETS || t == OpType::REDUCE_SEND_PACKETS || t == OpType::REDUCE_COPY_PACKETS ||
+                         t == OpType::REDUCE_COPY_SEND_PACKETS;  // (the first source and the first destination are plain)
+    if (!packets && t != OpType::REDUCE && t != OpType::REDUCE_SEND && t != OpType::READ_REDUCE && t != OpType::READ_REDUCE_SEND &&
+        t != OpType::GROUP_LOAD_REDUCE_STORE && t != OpType::GROUP_STORE)
+      return;
+    if (op.nSrc == 0) return;
+    const bool sliced = unit != 0 && op.src[0].size > unit;
+    if ((sliced ? unit : op.src[0].size) < 16) return;
+    uint64_t bits = sliced ? unit : 0;
+    for (int k = 0; k < (packets ? 1 : op.nSrc); k++) bits |= op.src[k].offset;
+    for (int k = 0; k < (packets && op.nDst > 1 ? 1 : op.nDst); k++) bits |= op.dst[k].offset;
+    if ((bits & 15) != 0)
+      throw Error("plan '" + p_.name + "': rank " + std::to_string(rank_) + "'s operation '" + name +
+                      "' has an operand that does not begin at a multiple of 16 bytes: the buffers, the plan's buffer_alignment and its "
+                      "pipeline units have to be multiples of 16",
+                  ErrorCode::ExecutorError);
+  }
+
+  // pipelineUnit: bytes per iteration of the pipeline that the operations are in, 0: in none
+  void emitOps(const json::Value& ops, std::vector<DevOp>& out, uint64_t pipelineUnit) {
+    const bool inPipeline = pipelineUnit != 0;
     for (size_t i = 0; i < ops.size(); i++) {
       const json::Value& op = ops.at(i);
       const std::string& name = op.at("name").asString();
@@ -329,7 +353,7 @@ class Resolver {
         begin.arg0 = static_cast<uint32_t>(std::max<uint64_t>(1, (chunks * l_.chunkUpper + unit - 1) / unit));
         begin.arg1 = static_cast<uint32_t>(unit);
         out.push_back(begin);
-        emitOps(op.at("ops"), out, true);
+        emitOps(op.at("ops"), out, unit);
         DevOp end{};
         end.type = static_cast<uint8_t>(OpType::PIPELINE_END);
         out.push_back(end);
@@ -376,6 +400,7 @@ class Resolver {
         d.arg1 = static_cast<uint32_t>(op.at("barrier_id").asUInt());
         if (d.arg1 >= static_cast<uint32_t>(kExecMaxBarriers)) throw Error("plan '" + p_.name + "': barrier id too large", ErrorCode::ExecutorError);
       }
+      checkWords(d, name, pipelineUnit);
       out.push_back(d);
     }
   }

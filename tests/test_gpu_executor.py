@@ -135,6 +135,52 @@ def test_allgather_reducescatter_alltoall_plans(world):
     _run_both(single_node.build("allgather_allpairs", world, in_place=False).to_json(), world, per, world * per, np.int32, inplace=False)
 
 
+def test_reduction_operands_that_begin_off_a_word_are_refused():
+    """Refused before anything is launched: a heap buffer that begins four bytes into a word, chunks that do (buffer_alignment 4), a pipeline unit that is no
+    multiple of 16. Chunks of less than a word still run."""
+    from mscclpp_b200 import SymmetricMemory, native
+    from mscclpp_b200.default_algos.single_node import make_spec
+    from mscclpp_b200.language.collectives import AllReduce
+    from mscclpp_b200.language.loop import LoopIterationContext
+    from mscclpp_b200.language.program import CollectiveProgram
+    from mscclpp_b200.language.rank import Rank
+
+    def plan(name, alignment, unit=0):
+        prog = CollectiveProgram.from_spec(make_spec(name, AllReduce(2, 2, True), 2, buffer_alignment=alignment))
+        with prog:
+            loop = LoopIterationContext(unit=unit, num_chunks=1) if unit else None
+            if loop:
+                loop.__enter__()
+            for r in range(2):
+                inp = Rank(r).get_input_buffer()
+                Rank(r).reduce(inp[1:2], [inp[2:3]], tb=0)
+            if loop:
+                loop.__exit__(None, None, None)
+        return n.ExecutionPlan.from_string(prog.to_json(), 0)
+
+    n = native()
+    symm = SymmetricMemory.emulated(2, nbytes=64 << 20, timeout_ms=1000)
+    t = symm.tensor((1024,), torch.float32, zero=True)
+    ex = n.Executor(symm.heap)
+    run = lambda p, offset, nbytes: ex.execute(0, t.data_ptr() + offset, t.data_ptr() + offset, nbytes, nbytes, n.DataType.float32, p, 0)
+    for p, offset, nbytes in ((plan("aligned", 16), 4, 1024), (plan("words", 4), 0, 1024 + 16), (plan("units", 16, unit=24), 0, 1024)):
+        with pytest.raises(Exception, match="multiple of 16 bytes"):
+            run(p, offset, nbytes)
+    for r in range(2):
+        symm.rank_view(t, r).copy_(torch.arange(1024) + 1024.0 * r)
+    run(plan("words", 4), 0, 48)  # four chunks of three elements
+    run(plan("units_of_words", 16, unit=32), 0, 1024)
+    torch.cuda.synchronize()
+    symm.check()
+    for r in range(2):
+        want = torch.arange(1024) + 1024.0 * r
+        want[3:6] += want[6:9].clone()
+        want[64:128] += want[128:192].clone()
+        assert torch.equal(symm.rank_view(t, r).cpu(), want)
+    ex.reset()
+    symm.destroy()
+
+
 def test_malformed_plan_is_rejected():
     from mscclpp_b200 import native
     from mscclpp_b200.default_algos import single_node
