@@ -71,7 +71,7 @@ struct MoeCombineArgs {
   int fp8;                      // 1: expertOut holds e4m3 with one fp32 scale per 128 elements in outScales (half the
                                 // bytes pulled over NVLink); the weighted sum is still taken in fp32
   const float* outScales;       // symmetric [capacity, hidden / 128] (fp8 only)
-  int blockStep, warpStep;      // set by launchMoeCombine: a warp's first unit of work is blockIdx.x * blockStep + warp * warpStep
+  int roundTheBlocks;           // set by launchMoeCombine for long pieces: units of work go round the thread blocks first, not round the warps of one
 };
 
 // Quantiser for the fp8 form of the combine (and for tests): q[r] = e4m3(x[r] / scale), scale = amax of each 128-element
